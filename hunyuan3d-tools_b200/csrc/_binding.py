@@ -112,6 +112,12 @@ class _Base:
         self._lib = configure(lib)
 
     # -- helpers -----------------------------------------------------------------------
+    @staticmethod
+    def _native():
+        """The native host path (torch_ext.cpp): the same calls for plain arguments, None otherwise."""
+        from .build import load_native
+        return load_native()
+
     def _check(self, status: int, what: str):
         if status != 0:
             msg = self._lib.hy3d_status_string(status).decode()
@@ -343,6 +349,10 @@ class TcGemmModule(_Base):
     def int8_linear_tc(self, x, w_int8, w_scale, bias, epilogue=EPI_LINEAR, cta_group=0, block_n=0):
         """x (M,K) f16/bf16, w_int8 (N,K), w_scale (N), bias (N) or empty -> (M,N) in x's
         dtype.  csrc/int8_gemm_tc.cu:312-320."""
+        if cta_group == 0 and block_n == 0 and isinstance(x, torch.Tensor) and x.dim() == 2:
+            y = self._native().linear_dense(x, w_int8, w_scale, bias, epilogue)
+            if y is not None:
+                return y
         self._req(x, "x", (torch.float16, torch.bfloat16), 2)
         self._req(w_int8, "w_int8", torch.int8, 2)
         M, K = x.shape
@@ -460,6 +470,10 @@ class SparseTcModule(_Base):
 
     def sparse_int8_linear_ex(self, x, w_comp, w_meta, w_scale, bias, path=-1, epilogue=EPI_LINEAR):
         """csrc/int8_sparse_tc.cu:2006-2025.  ``path`` is accepted and ignored."""
+        if isinstance(x, torch.Tensor) and x.dim() == 2:
+            y = self._native().linear_sparse(x, w_comp, w_meta, w_scale, bias, epilogue)
+            if y is not None:
+                return y
         self._req(x, "x", (torch.float16, torch.bfloat16), 2)
         self._req(w_comp, "w_comp", torch.int8, 2)
         self._req(w_meta, "w_meta", torch.int32, 2)

@@ -8,6 +8,9 @@ Mirrors the loader surface of the reference's ``csrc/build.py`` (``load_int8_ker
   ``ctypes`` -- no torch headers are involved, so a cold build takes seconds and the ``.so``
   sits in-tree next to its sources.
 
+Beside it sits ``hy3d_torch.so`` (``torch_ext.cpp``, compiled by ``g++`` against torch's headers): the
+native host path that the modules call, which allocates from torch and calls the same C ABI.
+
 The three ``load_*`` functions return small namespace objects exposing the reference's
 extension function names (see ``_binding.py``); all of them share the single library.
 """
@@ -27,6 +30,8 @@ _REPO_INCLUDE = os.path.normpath(os.path.join(_CSRC, "..", "..", "include"))
 _BUILD_DIR = os.path.join(_CSRC, "_build")
 LIB_NAME = "libhy3d_int8.so"
 LIB_PATH = os.path.join(_CSRC, LIB_NAME)
+EXT_PATH = os.path.join(_CSRC, "hy3d_torch.so")
+EXT_SOURCES = ["torch_ext.cpp", os.path.join(_REPO_INCLUDE, "hy3d_int8.h")]
 
 # hy3d_int8.cu is the only translation unit; it #includes the kernel files listed in HEADERS.
 SOURCES = ["hy3d_int8.cu"]
@@ -35,6 +40,7 @@ HEADERS = ["common.cuh", "quantize.cu", "prune_pack.cu", "gemm_dense.cu", "gemm_
 
 _lock = threading.Lock()
 _lib = None
+_native = None
 
 
 def _nvcc() -> str:
@@ -69,8 +75,8 @@ def _source_digest() -> str:
     return h.hexdigest()
 
 
-def _up_to_date(stamp: str, digest: str) -> bool:
-    if not (os.path.exists(LIB_PATH) and os.path.exists(stamp)):
+def _up_to_date(stamp: str, digest: str, product: str = LIB_PATH) -> bool:
+    if not (os.path.exists(product) and os.path.exists(stamp)):
         return False
     with open(stamp) as f:
         return f.read().strip() == digest
@@ -124,6 +130,85 @@ def _build_locked(stamp: str, digest: str, verbose: bool) -> str:
     with open(stamp, "w") as f:
         f.write(digest)
     return LIB_PATH
+
+
+def _ext_command() -> list[str]:
+    """g++ command of the torch extension; it lives in this torch's ABI."""
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    lib = os.path.join(root, "lib")
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-isystem", os.path.join(root, "include"),
+            "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+            "-isystem", os.path.join(cuda, "include"), "-isystem", sysconfig.get_paths()["include"],
+            os.path.join(_CSRC, EXT_SOURCES[0]),
+            "-L" + lib, "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+
+
+def _ext_digest() -> str:
+    """Hash of the extension's sources and of the torch and Python it is compiled against."""
+    import torch
+    h = hashlib.sha256(f"{torch.__version__} {sys.version_info[:2]}".encode())
+    for name in EXT_SOURCES:
+        path = name if os.path.isabs(name) else os.path.join(_CSRC, name)
+        with open(path, "rb") as f:
+            h.update(os.path.basename(name).encode())
+            h.update(f.read())
+    return h.hexdigest()
+
+
+def build_native(force: bool = False, verbose: bool = False) -> str:
+    """Compile ``hy3d_torch.so`` if its sources or torch changed; returns its path."""
+    stamp = os.path.join(_BUILD_DIR, "torch_ext_digest.txt")
+    digest = _ext_digest()
+    if not force and _up_to_date(stamp, digest, EXT_PATH):
+        return EXT_PATH
+    os.makedirs(_BUILD_DIR, exist_ok=True)
+    import fcntl
+    with open(os.path.join(_BUILD_DIR, "build.lock"), "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        try:
+            if not force and _up_to_date(stamp, digest, EXT_PATH):
+                return EXT_PATH
+            tmp = EXT_PATH + f".tmp{os.getpid()}"
+            cmd = _ext_command() + [f'-DHY3D_EXT_DIGEST="{digest}"', "-o", tmp]
+            r = subprocess.run(cmd, capture_output=True, text=True)
+            if verbose or r.returncode != 0:
+                sys.stderr.write(r.stdout + r.stderr)
+            if r.returncode != 0:
+                raise RuntimeError(f"g++ failed on {EXT_SOURCES[0]}:\n{r.stderr}")
+            os.replace(tmp, EXT_PATH)
+            with open(stamp, "w") as f:
+                f.write(digest)
+            return EXT_PATH
+        finally:
+            fcntl.flock(lock, fcntl.LOCK_UN)
+
+
+def load_native():
+    """The native host path (``torch_ext.cpp``), bound to the loaded kernel library."""
+    global _native
+    if _native is not None:
+        return _native
+    from . import _binding
+    _binding.configure(load_library())      # refuses a library of another ABI version
+    with _lock:
+        if _native is None:
+            import importlib.machinery
+            import importlib.util
+            path = build_native()
+            spec = importlib.util.spec_from_loader(
+                "hy3d_torch", importlib.machinery.ExtensionFileLoader("hy3d_torch", path))
+            mod = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(mod)
+            if mod.source_digest != _ext_digest():
+                raise RuntimeError("hy3d_torch.so was built from other sources; rebuild it with `python csrc/build.py`")
+            mod.open(LIB_PATH)
+            _native = mod
+        return _native
 
 
 def load_library(build_if_missing: bool = True) -> ctypes.CDLL:
@@ -184,3 +269,4 @@ if __name__ == "__main__":
     # Every target lives in the same library.
     print("Building", LIB_NAME, "for sm_100a ...")
     print("  ->", build(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print("  ->", build_native(force="--force" in sys.argv, verbose="-v" in sys.argv))

@@ -1,0 +1,397 @@
+// Native host path of the layers: takes torch tensors, allocates outputs and scratch from torch's
+// caching allocator, and calls the C ABI of libhy3d_int8.so (include/hy3d_int8.h) on the current
+// stream.  One call replaces the argument checks, allocations, device guard and 19-argument ctypes
+// call of `_binding.py`, which cost 30-35 us of host time per layer -- more than the kernels of every
+// layer below about 10 G multiply-adds.
+//
+// Every function answers Py_None, having done nothing, for arguments outside the plain case (another
+// dtype, a non-contiguous or CPU tensor, a tensor subclass, a size the kernels refuse); the caller then
+// takes the checked path of `_binding.py`, which either handles them or raises with its message.  Plain
+// CPython calling convention: no argument-conversion layer in between.
+#include <Python.h>
+#include <dlfcn.h>
+
+#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/core/Tensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/hy3d_int8.h"
+
+namespace {
+
+#define HY3D_FN(name) decltype(&::name) name = nullptr
+struct Api {
+  HY3D_FN(hy3d_linear_w8a8_dense);
+  HY3D_FN(hy3d_gemm_w8a8_dense);
+  HY3D_FN(hy3d_dense_splitk_plan);
+  HY3D_FN(hy3d_gemm_w8a8_dense_splitk);
+  HY3D_FN(hy3d_quantize_rows);
+  HY3D_FN(hy3d_linear_w8a8_sparse24);
+  HY3D_FN(hy3d_gemm_w8a8_sparse24);
+  HY3D_FN(hy3d_layernorm_quantize);
+  HY3D_FN(hy3d_groupnorm_nhwc);
+  HY3D_FN(hy3d_groupnorm_workspace_floats);
+  HY3D_FN(hy3d_status_string);
+} api;
+#undef HY3D_FN
+
+// A tensor the kernels can take as it is: plain strided CUDA storage, contiguous.
+const at::Tensor* plain(PyObject* o) {
+  if (!THPVariable_CheckExact(o)) return nullptr;   // torch.Tensor or Parameter, no other subclass
+  const at::Tensor& t = THPVariable_Unpack(o);
+  return t.is_cuda() && t.layout() == at::kStrided && t.is_contiguous() ? &t : nullptr;
+}
+
+int half_code(at::ScalarType t) {
+  return t == at::kHalf ? HY3D_F16 : t == at::kBFloat16 ? HY3D_BF16 : -1;
+}
+int param_code(at::ScalarType t) { return t == at::kFloat ? HY3D_F32 : half_code(t); }
+
+// Scratch of one call: taken from the allocator's pool of the stream it is used on and handed back when
+// the call has enqueued its kernels, which is when a tensor going out of scope would return it too.
+struct Scratch {
+  void* p = nullptr;
+  Scratch(size_t bytes, cudaStream_t s) : p(c10::cuda::CUDACachingAllocator::raw_alloc_with_stream(bytes, s)) {}
+  ~Scratch() { if (p) c10::cuda::CUDACachingAllocator::raw_delete(p); }
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  int8_t* at(size_t off) const { return static_cast<int8_t*>(p) + off; }
+};
+
+size_t align256(size_t n) { return (n + 255) & ~static_cast<size_t>(255); }
+
+PyObject* none() { Py_RETURN_NONE; }
+
+PyObject* failed(const char* what, int rc) {
+  PyErr_Format(PyExc_RuntimeError, "%s failed: %s (status %d)", what, api.hy3d_status_string(rc), rc);
+  return nullptr;
+}
+
+// Weight scales and the optional bias of a layer with N output rows.
+struct Params {
+  const void* ws = nullptr;
+  const void* bias = nullptr;
+  int ws_code = 0, bias_code = HY3D_F16;
+  bool ok = false;
+  Params(PyObject* scale, PyObject* b, int64_t N, c10::Device dev) {
+    const at::Tensor* s = plain(scale);
+    if (!s || s->dim() != 1 || s->size(0) != N || s->device() != dev) return;
+    ws_code = param_code(s->scalar_type());
+    ws = s->const_data_ptr();
+    if (ws_code < 0) return;
+    if (b != Py_None) {
+      const at::Tensor* t = plain(b);
+      if (!t || t->device() != dev) return;
+      if (t->numel() != 0) {
+        if (t->dim() != 1 || t->size(0) != N) return;
+        bias_code = param_code(t->scalar_type());
+        if (bias_code < 0) return;
+        bias = t->const_data_ptr();
+      }
+    }
+    ok = true;
+  }
+};
+
+// The output of a layer: the input's leading dimensions, `cols` columns.
+at::Tensor out_like(c10::IntArrayRef lead, int64_t cols, at::ScalarType type, c10::Device dev) {
+  c10::SmallVector<int64_t, 6> shape(lead.begin(), lead.end());
+  shape.push_back(cols);
+  return at::Tensor(at::detail::empty_cuda(shape, type, dev, std::nullopt));
+}
+
+bool small_int(PyObject* o, long lo, long hi, long* v) {
+  if (!PyLong_CheckExact(o)) return false;
+  *v = PyLong_AsLong(o);
+  return *v >= lo && *v <= hi;
+}
+
+// int8 GEMM + epilogue on codes that are already there; follows the library's split-K plan.
+int dense_gemm(const int8_t* q, const float* s, const at::Tensor& w, const Params& p, void* out, int out_code,
+               int64_t M, int64_t N, int64_t K, int epi, cudaStream_t st) {
+  int64_t bytes = 0;
+  const int splits = api.hy3d_dense_splitk_plan(M, N, K, epi, &bytes);
+  if (splits > 1) {
+    Scratch part(static_cast<size_t>(bytes), st);
+    return api.hy3d_gemm_w8a8_dense_splitk(q, w.const_data_ptr<int8_t>(), s, p.ws, p.ws_code, p.bias, p.bias_code,
+                                           out, out_code, M, N, K, epi, splits, part.p, bytes, st);
+  }
+  return api.hy3d_gemm_w8a8_dense(q, w.const_data_ptr<int8_t>(), s, p.ws, p.ws_code, p.bias, p.bias_code, out,
+                                  out_code, M, N, K, epi, 0, 0, st);
+}
+
+// linear_dense(x, w_int8 (N,K), w_scale, bias | None, epilogue) -> y | None
+PyObject* linear_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  long epi = 0;
+  if (n != 5 || !small_int(a[4], 0, 2, &epi)) return none();
+  const at::Tensor *x = plain(a[0]), *w = plain(a[1]);
+  if (!x || !w || x->dim() < 1 || w->dim() != 2 || w->scalar_type() != at::kChar || w->device() != x->device())
+    return none();
+  const int code = half_code(x->scalar_type());
+  const int64_t N = w->size(0), K = w->size(1);
+  const int64_t M = K > 0 ? x->numel() / K : 0;
+  if (code < 0 || M <= 0 || x->size(-1) != K || (K & 63) || (N & 15)) return none();
+  const Params p(a[2], a[3], N, x->device());
+  if (!p.ok) return none();
+  c10::cuda::CUDAGuard guard(x->device());
+  cudaStream_t st = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
+  at::Tensor y = out_like(x->sizes().slice(0, x->dim() - 1), epi == HY3D_EPI_GEGLU ? N / 2 : N, x->scalar_type(),
+                          x->device());
+  const size_t codes = align256(static_cast<size_t>(M) * K);
+  Scratch ws(codes + static_cast<size_t>(M) * 4, st);
+  int64_t bytes = 0;
+  int rc;
+  if (api.hy3d_dense_splitk_plan(M, N, K, static_cast<int>(epi), &bytes) > 1) {
+    rc = api.hy3d_quantize_rows(x->const_data_ptr(), code, M, K, K, ws.at(0), reinterpret_cast<float*>(ws.at(codes)), st);
+    if (rc == HY3D_OK)
+      rc = dense_gemm(ws.at(0), reinterpret_cast<float*>(ws.at(codes)), *w, p, y.mutable_data_ptr(), code, M, N, K,
+                      static_cast<int>(epi), st);
+  } else {
+    rc = api.hy3d_linear_w8a8_dense(x->const_data_ptr(), code, K, ws.at(0), reinterpret_cast<float*>(ws.at(codes)),
+                                    w->const_data_ptr<int8_t>(), p.ws, p.ws_code, p.bias, p.bias_code,
+                                    y.mutable_data_ptr(), code, M, N, K, static_cast<int>(epi), 0, 0, st);
+  }
+  if (rc != HY3D_OK) return failed("hy3d_linear_w8a8_dense", rc);
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// linear_sparse(x, w_comp (N,K/2), w_meta, w_scale, bias | None, epilogue) -> y | None
+PyObject* linear_sparse(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  long epi = 0;
+  if (n != 6 || !small_int(a[5], 0, 2, &epi)) return none();
+  const at::Tensor *x = plain(a[0]), *w = plain(a[1]), *e = plain(a[2]);
+  if (!x || !w || !e || x->dim() < 1 || w->dim() != 2 || e->dim() != 2 || w->scalar_type() != at::kChar ||
+      e->scalar_type() != at::kInt || w->device() != x->device() || e->device() != x->device())
+    return none();
+  const int code = half_code(x->scalar_type());
+  const int64_t N = w->size(0), K = 2 * w->size(1);
+  const int64_t M = K > 0 ? x->numel() / K : 0;
+  if (code < 0 || M <= 0 || x->size(-1) != K || (K & 63) || (N & 15) || e->size(0) != N) return none();
+  const Params p(a[3], a[4], N, x->device());
+  if (!p.ok) return none();
+  c10::cuda::CUDAGuard guard(x->device());
+  cudaStream_t st = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
+  at::Tensor y = out_like(x->sizes().slice(0, x->dim() - 1), epi == HY3D_EPI_GEGLU ? N / 2 : N, x->scalar_type(),
+                          x->device());
+  const size_t codes = align256(static_cast<size_t>(M) * K);
+  Scratch ws(codes + static_cast<size_t>(M) * 4, st);
+  const int rc = api.hy3d_linear_w8a8_sparse24(
+      x->const_data_ptr(), code, K, ws.at(0), reinterpret_cast<float*>(ws.at(codes)), w->const_data_ptr<int8_t>(),
+      reinterpret_cast<const uint32_t*>(e->const_data_ptr<int32_t>()), e->size(1), p.ws, p.ws_code, p.bias, p.bias_code,
+      y.mutable_data_ptr(), code, M, N, K, static_cast<int>(epi), 0, st);
+  if (rc != HY3D_OK) return failed("hy3d_linear_w8a8_sparse24", rc);
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// The two forms of a layer whose input arrives as codes and per-row scales: the logical leading shape
+// is given as a tuple (its last entry is K), the output type by an example tensor's code.
+bool lead_shape(PyObject* o, c10::SmallVector<int64_t, 6>* lead) {
+  if (!PyTuple_Check(o)) return false;
+  const Py_ssize_t d = PyTuple_GET_SIZE(o);
+  for (Py_ssize_t i = 0; i + 1 < d; ++i) {
+    PyObject* v = PyTuple_GET_ITEM(o, i);
+    if (!PyLong_Check(v)) return false;
+    lead->push_back(PyLong_AsLongLong(v));
+  }
+  return d >= 1;
+}
+
+// gemm_dense(q (M,K), scale (M), w_int8, w_scale, bias | None, is_bf16, epilogue, shape) -> y | None
+PyObject* gemm_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  long epi = 0, bf16 = 0;
+  c10::SmallVector<int64_t, 6> lead;
+  if (n != 8 || !small_int(a[5], 0, 1, &bf16) || !small_int(a[6], 0, 2, &epi) || !lead_shape(a[7], &lead)) return none();
+  const at::Tensor *q = plain(a[0]), *s = plain(a[1]), *w = plain(a[2]);
+  if (!q || !s || !w || q->dim() != 2 || s->dim() != 1 || w->dim() != 2 || q->scalar_type() != at::kChar ||
+      s->scalar_type() != at::kFloat || w->scalar_type() != at::kChar || w->device() != q->device() ||
+      s->device() != q->device())
+    return none();
+  const int64_t M = q->size(0), K = q->size(1), N = w->size(0);
+  if (M <= 0 || s->size(0) != M || w->size(1) != K || (K & 63) || (N & 15)) return none();
+  const Params p(a[3], a[4], N, q->device());
+  if (!p.ok) return none();
+  c10::cuda::CUDAGuard guard(q->device());
+  cudaStream_t st = c10::cuda::getCurrentCUDAStream(q->device().index()).stream();
+  at::Tensor y = out_like(lead, epi == HY3D_EPI_GEGLU ? N / 2 : N, bf16 ? at::kBFloat16 : at::kHalf, q->device());
+  const int rc = dense_gemm(q->const_data_ptr<int8_t>(), s->const_data_ptr<float>(), *w, p, y.mutable_data_ptr(),
+                            bf16 ? HY3D_BF16 : HY3D_F16, M, N, K, static_cast<int>(epi), st);
+  if (rc != HY3D_OK) return failed("hy3d_gemm_w8a8_dense", rc);
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// gemm_sparse(q, scale, w_comp, w_meta, w_scale, bias | None, is_bf16, epilogue, shape) -> y | None
+PyObject* gemm_sparse(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  long epi = 0, bf16 = 0;
+  c10::SmallVector<int64_t, 6> lead;
+  if (n != 9 || !small_int(a[6], 0, 1, &bf16) || !small_int(a[7], 0, 2, &epi) || !lead_shape(a[8], &lead)) return none();
+  const at::Tensor *q = plain(a[0]), *s = plain(a[1]), *w = plain(a[2]), *e = plain(a[3]);
+  if (!q || !s || !w || !e || q->dim() != 2 || s->dim() != 1 || w->dim() != 2 || e->dim() != 2 ||
+      q->scalar_type() != at::kChar || s->scalar_type() != at::kFloat || w->scalar_type() != at::kChar ||
+      e->scalar_type() != at::kInt || w->device() != q->device() || s->device() != q->device() ||
+      e->device() != q->device())
+    return none();
+  const int64_t M = q->size(0), K = q->size(1), N = w->size(0);
+  if (M <= 0 || s->size(0) != M || 2 * w->size(1) != K || (K & 63) || (N & 15) || e->size(0) != N) return none();
+  const Params p(a[4], a[5], N, q->device());
+  if (!p.ok) return none();
+  c10::cuda::CUDAGuard guard(q->device());
+  cudaStream_t st = c10::cuda::getCurrentCUDAStream(q->device().index()).stream();
+  at::Tensor y = out_like(lead, epi == HY3D_EPI_GEGLU ? N / 2 : N, bf16 ? at::kBFloat16 : at::kHalf, q->device());
+  const int rc = api.hy3d_gemm_w8a8_sparse24(
+      q->const_data_ptr<int8_t>(), s->const_data_ptr<float>(), w->const_data_ptr<int8_t>(),
+      reinterpret_cast<const uint32_t*>(e->const_data_ptr<int32_t>()), e->size(1), p.ws, p.ws_code, p.bias, p.bias_code,
+      y.mutable_data_ptr(), bf16 ? HY3D_BF16 : HY3D_F16, M, N, K, static_cast<int>(epi), 0, st);
+  if (rc != HY3D_OK) return failed("hy3d_gemm_w8a8_sparse24", rc);
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// gamma and beta of a normalisation: both of one type (or absent).
+struct Affine {
+  const void *gamma = nullptr, *beta = nullptr;
+  int code = HY3D_F32;
+  bool ok = false;
+  Affine(PyObject* g, PyObject* b, int64_t C, c10::Device dev) {
+    for (int i = 0; i < 2; ++i) {
+      PyObject* o = i ? b : g;
+      if (o == Py_None) continue;
+      const at::Tensor* t = plain(o);
+      if (!t || t->numel() != C || t->device() != dev) return;
+      const int c = param_code(t->scalar_type());
+      if (c < 0 || (i && gamma && c != code)) return;
+      code = c;
+      (i ? beta : gamma) = t->const_data_ptr();
+    }
+    ok = true;
+  }
+};
+
+// layernorm_quantize(x, gamma | None, beta | None, eps) -> (codes (M,K), scale (M)) | None
+PyObject* layernorm_quantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 4 || !PyFloat_Check(a[3])) return none();
+  const at::Tensor* x = plain(a[0]);
+  if (!x || x->dim() < 1) return none();
+  const int code = half_code(x->scalar_type());
+  const int64_t K = x->size(-1), M = K > 0 ? x->numel() / K : 0;
+  if (code < 0 || M <= 0) return none();
+  const Affine f(a[1], a[2], K, x->device());
+  if (!f.ok) return none();
+  c10::cuda::CUDAGuard guard(x->device());
+  cudaStream_t st = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
+  at::Tensor q = at::Tensor(at::detail::empty_cuda({M, K}, at::kChar, x->device(), std::nullopt));
+  at::Tensor s = at::Tensor(at::detail::empty_cuda({M}, at::kFloat, x->device(), std::nullopt));
+  const int rc = api.hy3d_layernorm_quantize(x->const_data_ptr(), code, M, K, K, f.gamma, f.beta, f.code,
+                                             static_cast<float>(PyFloat_AS_DOUBLE(a[3])), q.mutable_data_ptr<int8_t>(),
+                                             s.mutable_data_ptr<float>(), nullptr, st);
+  if (rc != HY3D_OK) return failed("hy3d_layernorm_quantize", rc);
+  PyObject* pq = THPVariable_Wrap(std::move(q));
+  PyObject* ps = pq ? THPVariable_Wrap(std::move(s)) : nullptr;
+  if (!ps) { Py_XDECREF(pq); return nullptr; }
+  PyObject* r = PyTuple_New(2);
+  if (!r) { Py_DECREF(pq); Py_DECREF(ps); return nullptr; }
+  PyTuple_SET_ITEM(r, 0, pq);
+  PyTuple_SET_ITEM(r, 1, ps);
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// groupnorm_nhwc(x channels_last, groups, gamma | None, beta | None, eps, silu, add (B,C) | None) -> y | None
+PyObject* groupnorm_nhwc(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  long groups = 0, silu = 0;
+  if (n != 7 || !small_int(a[1], 1, 1 << 20, &groups) || !PyFloat_Check(a[4])) return none();
+  silu = a[5] == Py_True ? 1 : 0;
+  if (!THPVariable_CheckExact(a[0])) return none();
+  const at::Tensor& x = THPVariable_Unpack(a[0]);
+  if (!x.is_cuda() || x.layout() != at::kStrided || x.dim() != 4 || !x.is_contiguous(at::MemoryFormat::ChannelsLast))
+    return none();
+  const int code = half_code(x.scalar_type());
+  const int64_t B = x.size(0), C = x.size(1), HW = x.size(2) * x.size(3);
+  if (code < 0 || B <= 0 || HW <= 0) return none();
+  const Affine f(a[2], a[3], C, x.device());
+  if (!f.ok) return none();
+  const void* add = nullptr;
+  if (a[6] != Py_None) {
+    const at::Tensor* t = plain(a[6]);
+    if (!t || t->dim() != 2 || t->size(0) != B || t->size(1) != C || t->scalar_type() != x.scalar_type() ||
+        t->device() != x.device())
+      return none();
+    add = t->const_data_ptr();
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  cudaStream_t st = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+  at::Tensor y = at::Tensor(at::detail::empty_cuda(x.sizes(), x.scalar_type(), x.device(), at::MemoryFormat::ChannelsLast));
+  Scratch ws(static_cast<size_t>(api.hy3d_groupnorm_workspace_floats(B, HW, static_cast<int>(groups)) + 4) * 4, st);
+  const int rc = api.hy3d_groupnorm_nhwc(x.const_data_ptr(), add, code, B, HW, C, static_cast<int>(groups), f.gamma, f.beta,
+                                         f.code, static_cast<float>(PyFloat_AS_DOUBLE(a[4])), static_cast<int>(silu),
+                                         y.mutable_data_ptr(), static_cast<float*>(ws.p), st);
+  if (rc != HY3D_OK) return failed("hy3d_groupnorm_nhwc", rc);
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// open(path): resolves the C ABI in the library at `path`, which the caller has loaded and checked.
+PyObject* open_library(PyObject*, PyObject* arg) {
+  const char* path = PyUnicode_AsUTF8(arg);
+  if (!path) return nullptr;
+  void* h = dlopen(path, RTLD_NOW | RTLD_LOCAL);
+  if (!h) {
+    PyErr_Format(PyExc_RuntimeError, "%s", dlerror());
+    return nullptr;
+  }
+#define HY3D_SYM(name)                                                                       \
+  do {                                                                                       \
+    api.name = reinterpret_cast<decltype(api.name)>(dlsym(h, #name));                        \
+    if (!api.name) {                                                                         \
+      PyErr_Format(PyExc_RuntimeError, "%s has no symbol %s", path, #name);                  \
+      return nullptr;                                                                        \
+    }                                                                                        \
+  } while (0)
+  HY3D_SYM(hy3d_linear_w8a8_dense);
+  HY3D_SYM(hy3d_gemm_w8a8_dense);
+  HY3D_SYM(hy3d_dense_splitk_plan);
+  HY3D_SYM(hy3d_gemm_w8a8_dense_splitk);
+  HY3D_SYM(hy3d_quantize_rows);
+  HY3D_SYM(hy3d_linear_w8a8_sparse24);
+  HY3D_SYM(hy3d_gemm_w8a8_sparse24);
+  HY3D_SYM(hy3d_layernorm_quantize);
+  HY3D_SYM(hy3d_groupnorm_nhwc);
+  HY3D_SYM(hy3d_groupnorm_workspace_floats);
+  HY3D_SYM(hy3d_status_string);
+#undef HY3D_SYM
+  Py_RETURN_NONE;
+}
+
+#define HY3D_FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {
+    {"open", open_library, METH_O, nullptr},
+    HY3D_FAST(linear_dense),
+    HY3D_FAST(linear_sparse),
+    HY3D_FAST(gemm_dense),
+    HY3D_FAST(gemm_sparse),
+    HY3D_FAST(layernorm_quantize),
+    HY3D_FAST(groupnorm_nhwc),
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "hy3d_torch", "Native host path of the INT8 layers.", -1, methods,
+                          nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit_hy3d_torch(void) {
+  PyObject* m = PyModule_Create(&module_def);
+  if (m) PyModule_AddStringConstant(m, "source_digest", HY3D_EXT_DIGEST);
+  return m;
+}

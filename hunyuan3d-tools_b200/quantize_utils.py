@@ -30,6 +30,7 @@ Differences from the reference, all of them additive:
 """
 from __future__ import annotations
 
+import math
 import os
 
 import torch
@@ -89,6 +90,23 @@ def sp_available() -> bool:
     return _load_sp() is not None
 
 
+_NATIVE = None
+
+
+def _load_native():
+    """Lazy-load the native host path (csrc/torch_ext.cpp) the modules call first.  Its functions
+    answer None for anything but plain contiguous CUDA tensors of sizes the kernels take; the modules
+    then go through the checked Python binding, which converts or raises."""
+    global _NATIVE
+    if _NATIVE is None:
+        try:
+            from .csrc.build import load_native
+            _NATIVE = load_native()
+        except Exception as e:  # noqa: BLE001 - reported with its type, then re-raised
+            _kernel_unavailable("INT8 layer host path", e)
+    return _NATIVE
+
+
 def _param_dtype(linear: nn.Linear) -> torch.dtype:
     dt = linear.weight.dtype
     return dt if dt in (torch.float16, torch.bfloat16) else torch.float16
@@ -123,10 +141,12 @@ class QuantizedActivation:
     def view(self, *shape):
         """Re-labels the leading dimensions (tokens stay tokens: the last dimension is fixed)."""
         shape = tuple(shape[0]) if len(shape) == 1 and isinstance(shape[0], (tuple, list, torch.Size)) else shape
-        probe = torch.empty(self.shape, device="meta").view(*shape)
-        if probe.shape[-1] != self.shape[-1]:
+        total, known = math.prod(self.shape), math.prod(shape)
+        if min(shape, default=-1) < 0 or known != total:      # -1 placeholders and errors: torch's own rules
+            shape = torch.empty(self.shape, device="meta").view(*shape).shape
+        if not shape or shape[-1] != self.shape[-1]:
             raise RuntimeError("a quantised activation can only be reshaped over its token dimensions")
-        return QuantizedActivation(self.q, self.scale, probe.shape, self.dtype)
+        return QuantizedActivation(self.q, self.scale, shape, self.dtype)
 
     reshape = view
 
@@ -149,6 +169,10 @@ class Int8LayerNorm(nn.Module):
         self._ik = None
 
     def forward(self, x: torch.Tensor) -> QuantizedActivation:
+        p = self._parameters
+        got = (_NATIVE or _load_native()).layernorm_quantize(x, p["weight"], p["bias"], self.eps)
+        if got is not None:
+            return QuantizedActivation(got[0], got[1], x.shape, x.dtype)
         if not x.is_cuda:
             raise RuntimeError("Int8LayerNorm runs on CUDA tensors only (no CPU fallback)")
         if self._ik is None:
@@ -348,6 +372,28 @@ class Int8Linear(nn.Module):
     _sp_ref = None
     _empty_bias = None
 
+    def _native_forward(self, x):
+        """The call on the native host path, or None where it declines.  Buffers come straight from
+        the module's dictionary: attribute look-ups through nn.Module cost as much as a launch."""
+        native = _NATIVE or _load_native()
+        b = self._buffers
+        bias = b["bias"] if "bias" in b else self.bias
+        epi = _EPILOGUES[self.epilogue]
+        quantized = type(x) is QuantizedActivation
+        if quantized and x.dtype not in (torch.float16, torch.bfloat16):
+            return None
+        if self.mode == "tc":
+            if quantized:
+                return native.gemm_dense(x.q, x.scale, b["weight_int8_nk"], b["weight_scale"], bias,
+                                         1 if x.dtype is torch.bfloat16 else 0, epi, x.shape)
+            return native.linear_dense(x, b["weight_int8_nk"], b["weight_scale"], bias, epi)
+        if self.mode == "sparse":
+            if quantized:
+                return native.gemm_sparse(x.q, x.scale, b["weight_sparse_comp"], b["weight_sparse_meta"],
+                                          b["weight_scale"], bias, 1 if x.dtype is torch.bfloat16 else 0, epi, x.shape)
+            return native.linear_sparse(x, b["weight_sparse_comp"], b["weight_sparse_meta"], b["weight_scale"], bias, epi)
+        return None
+
     def _bias_or_empty(self, x: torch.Tensor) -> torch.Tensor:
         """"No bias" crosses the extension boundary as a zero-element tensor
         (reference: quantize_utils.py:270-275)."""
@@ -387,6 +433,9 @@ class Int8Linear(nn.Module):
         return y.reshape(*x.shape[:-1], y.shape[-1])
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        y = self._native_forward(x)
+        if y is not None:
+            return y
         if isinstance(x, QuantizedActivation):
             return self._forward_quantized(x)
         if not x.is_cuda:

@@ -23,6 +23,8 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import quantize_utils as _qu
+
 
 def timestep_embedding(t: torch.Tensor, dim: int) -> torch.Tensor:
     """Sinusoidal embedding (flip_sin_to_cos, freq_shift 0 as in SD2.1)."""
@@ -51,14 +53,20 @@ class GroupNormNHWC(nn.GroupNorm):
         time-embedding projection of a ResNet block); the kernel path adds it on the fly."""
         if (self.fused and x.is_cuda and x.dim() == 4 and x.dtype in (torch.float16, torch.bfloat16)
                 and x.is_contiguous(memory_format=torch.channels_last)):
+            if add is not None and add.dtype != x.dtype:
+                add = add.to(x.dtype)
+            p = self._parameters
+            y = (_qu._NATIVE or _qu._load_native()).groupnorm_nhwc(
+                x, self.num_groups, p["weight"], p["bias"], self.eps, self.silu, add)
+            if y is not None:
+                return y
             if self._ik is None:
                 from .csrc.build import load_int8_kernels
                 self._ik = load_int8_kernels()
             if self._ws is None or self._ws.device != x.device:
                 self._ws = torch.empty(1 << 16, dtype=torch.float32, device=x.device)
             return self._ik.groupnorm_nhwc(x, self.num_groups, self.weight, self.bias, self.eps,
-                                           silu=self.silu, workspace=self._ws,
-                                           add=None if add is None else add.to(x.dtype))
+                                           silu=self.silu, workspace=self._ws, add=add)
         if add is not None:
             x = x + add[:, :, None, None]
         y = super().forward(x)
