@@ -122,14 +122,11 @@ __device__ __forceinline__ void slab_math(const uint32_t (&r)[32], float as, con
                                    static_cast<float>(static_cast<int32_t>(r[4 * q + 1])));
     const float2 a23 = make_float2(static_cast<float>(static_cast<int32_t>(r[4 * q + 2])),
                                    static_cast<float>(static_cast<int32_t>(r[4 * q + 3])));
-    const float2 y01 = __ffma2_rn(a01, s01, make_float2(b4.x, b4.y));
-    const float2 y23 = __ffma2_rn(a23, s23, make_float2(b4.z, b4.w));
-    float y0 = y01.x, y1 = y01.y, y2 = y23.x, y3 = y23.y;
-    if (kEpi == HY3D_EPI_GELU) {
-      y0 = gelu_erf(y0); y1 = gelu_erf(y1); y2 = gelu_erf(y2); y3 = gelu_erf(y3);
-    }
-    packed[2 * q] = pack2t<kBf16>(y0, y1);
-    packed[2 * q + 1] = pack2t<kBf16>(y2, y3);
+    float2 y01 = __ffma2_rn(a01, s01, make_float2(b4.x, b4.y));
+    float2 y23 = __ffma2_rn(a23, s23, make_float2(b4.z, b4.w));
+    if (kEpi == HY3D_EPI_GELU) { y01 = gelu_phi2(y01); y23 = gelu_phi2(y23); }
+    packed[2 * q] = pack2t<kBf16>(y01.x, y01.y);
+    packed[2 * q + 1] = pack2t<kBf16>(y23.x, y23.y);
   }
 }
 
@@ -138,18 +135,24 @@ template <bool kBf16>
 __device__ __forceinline__ void slab_math_geglu(const uint32_t (&rv)[16], const uint32_t (&rg)[16],
                                                 float as, const float* wsb, const float* bsb,
                                                 uint32_t* packed8) {
+  // `as * ws` and the fused multiply-add of four neighbouring columns, packed as in slab_math.
+  auto scaled4 = [&](const uint32_t* r, const float* w, const float* b, float2& lo, float2& hi) {
+    const float4 w4 = *reinterpret_cast<const float4*>(w);
+    const float4 b4 = *reinterpret_cast<const float4*>(b);
+    const float2 as2 = make_float2(as, as);
+    lo = __ffma2_rn(make_float2(static_cast<float>(static_cast<int32_t>(r[0])), static_cast<float>(static_cast<int32_t>(r[1]))),
+                    __fmul2_rn(as2, make_float2(w4.x, w4.y)), make_float2(b4.x, b4.y));
+    hi = __ffma2_rn(make_float2(static_cast<float>(static_cast<int32_t>(r[2])), static_cast<float>(static_cast<int32_t>(r[3]))),
+                    __fmul2_rn(as2, make_float2(w4.z, w4.w)), make_float2(b4.z, b4.w));
+  };
 #pragma unroll
-  for (int j = 0; j < 16; j += 2) {
-    float y[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const float v = fmaf(static_cast<float>(static_cast<int32_t>(rv[j + u])), as * wsb[j + u],
-                           bsb[j + u]);
-      const float g = fmaf(static_cast<float>(static_cast<int32_t>(rg[j + u])),
-                           as * wsb[16 + j + u], bsb[16 + j + u]);
-      y[u] = v * gelu_erf(g);
-    }
-    packed8[j >> 1] = pack2t<kBf16>(y[0], y[1]);
+  for (int j = 0; j < 16; j += 4) {
+    float2 v0, v1, g0, g1;
+    scaled4(rv + j, wsb + j, bsb + j, v0, v1);
+    scaled4(rg + j, wsb + 16 + j, bsb + 16 + j, g0, g1);
+    const float2 y0 = __fmul2_rn(v0, gelu_phi2(g0)), y1 = __fmul2_rn(v1, gelu_phi2(g1));
+    packed8[j >> 1] = pack2t<kBf16>(y0.x, y0.y);
+    packed8[(j >> 1) + 1] = pack2t<kBf16>(y1.x, y1.y);
   }
 }
 
@@ -656,7 +659,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
               y[j] = fmaf(static_cast<float>(static_cast<int32_t>(r[j])), as * wsb[c + j], bsb[c + j]);
-              if (gelu) y[j] = gelu_erf(y[j]);
+              if (gelu) y[j] = gelu_phi(y[j]);
             }
             uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) +
                                                   static_cast<int64_t>(m) * ldo + n);
@@ -683,7 +686,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                                    bsb[c + j]);
               const float g = fmaf(static_cast<float>(static_cast<int32_t>(rg[j])),
                                    as * wsb[c + 16 + j], bsb[c + 16 + j]);
-              y[j] = v * gelu_erf(g);
+              y[j] = v * gelu_phi(g);
             }
             uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) +
                                                   static_cast<int64_t>(m) * ldo + (n >> 1));
@@ -753,7 +756,7 @@ __device__ __forceinline__ void load8_as_float(const void* p, int dtype, int n, 
 
 // Split-K tail: sums the int32 partials of every K range (exact) and applies the layer's
 // epilogue with the formula and roundings of the GEMM kernel's own (acc * (as * ws) + b,
-// optional exact-erf GELU, one rounding to the 16-bit type).  One thread per 8 output columns.
+// optional exact-form GELU, one rounding to the 16-bit type).  One thread per 8 output columns.
 template <bool kBf16, int kEpi>
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const int32_t* __restrict__ partial, int splits, int64_t split_stride,
@@ -806,7 +809,7 @@ splitk_reduce_kernel(const int32_t* __restrict__ partial, int splits, int64_t sp
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         y[u] = __fmaf_rn(static_cast<float>(acc[j + u]), __fmul_rn(as, wsf[j + u]), bf[j + u]);
-        if (kEpi == HY3D_EPI_GELU) y[u] = gelu_erf(y[u]);
+        if (kEpi == HY3D_EPI_GELU) y[u] = gelu_phi(y[u]);
       }
       w[j >> 1] = pack2t<kBf16>(y[0], y[1]);
     }

@@ -274,7 +274,8 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       const int t0 = (tile / p.w_tiles) * p.block_t;
       const int n = w0 + row_in_tile;
       const bool n_ok = n < p.N;
-      float ws = 0.0f, bs = 0.0f;
+      float ws = 0.0f, bs = 0.0f;                            // direct stores: weight row n
+      float wsr[4] = {0.0f, 0.0f, 0.0f, 0.0f}, bsr[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // fragment rows
       float sc_next = 0.0f;
       if (p.out_dtype != HY3D_S32) {
         if (p.tma_store) {
@@ -282,11 +283,19 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
           // the tile needs no CTA-wide barrier.
           const int t = t0 + half * kSlabTokens + lane;
           if (half * kSlabTokens < p.block_t && t < p.M) sc_next = p.act_scale[t];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int nr = w0 + quarter * 32 + (lane >> 2) + 8 * i;
+            if (nr < p.N) {
+              wsr[i] = load_scalar(p.w_scale, p.ws_dtype, nr);
+              bsr[i] = p.bias ? load_scalar(p.bias, p.bias_dtype, nr) : 0.0f;
+            }
+          }
         } else {
           for (int c = et; c < p.block_t; c += kEpiThreads)
             ctrl->as[buf][c] = (t0 + c) < p.M ? p.act_scale[t0 + c] : 0.0f;
         }
-        if (n_ok) {
+        if (!p.tma_store && n_ok) {
           ws = load_scalar(p.w_scale, p.ws_dtype, n);
           bs = p.bias ? load_scalar(p.bias, p.bias_dtype, n) : 0.0f;
         }
@@ -302,14 +311,25 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       const float* asb = ctrl->as[buf];
       if (p.tma_store) {
         float* asw = &ctrl->as[0][0] + (warp - 2) * kSlabTokens;   // this warp's 32 scales
-        // Slabs of 32 tokens; this thread owns output column n, the warp 32 adjacent columns,
-        // so a slab is a 32 (tokens) x 64 B block of the output, staged with 64-byte swizzle.
+        // Slabs of 32 tokens x the warp's 32 weight rows, read from tensor memory in accumulator-
+        // fragment order: a thread then holds neighbouring tokens of four weight rows (r, r + 8 from
+        // lanes 0-15; r + 16, r + 24 from lanes 16-31, r = lane / 4), which is what a transposing
+        // stmatrix takes -- four of those write the slab, where one thread per output column needed
+        // 32 two-byte stores.  With GEGLU, weight rows come in blocks of 16 value rows and their 16
+        // gate rows, so value and gate of an output sit in the same register of the two loads: no
+        // exchange between lanes, and every lane works on a gate.
         const int nslab = p.block_t / kSlabTokens;
-        const uint32_t chunk = static_cast<uint32_t>(lane) >> 3;
-        const uint32_t in_chunk = (static_cast<uint32_t>(lane) & 7u) * 2u;
+        const int frag_tok = 2 * (lane & 3);
+        // Output rows in the staging buffer: 64 bytes with 64-byte swizzle (16-byte chunk c of token j
+        // at c ^ ((j >> 1) & 3)), or 32 bytes with 32-byte swizzle after the gate (c ^ ((j >> 2) & 1));
+        // either way the eight rows of a matrix fall into different banks.
+        const uint32_t st_row = static_cast<uint32_t>(lane) & 7u, st_mat = static_cast<uint32_t>(lane) >> 3;
+        const uint32_t st_addr =
+            geglu ? stage_buf + (8u * (st_mat >> 1) + st_row) * 32u + (((st_mat & 1u) ^ ((st_row >> 2) & 1u)) << 4)
+                  : stage_buf + st_row * 64u + ((st_mat ^ ((st_row >> 1) & 3u)) << 4);
         for (int s = half; s < nslab; s += kWarpsPerQuarter) {
           const int c0 = s * kSlabTokens;
-          uint32_t r[32];
+          uint32_t ra[16], rb[16];
           const float sc = sc_next;
           {
             const int sn = s + kWarpsPerQuarter;
@@ -318,53 +338,32 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
           }
           __syncwarp();
           asw[lane] = sc;
-          tmem_ld_x32(t_row + c0, r);
+          tmem_ld_16x256b_x4(t_row + c0, ra);
+          tmem_ld_16x256b_x4(t_row + (16u << 16) + c0, rb);
           tmem_ld_wait();
-          __syncwarp();
-          float y[32];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const float4 a4 = *reinterpret_cast<const float4*>(asw + 4 * q);
-            y[4 * q + 0] = fmaf(static_cast<float>(static_cast<int32_t>(r[4 * q + 0])), a4.x * ws, bs);
-            y[4 * q + 1] = fmaf(static_cast<float>(static_cast<int32_t>(r[4 * q + 1])), a4.y * ws, bs);
-            y[4 * q + 2] = fmaf(static_cast<float>(static_cast<int32_t>(r[4 * q + 2])), a4.z * ws, bs);
-            y[4 * q + 3] = fmaf(static_cast<float>(static_cast<int32_t>(r[4 * q + 3])), a4.w * ws, bs);
-          }
-          if (gelu) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) y[j] = gelu_erf(y[j]);
-          }
-          if (geglu) {
-            // Weight rows come in blocks of 32 = 16 value rows then their 16 gate rows: lanes
-            // 0-15 hold the values, lanes 16-31 the matching gates of the same tokens.
-#pragma unroll
-            for (int j = 0; j < 32; ++j) y[j] = y[j] * gelu_erf(__shfl_down_sync(0xffffffffu, y[j], 16));
-          }
           if (lane == 0) tma_store_wait_read<0>();
           __syncwarp();
-          if (!geglu) {
+          // `as * ws` and the fused multiply-add of two neighbouring tokens of one weight row
+          auto scaled = [&](uint32_t a0, uint32_t a1, float2 as2, int i) {
+            return __ffma2_rn(make_float2(static_cast<float>(static_cast<int32_t>(a0)), static_cast<float>(static_cast<int32_t>(a1))),
+                              __fmul2_rn(as2, make_float2(wsr[i], wsr[i])), make_float2(bsr[i], bsr[i]));
+          };
+          uint32_t pr[4];
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              // token rows j, j+1 of the slab (64 B each): 16-byte chunk c of row j sits at
-              // c ^ ((j >> 1) & 3), the same for both rows of a pair; one conversion packs both.
-              const uint32_t addr = stage_buf + static_cast<uint32_t>(j) * 64u +
-                                    ((chunk ^ ((static_cast<uint32_t>(j) >> 1) & 3u)) << 4) + in_chunk;
-              const uint32_t pr = pack2(y[j], y[j + 1], kOutDtype);
-              const uint16_t lo = static_cast<uint16_t>(pr & 0xFFFFu);
-              const uint16_t hi = static_cast<uint16_t>(pr >> 16);
-              asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr), "h"(lo) : "memory");
-              asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr + 64u), "h"(hi) : "memory");
-            }
-          } else if (lane < 16) {
-            // 16 output columns per token: plain 32-byte rows (the store's box is 32 B wide)
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              const uint32_t addr = stage_buf + static_cast<uint32_t>(j) * 32u + static_cast<uint32_t>(lane) * 2u;
-              const uint32_t pr = pack2(y[j], y[j + 1], kOutDtype);
-              const uint16_t lo = static_cast<uint16_t>(pr & 0xFFFFu);
-              const uint16_t hi = static_cast<uint16_t>(pr >> 16);
-              asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr), "h"(lo) : "memory");
-              asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr + 32u), "h"(hi) : "memory");
+          for (int o = 0; o < 4; ++o) {              // eight tokens at a time
+            const float2 as2 = *reinterpret_cast<const float2*>(asw + 8 * o + frag_tok);
+            float2 y0 = scaled(ra[4 * o], ra[4 * o + 1], as2, 0), y1 = scaled(ra[4 * o + 2], ra[4 * o + 3], as2, 1);
+            float2 y2 = scaled(rb[4 * o], rb[4 * o + 1], as2, 2), y3 = scaled(rb[4 * o + 2], rb[4 * o + 3], as2, 3);
+            if (geglu) {
+              y0 = __fmul2_rn(y0, gelu_phi2(y2));
+              y1 = __fmul2_rn(y1, gelu_phi2(y3));
+              pr[2 * (o & 1)] = pack2(y0.x, y0.y, kOutDtype);
+              pr[2 * (o & 1) + 1] = pack2(y1.x, y1.y, kOutDtype);
+              if (o & 1) stmatrix_x4_trans(st_addr + (o >> 1) * 512u, pr[0], pr[1], pr[2], pr[3]);
+            } else {
+              if (gelu) { y0 = gelu_phi2(y0); y1 = gelu_phi2(y1); y2 = gelu_phi2(y2); y3 = gelu_phi2(y3); }
+              stmatrix_x4_trans(st_addr + o * 512u, pack2(y0.x, y0.y, kOutDtype), pack2(y1.x, y1.y, kOutDtype),
+                                pack2(y2.x, y2.y, kOutDtype), pack2(y3.x, y3.y, kOutDtype));
             }
           }
           fence_proxy_async_smem();
@@ -400,10 +399,10 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             for (int j = 0; j < 16; ++j) {
               const int t = t0 + c + j;
               float y = fmaf(static_cast<float>(static_cast<int32_t>(r[j])), asb[c + j] * ws, bs);
-              if (gelu) y = gelu_erf(y);
+              if (gelu) y = gelu_phi(y);
               if (geglu) {
                 const float g = __shfl_down_sync(0xffffffffu, y, 16);
-                y = y * gelu_erf(g);
+                y = y * gelu_phi(g);
                 if (lane < 16 && n_ok && t < p.M)
                   store_one(p.out, p.out_dtype, static_cast<int64_t>(t) * ldo + out_col, y);
               } else if (n_ok && t < p.M) {
@@ -537,7 +536,7 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
     const bool geglu = epilogue == HY3D_EPI_GEGLU;
     const uint64_t row_bytes = static_cast<uint64_t>(geglu ? N / 2 : N) * 2;
     rc = encode_tmap_2d_u8(&tm_o, out, row_bytes, static_cast<uint64_t>(M), row_bytes, geglu ? 32 : 64,
-                           kSlabTokens, geglu ? 0 : 64);
+                           kSlabTokens, geglu ? 32 : 64);
     if (rc != HY3D_OK) return rc;
   } else {
     tm_o = tm_x;   // unused by the kernel

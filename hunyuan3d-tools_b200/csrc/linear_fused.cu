@@ -116,7 +116,7 @@ __device__ __forceinline__ void chunk_math_store(const uint32_t (&r)[16], float 
     float2 y01 = __ffma2_rn(a01, s01, make_float2(b4.x, b4.y));
     float2 y23 = __ffma2_rn(a23, s23, make_float2(b4.z, b4.w));
     if (kEpi == HY3D_EPI_GELU) {
-      y01.x = gelu_erf(y01.x); y01.y = gelu_erf(y01.y); y23.x = gelu_erf(y23.x); y23.y = gelu_erf(y23.y);
+      y01 = gelu_phi2(y01); y23 = gelu_phi2(y23);
     }
     packed[2 * q] = dense::pack2t<kBf16>(y01.x, y01.y);
     packed[2 * q + 1] = dense::pack2t<kBf16>(y23.x, y23.y);
