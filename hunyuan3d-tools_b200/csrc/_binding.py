@@ -49,6 +49,7 @@ SIGNATURES = {
                                       c_void_p],
     "hy3d_prune_pack_24": [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_int64,
                            c_void_p],
+    "hy3d_quantize_weight": [c_void_p, c_int, c_int64, c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_int, c_void_p],
     "hy3d_gemm_w8a8_sparse24": [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int,
                                 c_void_p, c_int, c_void_p, c_int, c_int64, c_int64, c_int64,
                                 c_int, c_int, c_void_p],
@@ -71,7 +72,7 @@ SIGNATURES = {
 }
 
 # The argument lists above belong to this ABI version of the library (hy3d_version()).
-ABI_VERSION = 201
+ABI_VERSION = 202
 
 
 def configure(lib: ctypes.CDLL) -> ctypes.CDLL:

@@ -309,6 +309,13 @@ int hy3d_prune_pack_24(const int8_t* w, int64_t N, int64_t K, int8_t* comp, uint
                        static_cast<cudaStream_t>(stream));
 }
 
+int hy3d_quantize_weight(const void* w, int w_dtype, int64_t N, int64_t K, int8_t* codes, uint32_t* meta,
+                         int64_t meta_ld, void* scale, int scale_dtype, void* stream) {
+  const int rc = check_device();
+  if (rc != HY3D_OK) return rc;
+  return quantize_weight(w, w_dtype, N, K, codes, meta, meta_ld, scale, scale_dtype, static_cast<cudaStream_t>(stream));
+}
+
 int hy3d_gemm_w8a8_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
                             const uint32_t* w_meta, int64_t meta_ld, const void* w_scale,
                             int w_scale_dtype, const void* bias, int bias_dtype, void* out,

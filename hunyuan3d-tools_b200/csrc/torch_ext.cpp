@@ -35,6 +35,7 @@ struct Api {
   HY3D_FN(hy3d_layernorm_quantize);
   HY3D_FN(hy3d_groupnorm_nhwc);
   HY3D_FN(hy3d_groupnorm_workspace_floats);
+  HY3D_FN(hy3d_quantize_weight);
   HY3D_FN(hy3d_status_string);
 } api;
 #undef HY3D_FN
@@ -342,6 +343,42 @@ PyObject* groupnorm_nhwc(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// quantize_weight(w (N,K), sparse) -> (codes, scale) or (compressed codes, metadata, scale) | None
+PyObject* quantize_weight(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 2) return none();
+  const at::Tensor* w = plain(a[0]);
+  if (!w || w->dim() != 2) return none();
+  const int code = param_code(w->scalar_type());
+  const int64_t N = w->size(0), K = w->size(1);
+  if (code < 0 || N <= 0 || K <= 0 || (K & 31) || (reinterpret_cast<uintptr_t>(w->const_data_ptr()) & 15)) return none();
+  const bool sparse = a[1] == Py_True;
+  c10::cuda::CUDAGuard guard(w->device());
+  cudaStream_t st = c10::cuda::getCurrentCUDAStream(w->device().index()).stream();
+  const auto dev = w->device();
+  const int64_t ld = 4 * ((K + 127) / 128);
+  at::Tensor out[3];
+  int count = 0;
+  out[count++] = at::Tensor(at::detail::empty_cuda({N, sparse ? K / 2 : K}, at::kChar, dev, std::nullopt));
+  if (sparse) out[count++] = at::Tensor(at::detail::empty_cuda({N, ld}, at::kInt, dev, std::nullopt));
+  const at::ScalarType st_type = w->scalar_type() == at::kBFloat16 ? at::kBFloat16 : at::kHalf;
+  out[count++] = at::Tensor(at::detail::empty_cuda({N}, st_type, dev, std::nullopt));
+  const int rc = api.hy3d_quantize_weight(
+      w->const_data_ptr(), code, N, K, out[0].mutable_data_ptr<int8_t>(),
+      sparse ? reinterpret_cast<uint32_t*>(out[1].mutable_data_ptr<int32_t>()) : nullptr, sparse ? ld : 0,
+      out[count - 1].mutable_data_ptr(), half_code(st_type), st);
+  if (rc != HY3D_OK) return failed("hy3d_quantize_weight", rc);
+  PyObject* r = PyTuple_New(count);
+  if (!r) return nullptr;
+  for (int i = 0; i < count; ++i) {
+    PyObject* o = THPVariable_Wrap(std::move(out[i]));
+    if (!o) { Py_DECREF(r); return nullptr; }
+    PyTuple_SET_ITEM(r, i, o);
+  }
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
 // open(path): resolves the C ABI in the library at `path`, which the caller has loaded and checked.
 PyObject* open_library(PyObject*, PyObject* arg) {
   const char* path = PyUnicode_AsUTF8(arg);
@@ -369,6 +406,7 @@ PyObject* open_library(PyObject*, PyObject* arg) {
   HY3D_SYM(hy3d_layernorm_quantize);
   HY3D_SYM(hy3d_groupnorm_nhwc);
   HY3D_SYM(hy3d_groupnorm_workspace_floats);
+  HY3D_SYM(hy3d_quantize_weight);
   HY3D_SYM(hy3d_status_string);
 #undef HY3D_SYM
   Py_RETURN_NONE;
@@ -383,6 +421,7 @@ PyMethodDef methods[] = {
     HY3D_FAST(gemm_sparse),
     HY3D_FAST(layernorm_quantize),
     HY3D_FAST(groupnorm_nhwc),
+    HY3D_FAST(quantize_weight),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "hy3d_torch", "Native host path of the INT8 layers.", -1, methods,

@@ -210,12 +210,7 @@ class Int8Linear(nn.Module):
 
     def __init__(self, in_features: int, out_features: int, bias: bool = True,
                  dtype: torch.dtype = torch.float16):
-        super().__init__()
-        self.in_features = in_features
-        self.out_features = out_features
-        # The reference's eligibility rule (quantize_utils.py:175-178).
-        self._tc_ok = (in_features % 64 == 0) and (out_features % 16 == 0)
-        self._sparse_ok = (in_features % 64 == 0) and (out_features % 16 == 0)
+        self._init_sizes(in_features, out_features)
         self.register_buffer("weight_int8_nk", torch.zeros(out_features, in_features, dtype=torch.int8))
         self.register_buffer("weight_scale", torch.ones(out_features, dtype=dtype))
         self.register_buffer("weight_sparse_comp", None)
@@ -225,14 +220,43 @@ class Int8Linear(nn.Module):
         else:
             self.bias = None
 
+    def _init_sizes(self, in_features: int, out_features: int):
+        super().__init__()
+        self.in_features = in_features
+        self.out_features = out_features
+        # The reference's eligibility rule (quantize_utils.py:175-178).
+        self._tc_ok = (in_features % 64 == 0) and (out_features % 16 == 0)
+        self._sparse_ok = (in_features % 64 == 0) and (out_features % 16 == 0)
+
     # -- construction ------------------------------------------------------------------
+    @staticmethod
+    def _assemble(linear, dt, codes, scale, comp=None, meta=None) -> "Int8Linear":
+        """A layer around finished buffers, without the placeholder tensors of ``__init__``."""
+        layer = Int8Linear.__new__(Int8Linear)
+        layer._init_sizes(linear.in_features, linear.out_features)
+        b = layer._buffers
+        b["weight_int8_nk"], b["weight_scale"] = codes, scale
+        b["weight_sparse_comp"], b["weight_sparse_meta"] = comp, meta
+        if linear.bias is not None:
+            b["bias"] = linear.bias.data.to(dt)
+        else:
+            layer.bias = None
+        if comp is not None:
+            layer.mode = "sparse"
+        return layer
+
     @staticmethod
     def from_linear(linear: nn.Linear) -> "Int8Linear":
         """Per-channel quantisation of an ``nn.Linear`` (reference: quantize_utils.py:203-223)."""
         has_bias = linear.bias is not None
         dt = _param_dtype(linear)
+        weight = linear.weight
+        if weight.is_cuda:
+            got = (_NATIVE or _load_native()).quantize_weight(weight, False)
+            if got is not None:
+                return Int8Linear._assemble(linear, dt, got[0], got[1])
         layer = Int8Linear(linear.in_features, linear.out_features, bias=has_bias, dtype=dt)
-        weight_f32 = linear.weight.data.float()
+        weight_f32 = weight.data.float()
         # Same expressions as the reference, evaluated on the weight's device.  (On CUDA torch
         # divides by a Python scalar through its reciprocal, so a scale can differ by one ulp
         # from the CPU value; the reference behaves the same way.)
@@ -250,13 +274,17 @@ class Int8Linear(nn.Module):
         """2:4-sparse conversion (reference: quantize_utils.py:226-260): quantise with the
         scale of the UNPRUNED row, then prune on int8 magnitudes, compress and pack on the
         GPU."""
-        sp_mod = _load_sp()
         has_bias = linear.bias is not None
         dt = _param_dtype(linear)
         device = linear.weight.device
         if device.type != "cuda":
             raise RuntimeError("from_linear_sparse needs the layer on a CUDA device "
                                "(pruning and packing run on the GPU)")
+        got = (_NATIVE or _load_native()).quantize_weight(linear.weight, True)
+        if got is not None:
+            return Int8Linear._assemble(linear, dt, torch.empty(0, dtype=torch.int8, device=device), got[2],
+                                        got[0], got[1])
+        sp_mod = _load_sp()
         layer = Int8Linear(linear.in_features, linear.out_features, bias=has_bias, dtype=dt)
         weight_f32 = linear.weight.data.float()
         scale = weight_f32.abs().amax(dim=1).clamp(min=1e-8) / 127.0

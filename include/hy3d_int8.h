@@ -253,6 +253,19 @@ int hy3d_prune_pack_24(const int8_t* w, int64_t N, int64_t K,
                        uint32_t* meta_packed, int64_t meta_ld, void* stream);
 
 /*
+ * Per-output-channel int8 quantisation of a weight matrix w (N,K) (HY3D_F16 / HY3D_BF16 / HY3D_F32), and,
+ * with meta != NULL, 2:4 pruning, compression and packing of the codes in the same pass.
+ *   dense:  scale = max(amax / 127, 1e-8);  sparse: scale = max(amax, 1e-8) / 127  (of the UNPRUNED row)
+ *   q = clamp(rint(w / scale), -128, 127)
+ * The division by 127 multiplies by its fp32 reciprocal, as torch does on CUDA for a scalar divisor.
+ * codes: (N,K) int8, or (N,K/2) compressed values; meta: (N, meta_ld) as hy3d_prune_pack_24 writes it;
+ * scale: (N) in scale_dtype (HY3D_F16 or HY3D_BF16).  Requires K % 32 == 0, 16-byte aligned w and codes.
+ * Replaces: quantize_utils.py:203-223 (from_linear), 226-260 (from_linear_sparse) on CUDA weights.
+ */
+int hy3d_quantize_weight(const void* w, int w_dtype, int64_t N, int64_t K, int8_t* codes, uint32_t* meta,
+                         int64_t meta_ld, void* scale, int scale_dtype, void* stream);
+
+/*
  * 2:4 structured-sparse W8A8 GEMM with the same epilogues as the dense one.
  *   acc[m,n] = sum_k X[m,k] * Wpruned[n,k]
  * X: (M,K) int8.  w_comp: (N,K/2) int8.  w_meta: (N, meta_ld) uint32 as written by

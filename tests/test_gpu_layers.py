@@ -115,6 +115,34 @@ def test_sparse_layer_numerics(qu, sp, K, N, M):
     assert torch.equal(layer.weight_sparse_meta.cpu(), O.pack_metadata(no, layer.weight_sparse_meta.shape[1]))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("N,K", [(16, 64), (19, 96), (640, 320), (77, 2048), (33, 2080), (48, 6144), (1, 16384)])
+def test_weight_conversion_equals_the_torch_expressions(qu, sp, dtype, N, K):
+    """One kernel against the operation-by-operation torch form on the same device: codes, scales,
+    survivors and metadata bit for bit (rows at both sides of every thread-group size, ragged metadata
+    padding, an all-zero row, tiny and huge rows)."""
+    torch.manual_seed(N + K)
+    lin = nn.Linear(K, N, device=DEV, dtype=dtype)
+    lin.weight.data.copy_(torch.randn(N, K, device=DEV) * 0.02)
+    lin.weight.data[0] = 0
+    lin.weight.data[-1] *= 1e4
+    lin.weight.data[N // 2] *= 1e-5
+    w = lin.weight.data.float()
+    amax = w.abs().amax(dim=1)
+    dt = dtype if dtype != torch.float32 else torch.float16
+    for make, scale in ((qu.Int8Linear.from_linear, (amax / 127.0).clamp(min=1e-8)),
+                        (qu.Int8Linear.from_linear_sparse, amax.clamp(min=1e-8) / 127.0)):
+        layer = make(lin)
+        codes = (w / scale[:, None]).round().clamp(-128, 127).to(torch.int8)
+        assert torch.equal(layer.weight_scale, scale.to(dt))
+        if layer.mode == "sparse":
+            comp, meta = sp.sparse_prune_and_pack(codes)
+            assert torch.equal(layer.weight_sparse_comp, comp) and torch.equal(layer.weight_sparse_meta, meta)
+            assert layer.weight_int8_nk.numel() == 0
+        else:
+            assert torch.equal(layer.weight_int8_nk, codes)
+
+
 def test_geglu_fused_layer(qu):
     torch.manual_seed(3)
     lin = nn.Linear(320, 2560).to(DEV).bfloat16()
