@@ -49,6 +49,9 @@ SIGNATURES = {
                                       c_void_p],
     "hy3d_prune_pack_24": [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_int64,
                            c_void_p],
+    "hy3d_linear_cluster_plan": [c_int64, c_int64, c_int64, c_int, c_void_p, c_void_p],
+    "hy3d_linear_w8a8_cluster": [c_void_p, c_int, c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_int, c_void_p, c_int,
+                                 c_void_p, c_int64, c_int64, c_int64, c_int, c_int, c_int, c_void_p],
     "hy3d_quantize_weight": [c_void_p, c_int, c_int64, c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_int, c_void_p],
     "hy3d_gemm_w8a8_sparse24": [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int,
                                 c_void_p, c_int, c_void_p, c_int, c_int64, c_int64, c_int64,

@@ -301,6 +301,21 @@ int hy3d_linear_w8a8_dense_fused(const void* x, int x_dtype, int64_t ldx, float*
                       out_dtype, M, N, K, epilogue, block_n, static_cast<cudaStream_t>(stream));
 }
 
+int hy3d_linear_cluster_plan(int64_t M, int64_t N, int64_t K, int sparse, int* block_t, int* ks) {
+  if (!block_t || !ks || check_device() != HY3D_OK) return 0;
+  return linear_cluster_plan(M, N, K, sparse != 0, block_t, ks) ? 1 : 0;
+}
+
+int hy3d_linear_w8a8_cluster(const void* x, int x_dtype, int64_t ldx, const int8_t* w, const uint32_t* w_meta,
+                             int64_t meta_ld, const void* w_scale, int w_scale_dtype, const void* bias, int bias_dtype,
+                             void* out, int64_t M, int64_t N, int64_t K, int epilogue, int block_t, int ks,
+                             void* stream) {
+  const int rc = check_device();
+  if (rc != HY3D_OK) return rc;
+  return linear_cluster(x, x_dtype, ldx, w, w_meta, meta_ld, w_scale, w_scale_dtype, bias, bias_dtype, out, M, N, K,
+                        epilogue, block_t, ks, static_cast<cudaStream_t>(stream));
+}
+
 int hy3d_prune_pack_24(const int8_t* w, int64_t N, int64_t K, int8_t* comp, uint8_t* meta_raw,
                        uint32_t* meta_packed, int64_t meta_ld, void* stream) {
   const int rc = check_device();

@@ -14,6 +14,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -30,6 +31,8 @@ struct Api {
   HY3D_FN(hy3d_dense_splitk_plan);
   HY3D_FN(hy3d_gemm_w8a8_dense_splitk);
   HY3D_FN(hy3d_quantize_rows);
+  HY3D_FN(hy3d_linear_cluster_plan);
+  HY3D_FN(hy3d_linear_w8a8_cluster);
   HY3D_FN(hy3d_linear_w8a8_sparse24);
   HY3D_FN(hy3d_gemm_w8a8_sparse24);
   HY3D_FN(hy3d_layernorm_quantize);
@@ -111,6 +114,13 @@ bool small_int(PyObject* o, long lo, long hi, long* v) {
   return *v >= lo && *v <= hi;
 }
 
+// Small layers in one launch: what a caller waits for there is its own thread's launches, not the device.
+// A captured graph replays without those, so capture keeps the two kernels, the faster form on the device.
+bool one_launch(int64_t M, int64_t N, int64_t K, int sparse, int* block_t, int* ks) {
+  return api.hy3d_linear_cluster_plan(M, N, K, sparse, block_t, ks) &&
+         c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None;
+}
+
 // int8 GEMM + epilogue on codes that are already there; follows the library's split-K plan.
 int dense_gemm(const int8_t* q, const float* s, const at::Tensor& w, const Params& p, void* out, int out_code,
                int64_t M, int64_t N, int64_t K, int epi, cudaStream_t st) {
@@ -126,27 +136,31 @@ int dense_gemm(const int8_t* q, const float* s, const at::Tensor& w, const Param
 }
 
 // linear_dense(x, w_int8 (N,K), w_scale, bias | None, epilogue) -> y | None
-PyObject* linear_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
+PyObject* linear_dense_impl(PyObject* px, PyObject* pw, PyObject* pscale, PyObject* pbias, long epi) {
   HANDLE_TH_ERRORS
-  long epi = 0;
-  if (n != 5 || !small_int(a[4], 0, 2, &epi)) return none();
-  const at::Tensor *x = plain(a[0]), *w = plain(a[1]);
+  const at::Tensor *x = plain(px), *w = plain(pw);
   if (!x || !w || x->dim() < 1 || w->dim() != 2 || w->scalar_type() != at::kChar || w->device() != x->device())
     return none();
   const int code = half_code(x->scalar_type());
   const int64_t N = w->size(0), K = w->size(1);
   const int64_t M = K > 0 ? x->numel() / K : 0;
   if (code < 0 || M <= 0 || x->size(-1) != K || (K & 63) || (N & 15)) return none();
-  const Params p(a[2], a[3], N, x->device());
+  const Params p(pscale, pbias, N, x->device());
   if (!p.ok) return none();
   c10::cuda::CUDAGuard guard(x->device());
   cudaStream_t st = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
   at::Tensor y = out_like(x->sizes().slice(0, x->dim() - 1), epi == HY3D_EPI_GEGLU ? N / 2 : N, x->scalar_type(),
                           x->device());
+  int rc, block_t = 0, ks = 0;
+  if (one_launch(M, N, K, 0, &block_t, &ks)) {
+    rc = api.hy3d_linear_w8a8_cluster(x->const_data_ptr(), code, K, w->const_data_ptr<int8_t>(), nullptr, 0, p.ws, p.ws_code,
+                                      p.bias, p.bias_code, y.mutable_data_ptr(), M, N, K, static_cast<int>(epi), block_t, ks, st);
+    if (rc != HY3D_OK) return failed("hy3d_linear_w8a8_cluster", rc);
+    return THPVariable_Wrap(std::move(y));
+  }
   const size_t codes = align256(static_cast<size_t>(M) * K);
   Scratch ws(codes + static_cast<size_t>(M) * 4, st);
   int64_t bytes = 0;
-  int rc;
   if (api.hy3d_dense_splitk_plan(M, N, K, static_cast<int>(epi), &bytes) > 1) {
     rc = api.hy3d_quantize_rows(x->const_data_ptr(), code, M, K, K, ws.at(0), reinterpret_cast<float*>(ws.at(codes)), st);
     if (rc == HY3D_OK)
@@ -162,12 +176,16 @@ PyObject* linear_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// linear_sparse(x, w_comp (N,K/2), w_meta, w_scale, bias | None, epilogue) -> y | None
-PyObject* linear_sparse(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
+PyObject* linear_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
   long epi = 0;
-  if (n != 6 || !small_int(a[5], 0, 2, &epi)) return none();
-  const at::Tensor *x = plain(a[0]), *w = plain(a[1]), *e = plain(a[2]);
+  if (n != 5 || !small_int(a[4], 0, 2, &epi)) return none();
+  return linear_dense_impl(a[0], a[1], a[2], a[3], epi);
+}
+
+// linear_sparse(x, w_comp (N,K/2), w_meta, w_scale, bias | None, epilogue) -> y | None
+PyObject* linear_sparse_impl(PyObject* px, PyObject* pw, PyObject* pmeta, PyObject* pscale, PyObject* pbias, long epi) {
+  HANDLE_TH_ERRORS
+  const at::Tensor *x = plain(px), *w = plain(pw), *e = plain(pmeta);
   if (!x || !w || !e || x->dim() < 1 || w->dim() != 2 || e->dim() != 2 || w->scalar_type() != at::kChar ||
       e->scalar_type() != at::kInt || w->device() != x->device() || e->device() != x->device())
     return none();
@@ -175,21 +193,36 @@ PyObject* linear_sparse(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t N = w->size(0), K = 2 * w->size(1);
   const int64_t M = K > 0 ? x->numel() / K : 0;
   if (code < 0 || M <= 0 || x->size(-1) != K || (K & 63) || (N & 15) || e->size(0) != N) return none();
-  const Params p(a[3], a[4], N, x->device());
+  const Params p(pscale, pbias, N, x->device());
   if (!p.ok) return none();
   c10::cuda::CUDAGuard guard(x->device());
   cudaStream_t st = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
   at::Tensor y = out_like(x->sizes().slice(0, x->dim() - 1), epi == HY3D_EPI_GEGLU ? N / 2 : N, x->scalar_type(),
                           x->device());
+  int rc, block_t = 0, ks = 0;
+  if (one_launch(M, N, K, 1, &block_t, &ks)) {
+    rc = api.hy3d_linear_w8a8_cluster(x->const_data_ptr(), code, K, w->const_data_ptr<int8_t>(),
+                                      reinterpret_cast<const uint32_t*>(e->const_data_ptr<int32_t>()), e->size(1), p.ws,
+                                      p.ws_code, p.bias, p.bias_code, y.mutable_data_ptr(), M, N, K, static_cast<int>(epi),
+                                      block_t, ks, st);
+    if (rc != HY3D_OK) return failed("hy3d_linear_w8a8_cluster", rc);
+    return THPVariable_Wrap(std::move(y));
+  }
   const size_t codes = align256(static_cast<size_t>(M) * K);
   Scratch ws(codes + static_cast<size_t>(M) * 4, st);
-  const int rc = api.hy3d_linear_w8a8_sparse24(
+  rc = api.hy3d_linear_w8a8_sparse24(
       x->const_data_ptr(), code, K, ws.at(0), reinterpret_cast<float*>(ws.at(codes)), w->const_data_ptr<int8_t>(),
       reinterpret_cast<const uint32_t*>(e->const_data_ptr<int32_t>()), e->size(1), p.ws, p.ws_code, p.bias, p.bias_code,
       y.mutable_data_ptr(), code, M, N, K, static_cast<int>(epi), 0, st);
   if (rc != HY3D_OK) return failed("hy3d_linear_w8a8_sparse24", rc);
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS
+}
+
+PyObject* linear_sparse(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  long epi = 0;
+  if (n != 6 || !small_int(a[5], 0, 2, &epi)) return none();
+  return linear_sparse_impl(a[0], a[1], a[2], a[3], a[4], epi);
 }
 
 // The two forms of a layer whose input arrives as codes and per-row scales: the logical leading shape
@@ -256,6 +289,54 @@ PyObject* gemm_sparse(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (rc != HY3D_OK) return failed("hy3d_gemm_w8a8_sparse24", rc);
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS
+}
+
+// layer_forward(layer, x) -> y | None: Int8Linear.forward on a plain tensor.  Mode, epilogue and buffers
+// come without the look-ups that nn.Module routes through Python, a third of what those cost.
+struct Names {
+  PyObject *dict, *buffers, *mode, *epilogue, *bias, *wq, *scale, *comp, *meta;
+} names;
+bool intern_names() {
+  struct { PyObject** at; const char* text; } all[] = {
+      {&names.dict, "__dict__"}, {&names.buffers, "_buffers"}, {&names.mode, "mode"}, {&names.epilogue, "epilogue"},
+      {&names.bias, "bias"}, {&names.wq, "weight_int8_nk"}, {&names.scale, "weight_scale"},
+      {&names.comp, "weight_sparse_comp"}, {&names.meta, "weight_sparse_meta"}};
+  for (auto& n : all)
+    if (!(*n.at = PyUnicode_InternFromString(n.text))) return false;
+  return true;
+}
+PyObject* layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 2 || !THPVariable_CheckExact(a[1])) return none();
+  PyObject* dict = PyObject_GetAttr(a[0], names.dict);
+  if (!dict) return nullptr;
+  Py_DECREF(dict);                            // the layer keeps it
+  PyObject* buffers = PyDict_Check(dict) ? PyDict_GetItemWithError(dict, names.buffers) : nullptr;
+  if (!buffers || !PyDict_Check(buffers)) return none();
+  PyObject* bias = PyDict_GetItemWithError(buffers, names.bias);
+  if (!bias) bias = PyDict_GetItemWithError(dict, names.bias);
+  PyObject* scale = PyDict_GetItemWithError(buffers, names.scale);
+  if (!bias || !scale) return none();
+  // instance or class attributes, compared by text
+  auto attribute_is_one_of = [&](PyObject* name, std::initializer_list<const char*> texts) {
+    PyObject* v = PyObject_GetAttr(a[0], name);
+    if (!v) { PyErr_Clear(); return -1; }
+    int found = -1, i = 0;
+    for (const char* t : texts) {
+      if (PyUnicode_Check(v) && PyUnicode_CompareWithASCIIString(v, t) == 0) { found = i; break; }
+      ++i;
+    }
+    Py_DECREF(v);
+    return found;
+  };
+  const int mode = attribute_is_one_of(names.mode, {"tc", "sparse"});
+  const int epi = attribute_is_one_of(names.epilogue, {"linear", "gelu", "geglu"});   // HY3D_EPI_* in order
+  if (mode < 0 || epi < 0) return none();
+  const bool sparse = mode == 1;
+  PyObject* w = PyDict_GetItemWithError(buffers, sparse ? names.comp : names.wq);
+  if (!w) return none();
+  if (!sparse) return linear_dense_impl(a[1], w, scale, bias, epi);
+  PyObject* meta = PyDict_GetItemWithError(buffers, names.meta);
+  return meta ? linear_sparse_impl(a[1], w, meta, scale, bias, epi) : none();
 }
 
 // gamma and beta of a normalisation: both of one type (or absent).
@@ -401,6 +482,8 @@ PyObject* open_library(PyObject*, PyObject* arg) {
   HY3D_SYM(hy3d_dense_splitk_plan);
   HY3D_SYM(hy3d_gemm_w8a8_dense_splitk);
   HY3D_SYM(hy3d_quantize_rows);
+  HY3D_SYM(hy3d_linear_cluster_plan);
+  HY3D_SYM(hy3d_linear_w8a8_cluster);
   HY3D_SYM(hy3d_linear_w8a8_sparse24);
   HY3D_SYM(hy3d_gemm_w8a8_sparse24);
   HY3D_SYM(hy3d_layernorm_quantize);
@@ -415,6 +498,7 @@ PyObject* open_library(PyObject*, PyObject* arg) {
 #define HY3D_FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     {"open", open_library, METH_O, nullptr},
+    HY3D_FAST(layer_forward),
     HY3D_FAST(linear_dense),
     HY3D_FAST(linear_sparse),
     HY3D_FAST(gemm_dense),
@@ -430,6 +514,7 @@ PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "hy3d_torch", "Native host path
 }  // namespace
 
 PyMODINIT_FUNC PyInit_hy3d_torch(void) {
+  if (!intern_names()) return nullptr;
   PyObject* m = PyModule_Create(&module_def);
   if (m) PyModule_AddStringConstant(m, "source_digest", HY3D_EXT_DIGEST);
   return m;

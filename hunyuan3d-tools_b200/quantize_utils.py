@@ -400,26 +400,21 @@ class Int8Linear(nn.Module):
     _sp_ref = None
     _empty_bias = None
 
-    def _native_forward(self, x):
-        """The call on the native host path, or None where it declines.  Buffers come straight from
-        the module's dictionary: attribute look-ups through nn.Module cost as much as a launch."""
+    def _native_quantized(self, x: "QuantizedActivation"):
+        """GEMM + epilogue on the native host path, or None where it declines.  Buffers come straight
+        from the module's dictionary: attribute look-ups through nn.Module cost as much as a launch."""
+        if x.dtype not in (torch.float16, torch.bfloat16):
+            return None
         native = _NATIVE or _load_native()
         b = self._buffers
         bias = b["bias"] if "bias" in b else self.bias
-        epi = _EPILOGUES[self.epilogue]
-        quantized = type(x) is QuantizedActivation
-        if quantized and x.dtype not in (torch.float16, torch.bfloat16):
-            return None
+        bf16 = 1 if x.dtype is torch.bfloat16 else 0
         if self.mode == "tc":
-            if quantized:
-                return native.gemm_dense(x.q, x.scale, b["weight_int8_nk"], b["weight_scale"], bias,
-                                         1 if x.dtype is torch.bfloat16 else 0, epi, x.shape)
-            return native.linear_dense(x, b["weight_int8_nk"], b["weight_scale"], bias, epi)
+            return native.gemm_dense(x.q, x.scale, b["weight_int8_nk"], b["weight_scale"], bias, bf16,
+                                     _EPILOGUES[self.epilogue], x.shape)
         if self.mode == "sparse":
-            if quantized:
-                return native.gemm_sparse(x.q, x.scale, b["weight_sparse_comp"], b["weight_sparse_meta"],
-                                          b["weight_scale"], bias, 1 if x.dtype is torch.bfloat16 else 0, epi, x.shape)
-            return native.linear_sparse(x, b["weight_sparse_comp"], b["weight_sparse_meta"], b["weight_scale"], bias, epi)
+            return native.gemm_sparse(x.q, x.scale, b["weight_sparse_comp"], b["weight_sparse_meta"],
+                                      b["weight_scale"], bias, bf16, _EPILOGUES[self.epilogue], x.shape)
         return None
 
     def _bias_or_empty(self, x: torch.Tensor) -> torch.Tensor:
@@ -461,11 +456,12 @@ class Int8Linear(nn.Module):
         return y.reshape(*x.shape[:-1], y.shape[-1])
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        y = self._native_forward(x)
+        y = (_NATIVE or _load_native()).layer_forward(self, x)
         if y is not None:
             return y
         if isinstance(x, QuantizedActivation):
-            return self._forward_quantized(x)
+            y = self._native_quantized(x)
+            return y if y is not None else self._forward_quantized(x)
         if not x.is_cuda:
             raise RuntimeError("Int8Linear runs on CUDA tensors only (no CPU fallback)")
         if x.dtype not in (torch.float16, torch.bfloat16):

@@ -253,6 +253,24 @@ int hy3d_prune_pack_24(const int8_t* w, int64_t N, int64_t K,
                        uint32_t* meta_packed, int64_t meta_ld, void* stream);
 
 /*
+ * 1 and a plan for hy3d_linear_w8a8_cluster where a layer of this size is small enough that one launch
+ * serves a caller better than two, 0 otherwise.
+ */
+int hy3d_linear_cluster_plan(int64_t M, int64_t N, int64_t K, int sparse, int* block_t, int* ks);
+
+/*
+ * Whole linear layer in one launch for small problems (dense, or 2:4 sparse with w_meta != NULL), output in
+ * x's type; same bits as quantise + GEMM.  block_t tokens per block (a multiple of 32, or of 16 when one
+ * block holds all M rows; <= 256), ks ranges of K (a cluster of that many CTAs, <= 8).  HY3D_ERR_SHAPE where
+ * the token block over a K range does not fit in shared memory, or a range would be empty.
+ * w: (N,K) int8, or (N,K/2) compressed.  K % 32 == 0 (% 64 sparse), K <= 16384, N % 16 == 0 (% 32 GEGLU).
+ */
+int hy3d_linear_w8a8_cluster(const void* x, int x_dtype, int64_t ldx, const int8_t* w, const uint32_t* w_meta,
+                             int64_t meta_ld, const void* w_scale, int w_scale_dtype, const void* bias, int bias_dtype,
+                             void* out, int64_t M, int64_t N, int64_t K, int epilogue, int block_t, int ks,
+                             void* stream);
+
+/*
  * Per-output-channel int8 quantisation of a weight matrix w (N,K) (HY3D_F16 / HY3D_BF16 / HY3D_F32), and,
  * with meta != NULL, 2:4 pruning, compression and packing of the codes in the same pass.
  *   dense:  scale = max(amax / 127, 1e-8);  sparse: scale = max(amax, 1e-8) / 127  (of the UNPRUNED row)

@@ -514,3 +514,64 @@ def test_dense_splitk_plan_leaves_the_unet_shapes_alone(tc):
     for M, K, N in [(49152, 320, 320), (12288, 640, 5120), (3072, 5120, 1280), (924, 1024, 1280)]:
         assert tc.dense_splitk_plan(M, N, K)[0] == 1
     assert tc.dense_splitk_plan(257, 1536, 6144)[0] > 1
+
+
+@pytest.mark.parametrize("sparse", [False, True])
+@pytest.mark.parametrize("M,K,N,block_t,ks", [
+    (1, 64, 16, 16, 1),            # smallest problem, one ragged K unit
+    (16, 128, 128, 16, 1),         # a full 16-token block
+    (12, 1280, 640, 16, 5),        # K split over a cluster
+    (31, 2688, 1296, 32, 7),       # ragged ranges, ragged weight rows, more units than pipeline stages
+    (33, 448, 272, 32, 2),         # second token block of one row
+    (100, 1024, 320, 64, 3),       # ranges of unequal length
+    (257, 512, 160, 96, 1),
+    (300, 192, 96, 160, 1),
+    (256, 256, 64, 256, 2)])       # widest block
+def test_one_launch_layer_equals_two_launches(tc, sp, sparse, M, K, N, block_t, ks):
+    """The one-launch layer (codes written straight to the operand tiles, K ranges over a cluster) against
+    quantiser + GEMM: same codes, same integer sums, same epilogue, so the same bits."""
+    if sparse and ks > 1 and (ks - 1) * -(-(-(-K // 256)) // ks) >= -(-K // 256):
+        pytest.skip("a range would be empty")
+    g = torch.Generator(device=DEV).manual_seed(M + K)
+    wq = torch.randint(-127, 128, (N, K), generator=g, device=DEV, dtype=torch.int8)
+    comp, meta = sp.sparse_prune_and_pack(wq) if sparse else (wq, None)
+    for dtype in (torch.bfloat16, torch.float16):
+        x = torch.randn(M, K, generator=g, device=DEV).to(dtype)
+        ws = (torch.rand(N, generator=g, device=DEV) * 1e-3).to(dtype)
+        b = torch.randn(N, generator=g, device=DEV).to(dtype)
+        code = 1 if dtype == torch.bfloat16 else 0
+        q, s = tc._quantize(x)
+        for epi in (0, 1, 2):
+            if epi == 2 and N % 32:
+                continue
+            ref = (sp.sparse_int8_gemm(q, s, comp, meta, ws, b, out_dtype=dtype, epilogue=epi) if sparse
+                   else tc.int8_gemm_tc(q, wq, s, ws, b, out_dtype=dtype, epilogue=epi))
+            out = torch.full_like(ref, float("nan"))
+            rc = tc._lib.hy3d_linear_w8a8_cluster(
+                x.data_ptr(), code, K, comp.data_ptr(), meta.data_ptr() if sparse else None, meta.shape[1] if sparse else 0,
+                ws.data_ptr(), code, b.data_ptr(), code, out.data_ptr(), M, N, K, epi, block_t, ks,
+                torch.cuda.current_stream().cuda_stream)
+            assert rc == 0 and torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gelu_epilogue_over_its_whole_range(tc, dtype):
+    """Pre-activations from -14 to 14 in steps of 1/512 (accumulator k, scale 1/512): v * Phi(v) in double
+    precision, plus the 5e-7 the fp32 form may add, plus the output type's unit roundoff (8 / 11 significant
+    bits: 2^-8 / 2^-11 of the value, and half of fp16's spacing of 2^-24 below its normal range)."""
+    a = torch.zeros(128, 64, dtype=torch.int8, device=DEV)
+    w = torch.zeros(64, 64, dtype=torch.int8, device=DEV)
+    v = torch.arange(-7168, 7169, device=DEV)[: 128 * 112].reshape(-1)
+    for chunk in v.split(128):
+        a.zero_()
+        n = chunk.numel()
+        a[:n, 0] = torch.div(chunk, 64, rounding_mode="floor").to(torch.int8)     # chunk = 64 * a0 + a1
+        a[:n, 1] = (chunk % 64).to(torch.int8)
+        w[:, 0], w[:, 1] = 64, 1
+        y = tc.int8_gemm_tc(a, w, torch.full((128,), 1.0 / 512, device=DEV), torch.ones(64, device=DEV), None,
+                            out_dtype=dtype, epilogue=1)[:n, 0].double()
+        x = chunk.double() / 512
+        ref = x * torch.special.ndtr(x)
+        u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+        tol = ref.abs() * u + 5e-7 + (2.0 ** -25 if dtype == torch.float16 else 0.0)
+        assert bool(((y - ref).abs() <= tol).all())
