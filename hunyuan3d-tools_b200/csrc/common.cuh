@@ -483,6 +483,8 @@ __host__ __device__ constexpr uint32_t make_idesc_i8(uint32_t m, uint32_t n, boo
 // ------------------------------------------------------------------------------------
 // Epilogue arithmetic shared by the dense and sparse GEMMs
 // ------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t pack2(float a, float b, int out_dtype);
+
 // Exact-form GELU, v * Phi(v) with Phi the normal distribution function, two values at a time:
 //     gelu(v) = max(v, 0) - |v| * Phi(-|v|),   Phi(-t) = 2^h(t)
 // h = log2 Phi(-t) is smooth, so one degree-8 polynomial serves every t >= 0 without a branch: a
@@ -490,19 +492,25 @@ __host__ __device__ constexpr uint32_t make_idesc_i8(uint32_t m, uint32_t n, boo
 // error of Phi below 6e-8 and a relative one below 6e-5; past 5.5 the negative leading coefficient
 // carries it to -infinity.  Against double precision over |v| <= 14 the largest absolute error is
 // 2.8e-7 (4.4e-7 for 0.5 * v * (1 + erf(v / sqrt 2)) in fp32, which also cancels to 5 % relative error
-// around v = -5).  15 issue slots and two exponentials for a pair; the erf form with its two-sided
+// around v = -5).  13 issue slots and two exponentials for a pair; the erf form with its two-sided
 // polynomials took the GEGLU epilogue of 49152 x 320 -> 2560 to 113 us where the plain one takes 55.
 __device__ __forceinline__ float ex2_approx(float v) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
   return r;
 }
-__device__ __forceinline__ float2 gelu_phi2(float2 v) {
-  // nt = -|v|; the coefficients of odd powers carry the sign
-  const float2 nt = make_float2(__uint_as_float(__float_as_uint(v.x) | 0x80000000u),
-                                __uint_as_float(__float_as_uint(v.y) | 0x80000000u));
-  float2 h = make_float2(-8.168350404957891e-07f, -8.168350404957891e-07f);
-#define HY3D_HORNER(c) h = __ffma2_rn(h, nt, make_float2(c, c))
+// kN pairs at once: every coefficient is set up once for all of them and their chains overlap.
+template <int kN>
+__device__ __forceinline__ void gelu_phi2n(const float2 (&v)[kN], float2 (&out)[kN]) {
+  float2 nt[kN], h[kN];              // nt = -|v|; the coefficients of odd powers carry the sign
+#pragma unroll
+  for (int i = 0; i < kN; ++i) {
+    nt[i] = make_float2(__uint_as_float(__float_as_uint(v[i].x) | 0x80000000u),
+                        __uint_as_float(__float_as_uint(v[i].y) | 0x80000000u));
+    h[i] = make_float2(-8.168350404957891e-07f, -8.168350404957891e-07f);
+  }
+#define HY3D_HORNER(c)  \
+  _Pragma("unroll") for (int i = 0; i < kN; ++i) h[i] = __ffma2_rn(h[i], nt[i], make_float2(c, c))
   HY3D_HORNER(-1.411904850101564e-05f);
   HY3D_HORNER(-6.25546817900613e-05f);
   HY3D_HORNER(0.00043832603842020035f);
@@ -512,10 +520,80 @@ __device__ __forceinline__ float2 gelu_phi2(float2 v) {
   HY3D_HORNER(1.1511142253875732f);
   HY3D_HORNER(-0.9999998211860657f);
 #undef HY3D_HORNER
-  const float2 e = make_float2(ex2_approx(h.x), ex2_approx(h.y));
-  return __ffma2_rn(nt, e, make_float2(fmaxf(v.x, 0.0f), fmaxf(v.y, 0.0f)));
+#pragma unroll
+  for (int i = 0; i < kN; ++i)
+    out[i] = __ffma2_rn(nt[i], make_float2(ex2_approx(h[i].x), ex2_approx(h[i].y)),
+                        make_float2(fmaxf(v[i].x, 0.0f), fmaxf(v[i].y, 0.0f)));
+}
+__device__ __forceinline__ float2 gelu_phi2(float2 v) {
+  const float2 in[1] = {v};
+  float2 out[1];
+  gelu_phi2n<1>(in, out);
+  return out[0];
 }
 __device__ __forceinline__ float gelu_phi(float v) { return gelu_phi2(make_float2(v, v)).x; }
+
+// The erf form, 0.5 * v * (1 + erf(v / sqrt 2)), whose bf16 roundings the GEGLU gate reproduces.
+__device__ __forceinline__ float gelu_erf(float v) {
+  return 0.5f * v * (1.0f + erff(v * 0.70710678118654752440f));
+}
+
+// value * gelu(gate) for eight pairs of outputs, packed to the 16-bit type; pair(j, v, g) gives the operands
+// of pair j.  A gate feeds an int8 quantiser and, through it, the rest of a deep network, where one changed
+// rounding grows to the noise of the 8-bit codes (1.6-2.4 % of a UNet's output).  So with bf16 outputs the
+// fast form is kept only where it must round to what the erf form rounds to: over every finite fp32 g
+// (compared exhaustively on the device) the two differ by at most 2.1e-7 |g|, the products then by that times
+// |value| plus three roundings of at most 6e-8 |value g| each, hence by less than 4.5e-7 |value g|.  Both
+// ends of that interval round alike for all but about one output in 3,000 of unit-variance rows; the others
+// are recomputed by the erf form at the end.  fp16 outputs, which have no such history, keep the fast form,
+// the more accurate one.  Issue-bound: 49152 x 320 -> 2560 takes 79 us, 113 with the erf form throughout
+// and 66 without the test of the roundings.
+template <bool kBf16, typename Pair>
+__device__ __forceinline__ void gated_pairs(uint32_t (&out)[8], Pair pair) {
+  constexpr int kType = kBf16 ? HY3D_BF16 : HY3D_F16;
+  uint32_t differ[8], any = 0;
+#pragma unroll
+  for (int q = 0; q < 8; q += 4) {
+    float2 v[4], g[4], y[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) pair(q + j, v[j], g[j]);
+    gelu_phi2n<4>(g, y);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      y[j] = __fmul2_rn(v[j], y[j]);
+      if (kBf16) {
+        const float2 w = __fmul2_rn(v[j], g[j]);
+        const float2 a = __ffma2_rn(w, make_float2(4.5e-7f, 4.5e-7f), y[j]);
+        const float2 b = __ffma2_rn(w, make_float2(-4.5e-7f, -4.5e-7f), y[j]);
+        out[q + j] = pack2(a.x, a.y, kType);
+        differ[q + j] = out[q + j] ^ pack2(b.x, b.y, kType);
+      } else {
+        out[q + j] = pack2(y[j].x, y[j].y, kType);
+      }
+    }
+    if (kBf16) any = any | (differ[q] | differ[q + 1]) | (differ[q + 2] | differ[q + 3]);
+  }
+  if (kBf16 && any) {
+    uint32_t mask = 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) mask |= differ[u] ? 1u << u : 0u;
+    while (mask) {
+      const int j = __ffs(static_cast<int>(mask)) - 1;
+      mask &= mask - 1;
+      float2 v = make_float2(0.0f, 0.0f), g = v;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (u == j) pair(u, v, g);
+      const uint32_t w = pack2(v.x * gelu_erf(g.x), v.y * gelu_erf(g.y), kType);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) out[u] = u == j ? w : out[u];
+    }
+  }
+}
+template <bool kBf16>
+__device__ __forceinline__ float gated1(float v, float g) {
+  return v * (kBf16 ? gelu_erf(g) : gelu_phi(g));
+}
 
 template <typename T>
 __device__ __forceinline__ float load_as_float(const void* p, int dtype, int64_t i);

@@ -134,26 +134,22 @@ __device__ __forceinline__ void slab_math(const uint32_t (&r)[32], float as, con
 template <bool kBf16>
 __device__ __forceinline__ void slab_math_geglu(const uint32_t (&rv)[16], const uint32_t (&rg)[16],
                                                 float as, const float* wsb, const float* bsb,
-                                                uint32_t* packed8) {
-  // `as * ws` and the fused multiply-add of four neighbouring columns, packed as in slab_math.
-  auto scaled4 = [&](const uint32_t* r, const float* w, const float* b, float2& lo, float2& hi) {
-    const float4 w4 = *reinterpret_cast<const float4*>(w);
-    const float4 b4 = *reinterpret_cast<const float4*>(b);
-    const float2 as2 = make_float2(as, as);
-    lo = __ffma2_rn(make_float2(static_cast<float>(static_cast<int32_t>(r[0])), static_cast<float>(static_cast<int32_t>(r[1]))),
-                    __fmul2_rn(as2, make_float2(w4.x, w4.y)), make_float2(b4.x, b4.y));
-    hi = __ffma2_rn(make_float2(static_cast<float>(static_cast<int32_t>(r[2])), static_cast<float>(static_cast<int32_t>(r[3]))),
-                    __fmul2_rn(as2, make_float2(w4.z, w4.w)), make_float2(b4.z, b4.w));
+                                                uint32_t (&packed8)[8]) {
+  // `as * ws` and the fused multiply-add of two neighbouring columns, packed as in slab_math.
+  const float2 as2 = make_float2(as, as);
+  // (16-byte loads of the parameters: the two pairs that share one are unrolled next to each other)
+  auto scaled2 = [&](const uint32_t* r, const float* w, const float* b, int half) {
+    const float4 w4 = *reinterpret_cast<const float4*>(w), b4 = *reinterpret_cast<const float4*>(b);
+    return __ffma2_rn(make_float2(static_cast<float>(static_cast<int32_t>(r[0])), static_cast<float>(static_cast<int32_t>(r[1]))),
+                      __fmul2_rn(as2, half ? make_float2(w4.z, w4.w) : make_float2(w4.x, w4.y)),
+                      half ? make_float2(b4.z, b4.w) : make_float2(b4.x, b4.y));
   };
-#pragma unroll
-  for (int j = 0; j < 16; j += 4) {
-    float2 v0, v1, g0, g1;
-    scaled4(rv + j, wsb + j, bsb + j, v0, v1);
-    scaled4(rg + j, wsb + 16 + j, bsb + 16 + j, g0, g1);
-    const float2 y0 = __fmul2_rn(v0, gelu_phi2(g0)), y1 = __fmul2_rn(v1, gelu_phi2(g1));
-    packed8[j >> 1] = pack2t<kBf16>(y0.x, y0.y);
-    packed8[(j >> 1) + 1] = pack2t<kBf16>(y1.x, y1.y);
-  }
+  auto pair = [&](int j, float2& v, float2& g) {
+    const int c = 4 * (j >> 1);
+    v = scaled2(rv + 2 * j, wsb + c, bsb + c, j & 1);
+    g = scaled2(rg + 2 * j, wsb + 16 + c, bsb + 16 + c, j & 1);
+  };
+  gated_pairs<kBf16>(packed8, pair);
 }
 
 // Writes one packed 32 x 32 slab row into the warp's staging buffer (64-byte swizzle: 16-byte
@@ -622,15 +618,22 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           for (int s = half; s < nslab; s += kWarpsPerQuarter) {
             const int c0 = s * acc_per_slab;
             uint32_t packed[16];
-            __syncwarp();
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
-              uint32_t rv[16], rg[16];
+              uint32_t rv[16], rg[16], out[8];
               const int cb = c0 + 32 * b;
+              __syncwarp();
               tmem_ld_x16(t_row + cb, rv);
               tmem_ld_x16(t_row + cb + 16, rg);
               tmem_ld_wait();
-              slab_math_geglu<kBf16>(rv, rg, as, wsb + cb, bsb + cb, packed + 8 * b);
+              if (b == 1 && s + kWarpsPerQuarter >= nslab) {
+                tc_fence_before_sync();
+                release_acc(smem_u32(&ctrl->tmem_empty[buf]));
+                arrived = true;
+              }
+              slab_math_geglu<kBf16>(rv, rg, as, wsb + cb, bsb + cb, out);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) packed[8 * b + j] = out[j];
             }
             slab_store(packed, stage_buf + sb * kSlabBytes, lane, pend, &tm_o, ((n0 + c0) >> 1) * 2,
                        out_row, rows_in && ((n0 + c0) >> 1) < ldo);
@@ -686,7 +689,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                                    bsb[c + j]);
               const float g = fmaf(static_cast<float>(static_cast<int32_t>(rg[j])),
                                    as * wsb[c + 16 + j], bsb[c + 16 + j]);
-              y[j] = v * gelu_phi(g);
+              y[j] = gated1<kBf16>(v, g);
             }
             uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) +
                                                   static_cast<int64_t>(m) * ldo + (n >> 1));

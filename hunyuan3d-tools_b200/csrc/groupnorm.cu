@@ -4,15 +4,17 @@
 // elements per (sample, group).  torch's own GroupNorm kernel takes NCHW only, so a model whose
 // convolutions run NHWC pays two layout copies around every normalisation.
 //
-// One launch: a cluster of up to eight CTAs owns one sample's slab of whole groups, each CTA a range of
-// its rows.
-//   pass 1  per-channel sum and sum of squares in fp32 registers, folded into per-group partials in a
-//           fixed order and exchanged through distributed shared memory (no atomics: results do not
-//           depend on timing)
+// One launch: a cluster of up to eight CTAs owns one sample's slab of whole groups.
+//   pass 1  per-channel sum and sum of squares in fp32 registers, chunk of rows by chunk, folded into
+//           per-group partials and exchanged through distributed shared memory
 //   pass 2  mean / rstd per group, then y = x * (rstd * gamma[c]) + (beta[c] - mean * rstd * gamma[c]) on
 //           the rows read again (from L2, where pass 1 left them), rounded to the activation type; with
 //           silu the rounded value goes through v / (1 + exp(-v)) and is rounded again (the two roundings
 //           of GroupNorm followed by SiLU as separate ops)
+// Results must not depend on how the work is spread: a statistic that moves in its last place changes some
+// rounding of the output, and behind an int8 quantiser a deep network turns that into 2 % of its result.  So
+// the order of every sum is a function of (B, HW, C, groups) alone -- row chunks, row lanes within a chunk,
+// channels within a group, chunk classes -- and slabs, ranks and sets only say who adds which part.
 // Bound by HBM at the large sizes (2 x 31.5 MB for 12 x 320 x 64 x 64: 9.7 us) beside two special-function
 // instructions per element of the SiLU (7 us), by latency at the small ones.  Two grid-wide launches with
 // partials in global memory took 27.1 us there and 11.5 us for 12 x 1280 x 8 x 8.
@@ -21,11 +23,14 @@
 
 namespace hy3d {
 int device_sm_count();
+int ensure_max_smem(const void* kernel, int bytes);
 namespace gnorm {
 namespace {
 
-constexpr int kMaxThreads = 384;
-constexpr int kTargetThreads = 384;
+// Three CTAs per SM: 56 registers a thread, 64 with the addend, which would spill otherwise.
+__host__ __device__ constexpr int narrow_threads(bool add) { return add ? 320 : 384; }
+constexpr int kWideThreads = 1024;
+constexpr int kOrderThreads = 320;    // lanes of a chunk: what 320 threads over whole rows make
 constexpr int kMaxRanks = 8;          // portable cluster size
 
 template <bool kBf16>
@@ -62,30 +67,40 @@ __device__ __forceinline__ void cluster_sync_release() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Threads are laid out as (row lane ty, vector column tx): tx = tid % (slab / 8) owns 8 adjacent
-// channels, ty = tid / (slab / 8) walks rows ty, ty + k, ...  blockDim.x = (slab / 8) * k.
-// grid.x = S (the cluster: row ranges), grid.y = slabs, grid.z = samples.
-template <bool kBf16, bool kAdd, bool kSilu>
-__global__ void __launch_bounds__(kMaxThreads, 3)
+// How a sample's sums are ordered: `chunks` ranges of `rows` rows; `lanes` row lanes walk a chunk with a
+// stride of `lanes`; lanes, then the channels of a group are added in order; a group's chunk sums go to
+// `classes` running sums (chunk modulo classes), added in order last.
+struct Order {
+  int chunks, rows, lanes, classes;
+};
+
+// Threads are laid out as (row lane ty, vector column tx): tx = tid % (slab / 8) owns 8 adjacent channels.
+// In pass 1 every `order.lanes` lanes form a set that works on a chunk at a time, `reps` of them before the
+// CTA folds; in pass 2 all lanes walk the rank's rows.  grid.x = S (the cluster), grid.y = slabs, grid.z =
+// samples.
+// kWide: up to 1024 threads, one CTA per SM, for grids that do not fill the chip.
+template <bool kBf16, bool kAdd, bool kSilu, bool kWide>
+__global__ void __launch_bounds__(kWide ? kWideThreads : narrow_threads(kAdd), kWide ? 1 : 3)
 groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ add, int64_t HW, int C, int cpg,
-                 int slab_groups, int rows_per_cta, const void* __restrict__ gamma, const void* __restrict__ beta,
-                 int gb_dtype, float eps, uint16_t* __restrict__ y) {
-  // [S][2 * slab_groups] group partials of every rank, then the fold's [k][2][slab] per-channel sums (the
-  // first slice later holds every channel's scale and shift)
+                 int slab_groups, int rows_per_cta, int chunks_per_rank, int reps, Order order,
+                 const void* __restrict__ gamma, const void* __restrict__ beta, int gb_dtype, float eps,
+                 uint16_t* __restrict__ y) {
+  // [chunks][2 * slab_groups] group partials, [classes][2 * slab_groups] their class sums, then the fold's
+  // [sets * reps][lanes][2][slab] per-channel sums (the first slice later holds every channel's scale and shift)
   extern __shared__ float smem[];
   const int slab = slab_groups * cpg;
   const int vec_cols = slab >> 3, row_vecs = C >> 3;
-  const int k = blockDim.x / vec_cols;
+  const int k = blockDim.x / vec_cols, sets = k / order.lanes;
   const int tx = threadIdx.x % vec_cols, ty = threadIdx.x / vec_cols;
+  const int set = ty / order.lanes, lane = ty - set * order.lanes;
   const int S = gridDim.x, rank = blockIdx.x, b = blockIdx.z;
   const int c0 = static_cast<int>(blockIdx.y) * slab + 8 * tx;      // this thread's first channel
   float* s_part = smem;
-  float* s_acc = s_part + (S * 2 * slab_groups + 3) / 4 * 4;
+  float* s_class = s_part + order.chunks * 2 * slab_groups;
+  float* s_acc = smem + ((order.chunks + order.classes) * 2 * slab_groups + 3) / 4 * 4;
   pdl_launch_dependents();
   if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   pdl_wait();
-  const int64_t r0 = static_cast<int64_t>(rank) * rows_per_cta;
-  const int64_t r1 = r0 + rows_per_cta < HW ? r0 + rows_per_cta : HW;
   const int64_t base = static_cast<int64_t>(b) * HW * C + c0;
   const uint4* src = reinterpret_cast<const uint4*>(x + base);
   float2 av[4];
@@ -93,64 +108,89 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ ad
   for (int j = 0; j < 4; ++j) av[j] = make_float2(0.0f, 0.0f);
   if (kAdd) unpack8f<kBf16>(__ldcs(reinterpret_cast<const uint4*>(add + static_cast<int64_t>(b) * C + c0)), av);
 
-  float2 s2[4], q2[4];
+  bool peers_run = S == 1;
+  const int set_floats = order.lanes * 2 * slab;
+  const int last_chunk = min(order.chunks, (rank + 1) * chunks_per_rank);
+  for (int first = rank * chunks_per_rank; first < last_chunk; first += sets * reps) {
+    const int here = min(sets * reps, last_chunk - first);       // chunks of this batch
+    for (int slot = set; slot < here; slot += sets) {
+      float2 s2[4], q2[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) { s2[j] = make_float2(0.0f, 0.0f); q2[j] = make_float2(0.0f, 0.0f); }
-  auto accumulate = [&](const uint4& v) {
-    float2 f[4];
-    unpack8f<kBf16>(v, f);
-    if (kAdd) add_round8<kBf16>(f, av);
+      for (int j = 0; j < 4; ++j) { s2[j] = make_float2(0.0f, 0.0f); q2[j] = make_float2(0.0f, 0.0f); }
+      auto accumulate = [&](const uint4& v) {
+        float2 f[4];
+        unpack8f<kBf16>(v, f);
+        if (kAdd) add_round8<kBf16>(f, av);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) { s2[j] = __fadd2_rn(s2[j], f[j]); q2[j] = __ffma2_rn(f[j], f[j], q2[j]); }
-  };
-  const int64_t step = static_cast<int64_t>(k) * row_vecs, at0 = (r0 + ty) * row_vecs;
-  int left = static_cast<int>((r1 - r0 - ty + k - 1) / k);          // rows of this thread (may be < 1)
-  const uint4* in = src + at0;
-  for (; left >= 4; left -= 4, in += 4 * step) {                    // four rows in flight per thread
-    uint4 v[4];
+        for (int j = 0; j < 4; ++j) { s2[j] = __fadd2_rn(s2[j], f[j]); q2[j] = __ffma2_rn(f[j], f[j], q2[j]); }
+      };
+      const int64_t r0 = static_cast<int64_t>(first + slot) * order.rows;
+      const int rows = static_cast<int>(r0 + order.rows < HW ? order.rows : HW - r0);
+      const int step = order.lanes * row_vecs;                        // at most 320 vectors and a row
+      int left = (rows - lane + order.lanes - 1) / order.lanes;       // rows of this lane (may be < 1)
+      const uint4* in = src + (r0 + lane) * row_vecs;
+      for (; left > 0; left -= 4, in += 4 * step) {                   // four rows in flight per thread, to the last
+        uint4 v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = in[u * step];
+        for (int u = 0; u < 4; ++u)
+          if (u < left) v[u] = in[u * step];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) accumulate(v[u]);
-  }
-  for (; left > 0; --left, in += step) accumulate(*in);
-
-  // Every row lane parks its sums in its own slice, channel c adds the k slices in order, group g its
-  // channels in order; the group sums go to every rank of the cluster.
-  float* mine = s_acc + static_cast<size_t>(ty) * 2 * slab + 8 * tx;
+        for (int u = 0; u < 4; ++u)
+          if (u < left) accumulate(v[u]);
+      }
+      // every row lane parks its sums in its own slice
+      float* mine = s_acc + slot * set_floats + lane * 2 * slab + 8 * tx;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    *reinterpret_cast<float2*>(mine + 2 * j) = s2[j];
-    *reinterpret_cast<float2*>(mine + slab + 2 * j) = q2[j];
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < 2 * slab; c += blockDim.x) {
-    float a = s_acc[c];
+      for (int j = 0; j < 4; ++j) {
+        *reinterpret_cast<float2*>(mine + 2 * j) = s2[j];
+        *reinterpret_cast<float2*>(mine + slab + 2 * j) = q2[j];
+      }
+    }
+    __syncthreads();
+    // Channel c adds the lanes of its chunk in order, group g its channels in order; the group sums of the
+    // chunk go to every rank of the cluster.
+    if (order.lanes > 1) {
+      for (int i = threadIdx.x; i < here * 2 * slab; i += blockDim.x) {
+        float* p = s_acc + i / (2 * slab) * set_floats + i % (2 * slab);
+        float a = *p;
 #pragma unroll 4
-    for (int lane = 1; lane < k; ++lane) a += s_acc[static_cast<size_t>(lane) * 2 * slab + c];
-    s_acc[c] = a;
+        for (int l = 1; l < order.lanes; ++l) a += p[l * 2 * slab];
+        *p = a;
+      }
+    }
+    if (!peers_run) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    peers_run = true;
+    __syncthreads();
+    for (int i = threadIdx.x; i < here * 2 * slab_groups; i += blockDim.x) {    // sums, then sums of squares
+      const int slot = i / (2 * slab_groups), g = i - slot * 2 * slab_groups;
+      const float* p = s_acc + slot * set_floats + g * cpg;
+      float a = 0.0f;
+#pragma unroll 4
+      for (int c = 0; c < cpg; ++c) a += p[c];
+      const uint32_t at = smem_u32(s_part + (first + slot) * 2 * slab_groups + g);
+      for (int peer = 0; peer < S; ++peer)
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_cta(at, static_cast<uint32_t>(peer))), "f"(a) : "memory");
+    }
+    __syncthreads();       // the slices are free again
   }
-  if (S > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // the peers run
-  __syncthreads();
-  for (int g = threadIdx.x; g < 2 * slab_groups; g += blockDim.x) {   // sums, then sums of squares
-    const float* p = s_acc + g * cpg;
+  if (!peers_run) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // a rank without chunks
+  if (S > 1) cluster_sync_release(); else __syncthreads();
+  for (int i = threadIdx.x; i < order.classes * 2 * slab_groups; i += blockDim.x) {
+    const int cls = i / (2 * slab_groups), g = i - cls * 2 * slab_groups;
     float a = 0.0f;
 #pragma unroll 4
-    for (int c = 0; c < cpg; ++c) a += p[c];
-    const uint32_t at = smem_u32(s_part + rank * 2 * slab_groups + g);
-    for (int peer = 0; peer < S; ++peer)
-      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_cta(at, static_cast<uint32_t>(peer))), "f"(a) : "memory");
+    for (int ch = cls; ch < order.chunks; ch += order.classes) a += s_part[ch * 2 * slab_groups + g];
+    s_class[i] = a;
   }
-  __syncwarp();
-  if (S > 1) cluster_sync_release(); else __syncthreads();
-  // One thread per channel of the slab turns the partials into scale and shift.
+  __syncthreads();
+  // One thread per channel of the slab turns the class sums into scale and shift.
   const float inv_n = 1.0f / (static_cast<float>(HW) * static_cast<float>(cpg));
   for (int c = threadIdx.x; c < slab; c += blockDim.x) {
     const int g = c / cpg;
     float a = 0.0f, q = 0.0f;
-    for (int peer = 0; peer < S; ++peer) {
-      a += s_part[peer * 2 * slab_groups + g];
-      q += s_part[peer * 2 * slab_groups + slab_groups + g];
+    for (int cls = 0; cls < order.classes; ++cls) {
+      a += s_class[cls * 2 * slab_groups + g];
+      q += s_class[cls * 2 * slab_groups + slab_groups + g];
     }
     const float mean = a * inv_n;
     const float rstd = rsqrtf(fmaxf(fmaf(-mean, mean, q * inv_n), 0.0f) + eps);
@@ -189,17 +229,22 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ ad
     }
     return make_uint4(w[0], w[1], w[2], w[3]);
   };
-  left = static_cast<int>((r1 - r0 - ty + k - 1) / k);
-  in = src + at0;
+  const int64_t r0 = static_cast<int64_t>(rank) * rows_per_cta;
+  const int rows = static_cast<int>(r0 + rows_per_cta < HW ? rows_per_cta : HW - r0);
+  const int64_t at0 = (r0 + ty) * row_vecs;
+  const int step = k * row_vecs;
+  int left = (rows - ty + k - 1) / k;                                 // may be < 1
+  const uint4* in = src + at0;
   uint4* out = dst + at0;
-  for (; left >= 4; left -= 4, in += 4 * step, out += 4 * step) {
+  for (; left > 0; left -= 4, in += 4 * step, out += 4 * step) {
     uint4 v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = __ldcs(in + u * step);
+    for (int u = 0; u < 4; ++u)
+      if (u < left) v[u] = __ldcs(in + u * step);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) out[u * step] = transform(v[u]);
+    for (int u = 0; u < 4; ++u)
+      if (u < left) out[u * step] = transform(v[u]);
   }
-  for (; left > 0; --left, in += step, out += step) *out = transform(__ldcs(in));
 }
 
 }  // namespace
@@ -222,37 +267,100 @@ int groupnorm_nhwc(const void* x, const void* add, int x_dtype, int64_t B, int64
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(add)) & 15)
     return HY3D_ERR_SHAPE;
   const int cpg = static_cast<int>(C / groups);
-  // Slab: the widest run of whole groups (a multiple of 8 channels, so that 16-byte vectors stay inside
-  // it) that still gives two CTAs per SM with clusters of eight; narrower than 32 channels only where
-  // nothing else divides, since a row of a slab is one contiguous piece.
+  // The order of the sums (see Order), fixed by the shape: chunks so that 320-thread blocks of whole rows
+  // would fill four per SM, at least eight rows each.
   const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
-  int slab_groups = 0;
-  for (int g = groups; g >= 1; --g) {
-    if (groups % g || (g * cpg) % 8 || g * cpg > 2560) continue;
-    if (slab_groups && g * cpg < 32) break;
-    slab_groups = g;
-    if (B * (groups / g) * kMaxRanks >= 2 * sms) break;
+  Order order;
+  {
+    int64_t want = static_cast<int64_t>(sms) * 4 / B;
+    want = want < 1 ? 1 : want > 64 ? 64 : want;
+    int64_t rows = (HW + want - 1) / want;
+    if (rows < 8) rows = 8;
+    order.chunks = static_cast<int>((HW + rows - 1) / rows);
+    order.rows = static_cast<int>((HW + order.chunks - 1) / order.chunks);
+    const int full_cols = static_cast<int>(C >> 3);
+    order.lanes = kOrderThreads / full_cols > 0 ? kOrderThreads / full_cols : 1;
+    order.classes = order.lanes * full_cols / groups > 0 ? order.lanes * full_cols / groups : 1;
+    if (order.lanes > order.rows) order.lanes = order.rows;     // the others would add zeros
   }
-  if (!slab_groups) return HY3D_ERR_SHAPE;
+  // A slab is a run of whole groups, a multiple of 8 channels (so that 16-byte vectors stay inside it) and,
+  // where the groups allow, at least 32 channels (one contiguous piece of a row); its partials take at most
+  // 32 KB.
+  int slab_groups = 0, ranks = 0, sets = 0;
+  bool wide = false;
+  auto slab_fits = [&](int g) {
+    return groups % g == 0 && (g * cpg) % 8 == 0 && static_cast<int64_t>(order.chunks) * g <= 4096;
+  };
+  // One round, one wave: the narrowest slab, and the fewest ranks (at best one: no exchange) with which every
+  // chunk has a set of its own and all CTAs are resident, as long as 64 CTAs remain; else the most ranks that
+  // do.  Against the rule below, 12 x 2560 x 8 x 8: 7.8 us for 11.2, 12 x 1920 x 32 x 32: 32.3 for 41.8,
+  // 4 x 96 x 96 x 96 (wide): 11.5 for 14.2.
+  {
+    int g = 1;
+    while (g < groups && !(slab_fits(g) && g * cpg >= 32)) ++g;
+    const int vec = g * cpg >> 3;
+    for (int w = 0; w < 2 && !ranks && slab_fits(g); ++w) {
+      for (int r = 1; r <= kMaxRanks; ++r) {
+        const int per_rank = (order.chunks + r - 1) / r;
+        if (r > 1 && (r - 1) * per_rank >= order.chunks) continue;      // a rank without chunks
+        const int64_t threads = static_cast<int64_t>(per_rank) * order.lanes * vec;
+        if (threads > (w ? kWideThreads : narrow_threads(add != nullptr))) continue;
+        const int64_t warps = (threads + 31) / 32;
+        int64_t resident = 65536 / ((w || add ? 64 : 56) * 32 * warps);        // by registers
+        if (resident > 64 / warps) resident = 64 / warps;
+        if (resident > 32) resident = 32;
+        const int64_t ctas = static_cast<int64_t>(r) * (groups / g) * B;
+        if (ctas * 20 > sms * resident * 19) continue;                  // clusters leave a few slots empty
+        slab_groups = g; ranks = r; sets = per_rank; wide = w != 0;
+        if (ctas >= 64) break;
+      }
+    }
+  }
+  // Otherwise the widest slab that still gives two CTAs per SM with clusters of eight; up to eight ranks
+  // while each has at least 16 rows and a chunk of its own; as many chunks at once as threads allow, evened
+  // out over the rounds.
+  if (!ranks) {
+    for (int g = groups; g >= 1; --g) {
+      if (!slab_fits(g)) continue;
+      if (slab_groups && g * cpg < 32) break;
+      slab_groups = g;
+      if (B * (groups / g) * kMaxRanks >= 2 * sms) break;
+    }
+    ranks = kMaxRanks;
+    while (ranks > 1 && (order.chunks < ranks || HW < static_cast<int64_t>(16) * ranks)) ranks >>= 1;
+    wide = static_cast<int64_t>(ranks) * (groups / slab_groups) * B <= sms;
+    sets = (wide ? kWideThreads : narrow_threads(add != nullptr)) / ((slab_groups * cpg >> 3) * order.lanes);
+    if (sets < 1) return HY3D_ERR_SHAPE;
+  }
   const int slab = slab_groups * cpg, vec_cols = slab >> 3;
-  // Rank count: up to eight, while every row lane keeps at least four rows.
-  int k = kTargetThreads / vec_cols > 0 ? kTargetThreads / vec_cols : 1;
-  int ranks = kMaxRanks;
-  while (ranks > 1 && HW < static_cast<int64_t>(4) * k * ranks && HW < static_cast<int64_t>(32) * ranks) ranks >>= 1;
+  // As many rounds as 40 KB of slices hold between two folds.
+  const int chunks_per_rank = (order.chunks + ranks - 1) / ranks;
+  const int rounds = (chunks_per_rank + sets - 1) / sets;
+  sets = (chunks_per_rank + rounds - 1) / rounds;
+  const int k = sets * order.lanes;
+  int reps = 40 * 1024 / (k * 2 * slab * 4);
+  reps = reps < 1 ? 1 : reps > rounds ? rounds : reps;
   const int64_t rows_per_cta = (HW + ranks - 1) / ranks;
-  if (rows_per_cta < k) k = static_cast<int>(rows_per_cta);
-  const size_t smem = (static_cast<size_t>(ranks * 2 * slab_groups + 3) + static_cast<size_t>(k) * 2 * slab) * sizeof(float);
+  const size_t smem = (static_cast<size_t>(order.chunks + order.classes) * 2 * slab_groups + 3 +
+                       static_cast<size_t>(reps) * k * 2 * slab) * sizeof(float);
   if (rows_per_cta > 0x7FFFFFFF || B > 65535 || groups / slab_groups > 65535) return HY3D_ERR_SHAPE;
   (void)workspace;
 
-  using KernelFn = void (*)(const uint16_t*, const uint16_t*, int64_t, int, int, int, int, const void*, const void*, int,
-                            float, uint16_t*);
-  static const KernelFn kernels[2][2][2] = {
-      {{groupnorm_kernel<false, false, false>, groupnorm_kernel<false, false, true>},
-       {groupnorm_kernel<false, true, false>, groupnorm_kernel<false, true, true>}},
-      {{groupnorm_kernel<true, false, false>, groupnorm_kernel<true, false, true>},
-       {groupnorm_kernel<true, true, false>, groupnorm_kernel<true, true, true>}}};
-  const KernelFn kernel = kernels[x_dtype == HY3D_BF16 ? 1 : 0][add ? 1 : 0][silu ? 1 : 0];
+  using KernelFn = void (*)(const uint16_t*, const uint16_t*, int64_t, int, int, int, int, int, int, Order, const void*,
+                            const void*, int, float, uint16_t*);
+#define HY3D_GN_ROW(W)                                                                           \
+  {{{groupnorm_kernel<false, false, false, W>, groupnorm_kernel<false, false, true, W>},         \
+    {groupnorm_kernel<false, true, false, W>, groupnorm_kernel<false, true, true, W>}},          \
+   {{groupnorm_kernel<true, false, false, W>, groupnorm_kernel<true, false, true, W>},           \
+    {groupnorm_kernel<true, true, false, W>, groupnorm_kernel<true, true, true, W>}}}
+  static const KernelFn kernels[2][2][2][2] = {HY3D_GN_ROW(false), HY3D_GN_ROW(true)};
+#undef HY3D_GN_ROW
+  const KernelFn kernel = kernels[wide ? 1 : 0][x_dtype == HY3D_BF16 ? 1 : 0][add ? 1 : 0][silu ? 1 : 0];
+  if (smem > 48 * 1024) {          // few samples of many chunks and narrow groups
+    const int rc = ensure_max_smem(reinterpret_cast<const void*>(kernel), 100 * 1024);
+    if (rc != HY3D_OK) return rc;
+    if (smem > 100 * 1024) return HY3D_ERR_SHAPE;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(ranks), static_cast<unsigned>(groups / slab_groups), static_cast<unsigned>(B));
   cfg.blockDim = dim3(static_cast<unsigned>(vec_cols * k));
@@ -268,7 +376,7 @@ int groupnorm_nhwc(const void* x, const void* add, int x_dtype, int64_t B, int64
   cfg.numAttrs = 2;
   const cudaError_t err = cudaLaunchKernelEx(
       &cfg, kernel, static_cast<const uint16_t*>(x), static_cast<const uint16_t*>(add), HW, static_cast<int>(C), cpg,
-      slab_groups, static_cast<int>(rows_per_cta), gamma, beta, gb_dtype, eps, static_cast<uint16_t*>(y));
+      slab_groups, static_cast<int>(rows_per_cta), chunks_per_rank, reps, order, gamma, beta, gb_dtype, eps, static_cast<uint16_t*>(y));
   if (err != cudaSuccess) {
     cudaGetLastError();
     return HY3D_ERR_CUDA;

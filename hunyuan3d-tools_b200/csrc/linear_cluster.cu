@@ -359,19 +359,25 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
       return __ffma2_rn(make_float2(static_cast<float>(static_cast<int32_t>(a0)), static_cast<float>(static_cast<int32_t>(a1))),
                         __fmul2_rn(as2, make_float2(wsr[i], wsr[i])), make_float2(bsr[i], bsr[i]));
     };
-    uint32_t pr[4];
+    if (geglu) {
+      // pair 2 o + h: tokens 8 o + frag_tok, + 1 of weight row r + 8 h and its gate row, 16 further on
+      uint32_t out[8];
+      auto pair = [&](int j, float2& v, float2& g) {
+        const int i = 2 * j, h = j & 1;
+        const float2 as2 = *reinterpret_cast<const float2*>(asw + 8 * (j >> 1) + frag_tok);
+        v = scaled(ra[i], ra[i + 1], as2, h);
+        g = scaled(rb[i], rb[i + 1], as2, 2 + h);
+      };
+      gated_pairs<kBf16>(out, pair);
+      __syncwarp();
+      stmatrix_x4_trans(st_addr, out[0], out[1], out[2], out[3]);
+      stmatrix_x4_trans(st_addr + 512u, out[4], out[5], out[6], out[7]);
+    } else {
 #pragma unroll
-    for (int o = 0; o < 4; ++o) {              // eight tokens at a time
-      const float2 as2 = *reinterpret_cast<const float2*>(asw + 8 * o + frag_tok);
-      float2 y0 = scaled(ra[4 * o], ra[4 * o + 1], as2, 0), y1 = scaled(ra[4 * o + 2], ra[4 * o + 3], as2, 1);
-      float2 y2 = scaled(rb[4 * o], rb[4 * o + 1], as2, 2), y3 = scaled(rb[4 * o + 2], rb[4 * o + 3], as2, 3);
-      if (geglu) {
-        y0 = __fmul2_rn(y0, gelu_phi2(y2));
-        y1 = __fmul2_rn(y1, gelu_phi2(y3));
-        pr[2 * (o & 1)] = pack2(y0.x, y0.y, kOutDtype);
-        pr[2 * (o & 1) + 1] = pack2(y1.x, y1.y, kOutDtype);
-        if (o & 1) stmatrix_x4_trans(st_addr + (o >> 1) * 512u, pr[0], pr[1], pr[2], pr[3]);
-      } else {
+      for (int o = 0; o < 4; ++o) {              // eight tokens at a time
+        const float2 as2 = *reinterpret_cast<const float2*>(asw + 8 * o + frag_tok);
+        float2 y0 = scaled(ra[4 * o], ra[4 * o + 1], as2, 0), y1 = scaled(ra[4 * o + 2], ra[4 * o + 3], as2, 1);
+        float2 y2 = scaled(rb[4 * o], rb[4 * o + 1], as2, 2), y3 = scaled(rb[4 * o + 2], rb[4 * o + 3], as2, 3);
         if (gelu) { y0 = gelu_phi2(y0); y1 = gelu_phi2(y1); y2 = gelu_phi2(y2); y3 = gelu_phi2(y3); }
         stmatrix_x4_trans(st_addr + o * 512u, pack2(y0.x, y0.y, kOutDtype), pack2(y1.x, y1.y, kOutDtype),
                           pack2(y2.x, y2.y, kOutDtype), pack2(y3.x, y3.y, kOutDtype));

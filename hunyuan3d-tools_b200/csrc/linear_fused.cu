@@ -532,8 +532,11 @@ linear_fused_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_const
               if (lane == 0) mbar_arrive(smem_u32(&ctrl->tmem_empty[buf]));
               arrived = true;
             }
-            dense::slab_math_geglu<kBf16>(rv, rg, as, wsb + j * kAps + 32 * b, bsb + j * kAps + 32 * b,
-                                          packed + 8 * b);
+            uint32_t out[8];
+            dense::slab_math_geglu<kBf16>(rv, rg, as, wsb + j * kAps + 32 * b, bsb + j * kAps + 32 * b, out);
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 8; ++u) packed[8 * b + u] = out[u];
           }
           const int out_col = (n0 + s * kAps) >> 1;
           dense::slab_store(packed, stage_buf + sb * kSlabBytes, lane, pend, &tm_o, out_col * 2, out_row,

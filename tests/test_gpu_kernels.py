@@ -575,3 +575,27 @@ def test_gelu_epilogue_over_its_whole_range(tc, dtype):
         u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
         tol = ref.abs() * u + 5e-7 + (2.0 ** -25 if dtype == torch.float16 else 0.0)
         assert bool(((y - ref).abs() <= tol).all())
+
+
+@pytest.mark.parametrize("sparse", [False, True])
+@pytest.mark.parametrize("M,K,N", [(200, 64, 32), (333, 320, 640), (1000, 1280, 480)])
+def test_bf16_gate_rounds_as_the_erf_form(tc, sp, sparse, M, K, N):
+    """The GEGLU epilogue computes most gates by another formula than 0.5 * g * (1 + erf(g / sqrt 2)) but
+    must round every bf16 output as that one does: torch's fp32 ops on the raw accumulators, bit for bit
+    (gates between about -10 and 10; without a bias the rescaled accumulator is one rounded product)."""
+    g = torch.Generator(device=DEV).manual_seed(K + N)
+    q = torch.randint(-127, 128, (M, K), generator=g, device=DEV, dtype=torch.int8)
+    w = torch.randint(-127, 128, (N, K), generator=g, device=DEV, dtype=torch.int8)
+    comp, meta = sp.sparse_prune_and_pack(w) if sparse else (w, None)
+    s = torch.rand(M, generator=g, device=DEV) * 2 + 0.5
+    ws = (torch.rand(N, generator=g, device=DEV) + 0.5) * 3.0 / (73.0 * 73.0 * K ** 0.5 * 1.25)
+    if sparse:
+        acc = sp.sparse_int8_gemm(q, None, comp, meta, None, None, out_dtype=torch.int32)
+        y = sp.sparse_int8_gemm(q, s, comp, meta, ws, None, out_dtype=torch.bfloat16, epilogue=2)
+    else:
+        acc = tc.int8_gemm_tc(q, w, None, None, None, out_dtype=torch.int32)
+        y = tc.int8_gemm_tc(q, w, s, ws, None, out_dtype=torch.bfloat16, epilogue=2)
+    v = (acc.double() * (s[:, None] * ws[None, :]).double()).float().view(M, N // 32, 2, 16)
+    value, gate = v[:, :, 0].reshape(M, -1), v[:, :, 1].reshape(M, -1)
+    ref = (value * (0.5 * gate * (1.0 + torch.erf(gate * 0.70710678118654752440)))).bfloat16()
+    assert torch.equal(y, ref)
