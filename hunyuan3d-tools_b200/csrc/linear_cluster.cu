@@ -177,16 +177,15 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     };
     auto write_row = [&](int r, float amax) {
       if (r >= rows) return;
-      const float scale = __fdiv_rn(fmaxf(amax, 1e-8f), 127.0f);
-      const float inv = __frcp_rn(scale);
-      if (sub == 0) ctrl->scale[r] = scale;
+      const quant::RowQuant rq = quant::row_quant(amax);
+      if (sub == 0) ctrl->scale[r] = rq.scale;
       const uint4* src = row_src(r);
       const uint32_t row_at = smem_base + static_cast<uint32_t>(r >> 3) * 1024u + static_cast<uint32_t>(r & 7) * 128u;
 #pragma unroll 2
       for (int c = sub; c < nvec; c += p.q_lanes) {
         float f[8];
         quant::unpack8<kBf16>(ld_l1(src + c), f);
-        const uint2 q = quant::quant8(f, scale, inv);
+        const uint2 q = quant::quant8(f, rq);
         // eight codes = half a 16-byte chunk of row r in token tile c / 16
         const uint32_t at = row_at + static_cast<uint32_t>(c >> 4) * tok_atom +
                             ((((static_cast<uint32_t>(c) >> 1) & 7u) ^ (static_cast<uint32_t>(r) & 7u)) << 4) +

@@ -198,8 +198,7 @@ __device__ __forceinline__ void quantiser_role(const FusedArgs& p, FusedCtrl* ct
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1)
       if (off < G) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-    const float scale = __fdiv_rn(fmaxf(amax, 1e-8f), 127.0f);
-    const float inv = __frcp_rn(scale);
+    const quant::RowQuant rq = quant::row_quant(amax);
     if (qw == 0 && lane == 0) HY3D_TRACE_FINE(0, tr, 8, idx);
     if (t == 0) {
       // The block's shared-memory tiles are free once the MMAs of the block that used them
@@ -210,8 +209,8 @@ __device__ __forceinline__ void quantiser_role(const FusedArgs& p, FusedCtrl* ct
         return false;
     }
     if (sub == 0) {
-      ctrl->as[blk & (kScaleSlots - 1)][row_local] = row_ok ? scale : 0.0f;
-      if (p.scale_out && row_ok) p.scale_out[row] = scale;
+      ctrl->as[blk & (kScaleSlots - 1)][row_local] = row_ok ? rq.scale : 0.0f;
+      if (p.scale_out && row_ok) p.scale_out[row] = rq.scale;
     }
     const uint32_t row_base = q.smem_base + static_cast<uint32_t>(abuf) * q.a_block_bytes +
                               static_cast<uint32_t>(row_local) * 128u;
@@ -222,7 +221,7 @@ __device__ __forceinline__ void quantiser_role(const FusedArgs& p, FusedCtrl* ct
       if (kLg > 0 || (i < V && sub + i * G < nvec)) {
         float f[8];
         quant::unpack8<kBf16>(v[i], f);
-        const uint2 c8 = quant::quant8(f, scale, inv);   // rows past M hold zeros: codes 0
+        const uint2 c8 = quant::quant8(f, rq);   // rows past M hold zeros: codes 0
         // byte offset of these 8 codes in the row: sub8 + 8 * G * i; with G fixed the second
         // term is a constant, so the swizzled address is a per-batch base plus an immediate
         const uint32_t kc = static_cast<uint32_t>(i * G) << 3;

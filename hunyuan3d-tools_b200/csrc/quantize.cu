@@ -4,16 +4,20 @@
 //     amax  = max_k |x[m,k]|                       (fp32)
 //     scale = max(amax, 1e-8f) / 127.0f            (IEEE division)
 //     q     = clamp(rint(x / scale), -128, 127)    (IEEE division, round-half-even)
-// The row is read ONCE with 16-byte loads and kept in registers between the absmax
-// reduction and the rounding pass, so the kernel moves 2*K + K + 4/M bytes per row.
-// 16-bit activations sit on a coarse grid, so quotients within rounding error of k + 0.5 are
-// common (about 0.2 % of the elements of a Gaussian bf16 row) and their codes depend on the
-// last bit of the IEEE quotient.  The quotient is therefore refined without a division
-// instruction: q0 = x * rcp(scale) with the correctly rounded reciprocal, then one residual
-// correction r = fma(-q0, scale, x); q = fma(r, rcp, q0).  A device-side enumeration of every
-// pair of 16-bit patterns (amax, x) with |x| <= amax -- 1.0e9 pairs for fp16, 1.07e9 for bf16,
-// i.e. every input this kernel can see -- found rint(q) == rint(__fdiv_rn(x, scale)) for all of
-// them (without the correction 16732 / 7424 pairs differ).
+// The row is read ONCE with 16-byte loads and kept in registers between the absmax reduction and the
+// rounding pass, so the kernel moves 2*K + K + 4/M bytes per row.
+//
+// The rounding costs one fused multiply-add per value, fma(x, mul, 1.5 * 2^23), with a multiplier that is
+// 1 / scale nudged by two units in the last place.  Why that is exact: x and amax carry at most 11 significant
+// bits, and x / amax = (2 k + 1) / 254 needs 127 to divide 2 k + 1 or the significand of amax (127 is prime).
+// So unless it divides the latter -- then scale * 127 == amax exactly and several ties exist -- the only tie is
+// x = amax / 2, between 63 and 64; every other quotient is at least 2.4e-4 away from one, far more than the
+// nudge (6e-5) and scale's own rounding move it.  At that tie the IEEE quotient of the rounded scale is 63.5 or
+// above (code 64, the even one) or below it (63); amax / scale, its double, tells which, and the nudge goes the
+// same way.  Rows whose scale is exact refine their quotient instead: q0 = x * rcp(scale), one residual
+// correction q = fma(fma(-q0, scale, x), rcp, q0).  A device-side enumeration of every pair of 16-bit patterns
+// (amax, x) with |x| <= amax -- 1.0e9 pairs for fp16, 1.07e9 for bf16, i.e. every input this kernel can see --
+// found rint(q) == rint(__fdiv_rn(x, scale)) for all of them.
 #include "common.cuh"
 
 namespace hy3d {
@@ -21,6 +25,8 @@ namespace quant {
 namespace {
 
 constexpr int kQuantThreads = 256;
+struct True { static constexpr bool value = true; };
+struct False { static constexpr bool value = false; };
 
 template <bool kBf16>
 __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
@@ -39,26 +45,20 @@ __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
   }
 }
 
-// Folds the eight 16-bit values of a 16-byte vector into a running packed |x| maximum
-// (two lanes per register), without widening them first.
+// Folds the eight 16-bit values of a 16-byte vector into a running packed maximum of |x| (two lanes per
+// register), without widening them first.  The signs of the result mean nothing.
 template <bool kBf16>
 __device__ __forceinline__ void absmax8(const uint4& v, uint32_t& acc) {
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    if (kBf16) {
-      const __nv_bfloat162 m = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&acc),
-                                       __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
-      acc = *reinterpret_cast<const uint32_t*>(&m);
-    } else {
-      const __half2 m = __hmax2(*reinterpret_cast<const __half2*>(&acc),
-                                __habs2(*reinterpret_cast<const __half2*>(&w[i])));
-      acc = *reinterpret_cast<const uint32_t*>(&m);
-    }
+    if (kBf16) asm("max.xorsign.abs.bf16x2 %0, %0, %1;" : "+r"(acc) : "r"(w[i]));
+    else asm("max.xorsign.abs.f16x2 %0, %0, %1;" : "+r"(acc) : "r"(w[i]));
   }
 }
 template <bool kBf16>
 __device__ __forceinline__ float absmax_to_float(uint32_t acc) {
+  acc &= 0x7FFF7FFFu;
   if (kBf16) {
     return fmaxf(__uint_as_float(acc << 16), __uint_as_float(acc & 0xFFFF0000u));
   }
@@ -66,33 +66,46 @@ __device__ __forceinline__ float absmax_to_float(uint32_t acc) {
   return fmaxf(t.x, t.y);
 }
 
-// Quantises eight values to eight int8 codes (two words).  Float <-> int conversion
-// instructions run at a fraction of the FMA rate on this architecture, so the final rounding
-// uses the 1.5 * 2^23 trick: adding that constant rounds |t| < 2^22 to the nearest integer
-// (ties to even, the FPU's own rounding) and leaves the two's-complement code in the low
-// mantissa byte, which a byte permute then gathers.  t is the refined quotient of the file
-// header, whose rounding equals that of the IEEE quotient for every 16-bit input.
-// No clamp is needed: scale = max|x| / 127 bounds |x / scale| by 127 (+ one rounding).
-__device__ __forceinline__ float refined_quotient(float x, float scale, float inv) {
-  const float q0 = x * inv;
-  return fmaf(fmaf(-q0, scale, x), inv, q0);
+// What a row's values are quantised with (see the file header).
+struct RowQuant {
+  float scale, mul, inv;
+  bool exact;      // scale * 127 == amax: refine the quotients
+};
+__device__ __forceinline__ RowQuant row_quant(float amax) {
+  RowQuant r;
+  const float a = fmaxf(amax, 1e-8f);
+  r.scale = __fdiv_rn(a, 127.0f);
+  r.inv = __frcp_rn(r.scale);
+  // The division's residual a - 127 scale is representable, so its sign and zero are the true ones; the IEEE
+  // quotient a / scale is 127 or more from half a unit in the last place (2^-18) below it on.
+  const float rest = fmaf(r.scale, -127.0f, a);
+  r.exact = rest == 0.0f;
+  r.mul = __int_as_float(__float_as_int(r.inv) + (fmaf(r.scale, 3.814697265625e-6f, rest) >= 0.0f ? 2 : -2));
+  return r;
 }
-// The same for two values at once with the packed fp32x2 instructions of sm_100 (each half is
-// an IEEE single-precision operation, so the results equal the scalar form bit for bit; the
-// point is half as many issue slots).  Returns refined quotient + 1.5 * 2^23.
-__device__ __forceinline__ float2 refined_quotient2_magic(float2 x, float scale, float inv) {
+
+// Quantises eight values to eight int8 codes (two words).  Float <-> int conversion instructions run at half
+// the FMA rate or less, so the rounding uses the 1.5 * 2^23 trick: adding that constant rounds |t| < 2^22 to
+// the nearest integer (ties to even, the FPU's own rounding) and leaves the two's-complement code in the low
+// mantissa byte, which a byte permute then gathers.  No clamp is needed: scale = max|x| / 127 bounds
+// |x / scale| by 127 (+ one rounding).  Packed fp32x2 instructions: two IEEE operations per issue slot.
+__device__ __forceinline__ float2 fast_code2(float2 x, float mul) {
+  return __ffma2_rn(x, make_float2(mul, mul), make_float2(12582912.0f, 12582912.0f));
+}
+__device__ __forceinline__ float2 refined_code2(float2 x, float scale, float inv) {
   const float2 inv2 = make_float2(inv, inv), nscale2 = make_float2(-scale, -scale);
   const float2 q0 = __fmul2_rn(x, inv2);
   const float2 r = __ffma2_rn(q0, nscale2, x);
   const float2 q = __ffma2_rn(r, inv2, q0);
   return __fadd2_rn(q, make_float2(12582912.0f, 12582912.0f));
 }
-
-__device__ __forceinline__ uint2 quant8(const float (&f)[8], float scale, float inv) {
+template <bool kExact>
+__device__ __forceinline__ uint2 quant8(const float (&f)[8], const RowQuant& r) {
   uint32_t b[8];
 #pragma unroll
   for (int j = 0; j < 8; j += 2) {
-    const float2 t = refined_quotient2_magic(make_float2(f[j], f[j + 1]), scale, inv);
+    const float2 x = make_float2(f[j], f[j + 1]);
+    const float2 t = kExact ? refined_code2(x, r.scale, r.inv) : fast_code2(x, r.mul);
     b[j] = __float_as_uint(t.x);
     b[j + 1] = __float_as_uint(t.y);
   }
@@ -100,109 +113,105 @@ __device__ __forceinline__ uint2 quant8(const float (&f)[8], float scale, float 
   const uint32_t p45 = __byte_perm(b[4], b[5], 0x0040), p67 = __byte_perm(b[6], b[7], 0x0040);
   return make_uint2(__byte_perm(p01, p23, 0x5410), __byte_perm(p45, p67, 0x5410));
 }
+__device__ __forceinline__ uint2 quant8(const float (&f)[8], const RowQuant& r) {
+  return r.exact ? quant8<true>(f, r) : quant8<false>(f, r);
+}
 
-// G threads cooperate on one row (G a power of two, 1..256); each holds up to kMaxV
-// 16-byte vectors.  A block of 256 threads covers 256/G rows.
-template <bool kBf16, int kMaxV>
-__global__ void __launch_bounds__(kQuantThreads, kMaxV <= 5 ? 4 : 3)
+// 2^lg threads cooperate on one row; each holds up to kMaxV 16-byte vectors.  A block of 256 threads covers
+// 256 >> lg rows; threads past the last row repeat it (same values to the same places).  kFull: every thread
+// has exactly kMaxV vectors.  Bound by HBM reads (the codes stay in L2 for the GEMM) and by issue slots:
+// about 35 instructions per 8 values.
+template <bool kBf16, int kMaxV, bool kFull>
+__global__ void __launch_bounds__(kQuantThreads, kMaxV <= 6 ? 5 : 4)
 quantize_rows_kernel(const uint16_t* __restrict__ x, int64_t ldx, int8_t* __restrict__ q,
-                     float* __restrict__ scale_out, int64_t M, int K, int G) {
+                     float* __restrict__ scale_out, int64_t M, int K, int lg) {
   __shared__ float s_part[kQuantThreads / 32];
   pdl_launch_dependents();
-  pdl_wait();   // x comes from the previous kernel in the stream
-  const int tid = threadIdx.x;
-  const int rows_per_block = kQuantThreads / G;
-  const int sub = tid % G;  // position within the row group
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * rows_per_block + tid / G;
-  const bool row_ok = row < M;
+  const int tid = threadIdx.x, G = 1 << lg;
+  const int sub = tid & (G - 1);  // position within the row group
+  int64_t row = static_cast<int64_t>(blockIdx.x) * (kQuantThreads >> lg) + (tid >> lg);
+  if (row >= M) row = M - 1;
   const int nvec = K >> 3;
+  const uint4* src = reinterpret_cast<const uint4*>(x + row * ldx) + sub;
+  uint2* dst = reinterpret_cast<uint2*>(q + row * static_cast<int64_t>(K)) + sub;
+  pdl_wait();   // x comes from the previous kernel in the stream
 
   uint4 v[kMaxV];
-  uint32_t amax2 = 0;
-  const uint4* src = reinterpret_cast<const uint4*>(x + (row_ok ? row : 0) * ldx);
 #pragma unroll
-  for (int i = 0; i < kMaxV; ++i) {
-    const int c = sub + i * G;
-    if (row_ok && c < nvec) {
-      v[i] = __ldcs(src + c);
-    } else {
-      v[i] = make_uint4(0, 0, 0, 0);
-    }
-  }
+  for (int i = 0; i < kMaxV; ++i)
+    v[i] = kFull || sub + i * G < nvec ? __ldcs(src + i * G) : make_uint4(0, 0, 0, 0);
+  uint32_t amax2 = 0;
 #pragma unroll
   for (int i = 0; i < kMaxV; ++i) absmax8<kBf16>(v[i], amax2);
   float amax = absmax_to_float<kBf16>(amax2);
-  // Reduce over the G threads of the row.
-  const int w = G < 32 ? G : 32;
-  for (int off = w >> 1; off > 0; off >>= 1)
+  // Reduce over the threads of the row.
+  for (int off = (G < 32 ? G : 32) >> 1; off > 0; off >>= 1)
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
   if (G > 32) {
     const int warp = tid >> 5;
     if ((tid & 31) == 0) s_part[warp] = amax;
     __syncthreads();
     const int warps_per_row = G >> 5;
-    const int first = (warp / warps_per_row) * warps_per_row;
+    const int first = warp & ~(warps_per_row - 1);
     amax = s_part[first];
     for (int i = 1; i < warps_per_row; ++i) amax = fmaxf(amax, s_part[first + i]);
   }
-  const float scale = __fdiv_rn(fmaxf(amax, 1e-8f), 127.0f);
-  const float inv = __frcp_rn(scale);
-  if (row_ok && sub == 0) scale_out[row] = scale;
-
-  uint2* dst = reinterpret_cast<uint2*>(q + (row_ok ? row : 0) * static_cast<int64_t>(K));
+  const RowQuant rq = row_quant(amax);
+  if (sub == 0) scale_out[row] = rq.scale;
+  auto write = [&](auto exact) {
 #pragma unroll
-  for (int i = 0; i < kMaxV; ++i) {
-    const int c = sub + i * G;
-    if (row_ok && c < nvec) {
-      float f[8];
-      unpack8<kBf16>(v[i], f);
-      dst[c] = quant8(f, scale, inv);
+    for (int i = 0; i < kMaxV; ++i) {
+      if (kFull || sub + i * G < nvec) {
+        float f[8];
+        unpack8<kBf16>(v[i], f);
+        dst[i * G] = quant8<decltype(exact)::value>(f, rq);
+      }
     }
-  }
+  };
+  if (rq.exact) write(True{}); else write(False{});
 }
 
 template <bool kBf16>
 int launch_quantize(const void* x, int64_t M, int64_t K, int64_t ldx, int8_t* q, float* scale,
                     cudaStream_t stream) {
   const int nvec = static_cast<int>(K >> 3);
-  // Choose the power-of-two group size G and vectors-per-thread V (<= 8) that cover the row
-  // with the fewest idle vector slots; among equals prefer V near 4 (enough loads in flight
-  // per thread without starving the block of rows).
-  int G = 0, maxv = 0, best = 1 << 30;
-  for (int g = 1; g <= kQuantThreads; g <<= 1) {
-    const int v = (nvec + g - 1) / g;
-    if (v > 8) continue;
-    const int score = (g * v - nvec) * 1000 / nvec * 16 + (v > 4 ? v - 4 : 4 - v);
-    if (score < best) { best = score; G = g; maxv = v; }
+  // Power-of-two group size and vectors per thread (<= 10) that cover the row with the fewest idle slots;
+  // among equals the fewest threads per row, since the row's reductions and divisions are repeated by every
+  // warp that holds a part of it -- unless the rows are too few to fill the chip that way.
+  int lg = -1, maxv = 0;
+  int64_t best = INT64_MAX;
+  const int64_t fill = static_cast<int64_t>(148) * 4 * kQuantThreads;
+  for (int l = 0; l <= 8; ++l) {
+    const int64_t g = int64_t{1} << l;
+    const int64_t v = (nvec + g - 1) / g;
+    if (v > 10) continue;
+    const int64_t idle = (g * v - nvec) * 64 / nvec;
+    const int64_t few = M * g < fill && l < 5 ? fill / (M * g + 1) : 0;     // a warp per row at most
+    const int64_t score = idle * 8 + few * 8 + l + (l > 5 ? 4 : 0);
+    if (score < best) { best = score; lg = l; maxv = static_cast<int>(v); }
   }
-  if (G == 0) return HY3D_ERR_SHAPE;
-  const int rows_per_block = kQuantThreads / G;
+  if (lg < 0) return HY3D_ERR_SHAPE;
+#ifdef HY3D_QTUNE
+  if (const char* e = getenv("HY3D_QLG")) { lg = atoi(e); maxv = (nvec + (1 << lg) - 1) >> lg; if (maxv > 10 || maxv < 1) return HY3D_ERR_SHAPE; }
+#endif
+  const int rows_per_block = kQuantThreads >> lg;
   const int64_t blocks = (M + rows_per_block - 1) / rows_per_block;
   if (blocks > 0x7FFFFFFF) return HY3D_ERR_SHAPE;
-  const uint16_t* xp = reinterpret_cast<const uint16_t*>(x);
-  dim3 grid(static_cast<unsigned>(blocks));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
+  cfg.gridDim = dim3(static_cast<unsigned>(blocks));
   cfg.blockDim = dim3(kQuantThreads);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1] = {pdl_attribute()};
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t err = cudaSuccess;
-  const int Ki = static_cast<int>(K);
-#define HY3D_LAUNCH_Q(V) \
-  err = cudaLaunchKernelEx(&cfg, quantize_rows_kernel<kBf16, V>, xp, ldx, q, scale, M, Ki, G)
-  switch (maxv) {
-    case 1: HY3D_LAUNCH_Q(1); break;
-    case 2: HY3D_LAUNCH_Q(2); break;
-    case 3: HY3D_LAUNCH_Q(3); break;
-    case 4: HY3D_LAUNCH_Q(4); break;
-    case 5: HY3D_LAUNCH_Q(5); break;
-    case 6: HY3D_LAUNCH_Q(6); break;
-    case 7: HY3D_LAUNCH_Q(7); break;
-    default: HY3D_LAUNCH_Q(8); break;
-  }
-#undef HY3D_LAUNCH_Q
+  using KernelFn = void (*)(const uint16_t*, int64_t, int8_t*, float*, int64_t, int, int);
+#define HY3D_Q(V) {quantize_rows_kernel<kBf16, V, false>, quantize_rows_kernel<kBf16, V, true>}
+  static const KernelFn kernels[10][2] = {HY3D_Q(1), HY3D_Q(2), HY3D_Q(3), HY3D_Q(4), HY3D_Q(5),
+                                          HY3D_Q(6), HY3D_Q(7), HY3D_Q(8), HY3D_Q(9), HY3D_Q(10)};
+#undef HY3D_Q
+  const KernelFn kernel = kernels[maxv - 1][(maxv << lg) == nvec ? 1 : 0];
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const uint16_t*>(x), ldx, q, scale, M,
+                                             static_cast<int>(K), lg);
   if (err != cudaSuccess) {
     cudaGetLastError();
     return HY3D_ERR_CUDA;
@@ -218,14 +227,16 @@ int launch_quantize(const void* x, int64_t M, int64_t K, int64_t ldx, int8_t* q,
 // and 2K + K for the quantiser).  Arithmetic, all fp32, fixed reduction order:
 //     mean = sum(x) / K;  var = sum((x - mean)^2) / K;  rstd = 1 / sqrt(var + eps)  (IEEE)
 //     y    = round16( fma((x - mean) * rstd, gamma, beta) )
-// G <= 32 lanes share a row (shuffle reductions); gamma / beta are staged once per block in
-// shared memory as fp32 and the block walks rows with a grid-stride loop.
-template <bool kBf16, int kMaxV>
-__global__ void __launch_bounds__(kQuantThreads, kMaxV <= 4 ? 3 : 2)
+// 2^lg <= 32 lanes share a row (shuffle reductions), each with up to kMaxV vectors; gamma / beta are staged
+// once per block in shared memory as fp32 and the block walks rows with a grid-stride loop, the next row's
+// vectors requested before the current row is worked on.  Issue-bound.  Everything that can be is decided at
+// compile time (kFull: no lane has a vector too few; kY: the normalised row is wanted too).
+template <bool kBf16, int kMaxV, bool kFull, bool kY>
+__global__ void __launch_bounds__(kQuantThreads, kMaxV <= 2 ? 4 : kMaxV <= 5 ? 3 : 2)
 layernorm_quantize_kernel(const uint16_t* __restrict__ x, int64_t ldx, const void* __restrict__ gamma,
                           const void* __restrict__ beta, int gb_dtype, float eps,
                           int8_t* __restrict__ q, float* __restrict__ scale_out,
-                          uint16_t* __restrict__ y_out, int64_t M, int K, int G) {
+                          uint16_t* __restrict__ y_out, int64_t M, int K, int lg) {
   extern __shared__ float s_gb[];            // gamma and beta as fp32, 2 * K floats in planes
   pdl_launch_dependents();
   // Four planes of K/8 float4 each: [gamma 0-3 | gamma 4-7 | beta 0-3 | beta 4-7] of every
@@ -237,30 +248,28 @@ layernorm_quantize_kernel(const uint16_t* __restrict__ x, int64_t ldx, const voi
     s_gb[at] = gamma ? load_scalar(gamma, gb_dtype, k) : 1.0f;
     s_gb[2 * plane + at] = beta ? load_scalar(beta, gb_dtype, k) : 0.0f;
   }
-  pdl_wait();   // x comes from the previous kernel in the stream; gamma / beta are parameters
-  __syncthreads();
-  const int tid = threadIdx.x;
-  const int rows_per_block = kQuantThreads / G;
-  const int sub = tid % G;
+  const int tid = threadIdx.x, G = 1 << lg;
+  const int sub = tid & (G - 1);
   const int nvec = K >> 3;
   const float inv_k = 1.0f / static_cast<float>(K);
-  // The next row's vectors are requested before the current row is worked on, so that every
-  // warp keeps loads in flight through its reductions.
+  const float* gb = s_gb + 4 * sub;
+  const int rows_per_block = kQuantThreads >> lg;
   const int64_t row_step = static_cast<int64_t>(gridDim.x) * rows_per_block;
+  int64_t row = static_cast<int64_t>(blockIdx.x) * rows_per_block + (tid >> lg);
+  // The trip count is the block's: a thread past the last row repeats that row (same values, same places).
+  const int trips = static_cast<int>((M - static_cast<int64_t>(blockIdx.x) * rows_per_block + row_step - 1) / row_step);
+  pdl_wait();   // x comes from the previous kernel in the stream; gamma / beta are parameters
+  __syncthreads();
   uint4 vn[kMaxV];
-  auto fetch = [&](int64_t r0) {
-    const int64_t r = r0 + tid / G;
-    const uint4* src = reinterpret_cast<const uint4*>(x + (r < M ? r : 0) * ldx);
+  auto fetch = [&](int64_t r) {
+    const uint4* src = reinterpret_cast<const uint4*>(x + (r < M ? r : M - 1) * ldx) + sub;
 #pragma unroll
-    for (int i = 0; i < kMaxV; ++i) {
-      const int c = sub + i * G;
-      vn[i] = (r < M && c < nvec) ? __ldcs(src + c) : make_uint4(0, 0, 0, 0);
-    }
+    for (int i = 0; i < kMaxV; ++i)
+      vn[i] = kFull || sub + i * G < nvec ? __ldcs(src + i * G) : make_uint4(0, 0, 0, 0);
   };
-  fetch(static_cast<int64_t>(blockIdx.x) * rows_per_block);
-  for (int64_t row0 = static_cast<int64_t>(blockIdx.x) * rows_per_block; row0 < M; row0 += row_step) {
-    const int64_t row = row0 + tid / G;
-    const bool row_ok = row < M;
+  fetch(row);
+  for (int trip = 0; trip < trips; ++trip, row += row_step) {
+    const int64_t at_row = row < M ? row : M - 1;
     // The row lives in registers as pairs; every step below is a packed fp32x2 instruction
     // (two IEEE single-precision operations per issue slot).
     float2 f[kMaxV][4];
@@ -275,7 +284,7 @@ layernorm_quantize_kernel(const uint16_t* __restrict__ x, int64_t ldx, const voi
         sum2 = __fadd2_rn(sum2, f[i][j]);
       }
     }
-    if (row0 + row_step < M) fetch(row0 + row_step);
+    if (trip + 1 < trips) fetch(row + row_step);
     float sum = sum2.x + sum2.y;
     for (int off = G >> 1; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
     const float mean = sum * inv_k;
@@ -283,8 +292,7 @@ layernorm_quantize_kernel(const uint16_t* __restrict__ x, int64_t ldx, const voi
     float2 ss2 = make_float2(0.0f, 0.0f);
 #pragma unroll
     for (int i = 0; i < kMaxV; ++i) {
-      const int c = sub + i * G;
-      if (c < nvec) {
+      if (kFull || sub + i * G < nvec) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           f[i][j] = __fadd2_rn(f[i][j], nmean2);          // centred from here on
@@ -301,13 +309,13 @@ layernorm_quantize_kernel(const uint16_t* __restrict__ x, int64_t ldx, const voi
     uint4 yv[kMaxV];
 #pragma unroll
     for (int i = 0; i < kMaxV; ++i) {
-      const int c = sub + i * G;
       yv[i] = make_uint4(0, 0, 0, 0);
-      if (c < nvec) {
-        const float4 g0 = *reinterpret_cast<const float4*>(s_gb + 4 * c);
-        const float4 g1 = *reinterpret_cast<const float4*>(s_gb + plane + 4 * c);
-        const float4 b0 = *reinterpret_cast<const float4*>(s_gb + 2 * plane + 4 * c);
-        const float4 b1 = *reinterpret_cast<const float4*>(s_gb + 3 * plane + 4 * c);
+      if (kFull || sub + i * G < nvec) {
+        const float* g = gb + 4 * i * G;
+        const float4 g0 = *reinterpret_cast<const float4*>(g);
+        const float4 g1 = *reinterpret_cast<const float4*>(g + plane);
+        const float4 b0 = *reinterpret_cast<const float4*>(g + 2 * plane);
+        const float4 b1 = *reinterpret_cast<const float4*>(g + 3 * plane);
         const float2 gg[4] = {make_float2(g0.x, g0.y), make_float2(g0.z, g0.w),
                               make_float2(g1.x, g1.y), make_float2(g1.z, g1.w)};
         const float2 bb[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w),
@@ -316,13 +324,7 @@ layernorm_quantize_kernel(const uint16_t* __restrict__ x, int64_t ldx, const voi
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const float2 y = __ffma2_rn(__fmul2_rn(f[i][j], rstd2), gg[j], bb[j]);
-          if (kBf16) {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(y.x, y.y);
-            w[j] = *reinterpret_cast<const uint32_t*>(&h);
-          } else {
-            const __half2 h = __floats2half2_rn(y.x, y.y);
-            w[j] = *reinterpret_cast<const uint32_t*>(&h);
-          }
+          w[j] = pack2(y.x, y.y, kBf16 ? HY3D_BF16 : HY3D_F16);
         }
         yv[i] = make_uint4(w[0], w[1], w[2], w[3]);
         absmax8<kBf16>(yv[i], amax2);
@@ -331,20 +333,25 @@ layernorm_quantize_kernel(const uint16_t* __restrict__ x, int64_t ldx, const voi
     float amax = absmax_to_float<kBf16>(amax2);
     for (int off = G >> 1; off > 0; off >>= 1)
       amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-    const float scale = __fdiv_rn(fmaxf(amax, 1e-8f), 127.0f);
-    const float inv = __frcp_rn(scale);
-    if (row_ok && sub == 0) scale_out[row] = scale;
-    uint2* dst = reinterpret_cast<uint2*>(q + (row_ok ? row : 0) * static_cast<int64_t>(K));
-    uint4* ydst = y_out ? reinterpret_cast<uint4*>(y_out + (row_ok ? row : 0) * static_cast<int64_t>(K)) : nullptr;
+    const RowQuant rq = row_quant(amax);
+    if (sub == 0) scale_out[at_row] = rq.scale;
+    uint2* dst = reinterpret_cast<uint2*>(q + at_row * static_cast<int64_t>(K)) + sub;
+    auto write = [&](auto exact) {
 #pragma unroll
-    for (int i = 0; i < kMaxV; ++i) {
-      const int c = sub + i * G;
-      if (row_ok && c < nvec) {
-        float fy[8];
-        unpack8<kBf16>(yv[i], fy);
-        dst[c] = quant8(fy, scale, inv);
-        if (ydst) ydst[c] = yv[i];
+      for (int i = 0; i < kMaxV; ++i) {
+        if (kFull || sub + i * G < nvec) {
+          float fy[8];
+          unpack8<kBf16>(yv[i], fy);
+          dst[i * G] = quant8<decltype(exact)::value>(fy, rq);
+        }
       }
+    };
+    if (rq.exact) write(True{}); else write(False{});
+    if (kY) {
+      uint4* ydst = reinterpret_cast<uint4*>(y_out + at_row * static_cast<int64_t>(K)) + sub;
+#pragma unroll
+      for (int i = 0; i < kMaxV; ++i)
+        if (kFull || sub + i * G < nvec) ydst[i * G] = yv[i];
     }
   }
 }
@@ -354,15 +361,27 @@ int launch_layernorm_quantize(const void* x, int64_t M, int64_t K, int64_t ldx, 
                               const void* beta, int gb_dtype, float eps, int8_t* q, float* scale,
                               void* y_out, cudaStream_t stream) {
   const int nvec = static_cast<int>(K >> 3);
-  // lanes per row: the power of two (<= 32) that leaves at most 5 vectors per lane
-  int G = 1;
-  while (G < 32 && (nvec + G - 1) / G > 5) G <<= 1;
-  const int maxv = (nvec + G - 1) / G;
+  // lanes per row: the power of two (<= 32) that leaves at most 5 vectors per lane.  (The number of lanes
+  // also fixes the order of the row's sums, hence their last bits.)
+  int lg = 0;
+  while (lg < 5 && ((nvec + (1 << lg) - 1) >> lg) > 5) ++lg;
+  const int maxv = (nvec + (1 << lg) - 1) >> lg;
   if (maxv > 8) return HY3D_ERR_SHAPE;
-  const int rows_per_block = kQuantThreads / G;
-  int64_t blocks = (M + rows_per_block - 1) / rows_per_block;
-  const int64_t cap = 148 * 8;
-  if (blocks > cap) blocks = cap;
+  const int rows_per_block = kQuantThreads >> lg;
+  const int64_t batches = (M + rows_per_block - 1) / rows_per_block;
+  using KernelFn = void (*)(const uint16_t*, int64_t, const void*, const void*, int, float, int8_t*, float*, uint16_t*,
+                            int64_t, int, int);
+#define HY3D_LNQ(V)                                                                              \
+  {{layernorm_quantize_kernel<kBf16, V, false, false>, layernorm_quantize_kernel<kBf16, V, false, true>}, \
+   {layernorm_quantize_kernel<kBf16, V, true, false>, layernorm_quantize_kernel<kBf16, V, true, true>}}
+  static const KernelFn kernels[8][2][2] = {HY3D_LNQ(1), HY3D_LNQ(2), HY3D_LNQ(3), HY3D_LNQ(4),
+                                            HY3D_LNQ(5), HY3D_LNQ(6), HY3D_LNQ(7), HY3D_LNQ(8)};
+#undef HY3D_LNQ
+  const KernelFn kernel = kernels[maxv - 1][(maxv << lg) == nvec ? 1 : 0][y_out ? 1 : 0];
+  // One wave of resident blocks, evened out: every block walks the same number of row batches (or one less).
+  const int64_t wave = static_cast<int64_t>(148) * (maxv <= 2 ? 4 : maxv <= 5 ? 3 : 2);
+  const int64_t trips = (batches + wave - 1) / wave;
+  const int64_t blocks = (batches + trips - 1) / trips;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(blocks));
   cfg.blockDim = dim3(kQuantThreads);
@@ -371,18 +390,8 @@ int launch_layernorm_quantize(const void* x, int64_t M, int64_t K, int64_t ldx, 
   cudaLaunchAttribute attr[1] = {pdl_attribute()};
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const uint16_t* xp = reinterpret_cast<const uint16_t*>(x);
-  uint16_t* yp = reinterpret_cast<uint16_t*>(y_out);
-  const int Ki = static_cast<int>(K);
-  cudaError_t err = cudaSuccess;
-#define HY3D_LAUNCH_LNQ(V) \
-  err = cudaLaunchKernelEx(&cfg, layernorm_quantize_kernel<kBf16, V>, xp, ldx, gamma, beta, gb_dtype, eps, \
-                           q, scale, yp, M, Ki, G)
-  if (maxv <= 2) HY3D_LAUNCH_LNQ(2);
-  else if (maxv <= 4) HY3D_LAUNCH_LNQ(4);
-  else if (maxv == 5) HY3D_LAUNCH_LNQ(5);
-  else HY3D_LAUNCH_LNQ(8);
-#undef HY3D_LAUNCH_LNQ
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const uint16_t*>(x), ldx, gamma, beta, gb_dtype,
+                                             eps, q, scale, reinterpret_cast<uint16_t*>(y_out), M, static_cast<int>(K), lg);
   if (err != cudaSuccess) {
     cudaGetLastError();
     return HY3D_ERR_CUDA;
@@ -401,8 +410,7 @@ __global__ void __launch_bounds__(256) quotient_enum_kernel() {
   const float amax = kBf16 ? __uint_as_float(a_bits << 16)
                            : __half2float(__ushort_as_half(static_cast<unsigned short>(a_bits)));
   if (!(amax == amax) || isinf(amax)) return;
-  const float scale = __fdiv_rn(fmaxf(amax, 1e-8f), 127.0f);
-  const float inv = __frcp_rn(scale);
+  const RowQuant rq = row_quant(amax);
   unsigned long long pairs = 0, bad = 0;
   // Two patterns per step, through the packed arithmetic the quantiser kernels run.
   for (uint32_t xb = 2 * threadIdx.x; xb < 65536u; xb += 2 * blockDim.x) {
@@ -411,13 +419,13 @@ __global__ void __launch_bounds__(256) quotient_enum_kernel() {
     for (int h = 0; h < 2; ++h)
       x[h] = kBf16 ? __uint_as_float((xb + h) << 16)
                    : __half2float(__ushort_as_half(static_cast<unsigned short>(xb + h)));
-    const float2 t = refined_quotient2_magic(make_float2(x[0], x[1]), scale, inv);
+    const float2 t = rq.exact ? refined_code2(make_float2(x[0], x[1]), rq.scale, rq.inv) : fast_code2(make_float2(x[0], x[1]), rq.mul);
     const uint32_t b[2] = {__float_as_uint(t.x), __float_as_uint(t.y)};
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       if (!(fabsf(x[h]) <= amax)) continue;
       const int code = static_cast<int>(static_cast<signed char>(b[h] & 0xFFu));
-      const int ref = static_cast<int>(rintf(__fdiv_rn(x[h], scale)));
+      const int ref = static_cast<int>(rintf(__fdiv_rn(x[h], rq.scale)));
       ++pairs;
       if (code != ref) ++bad;
     }
