@@ -17,8 +17,10 @@
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include "../../include/hy3d_int8.h"
 
@@ -37,7 +39,6 @@ struct Api {
   HY3D_FN(hy3d_gemm_w8a8_sparse24);
   HY3D_FN(hy3d_layernorm_quantize);
   HY3D_FN(hy3d_groupnorm_nhwc);
-  HY3D_FN(hy3d_groupnorm_workspace_floats);
   HY3D_FN(hy3d_quantize_weight);
   HY3D_FN(hy3d_status_string);
 } api;
@@ -291,54 +292,6 @@ PyObject* gemm_sparse(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// layer_forward(layer, x) -> y | None: Int8Linear.forward on a plain tensor.  Mode, epilogue and buffers
-// come without the look-ups that nn.Module routes through Python, a third of what those cost.
-struct Names {
-  PyObject *dict, *buffers, *mode, *epilogue, *bias, *wq, *scale, *comp, *meta;
-} names;
-bool intern_names() {
-  struct { PyObject** at; const char* text; } all[] = {
-      {&names.dict, "__dict__"}, {&names.buffers, "_buffers"}, {&names.mode, "mode"}, {&names.epilogue, "epilogue"},
-      {&names.bias, "bias"}, {&names.wq, "weight_int8_nk"}, {&names.scale, "weight_scale"},
-      {&names.comp, "weight_sparse_comp"}, {&names.meta, "weight_sparse_meta"}};
-  for (auto& n : all)
-    if (!(*n.at = PyUnicode_InternFromString(n.text))) return false;
-  return true;
-}
-PyObject* layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n != 2 || !THPVariable_CheckExact(a[1])) return none();
-  PyObject* dict = PyObject_GetAttr(a[0], names.dict);
-  if (!dict) return nullptr;
-  Py_DECREF(dict);                            // the layer keeps it
-  PyObject* buffers = PyDict_Check(dict) ? PyDict_GetItemWithError(dict, names.buffers) : nullptr;
-  if (!buffers || !PyDict_Check(buffers)) return none();
-  PyObject* bias = PyDict_GetItemWithError(buffers, names.bias);
-  if (!bias) bias = PyDict_GetItemWithError(dict, names.bias);
-  PyObject* scale = PyDict_GetItemWithError(buffers, names.scale);
-  if (!bias || !scale) return none();
-  // instance or class attributes, compared by text
-  auto attribute_is_one_of = [&](PyObject* name, std::initializer_list<const char*> texts) {
-    PyObject* v = PyObject_GetAttr(a[0], name);
-    if (!v) { PyErr_Clear(); return -1; }
-    int found = -1, i = 0;
-    for (const char* t : texts) {
-      if (PyUnicode_Check(v) && PyUnicode_CompareWithASCIIString(v, t) == 0) { found = i; break; }
-      ++i;
-    }
-    Py_DECREF(v);
-    return found;
-  };
-  const int mode = attribute_is_one_of(names.mode, {"tc", "sparse"});
-  const int epi = attribute_is_one_of(names.epilogue, {"linear", "gelu", "geglu"});   // HY3D_EPI_* in order
-  if (mode < 0 || epi < 0) return none();
-  const bool sparse = mode == 1;
-  PyObject* w = PyDict_GetItemWithError(buffers, sparse ? names.comp : names.wq);
-  if (!w) return none();
-  if (!sparse) return linear_dense_impl(a[1], w, scale, bias, epi);
-  PyObject* meta = PyDict_GetItemWithError(buffers, names.meta);
-  return meta ? linear_sparse_impl(a[1], w, meta, scale, bias, epi) : none();
-}
-
 // gamma and beta of a normalisation: both of one type (or absent).
 struct Affine {
   const void *gamma = nullptr, *beta = nullptr;
@@ -360,26 +313,31 @@ struct Affine {
 };
 
 // layernorm_quantize(x, gamma | None, beta | None, eps) -> (codes (M,K), scale (M)) | None
-PyObject* layernorm_quantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
-  if (n != 4 || !PyFloat_Check(a[3])) return none();
-  const at::Tensor* x = plain(a[0]);
-  if (!x || x->dim() < 1) return none();
+struct Quantized { at::Tensor q, s; };
+bool layernorm_quantize_impl(PyObject* px, PyObject* gamma, PyObject* beta, double eps, Quantized* out, int* status) {
+  const at::Tensor* x = plain(px);
+  if (!x || x->dim() < 1) return false;
   const int code = half_code(x->scalar_type());
   const int64_t K = x->size(-1), M = K > 0 ? x->numel() / K : 0;
-  if (code < 0 || M <= 0) return none();
-  const Affine f(a[1], a[2], K, x->device());
-  if (!f.ok) return none();
+  if (code < 0 || M <= 0) return false;
+  const Affine f(gamma, beta, K, x->device());
+  if (!f.ok) return false;
   c10::cuda::CUDAGuard guard(x->device());
   cudaStream_t st = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
-  at::Tensor q = at::Tensor(at::detail::empty_cuda({M, K}, at::kChar, x->device(), std::nullopt));
-  at::Tensor s = at::Tensor(at::detail::empty_cuda({M}, at::kFloat, x->device(), std::nullopt));
-  const int rc = api.hy3d_layernorm_quantize(x->const_data_ptr(), code, M, K, K, f.gamma, f.beta, f.code,
-                                             static_cast<float>(PyFloat_AS_DOUBLE(a[3])), q.mutable_data_ptr<int8_t>(),
-                                             s.mutable_data_ptr<float>(), nullptr, st);
+  out->q = at::Tensor(at::detail::empty_cuda({M, K}, at::kChar, x->device(), std::nullopt));
+  out->s = at::Tensor(at::detail::empty_cuda({M}, at::kFloat, x->device(), std::nullopt));
+  *status = api.hy3d_layernorm_quantize(x->const_data_ptr(), code, M, K, K, f.gamma, f.beta, f.code, static_cast<float>(eps),
+                                        out->q.mutable_data_ptr<int8_t>(), out->s.mutable_data_ptr<float>(), nullptr, st);
+  return true;
+}
+PyObject* layernorm_quantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Quantized z;
+  int rc = 0;
+  if (n != 4 || !PyFloat_Check(a[3]) || !layernorm_quantize_impl(a[0], a[1], a[2], PyFloat_AS_DOUBLE(a[3]), &z, &rc)) return none();
   if (rc != HY3D_OK) return failed("hy3d_layernorm_quantize", rc);
-  PyObject* pq = THPVariable_Wrap(std::move(q));
-  PyObject* ps = pq ? THPVariable_Wrap(std::move(s)) : nullptr;
+  PyObject* pq = THPVariable_Wrap(std::move(z.q));
+  PyObject* ps = pq ? THPVariable_Wrap(std::move(z.s)) : nullptr;
   if (!ps) { Py_XDECREF(pq); return nullptr; }
   PyObject* r = PyTuple_New(2);
   if (!r) { Py_DECREF(pq); Py_DECREF(ps); return nullptr; }
@@ -390,23 +348,20 @@ PyObject* layernorm_quantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // groupnorm_nhwc(x channels_last, groups, gamma | None, beta | None, eps, silu, add (B,C) | None) -> y | None
-PyObject* groupnorm_nhwc(PyObject*, PyObject* const* a, Py_ssize_t n) {
+PyObject* groupnorm_impl(PyObject* px, long groups, PyObject* gamma, PyObject* beta, double eps, bool silu, PyObject* padd) {
   HANDLE_TH_ERRORS
-  long groups = 0, silu = 0;
-  if (n != 7 || !small_int(a[1], 1, 1 << 20, &groups) || !PyFloat_Check(a[4])) return none();
-  silu = a[5] == Py_True ? 1 : 0;
-  if (!THPVariable_CheckExact(a[0])) return none();
-  const at::Tensor& x = THPVariable_Unpack(a[0]);
+  if (!THPVariable_CheckExact(px)) return none();
+  const at::Tensor& x = THPVariable_Unpack(px);
   if (!x.is_cuda() || x.layout() != at::kStrided || x.dim() != 4 || !x.is_contiguous(at::MemoryFormat::ChannelsLast))
     return none();
   const int code = half_code(x.scalar_type());
   const int64_t B = x.size(0), C = x.size(1), HW = x.size(2) * x.size(3);
   if (code < 0 || B <= 0 || HW <= 0) return none();
-  const Affine f(a[2], a[3], C, x.device());
+  const Affine f(gamma, beta, C, x.device());
   if (!f.ok) return none();
   const void* add = nullptr;
-  if (a[6] != Py_None) {
-    const at::Tensor* t = plain(a[6]);
+  if (padd != Py_None) {
+    const at::Tensor* t = plain(padd);
     if (!t || t->dim() != 2 || t->size(0) != B || t->size(1) != C || t->scalar_type() != x.scalar_type() ||
         t->device() != x.device())
       return none();
@@ -415,13 +370,18 @@ PyObject* groupnorm_nhwc(PyObject*, PyObject* const* a, Py_ssize_t n) {
   c10::cuda::CUDAGuard guard(x.device());
   cudaStream_t st = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
   at::Tensor y = at::Tensor(at::detail::empty_cuda(x.sizes(), x.scalar_type(), x.device(), at::MemoryFormat::ChannelsLast));
-  Scratch ws(static_cast<size_t>(api.hy3d_groupnorm_workspace_floats(B, HW, static_cast<int>(groups)) + 4) * 4, st);
+  // the kernel needs no workspace; the C ABI still asks for one
   const int rc = api.hy3d_groupnorm_nhwc(x.const_data_ptr(), add, code, B, HW, C, static_cast<int>(groups), f.gamma, f.beta,
-                                         f.code, static_cast<float>(PyFloat_AS_DOUBLE(a[4])), static_cast<int>(silu),
-                                         y.mutable_data_ptr(), static_cast<float*>(ws.p), st);
+                                         f.code, static_cast<float>(eps), silu ? 1 : 0, y.mutable_data_ptr(),
+                                         static_cast<float*>(y.mutable_data_ptr()), st);
   if (rc != HY3D_OK) return failed("hy3d_groupnorm_nhwc", rc);
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS
+}
+PyObject* groupnorm_nhwc(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  long groups = 0;
+  if (n != 7 || !small_int(a[1], 1, 1 << 20, &groups) || !PyFloat_Check(a[4])) return none();
+  return groupnorm_impl(a[0], groups, a[2], a[3], PyFloat_AS_DOUBLE(a[4]), a[5] == Py_True, a[6]);
 }
 
 // quantize_weight(w (N,K), sparse) -> (codes, scale) or (compressed codes, metadata, scale) | None
@@ -460,6 +420,197 @@ PyObject* quantize_weight(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// ---------------------------------------------------------------------------------------
+//  Modules
+// ---------------------------------------------------------------------------------------
+// The functions below are what calling an Int8Linear, Int8LayerNorm or GroupNormNHWC does when nothing
+// stands between the call and the kernels: nn.Module's own __call__ and attribute look-ups through Python cost
+// 1.5 us, more than half of a launch.  They answer None, having done nothing, for a subclass, a replaced
+// `forward`, any hook (of the instance or global), a compiled or traced call, and whatever the functions above
+// decline.
+struct Names {
+  PyObject *dict, *buffers, *parameters, *mode, *epilogue, *bias, *wq, *scale, *comp, *meta, *forward, *compiled, *weight,
+      *eps, *fused, *silu, *groups, *shape, *dtype, *q, *act_scale;
+  PyObject* hooks[4];
+} names;
+struct Registered {
+  PyTypeObject* type = nullptr;
+  PyObject* forward = nullptr;
+} linear_class, layernorm_class, groupnorm_class;
+PyTypeObject* quantized_class = nullptr;
+PyObject* global_hooks[4] = {};
+
+bool intern_names() {
+  struct { PyObject** at; const char* text; } all[] = {
+      {&names.dict, "__dict__"}, {&names.buffers, "_buffers"}, {&names.parameters, "_parameters"}, {&names.mode, "mode"},
+      {&names.epilogue, "epilogue"}, {&names.bias, "bias"}, {&names.wq, "weight_int8_nk"}, {&names.scale, "weight_scale"},
+      {&names.comp, "weight_sparse_comp"}, {&names.meta, "weight_sparse_meta"}, {&names.forward, "forward"},
+      {&names.compiled, "_compiled_call_impl"}, {&names.weight, "weight"}, {&names.eps, "eps"}, {&names.fused, "fused"},
+      {&names.silu, "silu"}, {&names.groups, "num_groups"}, {&names.shape, "shape"}, {&names.dtype, "dtype"},
+      {&names.q, "q"}, {&names.act_scale, "scale"}, {&names.hooks[0], "_backward_hooks"},
+      {&names.hooks[1], "_backward_pre_hooks"}, {&names.hooks[2], "_forward_hooks"}, {&names.hooks[3], "_forward_pre_hooks"}};
+  for (auto& n : all)
+    if (!(*n.at = PyUnicode_InternFromString(n.text))) return false;
+  return true;
+}
+
+// register_modules((Int8Linear, Int8LayerNorm, GroupNormNHWC | None), QuantizedActivation, 4 global hook dicts):
+// the classes with the `forward` they have now.
+PyObject* register_modules(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 3 || !PyTuple_Check(a[0]) || !PyType_Check(a[1]) || !PyTuple_Check(a[2]) || PyTuple_GET_SIZE(a[2]) != 4) {
+    PyErr_SetString(PyExc_TypeError, "register_modules(classes, quantized class, hook dicts)");
+    return nullptr;
+  }
+  Registered* regs[] = {&linear_class, &layernorm_class, &groupnorm_class};
+  for (Py_ssize_t i = 0; i < 3 && i < PyTuple_GET_SIZE(a[0]); ++i) {
+    PyObject* c = PyTuple_GET_ITEM(a[0], i);
+    if (c == Py_None) continue;
+    PyObject* f = PyType_Check(c) ? PyObject_GetAttr(c, names.forward) : nullptr;
+    if (!f) return nullptr;
+    Py_INCREF(c);
+    regs[i]->type = reinterpret_cast<PyTypeObject*>(c);
+    regs[i]->forward = f;
+  }
+  Py_INCREF(a[1]);
+  quantized_class = reinterpret_cast<PyTypeObject*>(a[1]);
+  for (int i = 0; i < 4; ++i) {
+    PyObject* d = PyTuple_GET_ITEM(a[2], i);
+    if (!PyDict_Check(d)) { PyErr_SetString(PyExc_TypeError, "hook dicts"); return nullptr; }
+    Py_INCREF(d);
+    global_hooks[i] = d;
+  }
+  Py_RETURN_NONE;
+}
+
+// The instance dictionary of a module nothing stands before (borrowed), or nullptr.
+PyObject* plain_module(PyObject* m, const Registered& reg) {
+  if (Py_TYPE(m) != reg.type || torch::jit::tracer::isTracing()) return nullptr;
+  if (_PyType_Lookup(reg.type, names.forward) != reg.forward) return nullptr;
+  PyObject* dict = PyObject_GetAttr(m, names.dict);
+  if (!dict) { PyErr_Clear(); return nullptr; }
+  Py_DECREF(dict);                            // the module keeps it
+  if (!PyDict_Check(dict) || PyDict_GetItemWithError(dict, names.forward) || PyDict_GetItemWithError(dict, names.compiled))
+    return nullptr;
+  for (int i = 0; i < 4; ++i) {
+    PyObject* h = PyDict_GetItemWithError(dict, names.hooks[i]);
+    if (!h || !PyDict_Check(h) || PyDict_GET_SIZE(h) != 0 || PyDict_GET_SIZE(global_hooks[i]) != 0) return nullptr;
+  }
+  return dict;
+}
+
+// The layer of instance dictionary `dict` on a tensor or a QuantizedActivation.
+PyObject* linear_of(PyObject* layer, PyObject* dict, PyObject* x) {
+  PyObject* buffers = PyDict_GetItemWithError(dict, names.buffers);
+  if (!buffers || !PyDict_Check(buffers)) return none();
+  PyObject* bias = PyDict_GetItemWithError(buffers, names.bias);
+  if (!bias) bias = PyDict_GetItemWithError(dict, names.bias);
+  PyObject* scale = PyDict_GetItemWithError(buffers, names.scale);
+  if (!bias || !scale) return none();
+  // instance or class attributes, compared by text
+  auto attribute_is_one_of = [&](PyObject* name, std::initializer_list<const char*> texts) {
+    PyObject* v = PyDict_GetItemWithError(dict, name);
+    if (!v) v = _PyType_Lookup(Py_TYPE(layer), name);
+    int i = 0;
+    for (const char* t : texts) {
+      if (v && PyUnicode_Check(v) && PyUnicode_CompareWithASCIIString(v, t) == 0) return i;
+      ++i;
+    }
+    return -1;
+  };
+  const int mode = attribute_is_one_of(names.mode, {"tc", "sparse"});
+  const int epi = attribute_is_one_of(names.epilogue, {"linear", "gelu", "geglu"});   // HY3D_EPI_* in order
+  if (mode < 0 || epi < 0) return none();
+  const bool sparse = mode == 1;
+  PyObject* w = PyDict_GetItemWithError(buffers, sparse ? names.comp : names.wq);
+  PyObject* meta = sparse ? PyDict_GetItemWithError(buffers, names.meta) : Py_None;
+  if (!w || !meta) return none();
+  if (THPVariable_CheckExact(x))
+    return sparse ? linear_sparse_impl(x, w, meta, scale, bias, epi) : linear_dense_impl(x, w, scale, bias, epi);
+  if (Py_TYPE(x) != quantized_class) return none();
+  PyObject* part[4] = {PyObject_GetAttr(x, names.q), PyObject_GetAttr(x, names.act_scale), PyObject_GetAttr(x, names.shape),
+                       PyObject_GetAttr(x, names.dtype)};
+  PyObject* r = nullptr;
+  if (part[0] && part[1] && part[2] && part[3]) {
+    const at::ScalarType type = THPDtype_Check(part[3]) ? reinterpret_cast<THPDtype*>(part[3])->scalar_type : at::kFloat;
+    if (half_code(type) < 0) {
+      r = none();
+    } else {
+      PyObject* bf16 = PyLong_FromLong(type == at::kBFloat16 ? 1 : 0);
+      PyObject* code = PyLong_FromLong(epi);
+      if (sparse) {
+        PyObject* args[] = {part[0], part[1], w, meta, scale, bias, bf16, code, part[2]};
+        r = gemm_sparse(nullptr, args, 9);
+      } else {
+        PyObject* args[] = {part[0], part[1], w, scale, bias, bf16, code, part[2]};
+        r = gemm_dense(nullptr, args, 8);
+      }
+      Py_XDECREF(bf16);
+      Py_XDECREF(code);
+    }
+  }
+  for (PyObject* p : part) Py_XDECREF(p);
+  return r;
+}
+
+// layer_call(layer, x) -> y | None: calling an Int8Linear
+PyObject* layer_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  PyObject* dict = n == 2 ? plain_module(a[0], linear_class) : nullptr;
+  return dict ? linear_of(a[0], dict, a[1]) : none();
+}
+// layer_forward(layer, x) -> y | None: Int8Linear.forward, also of subclasses
+PyObject* layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 2) return none();
+  PyObject* dict = PyObject_GetAttr(a[0], names.dict);
+  if (!dict) return nullptr;
+  Py_DECREF(dict);
+  return PyDict_Check(dict) ? linear_of(a[0], dict, a[1]) : none();
+}
+
+// norm_call(layer, x) -> QuantizedActivation | None: calling an Int8LayerNorm
+PyObject* norm_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  PyObject* dict = n == 2 && THPVariable_CheckExact(a[1]) ? plain_module(a[0], layernorm_class) : nullptr;
+  PyObject* params = dict ? PyDict_GetItemWithError(dict, names.parameters) : nullptr;
+  PyObject* eps = dict ? PyDict_GetItemWithError(dict, names.eps) : nullptr;
+  if (!params || !PyDict_Check(params) || !eps || !PyFloat_Check(eps)) return none();
+  PyObject* gamma = PyDict_GetItemWithError(params, names.weight);
+  PyObject* beta = PyDict_GetItemWithError(params, names.bias);
+  Quantized z;
+  int rc = 0;
+  if (!gamma || !beta || !layernorm_quantize_impl(a[1], gamma, beta, PyFloat_AS_DOUBLE(eps), &z, &rc)) return none();
+  if (rc != HY3D_OK) return failed("hy3d_layernorm_quantize", rc);
+  PyObject* r = quantized_class->tp_alloc(quantized_class, 0);
+  if (!r) return nullptr;
+  struct { PyObject *name, *value; } set[] = {{names.q, THPVariable_Wrap(std::move(z.q))},
+                                              {names.act_scale, THPVariable_Wrap(std::move(z.s))},
+                                              {names.shape, PyObject_GetAttr(a[1], names.shape)},
+                                              {names.dtype, PyObject_GetAttr(a[1], names.dtype)}};
+  bool bad = false;
+  for (auto& e : set) {
+    bad = bad || !e.value || PyObject_SetAttr(r, e.name, e.value) < 0;
+    Py_XDECREF(e.value);
+  }
+  if (bad) { Py_DECREF(r); return nullptr; }
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// groupnorm_call(layer, x, add | None) -> y | None: calling a GroupNormNHWC whose kernel path is on
+PyObject* groupnorm_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  PyObject* dict = n == 3 ? plain_module(a[0], groupnorm_class) : nullptr;
+  if (!dict || PyDict_GetItemWithError(dict, names.fused) != Py_True) return none();
+  PyObject* params = PyDict_GetItemWithError(dict, names.parameters);
+  PyObject* eps = PyDict_GetItemWithError(dict, names.eps);
+  PyObject* silu = PyDict_GetItemWithError(dict, names.silu);
+  PyObject* ng = PyDict_GetItemWithError(dict, names.groups);
+  long groups = 0;
+  if (!params || !PyDict_Check(params) || !eps || !PyFloat_Check(eps) || !silu || !ng || !small_int(ng, 1, 1 << 20, &groups))
+    return none();
+  PyObject* gamma = PyDict_GetItemWithError(params, names.weight);
+  PyObject* beta = PyDict_GetItemWithError(params, names.bias);
+  return gamma && beta ? groupnorm_impl(a[1], groups, gamma, beta, PyFloat_AS_DOUBLE(eps), silu == Py_True, a[2]) : none();
+}
+
 // open(path): resolves the C ABI in the library at `path`, which the caller has loaded and checked.
 PyObject* open_library(PyObject*, PyObject* arg) {
   const char* path = PyUnicode_AsUTF8(arg);
@@ -488,7 +639,6 @@ PyObject* open_library(PyObject*, PyObject* arg) {
   HY3D_SYM(hy3d_gemm_w8a8_sparse24);
   HY3D_SYM(hy3d_layernorm_quantize);
   HY3D_SYM(hy3d_groupnorm_nhwc);
-  HY3D_SYM(hy3d_groupnorm_workspace_floats);
   HY3D_SYM(hy3d_quantize_weight);
   HY3D_SYM(hy3d_status_string);
 #undef HY3D_SYM
@@ -498,7 +648,11 @@ PyObject* open_library(PyObject*, PyObject* arg) {
 #define HY3D_FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     {"open", open_library, METH_O, nullptr},
+    HY3D_FAST(register_modules),
+    HY3D_FAST(layer_call),
     HY3D_FAST(layer_forward),
+    HY3D_FAST(norm_call),
+    HY3D_FAST(groupnorm_call),
     HY3D_FAST(linear_dense),
     HY3D_FAST(linear_sparse),
     HY3D_FAST(gemm_dense),

@@ -242,3 +242,43 @@ def test_host_pipeline_matches_direct_calls(qu, pkg):
     pipe.synchronize()
     for a, b in zip(hy, ref):
         assert torch.equal(a, b)
+
+
+def test_direct_calls_leave_hooks_and_overrides_alone(qu):
+    """Calling a layer takes a direct way to the kernels; a hook, a replaced or overridden `forward` and a
+    keyword argument must still go through nn.Module."""
+    torch.manual_seed(5)
+    lin = nn.Linear(128, 64).to(DEV).bfloat16()
+    x = torch.randn(9, 128, device=DEV).bfloat16()
+    for make in (qu.Int8Linear.from_linear, qu.Int8Linear.from_linear_sparse):
+        layer = make(lin)
+        y = layer(x)
+        assert torch.equal(y, layer(x=x)) and torch.equal(y, layer.forward(x))
+        h = layer.register_forward_hook(lambda m, a, out: out + 1)
+        assert torch.equal(layer(x), y + 1)
+        h.remove()
+        h = layer.register_forward_pre_hook(lambda m, a: (a[0] * 0,))
+        assert torch.equal(layer(x), layer.forward(x * 0))
+        h.remove()
+        h = nn.modules.module.register_module_forward_hook(lambda m, a, out: out * 2)
+        assert torch.equal(layer(x), y * 2)
+        h.remove()
+        layer.forward = lambda t: t
+        assert layer(x) is x
+        del layer.forward
+        assert torch.equal(layer(x), y)
+
+    class Doubled(qu.Int8Linear):
+        def forward(self, t):
+            return super().forward(t) * 2
+    d = Doubled(128, 64, dtype=torch.bfloat16)
+    d.load_state_dict(qu.Int8Linear.from_linear(lin).state_dict())
+    assert torch.equal(d.to(DEV)(x), qu.Int8Linear.from_linear(lin)(x) * 2)
+    ln = qu.Int8LayerNorm(nn.LayerNorm(128).to(DEV).bfloat16())
+    seen = []
+    h = ln.register_forward_hook(lambda m, a, out: seen.append(out))
+    a = ln(x)
+    h.remove()
+    b = ln(x)
+    assert seen == [a] and torch.equal(a.q, b.q) and torch.equal(a.scale, b.scale)
+    assert b.shape == x.shape and b.dtype == x.dtype and torch.equal(layer(a), layer(b))
