@@ -71,11 +71,19 @@ SIGNATURES = {
     "hy3d_probe_tmem_ld": [c_int, c_int, c_int, c_void_p, c_void_p],
     "hy3d_groupnorm_nhwc": [c_void_p, c_void_p, c_int, c_int64, c_int64, c_int64, c_int, c_void_p, c_void_p,
                             c_int, ctypes.c_float, c_int, c_void_p, c_void_p, c_void_p],
+    "hy3d_groupnorm_nhwc_terms": [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int64, c_int64, c_int64, c_int, c_void_p,
+                                  c_void_p, c_int, ctypes.c_float, c_int, c_void_p, c_void_p],
+    "hy3d_add_bias_nhwc": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int64, c_void_p],
+    "hy3d_concat_nhwc": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p],
+    "hy3d_upsample2x_nhwc": [c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_void_p],
+    "hy3d_add_quantize_rows": [c_void_p, c_void_p, c_int, c_int64, c_int64, c_void_p, c_void_p, c_void_p],
+    "hy3d_add_layernorm_quantize": [c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int64, c_void_p, c_void_p, c_int,
+                                    ctypes.c_float, c_void_p, c_void_p, c_void_p],
     "hy3d_version": [],
 }
 
 # The argument lists above belong to this ABI version of the library (hy3d_version()).
-ABI_VERSION = 202
+ABI_VERSION = 203
 
 
 def configure(lib: ctypes.CDLL) -> ctypes.CDLL:

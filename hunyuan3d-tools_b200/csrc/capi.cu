@@ -178,8 +178,55 @@ int hy3d_groupnorm_nhwc(const void* x, const void* add, int x_dtype, int64_t B, 
                         int silu, void* y, float* workspace, void* stream) {
   const int rc = check_device();
   if (rc != HY3D_OK) return rc;
-  return gnorm::groupnorm_nhwc(x, add, x_dtype, B, HW, C, groups, gamma, beta, gb_dtype, eps, silu, y,
-                               workspace, static_cast<cudaStream_t>(stream));
+  (void)workspace;
+  return gnorm::groupnorm_nhwc(x, nullptr, add, C, x_dtype, B, HW, C, groups, gamma, beta, gb_dtype, eps, silu, y,
+                               static_cast<cudaStream_t>(stream));
+}
+
+int hy3d_groupnorm_nhwc_terms(const void* x, const void* bias, const void* add, int64_t add_ld, int x_dtype, int64_t B,
+                              int64_t HW, int64_t C, int groups, const void* gamma, const void* beta, int gb_dtype,
+                              float eps, int silu, void* y, void* stream) {
+  const int rc = check_device();
+  if (rc != HY3D_OK) return rc;
+  return gnorm::groupnorm_nhwc(x, bias, add, add_ld, x_dtype, B, HW, C, groups, gamma, beta, gb_dtype, eps, silu, y,
+                               static_cast<cudaStream_t>(stream));
+}
+
+int hy3d_add_bias_nhwc(const void* x, const void* bias_x, const void* h, const void* bias_h, int dtype, void* y,
+                       int64_t rows, int64_t C, void* stream) {
+  const int rc = check_device();
+  if (rc != HY3D_OK) return rc;
+  return nhwc::add_bias(x, bias_x, h, bias_h, dtype, y, rows, C, static_cast<cudaStream_t>(stream));
+}
+
+int hy3d_concat_nhwc(const void* a, int64_t Ca, const void* b, int64_t Cb, void* y, int64_t rows, void* stream) {
+  const int rc = check_device();
+  if (rc != HY3D_OK) return rc;
+  return nhwc::concat(a, Ca, b, Cb, y, rows, static_cast<cudaStream_t>(stream));
+}
+
+int hy3d_upsample2x_nhwc(const void* x, void* y, int64_t B, int64_t H, int64_t W, int64_t C, void* stream) {
+  const int rc = check_device();
+  if (rc != HY3D_OK) return rc;
+  return nhwc::upsample2x(x, y, B, H, W, C, static_cast<cudaStream_t>(stream));
+}
+
+int hy3d_add_quantize_rows(const void* x, const void* add, int x_dtype, int64_t M, int64_t K, int8_t* q, float* scale,
+                           void* stream) {
+  const int rc = check_device();
+  if (rc != HY3D_OK) return rc;
+  if (M > 0 && !add) return HY3D_ERR_ARG;
+  return quantize_rows(x, add, x_dtype, M, K, K, q, scale, static_cast<cudaStream_t>(stream));
+}
+
+int hy3d_add_layernorm_quantize(const void* x, const void* add, void* sum, int x_dtype, int64_t M, int64_t K,
+                                const void* gamma, const void* beta, int gb_dtype, float eps, int8_t* q, float* scale,
+                                void* stream) {
+  const int rc = check_device();
+  if (rc != HY3D_OK) return rc;
+  if (M > 0 && (!add || !sum)) return HY3D_ERR_ARG;
+  return layernorm_quantize(x, add, x_dtype, M, K, K, gamma, beta, gb_dtype, eps, q, scale, sum,
+                            static_cast<cudaStream_t>(stream));
 }
 
 int64_t hy3d_groupnorm_workspace_floats(int64_t B, int64_t HW, int groups) {
@@ -212,7 +259,7 @@ int hy3d_quantize_rows(const void* x, int x_dtype, int64_t M, int64_t K, int64_t
                        float* scale, void* stream) {
   const int rc = check_device();
   if (rc != HY3D_OK) return rc;
-  return quantize_rows(x, x_dtype, M, K, ldx, q, scale, static_cast<cudaStream_t>(stream));
+  return quantize_rows(x, nullptr, x_dtype, M, K, ldx, q, scale, static_cast<cudaStream_t>(stream));
 }
 
 int hy3d_layernorm_quantize(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx,
@@ -220,7 +267,7 @@ int hy3d_layernorm_quantize(const void* x, int x_dtype, int64_t M, int64_t K, in
                             float* scale, void* y_out, void* stream) {
   const int rc = check_device();
   if (rc != HY3D_OK) return rc;
-  return layernorm_quantize(x, x_dtype, M, K, ldx, gamma, beta, gb_dtype, eps, q, scale, y_out,
+  return layernorm_quantize(x, nullptr, x_dtype, M, K, ldx, gamma, beta, gb_dtype, eps, q, scale, y_out,
                             static_cast<cudaStream_t>(stream));
 }
 
@@ -279,7 +326,7 @@ int hy3d_linear_w8a8_dense(const void* x, int x_dtype, int64_t ldx, int8_t* q_ws
       linear_path(M, K, N, epilogue) == 1)
     return linear_fused(x, x_dtype, ldx, nullptr, B, w_scale, w_scale_dtype, bias, bias_dtype, out,
                         out_dtype, M, N, K, epilogue, 0, s);
-  rc = quantize_rows(x, x_dtype, M, K, ldx, q_ws, scale_ws, s);
+  rc = quantize_rows(x, nullptr, x_dtype, M, K, ldx, q_ws, scale_ws, s);
   if (rc != HY3D_OK) return rc;
   return gemm_dense(q_ws, B, scale_ws, w_scale, w_scale_dtype, bias, bias_dtype, out, out_dtype, M,
                     N, K, epilogue, cta_group, block_n, s);
@@ -352,7 +399,7 @@ int hy3d_linear_w8a8_sparse24(const void* x, int x_dtype, int64_t ldx, int8_t* q
   int rc = check_device();
   if (rc != HY3D_OK) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  rc = quantize_rows(x, x_dtype, M, K, ldx, q_ws, scale_ws, s);
+  rc = quantize_rows(x, nullptr, x_dtype, M, K, ldx, q_ws, scale_ws, s);
   if (rc != HY3D_OK) return rc;
   return gemm_sparse24(q_ws, scale_ws, w_comp, w_meta, meta_ld, w_scale, w_scale_dtype, bias,
                        bias_dtype, out, out_dtype, M, N, K, epilogue, block_m, s);

@@ -11,7 +11,7 @@
 
 #include "../../include/hy3d_int8.h"
 
-#define HY3D_ABI_VERSION 202
+#define HY3D_ABI_VERSION 203
 
 namespace hy3d {
 
@@ -613,6 +613,20 @@ __device__ __forceinline__ uint32_t pack2(float a, float b, int out_dtype) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// round(a + b) of eight 16-bit values, two at a time.  The packed add rounds the exact sum once; a sum in
+// fp32 that is rounded afterwards gives the same bits: it is exact unless the smaller operand lies more than
+// 13 (16 for bf16) binades below the larger, and then no sum is near a tie of the 16-bit type.
+template <bool kBf16>
+__device__ __forceinline__ uint32_t add2_16(uint32_t a, uint32_t b) {
+  uint32_t r;
+  if (kBf16) asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  else asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+template <bool kBf16>
+__device__ __forceinline__ uint4 add8_16(const uint4& a, const uint4& b) {
+  return make_uint4(add2_16<kBf16>(a.x, b.x), add2_16<kBf16>(a.y, b.y), add2_16<kBf16>(a.z, b.z), add2_16<kBf16>(a.w, b.w));
+}
 
 // Host side: launch attribute that lets a kernel start before its stream predecessor ends
 // (HY3D_PDL=0 in the environment turns it off).

@@ -27,7 +27,7 @@ int ensure_max_smem(const void* kernel, int bytes);
 namespace gnorm {
 namespace {
 
-// Three CTAs per SM: 56 registers a thread, 64 with the addend, which would spill otherwise.
+// Three CTAs per SM: 56 registers a thread, 64 with terms to add, which would spill otherwise.
 __host__ __device__ constexpr int narrow_threads(bool add) { return add ? 320 : 384; }
 constexpr int kWideThreads = 1024;
 constexpr int kOrderThreads = 320;    // lanes of a chunk: what 320 threads over whole rows make
@@ -44,16 +44,6 @@ __device__ __forceinline__ void unpack8f(const uint4& v, float2 (&f)[4]) {
   f[1] = unpack2f<kBf16>(v.y);
   f[2] = unpack2f<kBf16>(v.z);
   f[3] = unpack2f<kBf16>(v.w);
-}
-
-// x + add[b, c], rounded to the activation type as a separate broadcast add would have stored it.
-template <bool kBf16>
-__device__ __forceinline__ void add_round8(float2 (&f)[4], const float2 (&a)[4]) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 t = __fadd2_rn(f[j], a[j]);
-    f[j] = unpack2f<kBf16>(pack2(t.x, t.y, kBf16 ? HY3D_BF16 : HY3D_F16));
-  }
 }
 
 __device__ __forceinline__ float rcp_approx(float v) {
@@ -79,9 +69,12 @@ struct Order {
 // CTA folds; in pass 2 all lanes walk the rank's rows.  grid.x = S (the cluster), grid.y = slabs, grid.z =
 // samples.
 // kWide: up to 1024 threads, one CTA per SM, for grids that do not fill the chip.
-template <bool kBf16, bool kAdd, bool kSilu, bool kWide>
-__global__ void __launch_bounds__(kWide ? kWideThreads : narrow_threads(kAdd), kWide ? 1 : 3)
-groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ add, int64_t HW, int C, int cpg,
+// kAdd: 0 nothing, 1 a (B, C) term, 2 a (C) term and then the (B, C) one is added to x first, each rounded as
+// a separate broadcast add would have stored it.
+template <bool kBf16, int kAdd, bool kSilu, bool kWide>
+__global__ void __launch_bounds__(kWide ? kWideThreads : narrow_threads(kAdd > 0), kWide ? 1 : 3)
+groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ pre, const uint16_t* __restrict__ add,
+                 int64_t add_ld, int64_t HW, int C, int cpg,
                  int slab_groups, int rows_per_cta, int chunks_per_rank, int reps, Order order,
                  const void* __restrict__ gamma, const void* __restrict__ beta, int gb_dtype, float eps,
                  uint16_t* __restrict__ y) {
@@ -103,10 +96,13 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ ad
   pdl_wait();
   const int64_t base = static_cast<int64_t>(b) * HW * C + c0;
   const uint4* src = reinterpret_cast<const uint4*>(x + base);
-  float2 av[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) av[j] = make_float2(0.0f, 0.0f);
-  if (kAdd) unpack8f<kBf16>(__ldcs(reinterpret_cast<const uint4*>(add + static_cast<int64_t>(b) * C + c0)), av);
+  uint4 pv = make_uint4(0, 0, 0, 0), av = pv;
+  if (kAdd == 2) pv = __ldg(reinterpret_cast<const uint4*>(pre + c0));
+  if (kAdd) av = __ldcs(reinterpret_cast<const uint4*>(add + b * add_ld + c0));
+  auto with_terms = [&](uint4 v) {
+    if (kAdd == 2) v = add8_16<kBf16>(v, pv);
+    return kAdd ? add8_16<kBf16>(v, av) : v;
+  };
 
   bool peers_run = S == 1;
   const int set_floats = order.lanes * 2 * slab;
@@ -119,8 +115,7 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ ad
       for (int j = 0; j < 4; ++j) { s2[j] = make_float2(0.0f, 0.0f); q2[j] = make_float2(0.0f, 0.0f); }
       auto accumulate = [&](const uint4& v) {
         float2 f[4];
-        unpack8f<kBf16>(v, f);
-        if (kAdd) add_round8<kBf16>(f, av);
+        unpack8f<kBf16>(with_terms(v), f);
 #pragma unroll
         for (int j = 0; j < 4; ++j) { s2[j] = __fadd2_rn(s2[j], f[j]); q2[j] = __ffma2_rn(f[j], f[j], q2[j]); }
       };
@@ -211,8 +206,7 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ ad
   uint4* dst = reinterpret_cast<uint4*>(y + base);
   auto transform = [&](const uint4& v) {
     float2 f[4];
-    unpack8f<kBf16>(v, f);
-    if (kAdd) add_round8<kBf16>(f, av);
+    unpack8f<kBf16>(with_terms(v), f);
     uint32_t w[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -255,16 +249,17 @@ int64_t workspace_floats(int64_t B, int64_t HW, int groups) {
   return B * groups * 2;
 }
 
-int groupnorm_nhwc(const void* x, const void* add, int x_dtype, int64_t B, int64_t HW, int64_t C, int groups,
-                   const void* gamma, const void* beta, int gb_dtype, float eps, int silu,
-                   void* y, float* workspace, cudaStream_t stream) {
+int groupnorm_nhwc(const void* x, const void* pre, const void* add, int64_t add_ld, int x_dtype, int64_t B, int64_t HW,
+                   int64_t C, int groups, const void* gamma, const void* beta, int gb_dtype, float eps, int silu,
+                   void* y, cudaStream_t stream) {
   if (x_dtype != HY3D_F16 && x_dtype != HY3D_BF16) return HY3D_ERR_ARG;
   if ((gamma || beta) && (gb_dtype < HY3D_F16 || gb_dtype > HY3D_F32)) return HY3D_ERR_ARG;
   if (B < 0 || HW <= 0 || C <= 0 || groups <= 0 || (C & 7) || C % groups) return HY3D_ERR_SHAPE;
   if (C > 2560 || B > 65535 || HW > (1ll << 31)) return HY3D_ERR_SHAPE;
   if (B == 0) return HY3D_OK;
-  if (!x || !y || !workspace) return HY3D_ERR_ARG;
-  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(add)) & 15)
+  if (!x || !y || (pre && !add)) return HY3D_ERR_ARG;
+  if (add && (add_ld < C || (add_ld & 7))) return HY3D_ERR_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(add) | reinterpret_cast<uintptr_t>(pre)) & 15)
     return HY3D_ERR_SHAPE;
   const int cpg = static_cast<int>(C / groups);
   // The order of the sums (see Order), fixed by the shape: chunks so that 320-thread blocks of whole rows
@@ -344,18 +339,17 @@ int groupnorm_nhwc(const void* x, const void* add, int x_dtype, int64_t B, int64
   const size_t smem = (static_cast<size_t>(order.chunks + order.classes) * 2 * slab_groups + 3 +
                        static_cast<size_t>(reps) * k * 2 * slab) * sizeof(float);
   if (rows_per_cta > 0x7FFFFFFF || B > 65535 || groups / slab_groups > 65535) return HY3D_ERR_SHAPE;
-  (void)workspace;
 
-  using KernelFn = void (*)(const uint16_t*, const uint16_t*, int64_t, int, int, int, int, int, int, Order, const void*,
+  using KernelFn = void (*)(const uint16_t*, const uint16_t*, const uint16_t*, int64_t, int64_t, int, int, int, int, int, int, Order, const void*,
                             const void*, int, float, uint16_t*);
-#define HY3D_GN_ROW(W)                                                                           \
-  {{{groupnorm_kernel<false, false, false, W>, groupnorm_kernel<false, false, true, W>},         \
-    {groupnorm_kernel<false, true, false, W>, groupnorm_kernel<false, true, true, W>}},          \
-   {{groupnorm_kernel<true, false, false, W>, groupnorm_kernel<true, false, true, W>},           \
-    {groupnorm_kernel<true, true, false, W>, groupnorm_kernel<true, true, true, W>}}}
-  static const KernelFn kernels[2][2][2][2] = {HY3D_GN_ROW(false), HY3D_GN_ROW(true)};
+#define HY3D_GN_ADD(BF, A, W) {groupnorm_kernel<BF, A, false, W>, groupnorm_kernel<BF, A, true, W>}
+#define HY3D_GN_ROW(W)                                                                    \
+  {{HY3D_GN_ADD(false, 0, W), HY3D_GN_ADD(false, 1, W), HY3D_GN_ADD(false, 2, W)},        \
+   {HY3D_GN_ADD(true, 0, W), HY3D_GN_ADD(true, 1, W), HY3D_GN_ADD(true, 2, W)}}
+  static const KernelFn kernels[2][2][3][2] = {HY3D_GN_ROW(false), HY3D_GN_ROW(true)};
 #undef HY3D_GN_ROW
-  const KernelFn kernel = kernels[wide ? 1 : 0][x_dtype == HY3D_BF16 ? 1 : 0][add ? 1 : 0][silu ? 1 : 0];
+#undef HY3D_GN_ADD
+  const KernelFn kernel = kernels[wide ? 1 : 0][x_dtype == HY3D_BF16 ? 1 : 0][pre ? 2 : add ? 1 : 0][silu ? 1 : 0];
   if (smem > 48 * 1024) {          // few samples of many chunks and narrow groups
     const int rc = ensure_max_smem(reinterpret_cast<const void*>(kernel), 100 * 1024);
     if (rc != HY3D_OK) return rc;
@@ -375,7 +369,7 @@ int groupnorm_nhwc(const void* x, const void* add, int x_dtype, int64_t B, int64
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   const cudaError_t err = cudaLaunchKernelEx(
-      &cfg, kernel, static_cast<const uint16_t*>(x), static_cast<const uint16_t*>(add), HW, static_cast<int>(C), cpg,
+      &cfg, kernel, static_cast<const uint16_t*>(x), static_cast<const uint16_t*>(pre), static_cast<const uint16_t*>(add), add_ld, HW, static_cast<int>(C), cpg,
       slab_groups, static_cast<int>(rows_per_cta), chunks_per_rank, reps, order, gamma, beta, gb_dtype, eps, static_cast<uint16_t*>(y));
   if (err != cudaSuccess) {
     cudaGetLastError();

@@ -7,6 +7,7 @@
 #include "linear_fused.cu"
 #include "linear_cluster.cu"
 #include "groupnorm.cu"
+#include "nhwc_ops.cu"
 #include "capi.cu"
 #include "static_scratch.cu"
 #include "probes.cu"

@@ -121,9 +121,10 @@ __device__ __forceinline__ uint2 quant8(const float (&f)[8], const RowQuant& r) 
 // 256 >> lg rows; threads past the last row repeat it (same values to the same places).  kFull: every thread
 // has exactly kMaxV vectors.  Bound by HBM reads (the codes stay in L2 for the GEMM) and by issue slots:
 // about 35 instructions per 8 values.
-template <bool kBf16, int kMaxV, bool kFull>
-__global__ void __launch_bounds__(kQuantThreads, kMaxV <= 6 ? 5 : 4)
-quantize_rows_kernel(const uint16_t* __restrict__ x, int64_t ldx, int8_t* __restrict__ q,
+// kAdd: the rows are x + add, rounded to the 16-bit type and not stored.
+template <bool kBf16, int kMaxV, bool kFull, bool kAdd>
+__global__ void __launch_bounds__(kQuantThreads, kAdd ? 3 : kMaxV <= 6 ? 5 : 4)
+quantize_rows_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ add, int64_t ldx, int8_t* __restrict__ q,
                      float* __restrict__ scale_out, int64_t M, int K, int lg) {
   __shared__ float s_part[kQuantThreads / 32];
   pdl_launch_dependents();
@@ -140,6 +141,15 @@ quantize_rows_kernel(const uint16_t* __restrict__ x, int64_t ldx, int8_t* __rest
 #pragma unroll
   for (int i = 0; i < kMaxV; ++i)
     v[i] = kFull || sub + i * G < nvec ? __ldcs(src + i * G) : make_uint4(0, 0, 0, 0);
+  if (kAdd) {
+    const uint4* other = reinterpret_cast<const uint4*>(add + row * ldx) + sub;
+    uint4 w[kMaxV];
+#pragma unroll
+    for (int i = 0; i < kMaxV; ++i)
+      w[i] = kFull || sub + i * G < nvec ? __ldcs(other + i * G) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int i = 0; i < kMaxV; ++i) v[i] = add8_16<kBf16>(v[i], w[i]);
+  }
   uint32_t amax2 = 0;
 #pragma unroll
   for (int i = 0; i < kMaxV; ++i) absmax8<kBf16>(v[i], amax2);
@@ -172,7 +182,7 @@ quantize_rows_kernel(const uint16_t* __restrict__ x, int64_t ldx, int8_t* __rest
 }
 
 template <bool kBf16>
-int launch_quantize(const void* x, int64_t M, int64_t K, int64_t ldx, int8_t* q, float* scale,
+int launch_quantize(const void* x, const void* add, int64_t M, int64_t K, int64_t ldx, int8_t* q, float* scale,
                     cudaStream_t stream) {
   const int nvec = static_cast<int>(K >> 3);
   // Power-of-two group size and vectors per thread (<= 10) that cover the row with the fewest idle slots;
@@ -191,9 +201,6 @@ int launch_quantize(const void* x, int64_t M, int64_t K, int64_t ldx, int8_t* q,
     if (score < best) { best = score; lg = l; maxv = static_cast<int>(v); }
   }
   if (lg < 0) return HY3D_ERR_SHAPE;
-#ifdef HY3D_QTUNE
-  if (const char* e = getenv("HY3D_QLG")) { lg = atoi(e); maxv = (nvec + (1 << lg) - 1) >> lg; if (maxv > 10 || maxv < 1) return HY3D_ERR_SHAPE; }
-#endif
   const int rows_per_block = kQuantThreads >> lg;
   const int64_t blocks = (M + rows_per_block - 1) / rows_per_block;
   if (blocks > 0x7FFFFFFF) return HY3D_ERR_SHAPE;
@@ -204,13 +211,16 @@ int launch_quantize(const void* x, int64_t M, int64_t K, int64_t ldx, int8_t* q,
   cudaLaunchAttribute attr[1] = {pdl_attribute()};
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  using KernelFn = void (*)(const uint16_t*, int64_t, int8_t*, float*, int64_t, int, int);
-#define HY3D_Q(V) {quantize_rows_kernel<kBf16, V, false>, quantize_rows_kernel<kBf16, V, true>}
-  static const KernelFn kernels[10][2] = {HY3D_Q(1), HY3D_Q(2), HY3D_Q(3), HY3D_Q(4), HY3D_Q(5),
+  using KernelFn = void (*)(const uint16_t*, const uint16_t*, int64_t, int8_t*, float*, int64_t, int, int);
+#define HY3D_Q(V)                                                                                      \
+  {{quantize_rows_kernel<kBf16, V, false, false>, quantize_rows_kernel<kBf16, V, true, false>},        \
+   {quantize_rows_kernel<kBf16, V, false, true>, quantize_rows_kernel<kBf16, V, true, true>}}
+  static const KernelFn kernels[10][2][2] = {HY3D_Q(1), HY3D_Q(2), HY3D_Q(3), HY3D_Q(4), HY3D_Q(5),
                                           HY3D_Q(6), HY3D_Q(7), HY3D_Q(8), HY3D_Q(9), HY3D_Q(10)};
 #undef HY3D_Q
-  const KernelFn kernel = kernels[maxv - 1][(maxv << lg) == nvec ? 1 : 0];
-  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const uint16_t*>(x), ldx, q, scale, M,
+  const KernelFn kernel = kernels[maxv - 1][add ? 1 : 0][(maxv << lg) == nvec ? 1 : 0];
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const uint16_t*>(x),
+                                             reinterpret_cast<const uint16_t*>(add), ldx, q, scale, M,
                                              static_cast<int>(K), lg);
   if (err != cudaSuccess) {
     cudaGetLastError();
@@ -230,10 +240,12 @@ int launch_quantize(const void* x, int64_t M, int64_t K, int64_t ldx, int8_t* q,
 // 2^lg <= 32 lanes share a row (shuffle reductions), each with up to kMaxV vectors; gamma / beta are staged
 // once per block in shared memory as fp32 and the block walks rows with a grid-stride loop, the next row's
 // vectors requested before the current row is worked on.  Issue-bound.  Everything that can be is decided at
-// compile time (kFull: no lane has a vector too few; kY: the normalised row is wanted too).
-template <bool kBf16, int kMaxV, bool kFull, bool kY>
-__global__ void __launch_bounds__(kQuantThreads, kMaxV <= 2 ? 4 : kMaxV <= 5 ? 3 : 2)
-layernorm_quantize_kernel(const uint16_t* __restrict__ x, int64_t ldx, const void* __restrict__ gamma,
+// compile time (kFull: no lane has a vector too few; kOut 1: the normalised row is stored too; kOut 2: the rows
+// are x + add, rounded to the 16-bit type, and that sum is stored -- a transformer block's residual stream).
+__host__ __device__ constexpr int ln_blocks(int maxv, int out) { return maxv <= 2 ? 4 : maxv <= 5 && out < 2 ? 3 : 2; }
+template <bool kBf16, int kMaxV, bool kFull, int kOut>
+__global__ void __launch_bounds__(kQuantThreads, ln_blocks(kMaxV, kOut))
+layernorm_quantize_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ add, int64_t ldx, const void* __restrict__ gamma,
                           const void* __restrict__ beta, int gb_dtype, float eps,
                           int8_t* __restrict__ q, float* __restrict__ scale_out,
                           uint16_t* __restrict__ y_out, int64_t M, int K, int lg) {
@@ -260,9 +272,16 @@ layernorm_quantize_kernel(const uint16_t* __restrict__ x, int64_t ldx, const voi
   const int trips = static_cast<int>((M - static_cast<int64_t>(blockIdx.x) * rows_per_block + row_step - 1) / row_step);
   pdl_wait();   // x comes from the previous kernel in the stream; gamma / beta are parameters
   __syncthreads();
-  uint4 vn[kMaxV];
+  uint4 vn[kMaxV], an[kOut == 2 ? kMaxV : 1];
   auto fetch = [&](int64_t r) {
-    const uint4* src = reinterpret_cast<const uint4*>(x + (r < M ? r : M - 1) * ldx) + sub;
+    const int64_t off = (r < M ? r : M - 1) * ldx;
+    const uint4* src = reinterpret_cast<const uint4*>(x + off) + sub;
+    if (kOut == 2) {
+      const uint4* other = reinterpret_cast<const uint4*>(add + off) + sub;
+#pragma unroll
+      for (int i = 0; i < kMaxV; ++i)
+        an[kOut == 2 ? i : 0] = kFull || sub + i * G < nvec ? __ldcs(other + i * G) : make_uint4(0, 0, 0, 0);
+    }
 #pragma unroll
     for (int i = 0; i < kMaxV; ++i)
       vn[i] = kFull || sub + i * G < nvec ? __ldcs(src + i * G) : make_uint4(0, 0, 0, 0);
@@ -277,6 +296,11 @@ layernorm_quantize_kernel(const uint16_t* __restrict__ x, int64_t ldx, const voi
 #pragma unroll
     for (int i = 0; i < kMaxV; ++i) {
       float t[8];
+      if (kOut == 2) {
+        vn[i] = add8_16<kBf16>(vn[i], an[kOut == 2 ? i : 0]);
+        if (kFull || sub + i * G < nvec)
+          (reinterpret_cast<uint4*>(y_out + at_row * static_cast<int64_t>(K)) + sub)[i * G] = vn[i];
+      }
       unpack8<kBf16>(vn[i], t);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -347,7 +371,7 @@ layernorm_quantize_kernel(const uint16_t* __restrict__ x, int64_t ldx, const voi
       }
     };
     if (rq.exact) write(True{}); else write(False{});
-    if (kY) {
+    if (kOut == 1) {
       uint4* ydst = reinterpret_cast<uint4*>(y_out + at_row * static_cast<int64_t>(K)) + sub;
 #pragma unroll
       for (int i = 0; i < kMaxV; ++i)
@@ -357,7 +381,7 @@ layernorm_quantize_kernel(const uint16_t* __restrict__ x, int64_t ldx, const voi
 }
 
 template <bool kBf16>
-int launch_layernorm_quantize(const void* x, int64_t M, int64_t K, int64_t ldx, const void* gamma,
+int launch_layernorm_quantize(const void* x, const void* add, int64_t M, int64_t K, int64_t ldx, const void* gamma,
                               const void* beta, int gb_dtype, float eps, int8_t* q, float* scale,
                               void* y_out, cudaStream_t stream) {
   const int nvec = static_cast<int>(K >> 3);
@@ -369,17 +393,19 @@ int launch_layernorm_quantize(const void* x, int64_t M, int64_t K, int64_t ldx, 
   if (maxv > 8) return HY3D_ERR_SHAPE;
   const int rows_per_block = kQuantThreads >> lg;
   const int64_t batches = (M + rows_per_block - 1) / rows_per_block;
-  using KernelFn = void (*)(const uint16_t*, int64_t, const void*, const void*, int, float, int8_t*, float*, uint16_t*,
-                            int64_t, int, int);
-#define HY3D_LNQ(V)                                                                              \
-  {{layernorm_quantize_kernel<kBf16, V, false, false>, layernorm_quantize_kernel<kBf16, V, false, true>}, \
-   {layernorm_quantize_kernel<kBf16, V, true, false>, layernorm_quantize_kernel<kBf16, V, true, true>}}
-  static const KernelFn kernels[8][2][2] = {HY3D_LNQ(1), HY3D_LNQ(2), HY3D_LNQ(3), HY3D_LNQ(4),
-                                            HY3D_LNQ(5), HY3D_LNQ(6), HY3D_LNQ(7), HY3D_LNQ(8)};
+  using KernelFn = void (*)(const uint16_t*, const uint16_t*, int64_t, const void*, const void*, int, float, int8_t*,
+                            float*, uint16_t*, int64_t, int, int);
+#define HY3D_LNQ(V)                                                                                          \
+  {{layernorm_quantize_kernel<kBf16, V, false, 0>, layernorm_quantize_kernel<kBf16, V, false, 1>,            \
+    layernorm_quantize_kernel<kBf16, V, false, 2>},                                                          \
+   {layernorm_quantize_kernel<kBf16, V, true, 0>, layernorm_quantize_kernel<kBf16, V, true, 1>,              \
+    layernorm_quantize_kernel<kBf16, V, true, 2>}}
+  static const KernelFn kernels[6][2][3] = {HY3D_LNQ(1), HY3D_LNQ(2), HY3D_LNQ(3), HY3D_LNQ(4), HY3D_LNQ(5), HY3D_LNQ(8)};
 #undef HY3D_LNQ
-  const KernelFn kernel = kernels[maxv - 1][(maxv << lg) == nvec ? 1 : 0][y_out ? 1 : 0];
+  const int v = maxv <= 5 ? maxv : 8, out = add ? 2 : y_out ? 1 : 0;
+  const KernelFn kernel = kernels[maxv <= 5 ? maxv - 1 : 5][(v << lg) == nvec ? 1 : 0][out];
   // One wave of resident blocks, evened out: every block walks the same number of row batches (or one less).
-  const int64_t wave = static_cast<int64_t>(148) * (maxv <= 2 ? 4 : maxv <= 5 ? 3 : 2);
+  const int64_t wave = static_cast<int64_t>(148) * ln_blocks(v, out);
   const int64_t trips = (batches + wave - 1) / wave;
   const int64_t blocks = (batches + trips - 1) / trips;
   cudaLaunchConfig_t cfg = {};
@@ -390,8 +416,8 @@ int launch_layernorm_quantize(const void* x, int64_t M, int64_t K, int64_t ldx, 
   cudaLaunchAttribute attr[1] = {pdl_attribute()};
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const uint16_t*>(x), ldx, gamma, beta, gb_dtype,
-                                             eps, q, scale, reinterpret_cast<uint16_t*>(y_out), M, static_cast<int>(K), lg);
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const uint16_t*>(x),
+                                             reinterpret_cast<const uint16_t*>(add), ldx, gamma, beta, gb_dtype, eps, q, scale, reinterpret_cast<uint16_t*>(y_out), M, static_cast<int>(K), lg);
   if (err != cudaSuccess) {
     cudaGetLastError();
     return HY3D_ERR_CUDA;
@@ -467,20 +493,20 @@ dequant_bias_kernel(const int32_t* __restrict__ acc, const float* __restrict__ a
 
 }  // namespace
 
-int quantize_rows(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, int8_t* q,
+int quantize_rows(const void* x, const void* add, int x_dtype, int64_t M, int64_t K, int64_t ldx, int8_t* q,
                   float* scale, cudaStream_t stream) {
   if (x_dtype != HY3D_F16 && x_dtype != HY3D_BF16) return HY3D_ERR_ARG;
   if (M < 0 || K <= 0 || (K & 7) || K > 16384 || ldx < K || (ldx & 7)) return HY3D_ERR_SHAPE;
   if (M == 0) return HY3D_OK;
   if (!x || !q || !scale) return HY3D_ERR_ARG;
-  if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(q) & 7))
+  if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(add)) & 15) || (reinterpret_cast<uintptr_t>(q) & 7))
     return HY3D_ERR_SHAPE;
   if (M == 0) return HY3D_OK;
-  return x_dtype == HY3D_BF16 ? launch_quantize<true>(x, M, K, ldx, q, scale, stream)
-                              : launch_quantize<false>(x, M, K, ldx, q, scale, stream);
+  return x_dtype == HY3D_BF16 ? launch_quantize<true>(x, add, M, K, ldx, q, scale, stream)
+                              : launch_quantize<false>(x, add, M, K, ldx, q, scale, stream);
 }
 
-int layernorm_quantize(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, const void* gamma,
+int layernorm_quantize(const void* x, const void* add, int x_dtype, int64_t M, int64_t K, int64_t ldx, const void* gamma,
                        const void* beta, int gb_dtype, float eps, int8_t* q, float* scale, void* y_out,
                        cudaStream_t stream) {
   if (x_dtype != HY3D_F16 && x_dtype != HY3D_BF16) return HY3D_ERR_ARG;
@@ -488,13 +514,13 @@ int layernorm_quantize(const void* x, int x_dtype, int64_t M, int64_t K, int64_t
   if (M < 0 || K <= 0 || (K & 7) || K > 2048 || ldx < K || (ldx & 7)) return HY3D_ERR_SHAPE;
   if (!(eps >= 0.0f)) return HY3D_ERR_ARG;
   if (M == 0) return HY3D_OK;
-  if (!x || !q || !scale) return HY3D_ERR_ARG;
-  if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(q) & 7) ||
+  if (!x || !q || !scale || (add && !y_out)) return HY3D_ERR_ARG;
+  if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(add)) & 15) || (reinterpret_cast<uintptr_t>(q) & 7) ||
       (reinterpret_cast<uintptr_t>(y_out) & 15))
     return HY3D_ERR_SHAPE;
   return x_dtype == HY3D_BF16
-             ? launch_layernorm_quantize<true>(x, M, K, ldx, gamma, beta, gb_dtype, eps, q, scale, y_out, stream)
-             : launch_layernorm_quantize<false>(x, M, K, ldx, gamma, beta, gb_dtype, eps, q, scale, y_out, stream);
+             ? launch_layernorm_quantize<true>(x, add, M, K, ldx, gamma, beta, gb_dtype, eps, q, scale, y_out, stream)
+             : launch_layernorm_quantize<false>(x, add, M, K, ldx, gamma, beta, gb_dtype, eps, q, scale, y_out, stream);
 }
 
 int quantizer_enum_check(int x_dtype, unsigned long long* pairs, unsigned long long* mismatches,

@@ -67,7 +67,7 @@ int linear_dense_static(const void* x, int x_dtype, int64_t ldx, const int8_t* B
   if (rc != HY3D_OK) return rc;
   int8_t* q = reinterpret_cast<int8_t*>(base);
   float* scale = reinterpret_cast<float*>(base + kStaticQBytes);
-  rc = quantize_rows(x, x_dtype, M, K, ldx, q, scale, stream);
+  rc = quantize_rows(x, nullptr, x_dtype, M, K, ldx, q, scale, stream);
   if (rc != HY3D_OK) return rc;
   return gemm_dense(q, B, scale, w_scale, ws_dtype, bias, bias_dtype, out, out_dtype, M, N, K,
                     epilogue, 0, 0, stream);

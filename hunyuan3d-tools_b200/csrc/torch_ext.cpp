@@ -38,7 +38,12 @@ struct Api {
   HY3D_FN(hy3d_linear_w8a8_sparse24);
   HY3D_FN(hy3d_gemm_w8a8_sparse24);
   HY3D_FN(hy3d_layernorm_quantize);
-  HY3D_FN(hy3d_groupnorm_nhwc);
+  HY3D_FN(hy3d_groupnorm_nhwc_terms);
+  HY3D_FN(hy3d_add_bias_nhwc);
+  HY3D_FN(hy3d_concat_nhwc);
+  HY3D_FN(hy3d_upsample2x_nhwc);
+  HY3D_FN(hy3d_add_quantize_rows);
+  HY3D_FN(hy3d_add_layernorm_quantize);
   HY3D_FN(hy3d_quantize_weight);
   HY3D_FN(hy3d_status_string);
 } api;
@@ -49,6 +54,17 @@ const at::Tensor* plain(PyObject* o) {
   if (!THPVariable_CheckExact(o)) return nullptr;   // torch.Tensor or Parameter, no other subclass
   const at::Tensor& t = THPVariable_Unpack(o);
   return t.is_cuda() && t.layout() == at::kStrided && t.is_contiguous() ? &t : nullptr;
+}
+
+// The same in channels-last memory, f16 / bf16, whole 16-byte vectors of channels.
+const at::Tensor* plain_nhwc(PyObject* o) {
+  if (!THPVariable_CheckExact(o)) return nullptr;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  return t.is_cuda() && t.layout() == at::kStrided && t.dim() == 4 && (t.scalar_type() == at::kHalf || t.scalar_type() == at::kBFloat16) &&
+                 (t.size(1) & 7) == 0 && t.numel() > 0 && t.is_contiguous(at::MemoryFormat::ChannelsLast) &&
+                 (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15) == 0
+             ? &t
+             : nullptr;
 }
 
 int half_code(at::ScalarType t) {
@@ -313,8 +329,10 @@ struct Affine {
 };
 
 // layernorm_quantize(x, gamma | None, beta | None, eps) -> (codes (M,K), scale (M)) | None
-struct Quantized { at::Tensor q, s; };
-bool layernorm_quantize_impl(PyObject* px, PyObject* gamma, PyObject* beta, double eps, Quantized* out, int* status) {
+struct Quantized { at::Tensor q, s, sum; };
+// padd: rows to add first; the sum goes to out->sum.
+bool layernorm_quantize_impl(PyObject* px, PyObject* padd, PyObject* gamma, PyObject* beta, double eps, Quantized* out,
+                             int* status) {
   const at::Tensor* x = plain(px);
   if (!x || x->dim() < 1) return false;
   const int code = half_code(x->scalar_type());
@@ -326,6 +344,15 @@ bool layernorm_quantize_impl(PyObject* px, PyObject* gamma, PyObject* beta, doub
   cudaStream_t st = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
   out->q = at::Tensor(at::detail::empty_cuda({M, K}, at::kChar, x->device(), std::nullopt));
   out->s = at::Tensor(at::detail::empty_cuda({M}, at::kFloat, x->device(), std::nullopt));
+  if (padd) {
+    const at::Tensor* t = plain(padd);
+    if (!t || t->scalar_type() != x->scalar_type() || t->device() != x->device() || t->sizes() != x->sizes()) return false;
+    out->sum = at::Tensor(at::detail::empty_cuda(x->sizes(), x->scalar_type(), x->device(), std::nullopt));
+    *status = api.hy3d_add_layernorm_quantize(x->const_data_ptr(), t->const_data_ptr(), out->sum.mutable_data_ptr(), code, M, K,
+                                              f.gamma, f.beta, f.code, static_cast<float>(eps), out->q.mutable_data_ptr<int8_t>(),
+                                              out->s.mutable_data_ptr<float>(), st);
+    return true;
+  }
   *status = api.hy3d_layernorm_quantize(x->const_data_ptr(), code, M, K, K, f.gamma, f.beta, f.code, static_cast<float>(eps),
                                         out->q.mutable_data_ptr<int8_t>(), out->s.mutable_data_ptr<float>(), nullptr, st);
   return true;
@@ -334,7 +361,7 @@ PyObject* layernorm_quantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Quantized z;
   int rc = 0;
-  if (n != 4 || !PyFloat_Check(a[3]) || !layernorm_quantize_impl(a[0], a[1], a[2], PyFloat_AS_DOUBLE(a[3]), &z, &rc)) return none();
+  if (n != 4 || !PyFloat_Check(a[3]) || !layernorm_quantize_impl(a[0], nullptr, a[1], a[2], PyFloat_AS_DOUBLE(a[3]), &z, &rc)) return none();
   if (rc != HY3D_OK) return failed("hy3d_layernorm_quantize", rc);
   PyObject* pq = THPVariable_Wrap(std::move(z.q));
   PyObject* ps = pq ? THPVariable_Wrap(std::move(z.s)) : nullptr;
@@ -348,32 +375,42 @@ PyObject* layernorm_quantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // groupnorm_nhwc(x channels_last, groups, gamma | None, beta | None, eps, silu, add (B,C) | None) -> y | None
-PyObject* groupnorm_impl(PyObject* px, long groups, PyObject* gamma, PyObject* beta, double eps, bool silu, PyObject* padd) {
+PyObject* groupnorm_impl(PyObject* px, long groups, PyObject* gamma, PyObject* beta, double eps, bool silu, PyObject* padd,
+                         PyObject* pbias) {
   HANDLE_TH_ERRORS
-  if (!THPVariable_CheckExact(px)) return none();
-  const at::Tensor& x = THPVariable_Unpack(px);
-  if (!x.is_cuda() || x.layout() != at::kStrided || x.dim() != 4 || !x.is_contiguous(at::MemoryFormat::ChannelsLast))
-    return none();
+  const at::Tensor* px4 = plain_nhwc(px);
+  if (!px4) return none();
+  const at::Tensor& x = *px4;
   const int code = half_code(x.scalar_type());
   const int64_t B = x.size(0), C = x.size(1), HW = x.size(2) * x.size(3);
   if (code < 0 || B <= 0 || HW <= 0) return none();
   const Affine f(gamma, beta, C, x.device());
   if (!f.ok) return none();
-  const void* add = nullptr;
-  if (padd != Py_None) {
-    const at::Tensor* t = plain(padd);
-    if (!t || t->dim() != 2 || t->size(0) != B || t->size(1) != C || t->scalar_type() != x.scalar_type() ||
-        t->device() != x.device())
+  const void *add = nullptr, *bias = nullptr;
+  int64_t add_ld = C;
+  if (padd != Py_None) {            // rows may lie apart (a slice of stacked projections)
+    if (!THPVariable_CheckExact(padd)) return none();
+    const at::Tensor& t = THPVariable_Unpack(padd);
+    if (!t.is_cuda() || t.layout() != at::kStrided || t.dim() != 2 || t.size(0) != B || t.size(1) != C ||
+        t.scalar_type() != x.scalar_type() || t.device() != x.device() || t.stride(1) != 1)
       return none();
-    add = t->const_data_ptr();
+    add = t.const_data_ptr();
+    add_ld = B > 1 ? t.stride(0) : C;
+    if (add_ld < C || (add_ld & 7) || (reinterpret_cast<uintptr_t>(add) & 15)) return none();
+  }
+  if (pbias != Py_None) {
+    const at::Tensor* t = plain(pbias);
+    if (!add || !t || t->numel() != C || t->scalar_type() != x.scalar_type() || t->device() != x.device() ||
+        (reinterpret_cast<uintptr_t>(t->const_data_ptr()) & 15))
+      return none();
+    bias = t->const_data_ptr();
   }
   c10::cuda::CUDAGuard guard(x.device());
   cudaStream_t st = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
   at::Tensor y = at::Tensor(at::detail::empty_cuda(x.sizes(), x.scalar_type(), x.device(), at::MemoryFormat::ChannelsLast));
-  // the kernel needs no workspace; the C ABI still asks for one
-  const int rc = api.hy3d_groupnorm_nhwc(x.const_data_ptr(), add, code, B, HW, C, static_cast<int>(groups), f.gamma, f.beta,
-                                         f.code, static_cast<float>(eps), silu ? 1 : 0, y.mutable_data_ptr(),
-                                         static_cast<float*>(y.mutable_data_ptr()), st);
+  const int rc = api.hy3d_groupnorm_nhwc_terms(x.const_data_ptr(), bias, add, add_ld, code, B, HW, C, static_cast<int>(groups),
+                                               f.gamma, f.beta, f.code, static_cast<float>(eps), silu ? 1 : 0,
+                                               y.mutable_data_ptr(), st);
   if (rc != HY3D_OK) return failed("hy3d_groupnorm_nhwc", rc);
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS
@@ -381,7 +418,7 @@ PyObject* groupnorm_impl(PyObject* px, long groups, PyObject* gamma, PyObject* b
 PyObject* groupnorm_nhwc(PyObject*, PyObject* const* a, Py_ssize_t n) {
   long groups = 0;
   if (n != 7 || !small_int(a[1], 1, 1 << 20, &groups) || !PyFloat_Check(a[4])) return none();
-  return groupnorm_impl(a[0], groups, a[2], a[3], PyFloat_AS_DOUBLE(a[4]), a[5] == Py_True, a[6]);
+  return groupnorm_impl(a[0], groups, a[2], a[3], PyFloat_AS_DOUBLE(a[4]), a[5] == Py_True, a[6], Py_None);
 }
 
 // quantize_weight(w (N,K), sparse) -> (codes, scale) or (compressed codes, metadata, scale) | None
@@ -566,25 +603,14 @@ PyObject* layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return PyDict_Check(dict) ? linear_of(a[0], dict, a[1]) : none();
 }
 
-// norm_call(layer, x) -> QuantizedActivation | None: calling an Int8LayerNorm
-PyObject* norm_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
-  PyObject* dict = n == 2 && THPVariable_CheckExact(a[1]) ? plain_module(a[0], layernorm_class) : nullptr;
-  PyObject* params = dict ? PyDict_GetItemWithError(dict, names.parameters) : nullptr;
-  PyObject* eps = dict ? PyDict_GetItemWithError(dict, names.eps) : nullptr;
-  if (!params || !PyDict_Check(params) || !eps || !PyFloat_Check(eps)) return none();
-  PyObject* gamma = PyDict_GetItemWithError(params, names.weight);
-  PyObject* beta = PyDict_GetItemWithError(params, names.bias);
-  Quantized z;
-  int rc = 0;
-  if (!gamma || !beta || !layernorm_quantize_impl(a[1], gamma, beta, PyFloat_AS_DOUBLE(eps), &z, &rc)) return none();
-  if (rc != HY3D_OK) return failed("hy3d_layernorm_quantize", rc);
+// A QuantizedActivation of x's shape and type.
+PyObject* quantized_object(PyObject* x, at::Tensor&& q, at::Tensor&& s) {
   PyObject* r = quantized_class->tp_alloc(quantized_class, 0);
   if (!r) return nullptr;
-  struct { PyObject *name, *value; } set[] = {{names.q, THPVariable_Wrap(std::move(z.q))},
-                                              {names.act_scale, THPVariable_Wrap(std::move(z.s))},
-                                              {names.shape, PyObject_GetAttr(a[1], names.shape)},
-                                              {names.dtype, PyObject_GetAttr(a[1], names.dtype)}};
+  struct { PyObject *name, *value; } set[] = {{names.q, THPVariable_Wrap(std::move(q))},
+                                              {names.act_scale, THPVariable_Wrap(std::move(s))},
+                                              {names.shape, PyObject_GetAttr(x, names.shape)},
+                                              {names.dtype, PyObject_GetAttr(x, names.dtype)}};
   bool bad = false;
   for (auto& e : set) {
     bad = bad || !e.value || PyObject_SetAttr(r, e.name, e.value) < 0;
@@ -592,12 +618,132 @@ PyObject* norm_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   if (bad) { Py_DECREF(r); return nullptr; }
   return r;
+}
+
+// norm_call(layer, x) -> QuantizedActivation | None: calling an Int8LayerNorm
+// norm_call(layer, x, h) -> (x + h, QuantizedActivation of its LayerNorm) | None
+PyObject* norm_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  PyObject* dict = (n == 2 || n == 3) && THPVariable_CheckExact(a[1]) ? plain_module(a[0], layernorm_class) : nullptr;
+  PyObject* params = dict ? PyDict_GetItemWithError(dict, names.parameters) : nullptr;
+  PyObject* eps = dict ? PyDict_GetItemWithError(dict, names.eps) : nullptr;
+  if (!params || !PyDict_Check(params) || !eps || !PyFloat_Check(eps)) return none();
+  PyObject* gamma = PyDict_GetItemWithError(params, names.weight);
+  PyObject* beta = PyDict_GetItemWithError(params, names.bias);
+  Quantized z;
+  int rc = 0;
+  if (!gamma || !beta || !layernorm_quantize_impl(a[1], n == 3 ? a[2] : nullptr, gamma, beta, PyFloat_AS_DOUBLE(eps), &z, &rc))
+    return none();
+  if (rc != HY3D_OK) return failed("hy3d_layernorm_quantize", rc);
+  PyObject* r = quantized_object(a[1], std::move(z.q), std::move(z.s));
+  if (n == 2 || !r) return r;
+  PyObject* sum = THPVariable_Wrap(std::move(z.sum));
+  PyObject* pair = sum ? PyTuple_New(2) : nullptr;
+  if (!pair) { Py_XDECREF(sum); Py_DECREF(r); return nullptr; }
+  PyTuple_SET_ITEM(pair, 0, sum);
+  PyTuple_SET_ITEM(pair, 1, r);
+  return pair;
   END_HANDLE_TH_ERRORS
 }
 
-// groupnorm_call(layer, x, add | None) -> y | None: calling a GroupNormNHWC whose kernel path is on
+// add_quantize(x, h) -> QuantizedActivation of x + h | None
+PyObject* add_quantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const at::Tensor* x = n == 2 ? plain(a[0]) : nullptr;
+  const at::Tensor* h = x ? plain(a[1]) : nullptr;
+  if (!h || !quantized_class || x->dim() < 1 || h->scalar_type() != x->scalar_type() || h->device() != x->device() ||
+      h->sizes() != x->sizes())
+    return none();
+  const int code = half_code(x->scalar_type());
+  const int64_t K = x->size(-1), M = K > 0 ? x->numel() / K : 0;
+  if (code < 0 || M <= 0 || (K & 7)) return none();
+  c10::cuda::CUDAGuard guard(x->device());
+  cudaStream_t st = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
+  at::Tensor q = at::Tensor(at::detail::empty_cuda({M, K}, at::kChar, x->device(), std::nullopt));
+  at::Tensor s = at::Tensor(at::detail::empty_cuda({M}, at::kFloat, x->device(), std::nullopt));
+  const int rc = api.hy3d_add_quantize_rows(x->const_data_ptr(), h->const_data_ptr(), code, M, K, q.mutable_data_ptr<int8_t>(),
+                                            s.mutable_data_ptr<float>(), st);
+  if (rc != HY3D_OK) return failed("hy3d_add_quantize_rows", rc);
+  return quantized_object(a[0], std::move(q), std::move(s));
+  END_HANDLE_TH_ERRORS
+}
+
+// add_bias(x, bias_x | None, h | None, bias_h | None) -> round(round(x + bias_x) + round(h + bias_h)) | None
+PyObject* add_bias(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const at::Tensor* x = n == 4 ? plain_nhwc(a[0]) : nullptr;
+  const at::Tensor* h = x && a[2] != Py_None ? plain_nhwc(a[2]) : nullptr;
+  if (!x || (a[2] != Py_None && (!h || h->sizes() != x->sizes() || h->scalar_type() != x->scalar_type() || h->device() != x->device())))
+    return none();
+  const int64_t C = x->size(1);
+  const void* bias[2] = {nullptr, nullptr};
+  for (int i = 0; i < 2; ++i) {
+    PyObject* o = a[i ? 3 : 1];
+    if (o == Py_None) continue;
+    const at::Tensor* t = plain(o);
+    if (!t || t->numel() != C || t->scalar_type() != x->scalar_type() || t->device() != x->device() ||
+        (reinterpret_cast<uintptr_t>(t->const_data_ptr()) & 15) || (i && !h))
+      return none();
+    bias[i] = t->const_data_ptr();
+  }
+  c10::cuda::CUDAGuard guard(x->device());
+  cudaStream_t st = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
+  at::Tensor y = at::Tensor(at::detail::empty_cuda(x->sizes(), x->scalar_type(), x->device(), at::MemoryFormat::ChannelsLast));
+  const int rc = api.hy3d_add_bias_nhwc(x->const_data_ptr(), bias[0], h ? h->const_data_ptr() : nullptr, bias[1],
+                                        half_code(x->scalar_type()), y.mutable_data_ptr(), x->numel() / C, C, st);
+  if (rc != HY3D_OK) return failed("hy3d_add_bias_nhwc", rc);
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// concat_nhwc(a, b) -> torch.cat([a, b], 1) | None
+PyObject* concat_nhwc(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const at::Tensor* x = n == 2 ? plain_nhwc(a[0]) : nullptr;
+  const at::Tensor* h = x ? plain_nhwc(a[1]) : nullptr;
+  if (!h || h->scalar_type() != x->scalar_type() || h->device() != x->device() || h->size(0) != x->size(0) ||
+      h->size(2) != x->size(2) || h->size(3) != x->size(3))
+    return none();
+  c10::cuda::CUDAGuard guard(x->device());
+  cudaStream_t st = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
+  const int64_t Ca = x->size(1), Cb = h->size(1);
+  at::Tensor y = at::Tensor(at::detail::empty_cuda({x->size(0), Ca + Cb, x->size(2), x->size(3)}, x->scalar_type(), x->device(),
+                                                   at::MemoryFormat::ChannelsLast));
+  const int rc = api.hy3d_concat_nhwc(x->const_data_ptr(), Ca, h->const_data_ptr(), Cb, y.mutable_data_ptr(), x->numel() / Ca, st);
+  if (rc != HY3D_OK) return failed("hy3d_concat_nhwc", rc);
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// upsample2x_nhwc(x) -> nearest-neighbour twice the size | None
+PyObject* upsample2x_nhwc(PyObject*, PyObject* px) {
+  HANDLE_TH_ERRORS
+  const at::Tensor* x = plain_nhwc(px);
+  if (!x) return none();
+  c10::cuda::CUDAGuard guard(x->device());
+  cudaStream_t st = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
+  at::Tensor y = at::Tensor(at::detail::empty_cuda({x->size(0), x->size(1), 2 * x->size(2), 2 * x->size(3)}, x->scalar_type(),
+                                                   x->device(), at::MemoryFormat::ChannelsLast));
+  const int rc = api.hy3d_upsample2x_nhwc(x->const_data_ptr(), y.mutable_data_ptr(), x->size(0), x->size(2), x->size(3), x->size(1), st);
+  if (rc != HY3D_OK) return failed("hy3d_upsample2x_nhwc", rc);
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// unhooked(module, ...) -> True where calling each module is calling the `forward` of its class, so that a
+// caller may do that forward's work itself
+PyObject* unhooked(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    const Registered any{Py_TYPE(a[i]), _PyType_Lookup(Py_TYPE(a[i]), names.forward)};
+    if (!global_hooks[0] || !plain_module(a[i], any)) Py_RETURN_FALSE;
+  }
+  Py_RETURN_TRUE;
+}
+
+// groupnorm_call(layer, x, add | None, bias | None) -> y | None: calling a GroupNormNHWC whose kernel path is
+// on; `bias` is that of the convolution that made x and is added first
 PyObject* groupnorm_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  PyObject* dict = n == 3 ? plain_module(a[0], groupnorm_class) : nullptr;
+  PyObject* dict = n == 4 ? plain_module(a[0], groupnorm_class) : nullptr;
   if (!dict || PyDict_GetItemWithError(dict, names.fused) != Py_True) return none();
   PyObject* params = PyDict_GetItemWithError(dict, names.parameters);
   PyObject* eps = PyDict_GetItemWithError(dict, names.eps);
@@ -608,7 +754,7 @@ PyObject* groupnorm_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return none();
   PyObject* gamma = PyDict_GetItemWithError(params, names.weight);
   PyObject* beta = PyDict_GetItemWithError(params, names.bias);
-  return gamma && beta ? groupnorm_impl(a[1], groups, gamma, beta, PyFloat_AS_DOUBLE(eps), silu == Py_True, a[2]) : none();
+  return gamma && beta ? groupnorm_impl(a[1], groups, gamma, beta, PyFloat_AS_DOUBLE(eps), silu == Py_True, a[2], a[3]) : none();
 }
 
 // open(path): resolves the C ABI in the library at `path`, which the caller has loaded and checked.
@@ -638,7 +784,12 @@ PyObject* open_library(PyObject*, PyObject* arg) {
   HY3D_SYM(hy3d_linear_w8a8_sparse24);
   HY3D_SYM(hy3d_gemm_w8a8_sparse24);
   HY3D_SYM(hy3d_layernorm_quantize);
-  HY3D_SYM(hy3d_groupnorm_nhwc);
+  HY3D_SYM(hy3d_groupnorm_nhwc_terms);
+  HY3D_SYM(hy3d_add_bias_nhwc);
+  HY3D_SYM(hy3d_concat_nhwc);
+  HY3D_SYM(hy3d_upsample2x_nhwc);
+  HY3D_SYM(hy3d_add_quantize_rows);
+  HY3D_SYM(hy3d_add_layernorm_quantize);
   HY3D_SYM(hy3d_quantize_weight);
   HY3D_SYM(hy3d_status_string);
 #undef HY3D_SYM
@@ -653,6 +804,11 @@ PyMethodDef methods[] = {
     HY3D_FAST(layer_forward),
     HY3D_FAST(norm_call),
     HY3D_FAST(groupnorm_call),
+    HY3D_FAST(add_quantize),
+    HY3D_FAST(add_bias),
+    HY3D_FAST(concat_nhwc),
+    {"upsample2x_nhwc", upsample2x_nhwc, METH_O, nullptr},
+    HY3D_FAST(unhooked),
     HY3D_FAST(linear_dense),
     HY3D_FAST(linear_sparse),
     HY3D_FAST(gemm_dense),

@@ -164,14 +164,16 @@ def build_texture_unet(device, dtype=torch.bfloat16, quant: str = "mixed", seed:
     ``quant``: "mixed" (2:4 sparse where that kernel is the faster one -- or where
     K >= ``sparse_min_k`` if given -- dense elsewhere), "dense", "sparse" (the
     reference's sparse mode: small-K layers stay bf16) or "none".  ``fuse_qkv`` stacks the
-    q/k/v (self-attention) and k/v (cross-attention) projections that share an input.
+    q/k/v (self-attention) and k/v (cross-attention) projections that share an input, and over the whole model
+    the projections of the time embedding and of the context.
     ``init_on_device`` draws the random weights on the GPU instead of the CPU.  ``fuse_ln`` lets
     the transformer blocks' LayerNorms emit int8 codes for the projections that follow them.
     ``fused_gn`` runs GroupNorm (+ SiLU) through the library's channels-last kernel (default: on
     for the INT8 modes on a CUDA device with channels_last activations, off for "none", which
     stands for the stock PyTorch model)."""
     from . import quantize_utils as qu
-    from .unet import UNetSD21MV, fuse_geglu_layers, fuse_qkv_layers, fuse_layernorm_quant
+    from .unet import (UNetSD21MV, fuse_context_projections, fuse_geglu_layers, fuse_layernorm_quant, fuse_qkv_layers,
+                       fuse_time_projections)
     torch.manual_seed(seed)
     if init_on_device:
         # Random initialisation by the device's generator: seconds instead of a minute for the
@@ -200,6 +202,7 @@ def build_texture_unet(device, dtype=torch.bfloat16, quant: str = "mixed", seed:
         stats["geglu_fused"] = fuse_geglu_layers(unet)
     if fuse_qkv and quant != "none":
         stats["qkv_layers_removed"] = fuse_qkv_layers(unet)
+        stats["shared_input_layers_removed"] = fuse_time_projections(unet) + fuse_context_projections(unet)
     if fuse_ln and quant in ("mixed", "dense"):
         stats["layernorms_emitting_int8"] = fuse_layernorm_quant(unet)
     stats["groupnorms_nhwc_kernel"] = sum(1 for m in unet.modules() if getattr(m, "fused", False) is True)

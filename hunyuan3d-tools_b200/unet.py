@@ -34,6 +34,59 @@ def timestep_embedding(t: torch.Tensor, dim: int) -> torch.Tensor:
     return torch.cat([torch.cos(args), torch.sin(args)], dim=-1)
 
 
+# -----------------------------------------------------------------------------------------
+# Steps between the layers.  torch adds a convolution's bias, a residual, a concatenation or an upsampling in
+# passes of their own; where a model runs channels_last f16 / bf16 on the GPU without autograd, the extension
+# does several of them in one pass, with the roundings the separate ops would have made.  Its functions answer
+# None for anything else, and the torch ops run.
+# -----------------------------------------------------------------------------------------
+def _native():
+    return None if torch.is_grad_enabled() else _qu._NATIVE
+
+
+def _leaves_bias(native, *convs):
+    """Whether these convolutions may be run without their bias, which is added later."""
+    return all(type(c) is nn.Conv2d and c.padding_mode == "zeros" for c in convs) and native.unhooked(*convs)
+
+
+def _conv_without_bias(conv, x):
+    return torch.conv2d(x, conv._parameters["weight"], None, conv.stride, conv.padding, conv.dilation, conv.groups)
+
+
+def _conv_bias(conv):
+    return conv._parameters["bias"]
+
+
+def _add_bias(native, x, bias_x, h=None, bias_h=None):
+    """(x + bias_x) + (h + bias_h), each sum rounded; any of the last three may be None."""
+    y = native.add_bias(x, bias_x, h, bias_h)
+    if y is not None:
+        return y
+    if bias_x is not None:
+        x = x + bias_x[:, None, None]
+    if h is None:
+        return x
+    return x + (h if bias_h is None else h + bias_h[:, None, None])
+
+
+def _conv(conv, x):
+    native = _native()
+    if native is not None and conv.bias is not None and _leaves_bias(native, conv):
+        return _add_bias(native, _conv_without_bias(conv, x), _conv_bias(conv))
+    return conv(x)
+
+
+def _residual_norm(norm, x, h):
+    """x + h and its normalisation."""
+    native = _native()
+    if native is not None:
+        got = native.norm_call(norm, x, h)
+        if got is not None:
+            return got
+    x = x + h
+    return x, norm(x)
+
+
 class GroupNormNHWC(nn.GroupNorm):
     """``nn.GroupNorm`` (optionally followed by SiLU) that, once ``fused`` is set, runs the
     library's channels-last kernel on channels_last CUDA f16/bf16 inputs: torch's own kernel
@@ -51,7 +104,7 @@ class GroupNormNHWC(nn.GroupNorm):
     def __call__(self, x, add=None):
         # The direct way to the kernel where no hook, subclass or tracer stands in it.
         if _qu._NATIVE is not None:
-            y = _qu._NATIVE.groupnorm_call(self, x, add)
+            y = _qu._NATIVE.groupnorm_call(self, x, add, None)
             if y is not None:
                 return y
         return super().__call__(x) if add is None else super().__call__(x, add)
@@ -91,10 +144,35 @@ class ResnetBlock(nn.Module):
         self.conv2 = nn.Conv2d(cout, cout, 3, padding=1)
         self.conv_shortcut = nn.Conv2d(cin, cout, 1) if cin != cout else None
 
-    def forward(self, x, temb):
+    # (stacked projection of all blocks, first column, last column + 1), set by fuse_time_projections
+    _time_slice = None
+
+    def _term(self, temb):
+        act = F.silu(temb)
+        if self._time_slice is None:
+            return self.time_emb_proj(act)
+        layer, lo, hi = self._time_slice
+        return layer(act)[:, lo:hi]
+
+    def forward(self, x, temb, term=None):
+        """``term``: this block's projection of the time embedding, where the caller has it already."""
+        if term is None:
+            term = self._term(temb)
+        convs = (self.conv1, self.conv2) if self.conv_shortcut is None else (self.conv1, self.conv2, self.conv_shortcut)
+        native = _native() if self.norm2.fused else None
+        if native is not None and _leaves_bias(native, *convs):
+            h = _conv_without_bias(convs[0], self.norm1(x))
+            b1 = _conv_bias(convs[0])
+            # h + bias + time embedding feeds norm2 only, so both terms ride in the normalisation
+            g = native.groupnorm_call(self.norm2, h, term, b1)
+            h = self.norm2(_add_bias(native, h, b1), term) if g is None else g
+            h = _conv_without_bias(convs[1], h)
+            if len(convs) == 2:
+                return _add_bias(native, x, None, h, _conv_bias(convs[1]))
+            return _add_bias(native, _conv_without_bias(convs[2], x), _conv_bias(convs[2]), h, _conv_bias(convs[1]))
         h = self.conv1(self.norm1(x))              # GroupNorm + SiLU
         # h + time embedding feeds norm2 only, so the broadcast add rides in the normalisation
-        h = self.conv2(self.norm2(h, add=self.time_emb_proj(F.silu(temb))))
+        h = self.conv2(self.norm2(h, add=term))
         if self.conv_shortcut is not None:
             x = self.conv_shortcut(x)
         return x + h
@@ -116,7 +194,11 @@ class Attention(nn.Module):
         self.to_kv = None
         self.is_self = context_dim is None
 
-    def forward(self, x, context=None):
+    # (stacked k / v projections of all blocks, first column, last column + 1), set by fuse_context_projections
+    _kv_slice = None
+
+    def forward(self, x, context=None, kv=None):
+        """``kv``: keys and values of the context side by side, where the caller has them already."""
         b, n, c = x.shape
         if self.to_qkv is not None:           # self-attention with the three projections stacked
             q, k, v = self.to_qkv(x).split(c, dim=-1)
@@ -125,7 +207,12 @@ class Attention(nn.Module):
             context = x if context is None else context
             m = context.shape[1]
             q = self.to_q(x)
-            if self.to_kv is not None:
+            if kv is None and self._kv_slice is not None:
+                layer, lo, hi = self._kv_slice
+                kv = layer(context)[..., lo:hi]
+            if kv is not None:
+                k, v = kv.split(c, dim=-1)
+            elif self.to_kv is not None:
                 k, v = self.to_kv(context).split(c, dim=-1)
             else:
                 k, v = self.to_k(context), self.to_v(context)
@@ -166,14 +253,20 @@ class TransformerBlock(nn.Module):
         self.norm3 = nn.LayerNorm(dim)
         self.ff = GEGLUFeedForward(dim)
 
-    def forward(self, x, context):
-        x = x + self.attn1(self.norm1(x))
+    def parts(self, x, context, kv=None):
+        """The block's output as the two terms of its last residual sum."""
+        h = self.attn1(self.norm1(x))
         if self.num_views > 1:
             b, n, c = x.shape
-            xv = self.norm_mv(x).view(b // self.num_views, self.num_views * n, c)
-            x = x + self.attn_mv(xv).view(b, n, c)
-        x = x + self.attn2(self.norm2(x), context)
-        return x + self.ff(self.norm3(x))
+            x, y = _residual_norm(self.norm_mv, x, h)
+            h = self.attn_mv(y.view(b // self.num_views, self.num_views * n, c)).view(b, n, c)
+        x, y = _residual_norm(self.norm2, x, h)
+        x, y = _residual_norm(self.norm3, x, self.attn2(y, context) if kv is None else self.attn2(y, context, kv))
+        return x, self.ff(y)
+
+    def forward(self, x, context, kv=None):
+        x, h = self.parts(x, context, kv)
+        return x + h
 
 
 class SpatialTransformer(nn.Module):
@@ -184,10 +277,18 @@ class SpatialTransformer(nn.Module):
         self.block = TransformerBlock(dim, heads, context_dim, num_views)
         self.proj_out = nn.Linear(dim, dim)
 
-    def forward(self, x, context):
+    def forward(self, x, context, kv=None):
         b, c, h, w = x.shape
-        y = self.norm(x).permute(0, 2, 3, 1).reshape(b, h * w, c)
-        y = self.proj_out(self.block(self.proj_in(y), context))
+        y = self.proj_in(self.norm(x).permute(0, 2, 3, 1).reshape(b, h * w, c))
+        native = _native()
+        if (native is not None and type(self.block) is TransformerBlock and isinstance(self.proj_out, _qu.Int8Linear)
+                and native.unhooked(self.block)):
+            # the block's last sum feeds proj_out only: it is quantised as it is added, and not stored
+            y, z = self.block.parts(y, context, kv)
+            q = native.add_quantize(y, z)
+            y = self.proj_out(y + z if q is None else q)
+        else:
+            y = self.proj_out(self.block(y, context) if kv is None else self.block(y, context, kv))
         return x + y.view(b, h, w, c).permute(0, 3, 1, 2)
 
 
@@ -197,7 +298,7 @@ class Downsample(nn.Module):
         self.conv = nn.Conv2d(c, c, 3, stride=2, padding=1)
 
     def forward(self, x):
-        return self.conv(x)
+        return _conv(self.conv, x)
 
 
 class Upsample(nn.Module):
@@ -206,7 +307,9 @@ class Upsample(nn.Module):
         self.conv = nn.Conv2d(c, c, 3, padding=1)
 
     def forward(self, x):
-        return self.conv(F.interpolate(x, scale_factor=2.0, mode="nearest"))
+        native = _native()
+        y = native.upsample2x_nhwc(x) if native is not None else None
+        return _conv(self.conv, F.interpolate(x, scale_factor=2.0, mode="nearest") if y is None else y)
 
 
 class UNetSD21MV(nn.Module):
@@ -262,6 +365,17 @@ class UNetSD21MV(nn.Module):
         # NHWC activations: the convolutions run without layout conversions and the token
         # view (B, H*W, C) the transformer blocks take is free.  Set by use_channels_last().
         self.channels_last = False
+        # Projections of the time embedding / of the context for all blocks at once, in forward order; set by
+        # fuse_time_projections / fuse_context_projections.
+        self.time_proj_all = None
+        self.context_proj_all = None
+
+    def _resnets(self):
+        return ([l["res"] for l in self.down if "res" in l] + [self.mid_res1, self.mid_res2]
+                + [l["res"] for l in self.up])
+
+    def _transformers(self):
+        return ([l["attn"] for l in self.down if "attn" in l] + [self.mid_attn] + [l["attn"] for l in self.up if "attn" in l])
 
     def use_channels_last(self) -> "UNetSD21MV":
         self.to(memory_format=torch.channels_last)
@@ -283,24 +397,40 @@ class UNetSD21MV(nn.Module):
         temb = self.time_embedding(timestep_embedding(t, self.time_proj_dim).to(x.dtype))
         if self.channels_last:
             x = x.contiguous(memory_format=torch.channels_last)
-        h = self.conv_in(x)
+        terms = kvs = None
+        if self.time_proj_all is not None:
+            terms = iter(self.time_proj_all(F.silu(temb)).split([m.conv1.out_channels for m in self._resnets()], dim=-1))
+        if self.context_proj_all is not None:
+            kvs = iter(self.context_proj_all(context).split([2 * m.proj_in.out_features for m in self._transformers()], dim=-1))
+
+        def res(m, h):
+            return m(h, temb) if terms is None else m(h, temb, next(terms))
+
+        def attn(m, h):
+            return m(h, context) if kvs is None else m(h, context, next(kvs))
+
+        native = _native()
+        h = _conv(self.conv_in, x)
         skips = [h]
         for layer in self.down:
             if "down" in layer:
                 h = layer["down"](h)
             else:
-                h = layer["res"](h, temb)
+                h = res(layer["res"], h)
                 if "attn" in layer:
-                    h = layer["attn"](h, context)
+                    h = attn(layer["attn"], h)
             skips.append(h)
-        h = self.mid_res2(self.mid_attn(self.mid_res1(h, temb), context), temb)
+        h = res(self.mid_res1, h)
+        h = res(self.mid_res2, attn(self.mid_attn, h))
         for layer in self.up:
-            h = layer["res"](torch.cat([h, skips.pop()], dim=1), temb)
+            skip = skips.pop()
+            y = native.concat_nhwc(h, skip) if native is not None else None
+            h = res(layer["res"], torch.cat([h, skip], dim=1) if y is None else y)
             if "attn" in layer:
-                h = layer["attn"](h, context)
+                h = attn(layer["attn"], h)
             if "up" in layer:
                 h = layer["up"](h)
-        return self.conv_out(self.norm_out(h)).contiguous()
+        return _conv(self.conv_out, self.norm_out(h)).contiguous()
 
 
 def fuse_geglu_layers(model: nn.Module) -> int:
@@ -362,6 +492,47 @@ def fuse_qkv_layers(model: nn.Module) -> int:
             m.to_kv, m.to_k, m.to_v = fused, None, None
         removed += len(group) - 1
     return removed
+
+
+def _stack(layers):
+    """One layer of all of them, or None where they cannot be stacked."""
+    from .quantize_utils import Int8Linear
+    if not layers or not all(type(l) is Int8Linear and l.epilogue == "linear" for l in layers):
+        return None
+    try:
+        return Int8Linear.concat(layers)
+    except RuntimeError:        # of different modes, types or inputs
+        return None
+
+
+def fuse_time_projections(model: "UNetSD21MV") -> int:
+    """Stacks the ResNet blocks' projections of the time embedding: one SiLU and one GEMM per forward in place of
+    one per block; every output column keeps its bits.  Returns the number of layers removed."""
+    blocks = model._resnets()
+    layer = _stack([m.time_emb_proj for m in blocks])
+    if layer is None:
+        return 0
+    model.time_proj_all, at = layer, 0
+    for m in blocks:
+        m._time_slice = (layer, at, at + m.time_emb_proj.out_features)
+        at = m._time_slice[2]
+        m.time_emb_proj = None
+    return len(blocks) - 1
+
+
+def fuse_context_projections(model: "UNetSD21MV") -> int:
+    """Stacks the cross-attentions' k / v projections, which all read the context: it is quantised once and one
+    GEMM runs per forward.  Run after ``fuse_qkv_layers``.  Returns the number of layers removed."""
+    attns = [m.block.attn2 for m in model._transformers()]
+    layer = _stack([m.to_kv for m in attns])
+    if layer is None:
+        return 0
+    model.context_proj_all, at = layer, 0
+    for m in attns:
+        m._kv_slice = (layer, at, at + m.to_kv.out_features)
+        at = m._kv_slice[2]
+        m.to_kv = None
+    return len(attns) - 1
 
 
 # -----------------------------------------------------------------------------------------

@@ -102,7 +102,7 @@ int hy3d_layernorm_quantize(const void* x, int x_dtype, int64_t M, int64_t K, in
  * order).  y = x * (rstd * gamma[c]) + (beta[c] - mean * rstd * gamma[c]) rounded to x_dtype;
  * with silu != 0 the rounded value v becomes v / (1 + exp(-v)), rounded again.  gamma / beta:
  * (C) of gb_dtype or NULL.  workspace: hy3d_groupnorm_workspace_floats(B, HW, groups) floats of
- * device memory owned by the caller (per-chunk partial sums; no initialisation needed).
+ * device memory owned by the caller (not used any more; may be NULL).
  * add: optional (B, C) array of x_dtype added to every pixel of its sample before the
  * normalisation -- x + add[b, c] rounded to x_dtype, as a separate broadcast add would store it
  * (a UNet's time-embedding term) -- or NULL.
@@ -115,6 +115,38 @@ int hy3d_groupnorm_nhwc(const void* x, const void* add, int x_dtype, int64_t B, 
                         int groups, const void* gamma, const void* beta, int gb_dtype, float eps,
                         int silu, void* y, float* workspace, void* stream);
 int64_t hy3d_groupnorm_workspace_floats(int64_t B, int64_t HW, int groups);
+
+/*
+ * The same with another optional term: `bias` (C), of x_dtype, is added to every pixel before `add`, rounded as
+ * a separate pass would have stored it (the bias of the convolution that produced x).  add: rows of C values
+ * add_ld apart (a multiple of 8).  bias needs add.  No workspace.
+ */
+int hy3d_groupnorm_nhwc_terms(const void* x, const void* bias, const void* add, int64_t add_ld, int x_dtype, int64_t B,
+                              int64_t HW, int64_t C, int groups, const void* gamma, const void* beta, int gb_dtype,
+                              float eps, int silu, void* y, void* stream);
+
+/*
+ * Channels-last element-wise steps of the model around the layers, `rows` pixels of C channels (C % 8 == 0,
+ * 16-byte aligned pointers), f16 / bf16, with the roundings of the separate operations they stand for:
+ *   hy3d_add_bias_nhwc     y = round(round(x + bias_x) + round(h + bias_h)); bias_x, h, bias_h may be NULL
+ *   hy3d_concat_nhwc       y = [a | b] along the channels
+ *   hy3d_upsample2x_nhwc   nearest neighbour, (B,H,W,C) -> (B,2H,2W,C)
+ * y may equal x or h in the first.
+ */
+int hy3d_add_bias_nhwc(const void* x, const void* bias_x, const void* h, const void* bias_h, int dtype, void* y,
+                       int64_t rows, int64_t C, void* stream);
+int hy3d_concat_nhwc(const void* a, int64_t Ca, const void* b, int64_t Cb, void* y, int64_t rows, void* stream);
+int hy3d_upsample2x_nhwc(const void* x, void* y, int64_t B, int64_t H, int64_t W, int64_t C, void* stream);
+
+/*
+ * Residual forms of the quantisers, on rows x + add rounded to x_dtype (both (M,K), contiguous): the plain one
+ * does not store the sum, the LayerNorm one stores it in `sum` (x's shape and type).
+ */
+int hy3d_add_quantize_rows(const void* x, const void* add, int x_dtype, int64_t M, int64_t K, int8_t* q, float* scale,
+                           void* stream);
+int hy3d_add_layernorm_quantize(const void* x, const void* add, void* sum, int x_dtype, int64_t M, int64_t K,
+                                const void* gamma, const void* beta, int gb_dtype, float eps, int8_t* q, float* scale,
+                                void* stream);
 
 /*
  * Self-check of the quantiser's rounding (test hook, no reference counterpart).  The kernel

@@ -599,3 +599,54 @@ def test_bf16_gate_rounds_as_the_erf_form(tc, sp, sparse, M, K, N):
     value, gate = v[:, :, 0].reshape(M, -1), v[:, :, 1].reshape(M, -1)
     ref = (value * (0.5 * gate * (1.0 + torch.erf(gate * 0.70710678118654752440)))).bfloat16()
     assert torch.equal(y, ref)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", [(1, 8, 1, 1), (2, 24, 5, 7), (3, 320, 9, 16), (1, 2560, 4, 3), (2, 1032, 33, 17)])
+def test_nhwc_steps_equal_the_separate_torch_ops(qu, dtype, shape):
+    """Bias / residual sums, concatenation, upsampling and the normalisation's pre-added terms against torch's
+    separate ops, bit for bit (values over many binades, so that small addends round away and ties occur)."""
+    nat = qu._load_native()
+    B, C, H, W = shape
+    g = torch.Generator(device=DEV).manual_seed(C + H)
+
+    def rand(*s):
+        return (torch.randn(*s, generator=g, device=DEV) * torch.exp2(torch.randint(-12, 6, s, generator=g, device=DEV).float())).to(dtype)
+    cl = torch.channels_last
+    x, h = rand(*shape).contiguous(memory_format=cl), rand(*shape).contiguous(memory_format=cl)
+    bx, bh = rand(C), rand(C)
+    col = lambda b: b[:, None, None]   # noqa: E731
+    assert torch.equal(nat.add_bias(x, bx, None, None), x + col(bx))
+    assert torch.equal(nat.add_bias(x, None, h, bh), x + (h + col(bh)))
+    assert torch.equal(nat.add_bias(x, bx, h, bh), (x + col(bx)) + (h + col(bh)))
+    other = rand(B, 16, H, W).contiguous(memory_format=cl)
+    y = nat.concat_nhwc(x, other)
+    assert torch.equal(y, torch.cat([x, other], 1)) and y.is_contiguous(memory_format=cl)
+    y = nat.upsample2x_nhwc(x)
+    assert torch.equal(y, torch.nn.functional.interpolate(x, scale_factor=2.0, mode="nearest")) and y.is_contiguous(memory_format=cl)
+    assert nat.add_bias(x.contiguous(memory_format=cl).float(), bx, None, None) is None
+    # the normalisation with a bias and a strided (B, C) term equals normalising the sum made beforehand
+    groups = 8 if C % 64 == 0 else 1
+    terms = rand(B, C + 24)[:, 8:8 + C]
+    norm = __import__("importlib").import_module("hunyuan3d-tools_b200.unet").GroupNormNHWC(groups, C).to(DEV).to(dtype)
+    norm.requires_grad_(False).fused = True
+    x1 = ((x + col(bx)) + terms[:, :, None, None]).contiguous(memory_format=cl)
+    assert torch.equal(nat.groupnorm_call(norm, x, terms, bx), norm(x1))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K", [(1, 64), (33, 320), (257, 640), (1000, 1088), (5, 1280), (300, 2048), (70, 5120)])
+def test_residual_quantisers_equal_adding_first(qu, ik, dtype, M, K):
+    nat = qu._load_native()
+    g = torch.Generator(device=DEV).manual_seed(M + K)
+    x, h = (torch.randn(M, K, generator=g, device=DEV).to(dtype) for _ in range(2))
+    q, s = ik.fused_quantize_activation(x + h)
+    got = nat.add_quantize(x, h)
+    assert torch.equal(got.q, q) and torch.equal(got.scale, s) and got.shape == x.shape and got.dtype == dtype
+    if K <= 2048:
+        ln = torch.nn.LayerNorm(K, device=DEV, dtype=dtype)
+        ln.weight.data.copy_(1 + 0.2 * torch.randn(K, generator=g, device=DEV))
+        norm = qu.Int8LayerNorm(ln)
+        total, z = nat.norm_call(norm, x, h)
+        ref = norm(x + h)
+        assert torch.equal(total, x + h) and torch.equal(z.q, ref.q) and torch.equal(z.scale, ref.scale)
