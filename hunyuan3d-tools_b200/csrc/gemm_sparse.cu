@@ -471,37 +471,42 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
        reinterpret_cast<uintptr_t>(w_meta) | reinterpret_cast<uintptr_t>(out)) & 15)
     return HY3D_ERR_SHAPE;
 
-  if (block_t == 0) {
-    // Token-tile width that minimises rounds x time per tile: rounds = ceil(tiles / SMs), a
-    // tile costs its width plus a fixed overhead worth ~94 columns of MMA time (the same
-    // model as the dense kernel; measured on B200 the widest tile wins whenever the grid is
-    // full, the narrowest when the whole problem is a single round).
-    const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
-    const int64_t w_tiles = (N + kTileW - 1) / kTileW;
-    int64_t best = -1;
-    for (int bt = 224; bt >= 128; bt -= 32) {
-      const int64_t tiles = w_tiles * ((M + bt - 1) / bt);
-      const int64_t cost = ((tiles + sms - 1) / sms) * (bt + 94);
-      if (best < 0 || cost < best) { best = cost; block_t = bt; }
-    }
-    if (M < block_t) block_t = static_cast<int>((M + 31) / 32 * 32);
-  }
-  if (block_t < 16 || block_t > kMaxBlockT || (block_t & 15)) return HY3D_ERR_SHAPE;
-
-  // CTA pairs (256 weight rows sharing one token tile) halve each CTA's activation traffic
-  // into shared memory, which is what paces deep-K stages (measured: 8192^3 384 -> 273 us,
-  // M=3072 K=5120 N=1280 21.3 -> 15.7 us); on short K the per-tile hand-offs of a pair cost
-  // more than that saves, and a weight matrix that fills its last 256-row tile badly (N = 320)
-  // wastes the second CTA; launch-bound problems (M = 924) are faster with single CTAs.
+  // Tile shape.  CTA pairs (256 weight rows sharing one token tile) halve each CTA's activation traffic into
+  // shared memory, which is what paces deep-K stages, and cost more per tile hand-off; a wide token tile
+  // amortises the weights, a narrow one spreads few tokens over the chip.  Both come from one cost model, in
+  // microseconds, fitted to 98 shapes x all tiles (7 % rms; the tile it picks is 1 % from the best on average,
+  // where a fixed threshold for pairs and tiles of 128 tokens or more were 10 %):
+  //   2335 x 4864 -> 688: 12.3 -> 10.6 us, 3451 x 3328 -> 640: 15.1 -> 8.7, 279 x 704 -> 1120: 4.8 -> 4.0
   int group = 1;
   {
-    const int64_t padded = ((N + 2 * kTileW - 1) / (2 * kTileW)) * (2 * kTileW);
-    if (K >= 1024 && M >= 2048 && (block_t & 31) == 0 && padded * 4 <= N * 5) group = 2;
+    const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
+    double best = 1e30;
+    int best_t = 0;
+    for (int g = 1; g <= (K >= 1024 ? 2 : 1); ++g) {
+      for (int bt = 32; bt <= 224; bt += 32) {
+        if (block_t != 0 && bt != 32) break;             // the caller's width, one pass per group
+        const int t = block_t != 0 ? block_t : bt;
+        if (t < 16 || t > kMaxBlockT || (t & 15) || (g == 2 && (t & 31))) continue;
+        if (block_t == 0 && bt > 32 && bt >= M + 32) break;
+        if (block_t == 0 && bt == 32 && M > 1024) continue;      // one store per 32 tokens and 32 columns
+        const double tiles = static_cast<double>((N + kTileW * g - 1) / (kTileW * g)) * static_cast<double>((M + t - 1) / t);
+        const double rounds = static_cast<double>((static_cast<int64_t>(tiles) + sms / g - 1) / (sms / g));
+        const double w = t / 100.0;
+        double stage = g == 1 ? 0.196 + 0.130 * w : 0.327 + 0.036 * w;
+        const double floor_us = g == 1 ? 0.273 : 0.351;
+        if (stage < floor_us) stage = floor_us;
+        const double operand_mb = tiles * g * static_cast<double>(kblocks) * (kABytes + kEBytes + 256.0 * t / g) / 1e7;
+        const double us = 3.0 + rounds * (static_cast<double>(kblocks) * stage + 0.08 + 0.55 * w) + 0.096 * operand_mb + (g == 2 ? 0.61 : 0.0);
+        if (us < best) { best = us; best_t = t; group = g; }
+      }
+    }
+    block_t = best_t;
 #ifdef HY3D_TRACE
     if (const char* e = getenv("HY3D_SPARSE_CTA_GROUP")) group = atoi(e) == 2 ? 2 : 1;
 #endif
-    if (group == 2 && (block_t & 31)) group = 1;
   }
+  if (block_t < 16 || block_t > kMaxBlockT || (block_t & 15)) return HY3D_ERR_SHAPE;
+  if (group == 2 && (block_t & 31)) group = 1;
 
   SparseArgs p;
   p.act_scale = act_scale; p.w_scale = w_scale; p.bias = bias; p.out = out;
