@@ -820,30 +820,98 @@ splitk_reduce_kernel(const int32_t* __restrict__ partial, int splits, int64_t sp
   }
 }
 
+struct TilePlan {
+  int block_n = 0, group = 0;
+  double us = 0.0;
+};
+
+// Tile width and CTA grouping for a launch of `splits` K ranges, with its expected device time.  Pairs halve the
+// B traffic into shared memory, which is what bounds the tensor pipe on deep K, and cost more per hand-off; wide
+// tiles re-read A less often, narrow ones spread few tiles over the chip.  All of it from one cost model, in
+// microseconds: rounds of the persistent grid x (K blocks x the slower of issue and operand fill + the tile's
+// epilogue) + operand traffic through L2 + a fixed part.  Fitted to 210 shapes x all tiles (6 % rms); the tile it
+// picks is 0.5 % from the best on average (4 % with the rule before it: tiles of 128 to 256 columns by rounds x
+// (width + 94), pairs by thresholds on K and the tile count): 7215 x 4800 -> 816 30.7 -> 25.5 us,
+// 902 x 2816 -> 4480 13.4 -> 11.4, 348 x 896 -> 912 5.2 -> 4.6.
+TilePlan search_tile(int64_t M, int64_t N, int64_t K, bool geglu, int cta_group, int block_n, int splits) {
+  TilePlan best;
+  best.us = 1e30;
+  const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
+  const int step = geglu ? 64 : 32;
+  const int64_t nk = ((K + kBlockKBytes - 1) / kBlockKBytes + splits - 1) / splits;
+  for (int g = 1; g <= 2; ++g) {
+    if (cta_group != 0 ? g != cta_group : (g == 2 && (K < 1024 || splits > 1))) continue;
+    for (int bn = 64; bn <= 256; bn += step) {
+      const int w = block_n != 0 ? block_n : N <= 128 ? static_cast<int>(N) : bn;
+      if (w != bn && bn != 64) break;                    // a width that is given: once per group
+      if (w == bn && bn >= N + 32 && bn > 64) break;
+      if (g == 2 && (w & 31) && cta_group == 0) continue;
+      const int64_t nt = (N + w - 1) / w;
+      const int64_t tiles = ((M + kTileM * g - 1) / (kTileM * g)) * nt * splits;
+      int64_t slots = sms / g;
+      if (nt > 1 && nt <= slots / 4) slots -= slots % nt;     // every CTA keeps one tile column, see the launch
+      const double rounds = static_cast<double>((tiles + slots - 1) / slots);
+      const bool resident = g == 1 && splits == 1 && nt <= sms / 4 && tiles >= 2 * slots &&
+                            nk * w * kBlockKBytes + 4 * kTileM * kBlockKBytes + 33000 <= kSmemLimit;
+      const double c = w / 100.0;
+      double block = g == 2 ? 0.148 + 0.031 * c : resident ? 0.050 + 0.030 * c : 0.072 + 0.070 * c;
+      const double least = g == 2 ? 0.019 : resident ? 0.220 : 0.207;
+      if (block < least) block = least;
+      const double operand = tiles * g * static_cast<double>(nk) * kBlockKBytes * (kTileM + (resident ? 0.0 : static_cast<double>(w) / g)) / 1e7;
+      const double us = 3.09 + rounds * (static_cast<double>(nk) * block + 0.124 + 0.423 * c) + 0.078 * operand + (g == 2 ? 1.19 : 0.0);
+      if (us < best.us) { best.us = us; best.block_n = w; best.group = g; }
+    }
+  }
+  return best;
+}
+
+// Sizes recur in every step of a model, so each thread keeps its last few answers (a search takes ~0.3 us, a
+// split-K plan fifteen of them).
+template <typename Value>
+struct Memo {
+  struct Entry { int64_t M, N, K, rest; Value value; } entries[64] = {};
+  template <typename Search>
+  Value get(int64_t M, int64_t N, int64_t K, int64_t rest, Search search) {
+    Entry& e = entries[(static_cast<uint64_t>(M) * 31 + static_cast<uint64_t>(N) * 7 + static_cast<uint64_t>(K >> 4) * 3 +
+                        static_cast<uint64_t>(rest) * 5) & 63];
+    if (e.M != M || e.N != N || e.K != K || e.rest != rest) e = {M, N, K, rest, search()};
+    return e.value;
+  }
+};
+
+TilePlan plan_tile(int64_t M, int64_t N, int64_t K, bool geglu, int cta_group, int block_n, int splits) {
+  static thread_local Memo<TilePlan> memo;
+  const int64_t rest = (geglu ? 1 : 0) | cta_group << 1 | block_n << 3 | static_cast<int64_t>(splits) << 12;
+  return memo.get(M, N, K, rest, [&] { return search_tile(M, N, K, geglu, cta_group, block_n, splits); });
+}
+
+int search_splits(int64_t M, int64_t N, int64_t K) {
+  const int64_t num_kb = (K + kBlockKBytes - 1) / kBlockKBytes;
+  const int64_t part_rows = (M + kTileM - 1) / kTileM * kTileM;
+  const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
+  if (num_kb < 16 || part_rows / kTileM * ((N + 255) / 256) * 2 > sms) return 1;
+  // Every range writes and re-reads an M-padded int32 matrix at ~8 TB/s (it stays in L2) and is one more stream for
+  // the second launch, which costs ~1.2 us: fitted to 67 (shape, split) pairs, 0.8 us rms, 1 % from the best split
+  // on average.  132 x 4160 -> 1200 9.9 -> 8.2 us, 900 x 5120 -> 640 11.8 -> 10.6, 200 x 5952 -> 2992 13.4 -> 11.5.
+  const double part_us = static_cast<double>(part_rows) * N * 4.0 * 2.0 / 8.3e6 + 0.2;
+  double best = search_tile(M, N, K, false, 0, 0, 1).us * 0.95;
+  int best_s = 1;
+  for (int sp = 2; sp <= 16 && static_cast<int64_t>(sp) * 4 <= num_kb; ++sp) {
+    const double t = search_tile(M, N, K, false, 1, 0, sp).us + sp * part_us + 1.2;
+    if (t < best) { best = t; best_s = sp; }
+  }
+  return best_s;
+}
+
 }  // namespace
 
 // Split-K plan for a dense layer: how many K ranges pay (1 = none).  Splitting serves launches
 // whose tiles leave most SMs idle while each tile walks a long K alone (the M = 257 image-encoder
 // layers with K = 6144): the ranges run side by side and a second small kernel adds them up.
 int dense_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue) {
-  if (epilogue == HY3D_EPI_GEGLU || (N & 7) || M <= 0) return 1;
-  const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
-  const int64_t bn = N <= 128 ? N : 256;
-  const int64_t tiles = ((M + kTileM - 1) / kTileM) * ((N + bn - 1) / bn);
-  const int64_t num_kb = (K + kBlockKBytes - 1) / kBlockKBytes;
-  if (tiles * 2 > sms || num_kb < 16) return 1;
-  // Measured cost model (microseconds): a tile walks its K blocks at ~0.27 us each; every range
-  // writes and re-reads an M-padded int32 matrix at ~5 TB/s; two launches cost ~6 us of fixed
-  // time against ~3.5 us for one.  The split has to win by a tenth to be taken.
-  const double part_us = static_cast<double>((M + kTileM - 1) / kTileM * kTileM) * N * 4.0 * 2.0 / 5.0e6;
-  const double single = num_kb * 0.27 + 3.5;
-  double best = single * 0.9;
-  int best_s = 1;
-  for (int64_t sp = 2; sp <= 16 && sp * tiles <= sms && sp * 4 <= num_kb; ++sp) {
-    const double t = ((num_kb + sp - 1) / sp) * 0.27 + sp * part_us + 6.0;
-    if (t < best) { best = t; best_s = static_cast<int>(sp); }
-  }
-  return best_s;
+  if (epilogue == HY3D_EPI_GEGLU || (N & 7) || M <= 0 || N <= 0 || K <= 0) return 1;
+  static thread_local Memo<int> memo;
+  return memo.get(M, N, K, 0, [&] { return search_splits(M, N, K); });
 }
 
 int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const void* w_scale,
@@ -874,48 +942,18 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
        reinterpret_cast<uintptr_t>(out)) & 15)
     return HY3D_ERR_SHAPE;
 
-  if (block_n == 0) {
-    if (N <= 128) {
-      block_n = static_cast<int>(N);
-    } else {
-      // Tile width (a multiple of the TMA-store slab) that minimises rounds x time per tile,
-      // where rounds = ceil(tiles / SMs) and a tile costs its width plus a fixed per-stage
-      // overhead worth ~94 columns of MMA time (measured).  A last tile that sticks out of N
-      // is zero-filled on load and clipped on store.
-      const int sms = device_sm_count();
-      const int64_t m_tiles = (M + kTileM - 1) / kTileM;
-      const int step = geglu ? 64 : 32;
-      int64_t best = -1;
-      const int nsm = sms > 0 ? sms : 148;
-      for (int bn = 256; bn >= 128; bn -= step) {
-        const int64_t n_tiles = (N + bn - 1) / bn;
-        const int64_t tiles = m_tiles * n_tiles;
-        // The grid is rounded down to a multiple of the column count (see the launch below).
-        const int64_t grid = n_tiles <= nsm / 4 ? nsm - nsm % n_tiles : nsm;
-        const int64_t rounds = (tiles + grid - 1) / grid;
-        const int64_t cost = rounds * (bn + 94);
-        if (best < 0 || cost < best) { best = cost; block_n = bn; }
-      }
-    }
-  }
-  if (block_n < 16 || block_n > 256 || (block_n & 15) || (geglu && (block_n & 31)))
-    return HY3D_ERR_SHAPE;
-
-  // CTA pairs need an even split of the B tile into two multiples of 16 rows.
   int group = cta_group;
-  if (group == 0) {
-    // CTA pairs halve the B traffic into shared memory, which is what bounds the tensor pipe
-    // on deep-K problems (measured: 8192^3 2768 vs 2332 TOPS); with K >= 2048 they pay off
-    // as soon as most SM pairs have a tile, with K >= 1024 once the grid holds several rounds
-    // of 256-row tile pairs; on shorter K the per-tile hand-offs of a pair cost more.
-    const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
-    const int64_t pair_tiles = ((M + 2 * kTileM - 1) / (2 * kTileM)) * ((N + block_n - 1) / block_n);
-    const int64_t min_pair_tiles = K >= 2048 ? (sms / 2) * 4 / 5 : 4 * (sms / 2);
-    group = (K >= 1024 && (block_n & 31) == 0 && pair_tiles >= min_pair_tiles) ? 2 : 1;
+  if (block_n == 0 || group == 0) {
+    const TilePlan t = plan_tile(M, N, K, geglu, cta_group, block_n, splits);
+    block_n = t.block_n;
+    group = t.group;
 #ifdef HY3D_TRACE
     if (const char* e = getenv("HY3D_CTA_GROUP")) group = atoi(e) == 2 ? 2 : 1;
 #endif
   }
+  if (block_n < 16 || block_n > 256 || (block_n & 15) || (geglu && (block_n & 31)))
+    return HY3D_ERR_SHAPE;
+  // CTA pairs need an even split of the B tile into two multiples of 16 rows.
   if (group == 2 && (block_n & 31)) {
     if (cta_group == 2) return HY3D_ERR_SHAPE;
     group = 1;
