@@ -885,22 +885,42 @@ TilePlan plan_tile(int64_t M, int64_t N, int64_t K, bool geglu, int cta_group, i
   return memo.get(M, N, K, rest, [&] { return search_tile(M, N, K, geglu, cta_group, block_n, splits); });
 }
 
-int search_splits(int64_t M, int64_t N, int64_t K) {
+// What the calling thread spends on a layer of two launches (quantise, GEMM) and of three (and a reduction).
+constexpr double kTwoLaunchesUs = 7.5, kThreeLaunchesUs = 10.0;
+
+struct LayerPlan {
+  int splits = 1;
+  double us = 0.0;
+};
+
+// Split-K plan and expected time of a whole layer, quantisation included: the greater of the device's time and the
+// calling thread's.  A split pays one more launch, and every range writes and re-reads an M-padded int32 matrix
+// (~11 TB/s, it stays in L2).  Fitted to 130 layers of random size x all splits (0.6 us rms).
+//   257 x 6144 -> 1536 13.4 -> 11.0 us (GEMM), 132 x 4160 -> 1200 9.9 -> 8.2, 200 x 5952 -> 2992 13.4 -> 11.5
+LayerPlan search_layer(int64_t M, int64_t N, int64_t K) {
   const int64_t num_kb = (K + kBlockKBytes - 1) / kBlockKBytes;
   const int64_t part_rows = (M + kTileM - 1) / kTileM * kTileM;
   const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
-  if (num_kb < 16 || part_rows / kTileM * ((N + 255) / 256) * 2 > sms) return 1;
-  // Every range writes and re-reads an M-padded int32 matrix at ~8 TB/s (it stays in L2) and is one more stream for
-  // the second launch, which costs ~1.2 us: fitted to 67 (shape, split) pairs, 0.8 us rms, 1 % from the best split
-  // on average.  132 x 4160 -> 1200 9.9 -> 8.2 us, 900 x 5120 -> 640 11.8 -> 10.6, 200 x 5952 -> 2992 13.4 -> 11.5.
-  const double part_us = static_cast<double>(part_rows) * N * 4.0 * 2.0 / 8.3e6 + 0.2;
-  double best = search_tile(M, N, K, false, 0, 0, 1).us * 0.95;
-  int best_s = 1;
+  const double act = static_cast<double>(M) * K / 1e6, weights = static_cast<double>(N) * K / 1e7;
+  LayerPlan best;
+  best.us = 0.9 + search_tile(M, N, K, false, 0, 0, 1).us + 0.46 * act + 1.7 * weights;
+  if (best.us < kTwoLaunchesUs) best.us = kTwoLaunchesUs;
+  if (best.us <= kThreeLaunchesUs || num_kb < 16 || part_rows / kTileM * ((N + 255) / 256) * 2 > sms) return best;
+  const double part_us = 0.21 + 0.09 * static_cast<double>(part_rows) * N * 8.0 / 1e6;
+  const double single_us = best.us;
+  best.us *= 0.9;                                   // a split has to be worth its workspace
   for (int sp = 2; sp <= 16 && static_cast<int64_t>(sp) * 4 <= num_kb; ++sp) {
-    const double t = search_tile(M, N, K, false, 1, 0, sp).us + sp * part_us + 1.2;
-    if (t < best) { best = t; best_s = sp; }
+    double us = 2.8 + search_tile(M, N, K, false, 1, 0, sp).us + sp * part_us + 0.42 * act + weights;
+    if (us < kThreeLaunchesUs) us = kThreeLaunchesUs + 0.01 * us;
+    if (us < best.us) { best.us = us; best.splits = sp; }
   }
-  return best_s;
+  if (best.splits == 1) best.us = single_us;
+  return best;
+}
+
+LayerPlan plan_layer(int64_t M, int64_t N, int64_t K) {
+  static thread_local Memo<LayerPlan> memo;
+  return memo.get(M, N, K, 0, [&] { return search_layer(M, N, K); });
 }
 
 }  // namespace
@@ -910,9 +930,11 @@ int search_splits(int64_t M, int64_t N, int64_t K) {
 // layers with K = 6144): the ranges run side by side and a second small kernel adds them up.
 int dense_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue) {
   if (epilogue == HY3D_EPI_GEGLU || (N & 7) || M <= 0 || N <= 0 || K <= 0) return 1;
-  static thread_local Memo<int> memo;
-  return memo.get(M, N, K, 0, [&] { return search_splits(M, N, K); });
+  return plan_layer(M, N, K).splits;
 }
+
+// Expected time of a layer that quantises and multiplies in separate launches, in microseconds.
+double dense_layer_us(int64_t M, int64_t N, int64_t K) { return plan_layer(M, N, K).us; }
 
 int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const void* w_scale,
                int ws_dtype, const void* bias, int bias_dtype, void* out, int out_dtype, int64_t M,
@@ -1157,6 +1179,7 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
 }  // namespace dense
 
 using dense::gemm_dense;
+using dense::dense_layer_us;
 using dense::dense_splitk_plan;
 
 }  // namespace hy3d

@@ -19,6 +19,7 @@
 // The CTAs of a cluster wait for one another only at hardware cluster barriers; every mbarrier wait is
 // bounded as in the other kernels.
 #include "common.cuh"
+#include <atomic>
 #include <cstdlib>
 
 namespace hy3d {
@@ -445,9 +446,42 @@ double plan_us(const Plan& p, int64_t M, bool sparse) {
          (p.ks > 1 ? 1.5 + 0.41 * slabs : 0.0) + 0.23 * slabs;
 }
 
-// Up to here one launch is taken.  The two launches need 6-8 us on the device for such shapes but about
-// 9 us of the calling thread, which then is what a caller waits for; one launch saves 2.4 us of that.
-constexpr double kOneLaunchUs = 8.5;
+// What a caller sees of a plan beside dense_layer_us: fitted to 117 dense layers of random size.
+double plan_layer_us(const Plan& p, int64_t M, int64_t N, int64_t K) {
+  return 1.156 * plan_us(p, M, false) - 0.4 + 0.25 * static_cast<double>(N) * K / 1e7 + (p.ks > 1 ? 0.2 : 0.0);
+}
+
+// Clusters of `ks` CTAs that run at the same time, one CTA an SM: the GPCs have 16 to 20 SMs, and what is left
+// over in each stays idle.  A second wave doubles the time (253 x 1792 -> 224 in 16 clusters of 7: 14.3 us, two
+// launches 7.8).
+int resident_clusters(int ks, int sms) {
+  static std::atomic<int> known[kMaxRanks + 1];
+  int n = known[ks].load(std::memory_order_relaxed);
+  if (n == 0) {
+    const void* kernel = reinterpret_cast<const void*>(linear_cluster_kernel<false, false, HY3D_EPI_LINEAR>);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(ks) * 64);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmemLimit;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(ks);
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (ensure_max_smem(kernel, kSmemLimit) != HY3D_OK || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = sms * 3 / 4 / ks;
+    }
+    known[ks].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+// Sparse layers take one launch up to here.  The two launches need 6-8 us on the device for such shapes and about
+// as much of the calling thread, which then is what a caller waits for; one launch saves 2.4 us of that.
+constexpr double kSparseOneLaunchUs = 8.5;
 
 }  // namespace
 
@@ -460,16 +494,19 @@ bool linear_cluster_plan(int64_t M, int64_t N, int64_t K, bool sparse, int* bloc
   if (e.M != M || e.N != N || e.K != K || e.sparse != (sparse ? 1 : 0)) {
     e = {M, N, K, sparse ? 1 : 0, 0, 0};
     const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
-    double best = kOneLaunchUs;
+    // Dense layers take the one launch where it is expected to be the shorter one: below the host's time for two
+    // launches, and for few tokens and many weights, which the cluster's K split streams over the whole chip
+    // (5 x 2816 -> 7872 14.5 -> 10.5 us, 13 x 4736 -> 5440 14.7 -> 11.4).
+    double best = sparse ? kSparseOneLaunchUs : dense_layer_us(M, N, K);
     // more than 148 blocks of 160 tokens and one weight tile: never one wave
     for (int bt = M <= 16 ? 16 : 32; M > 0 && M <= 148 * 160 && K <= 16384 && bt <= 160; bt = bt == 16 ? 32 : bt + 32) {
       for (int k = 1; k <= kMaxRanks; ++k) {
         Plan p;
         p.block_t = bt; p.ks = k;
         if (!complete(&p, M, N, K, sparse)) continue;
-        // clusters leave some SMs of a GPC unused
-        if (static_cast<int64_t>(p.t_tiles) * p.w_tiles * k > (k > 1 ? sms * 7 / 8 : sms)) continue;
-        const double t = plan_us(p, M, sparse);
+        const int64_t clusters = static_cast<int64_t>(p.t_tiles) * p.w_tiles;
+        if (clusters * k > (k > 1 ? sms * 7 / 8 : sms) || (k > 1 && clusters > resident_clusters(k, sms))) continue;
+        const double t = sparse ? plan_us(p, M, sparse) : plan_layer_us(p, M, N, K);
         if (t < best) { best = t; e.block_t = bt; e.ks = k; }
       }
       if (bt >= M) break;

@@ -526,7 +526,8 @@ def test_dense_splitk_plan_leaves_the_unet_shapes_alone(tc):
     (100, 1024, 320, 64, 3),       # ranges of unequal length
     (257, 512, 160, 96, 1),
     (300, 192, 96, 160, 1),
-    (256, 256, 64, 256, 2)])       # widest block
+    (256, 256, 64, 256, 2),        # widest block
+    (5, 2816, 7872, 16, 2)])       # few tokens, more weight tiles than half the SMs
 def test_one_launch_layer_equals_two_launches(tc, sp, sparse, M, K, N, block_t, ks):
     """The one-launch layer (codes written straight to the operand tiles, K ranges over a cluster) against
     quantiser + GEMM: same codes, same integer sums, same epilogue, so the same bits."""
