@@ -858,7 +858,13 @@ TilePlan search_tile(int64_t M, int64_t N, int64_t K, bool geglu, int cta_group,
       const double least = g == 2 ? 0.019 : resident ? 0.220 : 0.207;
       if (block < least) block = least;
       const double operand = tiles * g * static_cast<double>(nk) * kBlockKBytes * (kTileM + (resident ? 0.0 : static_cast<double>(w) / g)) / 1e7;
-      const double us = 3.09 + rounds * (static_cast<double>(nk) * block + 0.124 + 0.423 * c) + 0.078 * operand + (g == 2 ? 1.19 : 0.0);
+      double us = 3.09 + rounds * (static_cast<double>(nk) * block + 0.124 + 0.423 * c) + 0.078 * operand + (g == 2 ? 1.19 : 0.0);
+      // A CTA does not fit beside a quantiser's, so a grid that wants nearly every SM starts late behind one: it
+      // needs a few SMs to spare (257 x 1536 -> 4608, whole layer: 144 tiles 9.0 us, 108 tiles 8.1).
+      if (splits == 1 && rounds == 1.0 && tiles * g * 5 > sms * 4) us += 0.7;
+      // Pairs lean less on L2, which the real operands' traffic shares: they win where the model sees them equal
+      // (49152 x 1280 -> 320 in the layer: 61.0 -> 58.6 us).
+      if (g == 2 && rounds >= 4.0) us *= 0.985;
       if (us < best.us) { best.us = us; best.block_n = w; best.group = g; }
     }
   }

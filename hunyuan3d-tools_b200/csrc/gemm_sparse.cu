@@ -447,7 +447,49 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   }
 }
 
+// Tile shape.  CTA pairs (256 weight rows sharing one token tile) halve each CTA's activation traffic into
+// shared memory, which is what paces deep-K stages, and cost more per tile hand-off; a wide token tile
+// amortises the weights, a narrow one spreads few tokens over the chip.  Both come from one cost model, in
+// microseconds, fitted to 98 shapes x all tiles (7 % rms; the tile it picks is 1 % from the best on average,
+// where a fixed threshold for pairs and tiles of 128 tokens or more were 10 %):
+//   2335 x 4864 -> 688: 12.3 -> 10.6 us, 3451 x 3328 -> 640: 15.1 -> 8.7, 279 x 704 -> 1120: 4.8 -> 4.0
+struct SparseTile {
+  int block_t = 0, group = 1;
+  double us = 1e30;
+};
+SparseTile search_tile(int64_t M, int64_t N, int64_t K, int block_t) {
+  SparseTile best;
+  const int64_t kblocks = (K + kBlockK - 1) / kBlockK;
+  const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
+  for (int g = 1; g <= (K >= 1024 ? 2 : 1); ++g) {
+    for (int bt = 32; bt <= 224; bt += 32) {
+      if (block_t != 0 && bt != 32) break;             // the caller's width, one pass per group
+      const int t = block_t != 0 ? block_t : bt;
+      if (t < 16 || t > kMaxBlockT || (t & 15) || (g == 2 && (t & 31))) continue;
+      if (block_t == 0 && bt > 32 && bt >= M + 32) break;
+      if (block_t == 0 && bt == 32 && M > 1024) continue;      // one store per 32 tokens and 32 columns
+      const double tiles = static_cast<double>((N + kTileW * g - 1) / (kTileW * g)) * static_cast<double>((M + t - 1) / t);
+      const double rounds = static_cast<double>((static_cast<int64_t>(tiles) + sms / g - 1) / (sms / g));
+      const double w = t / 100.0;
+      double stage = g == 1 ? 0.196 + 0.130 * w : 0.327 + 0.036 * w;
+      const double floor_us = g == 1 ? 0.273 : 0.351;
+      if (stage < floor_us) stage = floor_us;
+      const double operand_mb = tiles * g * static_cast<double>(kblocks) * (kABytes + kEBytes + 256.0 * t / g) / 1e7;
+      const double us = 3.0 + rounds * (static_cast<double>(kblocks) * stage + 0.08 + 0.55 * w) + 0.096 * operand_mb + (g == 2 ? 0.61 : 0.0);
+      if (us < best.us) { best.us = us; best.block_t = t; best.group = g; }
+    }
+  }
+  return best;
+}
+
 }  // namespace
+
+// Expected time of a layer that quantises and multiplies in separate launches, in microseconds: the greater of
+// the device's and the calling thread's (7.5), fitted to 110 layers of random size (0.2 us rms).
+double sparse_layer_us(int64_t M, int64_t N, int64_t K) {
+  const double us = 1.271 * search_tile(M, N, K, 0).us + 0.424 * static_cast<double>(M) * K / 1e6 - 0.08;
+  return us > 7.5 ? us : 7.5;
+}
 
 
 int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
@@ -471,40 +513,12 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
        reinterpret_cast<uintptr_t>(w_meta) | reinterpret_cast<uintptr_t>(out)) & 15)
     return HY3D_ERR_SHAPE;
 
-  // Tile shape.  CTA pairs (256 weight rows sharing one token tile) halve each CTA's activation traffic into
-  // shared memory, which is what paces deep-K stages, and cost more per tile hand-off; a wide token tile
-  // amortises the weights, a narrow one spreads few tokens over the chip.  Both come from one cost model, in
-  // microseconds, fitted to 98 shapes x all tiles (7 % rms; the tile it picks is 1 % from the best on average,
-  // where a fixed threshold for pairs and tiles of 128 tokens or more were 10 %):
-  //   2335 x 4864 -> 688: 12.3 -> 10.6 us, 3451 x 3328 -> 640: 15.1 -> 8.7, 279 x 704 -> 1120: 4.8 -> 4.0
-  int group = 1;
-  {
-    const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
-    double best = 1e30;
-    int best_t = 0;
-    for (int g = 1; g <= (K >= 1024 ? 2 : 1); ++g) {
-      for (int bt = 32; bt <= 224; bt += 32) {
-        if (block_t != 0 && bt != 32) break;             // the caller's width, one pass per group
-        const int t = block_t != 0 ? block_t : bt;
-        if (t < 16 || t > kMaxBlockT || (t & 15) || (g == 2 && (t & 31))) continue;
-        if (block_t == 0 && bt > 32 && bt >= M + 32) break;
-        if (block_t == 0 && bt == 32 && M > 1024) continue;      // one store per 32 tokens and 32 columns
-        const double tiles = static_cast<double>((N + kTileW * g - 1) / (kTileW * g)) * static_cast<double>((M + t - 1) / t);
-        const double rounds = static_cast<double>((static_cast<int64_t>(tiles) + sms / g - 1) / (sms / g));
-        const double w = t / 100.0;
-        double stage = g == 1 ? 0.196 + 0.130 * w : 0.327 + 0.036 * w;
-        const double floor_us = g == 1 ? 0.273 : 0.351;
-        if (stage < floor_us) stage = floor_us;
-        const double operand_mb = tiles * g * static_cast<double>(kblocks) * (kABytes + kEBytes + 256.0 * t / g) / 1e7;
-        const double us = 3.0 + rounds * (static_cast<double>(kblocks) * stage + 0.08 + 0.55 * w) + 0.096 * operand_mb + (g == 2 ? 0.61 : 0.0);
-        if (us < best) { best = us; best_t = t; group = g; }
-      }
-    }
-    block_t = best_t;
+  const SparseTile tile = search_tile(M, N, K, block_t);
+  block_t = tile.block_t;
+  int group = tile.group;
 #ifdef HY3D_TRACE
-    if (const char* e = getenv("HY3D_SPARSE_CTA_GROUP")) group = atoi(e) == 2 ? 2 : 1;
+  if (const char* e = getenv("HY3D_SPARSE_CTA_GROUP")) group = atoi(e) == 2 ? 2 : 1;
 #endif
-  }
   if (block_t < 16 || block_t > kMaxBlockT || (block_t & 15)) return HY3D_ERR_SHAPE;
   if (group == 2 && (block_t & 31)) group = 1;
 
@@ -593,5 +607,6 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
 }  // namespace sparse
 
 using sparse::gemm_sparse24;
+using sparse::sparse_layer_us;
 
 }  // namespace hy3d

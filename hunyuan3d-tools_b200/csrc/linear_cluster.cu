@@ -446,9 +446,12 @@ double plan_us(const Plan& p, int64_t M, bool sparse) {
          (p.ks > 1 ? 1.5 + 0.41 * slabs : 0.0) + 0.23 * slabs;
 }
 
-// What a caller sees of a plan beside dense_layer_us: fitted to 117 dense layers of random size.
-double plan_layer_us(const Plan& p, int64_t M, int64_t N, int64_t K) {
-  return 1.156 * plan_us(p, M, false) - 0.4 + 0.25 * static_cast<double>(N) * K / 1e7 + (p.ks > 1 ? 0.2 : 0.0);
+// What a caller sees of a plan beside dense_layer_us / sparse_layer_us: fitted to 117 dense and 110 sparse layers
+// of random size.  The sparse MMA's metadata chain makes one CTA's K units dearer where there are many weights.
+double plan_layer_us(const Plan& p, int64_t M, int64_t N, int64_t K, bool sparse) {
+  const double weights = static_cast<double>(N) * K / 1e7;
+  return sparse ? 1.289 * plan_us(p, M, true) - 0.96 + 0.38 * weights - (p.ks > 1 ? 0.46 : 0.0)
+                : 1.156 * plan_us(p, M, false) - 0.4 + 0.25 * weights + (p.ks > 1 ? 0.2 : 0.0);
 }
 
 // Clusters of `ks` CTAs that run at the same time, one CTA an SM: the GPCs have 16 to 20 SMs, and what is left
@@ -479,10 +482,6 @@ int resident_clusters(int ks, int sms) {
   return n;
 }
 
-// Sparse layers take one launch up to here.  The two launches need 6-8 us on the device for such shapes and about
-// as much of the calling thread, which then is what a caller waits for; one launch saves 2.4 us of that.
-constexpr double kSparseOneLaunchUs = 8.5;
-
 }  // namespace
 
 // Whether a layer of this size should run as one launch, and with which plan.  Sizes recur in every step of
@@ -494,10 +493,10 @@ bool linear_cluster_plan(int64_t M, int64_t N, int64_t K, bool sparse, int* bloc
   if (e.M != M || e.N != N || e.K != K || e.sparse != (sparse ? 1 : 0)) {
     e = {M, N, K, sparse ? 1 : 0, 0, 0};
     const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
-    // Dense layers take the one launch where it is expected to be the shorter one: below the host's time for two
-    // launches, and for few tokens and many weights, which the cluster's K split streams over the whole chip
-    // (5 x 2816 -> 7872 14.5 -> 10.5 us, 13 x 4736 -> 5440 14.7 -> 11.4).
-    double best = sparse ? kSparseOneLaunchUs : dense_layer_us(M, N, K);
+    // A layer takes the one launch where it is expected to be the shorter one: below the host's time for two
+    // launches, and for few tokens and many dense weights, which the cluster's K split streams over the whole
+    // chip (5 x 2816 -> 7872 14.5 -> 10.5 us, 13 x 4736 -> 5440 14.7 -> 11.4).
+    double best = sparse ? sparse_layer_us(M, N, K) : dense_layer_us(M, N, K);
     // more than 148 blocks of 160 tokens and one weight tile: never one wave
     for (int bt = M <= 16 ? 16 : 32; M > 0 && M <= 148 * 160 && K <= 16384 && bt <= 160; bt = bt == 16 ? 32 : bt + 32) {
       for (int k = 1; k <= kMaxRanks; ++k) {
@@ -506,7 +505,7 @@ bool linear_cluster_plan(int64_t M, int64_t N, int64_t K, bool sparse, int* bloc
         if (!complete(&p, M, N, K, sparse)) continue;
         const int64_t clusters = static_cast<int64_t>(p.t_tiles) * p.w_tiles;
         if (clusters * k > (k > 1 ? sms * 7 / 8 : sms) || (k > 1 && clusters > resident_clusters(k, sms))) continue;
-        const double t = sparse ? plan_us(p, M, sparse) : plan_layer_us(p, M, N, K);
+        const double t = plan_layer_us(p, M, N, K, sparse);
         if (t < best) { best = t; e.block_t = bt; e.ks = k; }
       }
       if (bt >= M) break;
