@@ -242,17 +242,24 @@ PyObject* linear_sparse(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return linear_sparse_impl(a[0], a[1], a[2], a[3], a[4], epi);
 }
 
-// The two forms of a layer whose input arrives as codes and per-row scales: the logical leading shape
-// is given as a tuple (its last entry is K), the output type by an example tensor's code.
-bool lead_shape(PyObject* o, c10::SmallVector<int64_t, 6>* lead) {
+// The two forms of a layer whose input arrives as codes and per-row scales: the logical shape is given as a
+// tuple, the output type by a code.  The output is allocated from the leading entries and the kernel writes M
+// rows, so the tuple has to describe exactly M rows of K.
+bool lead_shape(PyObject* o, int64_t M, int64_t K, c10::SmallVector<int64_t, 6>* lead) {
   if (!PyTuple_Check(o)) return false;
   const Py_ssize_t d = PyTuple_GET_SIZE(o);
-  for (Py_ssize_t i = 0; i + 1 < d; ++i) {
+  int64_t rows = 1;
+  for (Py_ssize_t i = 0; i < d; ++i) {
     PyObject* v = PyTuple_GET_ITEM(o, i);
     if (!PyLong_Check(v)) return false;
-    lead->push_back(PyLong_AsLongLong(v));
+    const int64_t n = PyLong_AsLongLong(v);
+    if (n == -1 && PyErr_Occurred()) PyErr_Clear();
+    if (i + 1 == d) return n == K && rows == M;
+    if (n < 1 || rows > M / n) return false;
+    rows *= n;
+    lead->push_back(n);
   }
-  return d >= 1;
+  return false;
 }
 
 // gemm_dense(q (M,K), scale (M), w_int8, w_scale, bias | None, is_bf16, epilogue, shape) -> y | None
@@ -260,14 +267,14 @@ PyObject* gemm_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   long epi = 0, bf16 = 0;
   c10::SmallVector<int64_t, 6> lead;
-  if (n != 8 || !small_int(a[5], 0, 1, &bf16) || !small_int(a[6], 0, 2, &epi) || !lead_shape(a[7], &lead)) return none();
+  if (n != 8 || !small_int(a[5], 0, 1, &bf16) || !small_int(a[6], 0, 2, &epi)) return none();
   const at::Tensor *q = plain(a[0]), *s = plain(a[1]), *w = plain(a[2]);
   if (!q || !s || !w || q->dim() != 2 || s->dim() != 1 || w->dim() != 2 || q->scalar_type() != at::kChar ||
       s->scalar_type() != at::kFloat || w->scalar_type() != at::kChar || w->device() != q->device() ||
       s->device() != q->device())
     return none();
   const int64_t M = q->size(0), K = q->size(1), N = w->size(0);
-  if (M <= 0 || s->size(0) != M || w->size(1) != K || (K & 63) || (N & 15)) return none();
+  if (M <= 0 || s->size(0) != M || w->size(1) != K || (K & 63) || (N & 15) || !lead_shape(a[7], M, K, &lead)) return none();
   const Params p(a[3], a[4], N, q->device());
   if (!p.ok) return none();
   c10::cuda::CUDAGuard guard(q->device());
@@ -285,7 +292,7 @@ PyObject* gemm_sparse(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   long epi = 0, bf16 = 0;
   c10::SmallVector<int64_t, 6> lead;
-  if (n != 9 || !small_int(a[6], 0, 1, &bf16) || !small_int(a[7], 0, 2, &epi) || !lead_shape(a[8], &lead)) return none();
+  if (n != 9 || !small_int(a[6], 0, 1, &bf16) || !small_int(a[7], 0, 2, &epi)) return none();
   const at::Tensor *q = plain(a[0]), *s = plain(a[1]), *w = plain(a[2]), *e = plain(a[3]);
   if (!q || !s || !w || !e || q->dim() != 2 || s->dim() != 1 || w->dim() != 2 || e->dim() != 2 ||
       q->scalar_type() != at::kChar || s->scalar_type() != at::kFloat || w->scalar_type() != at::kChar ||
@@ -293,7 +300,9 @@ PyObject* gemm_sparse(PyObject*, PyObject* const* a, Py_ssize_t n) {
       e->device() != q->device())
     return none();
   const int64_t M = q->size(0), K = q->size(1), N = w->size(0);
-  if (M <= 0 || s->size(0) != M || 2 * w->size(1) != K || (K & 63) || (N & 15) || e->size(0) != N) return none();
+  if (M <= 0 || s->size(0) != M || 2 * w->size(1) != K || (K & 63) || (N & 15) || e->size(0) != N ||
+      !lead_shape(a[8], M, K, &lead))
+    return none();
   const Params p(a[4], a[5], N, q->device());
   if (!p.ok) return none();
   c10::cuda::CUDAGuard guard(q->device());

@@ -282,3 +282,24 @@ def test_direct_calls_leave_hooks_and_overrides_alone(qu):
     b = ln(x)
     assert seen == [a] and torch.equal(a.q, b.q) and torch.equal(a.scale, b.scale)
     assert b.shape == x.shape and b.dtype == x.dtype and torch.equal(layer(a), layer(b))
+
+
+@pytest.mark.parametrize("sparse", [False, True])
+def test_quantised_activation_of_another_shape_is_refused(qu, sparse):
+    """The output is allocated from the activation's shape while the kernel writes one row per code row, so a
+    shape that does not describe the codes has to raise instead of reaching the kernel."""
+    torch.manual_seed(8)
+    layer = (qu.Int8Linear.from_linear_sparse if sparse else qu.Int8Linear.from_linear)(nn.Linear(128, 64).to(DEV).bfloat16())
+    act = qu.Int8LayerNorm(nn.LayerNorm(128).to(DEV).bfloat16())(torch.randn(24, 128, device=DEV).bfloat16())
+    y = layer(act)
+    for shape in ((4, 6, 128), (24, 1, 128), (2, 3, 4, 128)):
+        assert torch.equal(layer(act.view(*shape)), y.view(*shape[:-1], 64))
+    for shape in ((1, 128), (23, 128), (4, 5, 128), (25, 128), (48, 128), (0, 128), (128,), (24, 2, 128)):
+        with pytest.raises(RuntimeError):
+            layer(qu.QuantizedActivation(act.q, act.scale, shape, act.dtype))
+    native = qu._load_native()
+    w, meta = (layer.weight_sparse_comp, (layer.weight_sparse_meta,)) if sparse else (layer.weight_int8_nk, ())
+    gemm = native.gemm_sparse if sparse else native.gemm_dense
+    for shape in ((24, 64), (-24, 128), (1 << 70, 128), (24, 1 << 70), (1 << 62, 1 << 62, 24, 128), (), ("24", 128)):
+        assert gemm(act.q, act.scale, w, *meta, layer.weight_scale, layer.bias, 1, 0, shape) is None
+    assert torch.equal(layer(act), y)
