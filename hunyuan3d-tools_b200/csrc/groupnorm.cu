@@ -153,6 +153,7 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ pr
         *p = a;
       }
     }
+    __syncwarp();          // the fold's trip counts differ by thread; the barrier is for converged warps
     if (!peers_run) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     peers_run = true;
     __syncthreads();

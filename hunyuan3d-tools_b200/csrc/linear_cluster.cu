@@ -201,6 +201,7 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
       for (int i = 0; i < rounds; ++i) {
         const int r = first + i * step;
         const float a = row_amax(r);
+        __syncwarp();                          // row_amax's trip counts differ by lane
         if (!waited) cluster_wait();           // the peers run: their shared memory may be written
         waited = true;
         if (r < rows && sub == 0)
