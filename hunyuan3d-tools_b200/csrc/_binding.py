@@ -292,6 +292,12 @@ class TcGemmModule(_Base):
         splits = self._lib.hy3d_dense_splitk_plan(M, N, K, epilogue, ctypes.byref(nbytes))
         return int(splits), int(nbytes.value)
 
+    def _planned_splits(self, M, N, K, epilogue, w_scale, bias):
+        """The plan's K ranges, or 1 where the reduction behind them could not read the parameters: it takes
+        scales and bias by 16-byte vectors, the single launch at any address."""
+        addresses = (w_scale.data_ptr() if w_scale is not None else 0) | (self._opt_bias(bias)[0] or 0)
+        return self.dense_splitk_plan(M, N, K, epilogue)[0] if addresses % 16 == 0 else 1
+
     def int8_gemm_tc(self, A, B, act_scale, w_scale, bias, out_dtype=None, epilogue=EPI_LINEAR,
                      cta_group=0, block_n=0, splits=None):
         """A (M,K) s8, B (N,K) s8, act_scale (M) f32, w_scale (N), bias (N) or empty ->
@@ -309,7 +315,7 @@ class TcGemmModule(_Base):
         out = torch.empty(self._out_shape(M, N, epilogue), dtype=out_dtype, device=A.device)
         bptr, bcode = self._opt_bias(bias)
         if splits is None:
-            splits = self.dense_splitk_plan(M, N, K, epilogue)[0] if (
+            splits = self._planned_splits(M, N, K, epilogue, w_scale, bias) if (
                 out_dtype in (torch.float16, torch.bfloat16) and cta_group == 0 and block_n == 0) else 1
         if splits > 1:
             ws = torch.empty((splits, (M + 127) // 128 * 128, N), dtype=torch.int32, device=A.device)
@@ -371,7 +377,7 @@ class TcGemmModule(_Base):
         N = w_int8.shape[0]
         if w_int8.shape[1] != K:
             raise RuntimeError(f"K mismatch: x has {K}, w_int8 has {w_int8.shape[1]}")
-        if cta_group == 0 and block_n == 0 and self.dense_splitk_plan(M, N, K, epilogue)[0] > 1:
+        if cta_group == 0 and block_n == 0 and self._planned_splits(M, N, K, epilogue, w_scale, bias) > 1:
             q, s = self._quantize(x)                     # few rows, deep K: split-K GEMM
             return self.int8_gemm_tc(q, w_int8, s, w_scale, bias, out_dtype=x.dtype, epilogue=epilogue)
         q = torch.empty((M, K), dtype=torch.int8, device=x.device)

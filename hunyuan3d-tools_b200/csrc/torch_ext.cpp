@@ -98,6 +98,8 @@ struct Params {
   const void* bias = nullptr;
   int ws_code = 0, bias_code = HY3D_F16;
   bool ok = false;
+  // The reduction behind a split K reads scales and bias by 16-byte vectors; the other kernels take any address.
+  bool may_split() const { return ((reinterpret_cast<uintptr_t>(ws) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0; }
   Params(PyObject* scale, PyObject* b, int64_t N, c10::Device dev) {
     const at::Tensor* s = plain(scale);
     if (!s || s->dim() != 1 || s->size(0) != N || s->device() != dev) return;
@@ -142,7 +144,7 @@ bool one_launch(int64_t M, int64_t N, int64_t K, int sparse, int* block_t, int* 
 int dense_gemm(const int8_t* q, const float* s, const at::Tensor& w, const Params& p, void* out, int out_code,
                int64_t M, int64_t N, int64_t K, int epi, cudaStream_t st) {
   int64_t bytes = 0;
-  const int splits = api.hy3d_dense_splitk_plan(M, N, K, epi, &bytes);
+  const int splits = p.may_split() ? api.hy3d_dense_splitk_plan(M, N, K, epi, &bytes) : 1;
   if (splits > 1) {
     Scratch part(static_cast<size_t>(bytes), st);
     return api.hy3d_gemm_w8a8_dense_splitk(q, w.const_data_ptr<int8_t>(), s, p.ws, p.ws_code, p.bias, p.bias_code,
@@ -178,7 +180,7 @@ PyObject* linear_dense_impl(PyObject* px, PyObject* pw, PyObject* pscale, PyObje
   const size_t codes = align256(static_cast<size_t>(M) * K);
   Scratch ws(codes + static_cast<size_t>(M) * 4, st);
   int64_t bytes = 0;
-  if (api.hy3d_dense_splitk_plan(M, N, K, static_cast<int>(epi), &bytes) > 1) {
+  if (p.may_split() && api.hy3d_dense_splitk_plan(M, N, K, static_cast<int>(epi), &bytes) > 1) {
     rc = api.hy3d_quantize_rows(x->const_data_ptr(), code, M, K, K, ws.at(0), reinterpret_cast<float*>(ws.at(codes)), st);
     if (rc == HY3D_OK)
       rc = dense_gemm(ws.at(0), reinterpret_cast<float*>(ws.at(codes)), *w, p, y.mutable_data_ptr(), code, M, N, K,

@@ -651,3 +651,21 @@ def test_residual_quantisers_equal_adding_first(qu, ik, dtype, M, K):
         total, z = nat.norm_call(norm, x, h)
         ref = norm(x + h)
         assert torch.equal(total, x + h) and torch.equal(z.q, ref.q) and torch.equal(z.scale, ref.scale)
+
+
+@pytest.mark.parametrize("M,K,N", [(132, 4160, 1200), (257, 6144, 1536)])
+def test_planned_split_takes_parameters_at_any_address(qu, tc, M, K, N):
+    """Scales and bias that do not start on 16 bytes: the reduction behind a split K refuses them, so a shape the
+    plan would split runs as one launch, with the same bits."""
+    assert tc.dense_splitk_plan(M, N, K)[0] > 1
+    g = torch.Generator(device=DEV).manual_seed(K)
+    x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+    w = torch.randint(-127, 128, (N, K), generator=g, device=DEV, dtype=torch.int8)
+    ws, b = (torch.rand(N + 1, generator=g, device=DEV).bfloat16() for _ in range(2))
+    ref = tc.int8_linear_tc(x, w, ws[1:].clone(), b[1:].clone())
+    q, s = tc._quantize(x)
+    native = qu._load_native()
+    for scale, bias in ((ws[1:], b[1:]), (ws[1:].clone(), b[1:]), (ws[1:], b[1:].clone())):
+        assert torch.equal(tc.int8_linear_tc(x, w, scale, bias), ref)
+        assert torch.equal(tc.int8_gemm_tc(q, w, s, scale, bias, out_dtype=torch.bfloat16), ref)
+        assert torch.equal(native.gemm_dense(q, s, w, scale, bias, 1, 0, (M, K)), ref)
