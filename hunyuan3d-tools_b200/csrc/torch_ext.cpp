@@ -129,8 +129,9 @@ at::Tensor out_like(c10::IntArrayRef lead, int64_t cols, at::ScalarType type, c1
 
 bool small_int(PyObject* o, long lo, long hi, long* v) {
   if (!PyLong_CheckExact(o)) return false;
-  *v = PyLong_AsLong(o);
-  return *v >= lo && *v <= hi;
+  int overflow = 0;
+  *v = PyLong_AsLongAndOverflow(o, &overflow);
+  return !overflow && *v >= lo && *v <= hi;
 }
 
 // Small layers in one launch: what a caller waits for there is its own thread's launches, not the device.
@@ -254,8 +255,8 @@ bool lead_shape(PyObject* o, int64_t M, int64_t K, c10::SmallVector<int64_t, 6>*
   for (Py_ssize_t i = 0; i < d; ++i) {
     PyObject* v = PyTuple_GET_ITEM(o, i);
     if (!PyLong_Check(v)) return false;
-    const int64_t n = PyLong_AsLongLong(v);
-    if (n == -1 && PyErr_Occurred()) PyErr_Clear();
+    int overflow = 0;
+    const int64_t n = PyLong_AsLongLongAndOverflow(v, &overflow);      // -1 and no exception where it does not fit
     if (i + 1 == d) return n == K && rows == M;
     if (n < 1 || rows > M / n) return false;
     rows *= n;

@@ -219,3 +219,13 @@ def test_measured_sparse_rule(qu):
     assert qu.sparse_pays(1280, 10240) and qu.sparse_pays(5120, 1280)
     for k, n in [(320, 2560), (640, 5120), (1280, 320), (1280, 1280), (2560, 640), (1024, 1280)]:
         assert not qu.sparse_pays(k, n)
+
+
+def test_native_path_declines_integers_of_any_size(qu):
+    """The native functions answer None for what they do not take, without leaving an exception behind."""
+    native = qu._load_native()
+    x, w, s = torch.zeros(1, 64).half(), torch.zeros(16, 64, dtype=torch.int8), torch.ones(16).half()
+    for epilogue in (1 << 70, -(1 << 70), -1, 3, 0):
+        assert native.linear_dense(x, w, s, None, epilogue) is None
+        assert native.linear_sparse(x, w, w, s, None, epilogue) is None
+        assert native.groupnorm_nhwc(x, epilogue, None, None, 1e-5, False, None) is None
