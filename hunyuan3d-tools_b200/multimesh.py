@@ -168,9 +168,9 @@ def build_texture_unet(device, dtype=torch.bfloat16, quant: str = "mixed", seed:
     the projections of the time embedding and of the context.
     ``init_on_device`` draws the random weights on the GPU instead of the CPU.  ``fuse_ln`` lets
     the transformer blocks' LayerNorms emit int8 codes for the projections that follow them.
-    ``fused_gn`` runs GroupNorm (+ SiLU) through the library's channels-last kernel (default: on
-    for the INT8 modes on a CUDA device with channels_last activations, off for "none", which
-    stands for the stock PyTorch model)."""
+    ``fused_gn`` runs GroupNorm (+ SiLU) and the element-wise passes between the layers through the library's
+    channels-last kernels (default: on for the INT8 modes on a CUDA device with channels_last activations, off
+    for "none", which stands for the stock PyTorch model)."""
     from . import quantize_utils as qu
     from .unet import (UNetSD21MV, fuse_context_projections, fuse_geglu_layers, fuse_layernorm_quant, fuse_qkv_layers,
                        fuse_time_projections)

@@ -36,12 +36,15 @@ def timestep_embedding(t: torch.Tensor, dim: int) -> torch.Tensor:
 
 # -----------------------------------------------------------------------------------------
 # Steps between the layers.  torch adds a convolution's bias, a residual, a concatenation or an upsampling in
-# passes of their own; where a model runs channels_last f16 / bf16 on the GPU without autograd, the extension
-# does several of them in one pass, with the roundings the separate ops would have made.  Its functions answer
-# None for anything else, and the torch ops run.
+# passes of their own; in a model that asks for it (``use_fused_groupnorm``) and runs channels_last f16 / bf16 on
+# the GPU without autograd, the extension does several of them in one pass, with the roundings the separate ops
+# would have made.  Its functions answer None for anything else, and the torch ops run.
 # -----------------------------------------------------------------------------------------
-def _native():
-    return None if torch.is_grad_enabled() else _qu._NATIVE
+def _native(module, x):
+    """The extension, loaded on first use, for a module whose ``fused_steps`` is set."""
+    if not module.fused_steps or not x.is_cuda or torch.is_grad_enabled():
+        return None
+    return _qu._NATIVE or _qu._load_native()
 
 
 def _leaves_bias(native, *convs):
@@ -69,8 +72,7 @@ def _add_bias(native, x, bias_x, h=None, bias_h=None):
     return x + (h if bias_h is None else h + bias_h[:, None, None])
 
 
-def _conv(conv, x):
-    native = _native()
+def _conv(native, conv, x):
     if native is not None and conv.bias is not None and _leaves_bias(native, conv):
         return _add_bias(native, _conv_without_bias(conv, x), _conv_bias(conv))
     return conv(x)
@@ -78,9 +80,8 @@ def _conv(conv, x):
 
 def _residual_norm(norm, x, h):
     """x + h and its normalisation."""
-    native = _native()
-    if native is not None:
-        got = native.norm_call(norm, x, h)
+    if type(norm) is _qu.Int8LayerNorm and not torch.is_grad_enabled():
+        got = (_qu._NATIVE or _qu._load_native()).norm_call(norm, x, h)
         if got is not None:
             return got
     x = x + h
@@ -144,6 +145,7 @@ class ResnetBlock(nn.Module):
         self.conv2 = nn.Conv2d(cout, cout, 3, padding=1)
         self.conv_shortcut = nn.Conv2d(cin, cout, 1) if cin != cout else None
 
+    fused_steps = False
     # (stacked projection of all blocks, first column, last column + 1), set by fuse_time_projections
     _time_slice = None
 
@@ -159,7 +161,7 @@ class ResnetBlock(nn.Module):
         if term is None:
             term = self._term(temb)
         convs = (self.conv1, self.conv2) if self.conv_shortcut is None else (self.conv1, self.conv2, self.conv_shortcut)
-        native = _native() if self.norm2.fused else None
+        native = _native(self, x)
         if native is not None and _leaves_bias(native, *convs):
             h = _conv_without_bias(convs[0], self.norm1(x))
             b1 = _conv_bias(convs[0])
@@ -280,9 +282,10 @@ class SpatialTransformer(nn.Module):
     def forward(self, x, context, kv=None):
         b, c, h, w = x.shape
         y = self.proj_in(self.norm(x).permute(0, 2, 3, 1).reshape(b, h * w, c))
-        native = _native()
-        if (native is not None and type(self.block) is TransformerBlock and isinstance(self.proj_out, _qu.Int8Linear)
-                and native.unhooked(self.block)):
+        native = None
+        if type(self.block) is TransformerBlock and isinstance(self.proj_out, _qu.Int8Linear) and not torch.is_grad_enabled():
+            native = _qu._NATIVE or _qu._load_native()
+        if native is not None and native.unhooked(self.block):
             # the block's last sum feeds proj_out only: it is quantised as it is added, and not stored
             y, z = self.block.parts(y, context, kv)
             q = native.add_quantize(y, z)
@@ -293,27 +296,33 @@ class SpatialTransformer(nn.Module):
 
 
 class Downsample(nn.Module):
+    fused_steps = False
+
     def __init__(self, c):
         super().__init__()
         self.conv = nn.Conv2d(c, c, 3, stride=2, padding=1)
 
     def forward(self, x):
-        return _conv(self.conv, x)
+        return _conv(_native(self, x), self.conv, x)
 
 
 class Upsample(nn.Module):
+    fused_steps = False
+
     def __init__(self, c):
         super().__init__()
         self.conv = nn.Conv2d(c, c, 3, padding=1)
 
     def forward(self, x):
-        native = _native()
+        native = _native(self, x)
         y = native.upsample2x_nhwc(x) if native is not None else None
-        return _conv(self.conv, F.interpolate(x, scale_factor=2.0, mode="nearest") if y is None else y)
+        return _conv(native, self.conv, F.interpolate(x, scale_factor=2.0, mode="nearest") if y is None else y)
 
 
 class UNetSD21MV(nn.Module):
     """UNet2DConditionModel of the Hunyuan3D-2.1 paint configuration + multiview attention."""
+
+    fused_steps = False
 
     def __init__(self, in_channels=4, out_channels=4, block_out_channels=(320, 640, 1280, 1280),
                  layers_per_block=2, attention_heads=(5, 10, 20, 20), cross_attention_dim=1024,
@@ -383,11 +392,14 @@ class UNetSD21MV(nn.Module):
         return self
 
     def use_fused_groupnorm(self, on: bool = True) -> "UNetSD21MV":
-        """GroupNorm (+ SiLU) through the library's channels-last kernel (CUDA, f16/bf16,
-        channels_last activations); elsewhere the torch ops keep running."""
+        """GroupNorm (+ SiLU), and the bias, residual, concatenation and upsampling passes between the layers,
+        through the library's channels-last kernels (CUDA, f16/bf16, channels_last activations); elsewhere the
+        torch ops keep running."""
         for m in self.modules():
             if isinstance(m, GroupNormNHWC):
                 m.fused = on
+            elif isinstance(m, (ResnetBlock, Downsample, Upsample, UNetSD21MV)):
+                m.fused_steps = on
         return self
 
     def forward(self, x, t, context):
@@ -409,8 +421,8 @@ class UNetSD21MV(nn.Module):
         def attn(m, h):
             return m(h, context) if kvs is None else m(h, context, next(kvs))
 
-        native = _native()
-        h = _conv(self.conv_in, x)
+        native = _native(self, x)
+        h = _conv(native, self.conv_in, x)
         skips = [h]
         for layer in self.down:
             if "down" in layer:
@@ -430,7 +442,7 @@ class UNetSD21MV(nn.Module):
                 h = attn(layer["attn"], h)
             if "up" in layer:
                 h = layer["up"](h)
-        return _conv(self.conv_out, self.norm_out(h)).contiguous()
+        return _conv(native, self.conv_out, self.norm_out(h)).contiguous()
 
 
 def fuse_geglu_layers(model: nn.Module) -> int:

@@ -1,6 +1,7 @@
 """CPU: the C-ABI library loads and exports what the header declares; the host-side mirror of
 the reference's module behaves like it where no GPU is needed, and fails loudly where one is."""
 import ctypes
+import importlib
 import os
 import re
 
@@ -229,3 +230,26 @@ def test_native_path_declines_integers_of_any_size(qu):
         assert native.linear_dense(x, w, s, None, epilogue) is None
         assert native.linear_sparse(x, w, w, s, None, epilogue) is None
         assert native.groupnorm_nhwc(x, epilogue, None, None, 1e-5, False, None) is None
+
+
+def test_stock_model_does_not_depend_on_what_ran_before(qu, pkg, monkeypatch):
+    """A model that did not ask for the fused passes between its layers runs torch's ops, also once an INT8 layer
+    has loaded the extension: the same bits, and no call into it."""
+    un = importlib.import_module(pkg.__name__ + ".unet")
+    torch.manual_seed(0)
+    net = un.UNetSD21MV(block_out_channels=(32, 32), layers_per_block=1, attention_heads=(1, 1), cross_attention_dim=16,
+                        attn_levels=(True, True), num_views=2).eval().bfloat16().use_channels_last()
+    x, ctx, t = torch.randn(2, 4, 8, 8).bfloat16(), torch.randn(2, 3, 16).bfloat16(), torch.full((2,), 10)
+
+    class Untouched:
+        def __getattr__(self, name):
+            if name == "groupnorm_call":          # GroupNormNHWC asks; the function declines a module that is not fused
+                return lambda *a: None
+            raise AssertionError(f"extension function {name} called")
+    with torch.no_grad():
+        monkeypatch.setattr(qu, "_NATIVE", None)
+        before = net(x, t, ctx)
+        monkeypatch.setattr(qu, "_NATIVE", Untouched())
+        assert torch.equal(net(x, t, ctx), before)
+        net.use_fused_groupnorm()                 # CPU tensors: torch's ops all the same
+        assert torch.equal(net(x, t, ctx), before)
