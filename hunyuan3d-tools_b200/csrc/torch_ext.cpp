@@ -12,6 +12,8 @@
 #include <dlfcn.h>
 
 #include <ATen/cuda/EmptyTensor.h>
+#include <ATen/Context.h>
+#include <ATen/autocast_mode.h>
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
@@ -479,7 +481,7 @@ PyObject* quantize_weight(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // decline.
 struct Names {
   PyObject *dict, *buffers, *parameters, *mode, *epilogue, *bias, *wq, *scale, *comp, *meta, *forward, *compiled, *weight,
-      *eps, *fused, *silu, *groups, *shape, *dtype, *q, *act_scale;
+      *eps, *fused, *silu, *groups, *shape, *dtype, *q, *act_scale, *conv_groups;
   PyObject* hooks[4];
 } names;
 struct Registered {
@@ -496,7 +498,7 @@ bool intern_names() {
       {&names.comp, "weight_sparse_comp"}, {&names.meta, "weight_sparse_meta"}, {&names.forward, "forward"},
       {&names.compiled, "_compiled_call_impl"}, {&names.weight, "weight"}, {&names.eps, "eps"}, {&names.fused, "fused"},
       {&names.silu, "silu"}, {&names.groups, "num_groups"}, {&names.shape, "shape"}, {&names.dtype, "dtype"},
-      {&names.q, "q"}, {&names.act_scale, "scale"}, {&names.hooks[0], "_backward_hooks"},
+      {&names.q, "q"}, {&names.conv_groups, "groups"}, {&names.act_scale, "scale"}, {&names.hooks[0], "_backward_hooks"},
       {&names.hooks[1], "_backward_pre_hooks"}, {&names.hooks[2], "_forward_hooks"}, {&names.hooks[3], "_forward_pre_hooks"}};
   for (auto& n : all)
     if (!(*n.at = PyUnicode_InternFromString(n.text))) return false;
@@ -752,6 +754,37 @@ PyObject* unhooked(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Py_RETURN_TRUE;
 }
 
+// bias_apart(x, conv, ...) -> True where running these convolutions on x without their bias and adding it after
+// gives the bits of running them whole.  That is how torch itself runs a cuDNN convolution of a 16-bit type; with
+// autocast the operands change type on the way, the depthwise and the non-cuDNN kernels add the bias before they
+// round, and a hook or a replaced forward has to see the whole call.
+PyObject* bias_apart(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n < 2 || !THPVariable_CheckExact(a[0]) || !global_hooks[0]) Py_RETURN_FALSE;
+  const at::Tensor& x = THPVariable_Unpack(a[0]);
+  if (!x.is_cuda() || half_code(x.scalar_type()) < 0 || at::autocast::is_autocast_enabled(at::kCUDA) ||
+      !at::globalContext().userEnabledCuDNN())
+    Py_RETURN_FALSE;
+  for (Py_ssize_t i = 1; i < n; ++i) {
+    const Registered any{Py_TYPE(a[i]), _PyType_Lookup(Py_TYPE(a[i]), names.forward)};
+    PyObject* dict = plain_module(a[i], any);
+    PyObject* params = dict ? PyDict_GetItemWithError(dict, names.parameters) : nullptr;
+    PyObject* conv_groups = dict ? PyDict_GetItemWithError(dict, names.conv_groups) : nullptr;
+    long one = 0;
+    if (!params || !PyDict_Check(params) || !conv_groups || !small_int(conv_groups, 1, 1, &one)) Py_RETURN_FALSE;
+    for (PyObject* name : {names.weight, names.bias}) {
+      PyObject* o = PyDict_GetItemWithError(params, name);
+      if (!o || (o == Py_None && name == names.weight)) Py_RETURN_FALSE;
+      if (o == Py_None) continue;
+      if (!THPVariable_CheckExact(o)) Py_RETURN_FALSE;
+      const at::Tensor& t = THPVariable_Unpack(o);
+      if (t.scalar_type() != x.scalar_type() || t.device() != x.device()) Py_RETURN_FALSE;
+    }
+  }
+  Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
+}
+
 // groupnorm_call(layer, x, add | None, bias | None) -> y | None: calling a GroupNormNHWC whose kernel path is
 // on; `bias` is that of the convolution that made x and is added first
 PyObject* groupnorm_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -821,6 +854,7 @@ PyMethodDef methods[] = {
     HY3D_FAST(concat_nhwc),
     {"upsample2x_nhwc", upsample2x_nhwc, METH_O, nullptr},
     HY3D_FAST(unhooked),
+    HY3D_FAST(bias_apart),
     HY3D_FAST(linear_dense),
     HY3D_FAST(linear_sparse),
     HY3D_FAST(gemm_dense),

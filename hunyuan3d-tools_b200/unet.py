@@ -47,9 +47,9 @@ def _native(module, x):
     return _qu._NATIVE or _qu._load_native()
 
 
-def _leaves_bias(native, *convs):
-    """Whether these convolutions may be run without their bias, which is added later."""
-    return all(type(c) is nn.Conv2d and c.padding_mode == "zeros" for c in convs) and native.unhooked(*convs)
+def _leaves_bias(native, x, *convs):
+    """Whether these convolutions, on x's type, may be run without their bias, which is added later."""
+    return all(type(c) is nn.Conv2d and c.padding_mode == "zeros" for c in convs) and native.bias_apart(x, *convs)
 
 
 def _conv_without_bias(conv, x):
@@ -73,7 +73,7 @@ def _add_bias(native, x, bias_x, h=None, bias_h=None):
 
 
 def _conv(native, conv, x):
-    if native is not None and conv.bias is not None and _leaves_bias(native, conv):
+    if native is not None and conv.bias is not None and _leaves_bias(native, x, conv):
         return _add_bias(native, _conv_without_bias(conv, x), _conv_bias(conv))
     return conv(x)
 
@@ -162,7 +162,7 @@ class ResnetBlock(nn.Module):
             term = self._term(temb)
         convs = (self.conv1, self.conv2) if self.conv_shortcut is None else (self.conv1, self.conv2, self.conv_shortcut)
         native = _native(self, x)
-        if native is not None and _leaves_bias(native, *convs):
+        if native is not None and _leaves_bias(native, x, *convs):
             h = _conv_without_bias(convs[0], self.norm1(x))
             b1 = _conv_bias(convs[0])
             # h + bias + time embedding feeds norm2 only, so both terms ride in the normalisation

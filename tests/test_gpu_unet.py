@@ -189,3 +189,55 @@ def test_nhwc_groupnorm_kernel_keeps_the_model_output():
     with torch.no_grad():
         ym = m(x.bfloat16(), t, ctx.bfloat16())
     assert not torch.isnan(ym).any()
+
+
+def test_convolutions_keep_their_bias_where_adding_it_later_would_differ():
+    """A convolution leaves its bias to the pass behind it only where that gives the bits, and the type, of the whole
+    call: not under autocast, not with parameters of another type, not depthwise, not without cuDNN, not when hooked."""
+    qu = importlib.import_module(PKG_NAME + ".quantize_utils")
+    un = importlib.import_module(PKG_NAME + ".unet")
+    native = qu._load_native()
+    torch.manual_seed(0)
+    cl = torch.channels_last
+    x = torch.randn(2, 64, 8, 8, device=DEV).bfloat16().contiguous(memory_format=cl)
+
+    def down(dtype, groups=1):
+        m = un.Downsample(64)
+        m.conv = nn.Conv2d(64, 64, 3, stride=2, padding=1, groups=groups)
+        m = m.to(DEV).to(dtype).to(memory_format=cl)
+        m.fused_steps = True
+        return m
+
+    def same(m, a):
+        y, ref = m(a), m.conv(a)
+        return y.dtype == ref.dtype and torch.equal(y, ref)
+    with torch.no_grad():
+        m = down(torch.bfloat16)
+        assert native.bias_apart(x, m.conv) and same(m, x)
+        assert not native.bias_apart(x.float(), m.conv)
+        for dtype in (torch.float32, torch.bfloat16):
+            for cast in (torch.bfloat16, torch.float16):
+                m = down(dtype)
+                with torch.autocast("cuda", cast):
+                    assert not native.bias_apart(x, m.conv) and same(m, x) and same(m, x.float())
+        m = down(torch.bfloat16, groups=64)
+        assert not native.bias_apart(x, m.conv) and same(m, x)
+        m = down(torch.bfloat16)
+        with torch.backends.cudnn.flags(enabled=False):
+            assert not native.bias_apart(x, m.conv) and same(m, x)
+        h = m.conv.register_forward_hook(lambda mod, a, out: out + 1)
+        assert not native.bias_apart(x, m.conv) and same(m, x)
+        h.remove()
+        assert native.bias_apart(x, m.conv, down(torch.bfloat16).conv)
+        assert not native.bias_apart(x, m.conv, down(torch.float16).conv)
+    # a whole block: under autocast every step behind the first convolution sees the type it would have seen
+    block = un.ResnetBlock(64, 128, 32).to(DEV).bfloat16().to(memory_format=cl).eval()
+    temb = torch.randn(2, 32, device=DEV).bfloat16()
+    with torch.no_grad():
+        for cast in (None, torch.float16):
+            with torch.autocast("cuda", cast or torch.float16, enabled=cast is not None):
+                ref = block(x, temb)
+                block.fused_steps = True
+                y = block(x, temb)
+                block.fused_steps = False
+            assert y.dtype == ref.dtype and torch.equal(y, ref)
