@@ -47,9 +47,13 @@ def _native(module, x):
     return _qu._NATIVE or _qu._load_native()
 
 
+_CONV2D_FORWARD = nn.Conv2d.forward
+
+
 def _leaves_bias(native, x, *convs):
     """Whether these convolutions, on x's type, may be run without their bias, which is added later."""
-    return all(type(c) is nn.Conv2d and c.padding_mode == "zeros" for c in convs) and native.bias_apart(x, *convs)
+    return (all(type(c) is nn.Conv2d and c.padding_mode == "zeros" for c in convs)
+            and nn.Conv2d.forward is _CONV2D_FORWARD and native.bias_apart(x, *convs))
 
 
 def _conv_without_bias(conv, x):
@@ -271,6 +275,9 @@ class TransformerBlock(nn.Module):
         return x + h
 
 
+_BLOCK_FORWARD, _LINEAR_FORWARD = TransformerBlock.forward, _qu.Int8Linear.forward
+
+
 class SpatialTransformer(nn.Module):
     def __init__(self, dim: int, heads: int, context_dim: int, num_views: int):
         super().__init__()
@@ -283,9 +290,10 @@ class SpatialTransformer(nn.Module):
         b, c, h, w = x.shape
         y = self.proj_in(self.norm(x).permute(0, 2, 3, 1).reshape(b, h * w, c))
         native = None
-        if type(self.block) is TransformerBlock and isinstance(self.proj_out, _qu.Int8Linear) and not torch.is_grad_enabled():
+        if type(self.block) is TransformerBlock and type(self.proj_out) is _qu.Int8Linear and not torch.is_grad_enabled():
             native = _qu._NATIVE or _qu._load_native()
-        if native is not None and native.unhooked(self.block):
+        if (native is not None and TransformerBlock.forward is _BLOCK_FORWARD and _qu.Int8Linear.forward is _LINEAR_FORWARD
+                and native.unhooked(self.block, self.proj_out)):
             # the block's last sum feeds proj_out only: it is quantised as it is added, and not stored
             y, z = self.block.parts(y, context, kv)
             q = native.add_quantize(y, z)

@@ -241,3 +241,43 @@ def test_convolutions_keep_their_bias_where_adding_it_later_would_differ():
                 y = block(x, temb)
                 block.fused_steps = False
             assert y.dtype == ref.dtype and torch.equal(y, ref)
+
+
+def test_hooks_and_overrides_around_the_output_projection_see_tensors(monkeypatch):
+    """The transformer's last residual sum is handed to the projection behind it as codes only where nobody looks:
+    a hook, a subclass or a replaced forward of either gets the tensors it always got, and the result is the same."""
+    qu = importlib.import_module(PKG_NAME + ".quantize_utils")
+    un = importlib.import_module(PKG_NAME + ".unet")
+    torch.manual_seed(0)
+    net = un.SpatialTransformer(128, 2, 128, 2).eval().bfloat16().to(DEV)
+    qu.quantize_model_tensorcore(net, verbose=False)
+    x = torch.randn(2, 128, 8, 8, device=DEV).bfloat16().contiguous(memory_format=torch.channels_last)
+    ctx = torch.randn(2, 7, 128, device=DEV).bfloat16()
+    seen = []
+    with torch.no_grad():
+        y = net(x, ctx)
+        for hook in (lambda: net.proj_out.register_forward_pre_hook(lambda m, a: seen.append(a[0])),
+                     lambda: net.proj_out.register_forward_hook(lambda m, a, out: seen.append(a[0])),
+                     lambda: net.block.register_forward_hook(lambda m, a, out: seen.append(out)),
+                     lambda: nn.modules.module.register_module_forward_pre_hook(
+                         lambda m, a: seen.append(a[0]) if m is net.proj_out else None)):
+            h = hook()
+            assert torch.equal(net(x, ctx), y)
+            h.remove()
+        plain, forward = net.proj_out, type(net.proj_out).forward
+
+        class Watched(qu.Int8Linear):
+            def forward(self, t):
+                seen.append(t)
+                return super().forward(t)
+        net.proj_out = Watched(128, 128, dtype=torch.bfloat16).to(DEV)
+        net.proj_out.load_state_dict(plain.state_dict())
+        assert torch.equal(net(x, ctx), y)
+        net.proj_out = plain
+        plain.forward = lambda t: seen.append(t) or forward(plain, t)
+        assert torch.equal(net(x, ctx), y)
+        del plain.forward
+        block_forward = un.TransformerBlock.forward
+        monkeypatch.setattr(un.TransformerBlock, "forward", lambda self, *a: seen.append(block_forward(self, *a)) or seen[-1])
+        assert torch.equal(net(x, ctx), y)
+    assert len(seen) == 7 and all(type(t) is torch.Tensor and t.shape == (2, 64, 128) for t in seen)
