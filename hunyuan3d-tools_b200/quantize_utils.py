@@ -383,6 +383,23 @@ class Int8Linear(nn.Module):
         out.mode = first.mode
         return out
 
+    @staticmethod
+    def concat_state(state_dict, prefix, parts):
+        """Replaces the entries of separate layers in a state dict by those of the layer ``concat`` makes of them,
+        in place; leaves the dict alone unless it has all of the parts, in one mode, and not the whole."""
+        names = ("weight_int8_nk", "weight_scale", "weight_sparse_comp", "weight_sparse_meta", "bias")
+        have = [[n for n in names if part + n in state_dict] for part in parts]
+        extra = [state_dict.get(part + "_extra_state") for part in parts]
+        if prefix + "weight_scale" in state_dict or not all("weight_scale" in h and h == have[0] for h in have) \
+                or any(e != extra[0] for e in extra):
+            return
+        for n in have[0]:       # (a sparse layer's empty dense buffers join to an empty one)
+            state_dict[prefix + n] = torch.cat([state_dict.pop(part + n) for part in parts])
+        for part in parts:
+            state_dict.pop(part + "_extra_state", None)
+        if extra[0] is not None:
+            state_dict[prefix + "_extra_state"] = extra[0]
+
     def interleave_geglu_rows(self) -> "Int8Linear":
         """Re-orders a GEGLU up-projection ([value(H) | gate(H)] output rows) into blocks of
         16 value rows followed by their 16 gate rows and switches the layer to the fused

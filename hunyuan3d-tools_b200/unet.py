@@ -394,6 +394,16 @@ class UNetSD21MV(nn.Module):
     def _transformers(self):
         return ([l["attn"] for l in self.down if "attn" in l] + [self.mid_attn] + [l["attn"] for l in self.up if "attn" in l])
 
+    def _load_from_state_dict(self, state_dict, prefix, *args):
+        # A checkpoint from before the blocks' projections were stacked holds them block by block; the stacked
+        # layers hold the same rows one below the other.
+        names = {id(m): name for name, m in self.named_modules()}
+        for attr, parts in (("time_proj_all", [names[id(m)] + ".time_emb_proj." for m in self._resnets()]),
+                            ("context_proj_all", [names[id(m.block.attn2)] + ".to_kv." for m in self._transformers()])):
+            if isinstance(getattr(self, attr, None), _qu.Int8Linear):
+                _qu.Int8Linear.concat_state(state_dict, prefix + attr + ".", [prefix + part for part in parts])
+        super()._load_from_state_dict(state_dict, prefix, *args)
+
     def use_channels_last(self) -> "UNetSD21MV":
         self.to(memory_format=torch.channels_last)
         self.channels_last = True
@@ -418,9 +428,9 @@ class UNetSD21MV(nn.Module):
         if self.channels_last:
             x = x.contiguous(memory_format=torch.channels_last)
         terms = kvs = None
-        if self.time_proj_all is not None:
+        if getattr(self, "time_proj_all", None) is not None:      # absent from a model pickled before it existed
             terms = iter(self.time_proj_all(F.silu(temb)).split([m.conv1.out_channels for m in self._resnets()], dim=-1))
-        if self.context_proj_all is not None:
+        if getattr(self, "context_proj_all", None) is not None:
             kvs = iter(self.context_proj_all(context).split([2 * m.proj_in.out_features for m in self._transformers()], dim=-1))
 
         def res(m, h):

@@ -253,3 +253,41 @@ def test_stock_model_does_not_depend_on_what_ran_before(qu, pkg, monkeypatch):
         assert torch.equal(net(x, t, ctx), before)
         net.use_fused_groupnorm()                 # CPU tensors: torch's ops all the same
         assert torch.equal(net(x, t, ctx), before)
+
+
+def test_checkpoint_of_separate_projections_loads_into_the_stacked_model(qu, pkg):
+    """State dicts written before the blocks' time and context projections were stacked keep loading, strictly; so do
+    those written since, and a model pickled before the stacked layers existed runs."""
+    un = importlib.import_module(pkg.__name__ + ".unet")
+
+    def model(seed):
+        torch.manual_seed(seed)
+        net = un.UNetSD21MV(block_out_channels=(128, 128), layers_per_block=1, attention_heads=(2, 2),
+                            cross_attention_dim=128, attn_levels=(True, False), num_views=2)
+        qu.quantize_model_tensorcore(net, verbose=False)
+        assert un.fuse_qkv_layers(net) > 0
+        return net
+    separate, stacked = model(1), model(2)
+    old = separate.state_dict()
+    assert un.fuse_time_projections(stacked) == 7 and un.fuse_context_projections(stacked) == 3
+    keys = set(stacked.state_dict())
+    stacked.load_state_dict(old)
+    assert any("time_emb_proj" in k for k in old)              # the caller's dict is not touched
+    un.fuse_time_projections(separate), un.fuse_context_projections(separate)
+    new = separate.state_dict()
+    assert set(new) == keys
+    for k, v in stacked.state_dict().items():
+        assert torch.equal(v, new[k]) if torch.is_tensor(v) else v == new[k]
+    again = model(3)
+    un.fuse_time_projections(again), un.fuse_context_projections(again)
+    again.load_state_dict(new)
+    assert torch.equal(again.time_proj_all.weight_int8_nk, separate.time_proj_all.weight_int8_nk)
+    broken = {k: v for k, v in old.items() if not k.startswith("mid_res1.time_emb_proj")}
+    with pytest.raises(RuntimeError):
+        again.load_state_dict(broken)
+    stock = un.UNetSD21MV(block_out_channels=(32, 32), layers_per_block=1, attention_heads=(1, 1), cross_attention_dim=16,
+                          num_views=1)
+    for attr in ("time_proj_all", "context_proj_all"):
+        delattr(stock, attr)
+    with torch.no_grad():
+        assert stock(torch.randn(1, 4, 8, 8), torch.tensor([3]), torch.randn(1, 3, 16)).shape == (1, 4, 8, 8)
