@@ -541,15 +541,26 @@ __device__ __forceinline__ float gelu_erf(float v) {
 // value * gelu(gate) for eight pairs of outputs, packed to the 16-bit type; pair(j, v, g) gives the operands
 // of pair j.  A gate feeds an int8 quantiser and, through it, the rest of a deep network, where one changed
 // rounding grows to the noise of the 8-bit codes (1.6-2.4 % of a UNet's output).  So with bf16 outputs the
-// fast form is kept only where it must round to what the erf form rounds to: over every finite fp32 g
-// (compared exhaustively on the device) the two differ by at most 2.1e-7 |g|, the products then by that times
-// |value| plus three roundings of at most 6e-8 |value g| each, hence by less than 4.5e-7 |value g|.  Both
+// fast form is kept only where it must round to what the erf form rounds to: over every normal fp32 g the two
+// differ by at most 2.1e-7 |g| (hy3d_gelu_enum_check compares them all on the device), the products then by that
+// times |value| plus three roundings of at most 6e-8 |value g| each, hence by less than 4.5e-7 |value g|.  Both
 // ends of that interval round alike for all but about one output in 3,000 of unit-variance rows; the others
-// are recomputed by the erf form at the end.  fp16 outputs, which have no such history, keep the fast form,
-// the more accurate one.  Issue-bound: 49152 x 320 -> 2560 takes 79 us, 113 with the erf form throughout
-// and 66 without the test of the roundings.
+// are recomputed by the erf form at the end.
+// Below about -3.7 the interval is wider than the rounding step of the small result, and every such gate is
+// recomputed.  With gates of a standard deviation above 1.5 that is several lanes in each group, and the loop
+// costs more than the erf form for everybody: `wide`, the same for all lanes of a warp, then sends the warp's next
+// group that way (gated_pairs_wide), whose result is the same bits.  49152 x 320 -> 2560, us for gates of standard
+// deviation 0.5 / 1 / 1.5 / 2 / 3 / 8: 83 / 92 / 112 / 109 / 110 / 111; without `wide` 81 / 90 / 113 / 140 / 180 /
+// 232; the erf form throughout 114.
+// fp16 outputs keep the fast form unsettled, 69 us at any width.  It is the more accurate one, but an fp16 UNet's
+// output is not that of the erf form: it moves by 1.3-1.6 % (of 6 views of 64 x 64 at width 320, 2 of 32 x 32 at
+// 128, 3 of 40 x 40 at 192), as under any other change of rounding.  The interval leaves about one fp16 output in
+// 400 open; the one form of settling them that was timed took 111 to 154 us.
+constexpr int kWideEnter = 6, kWideLeave = 5;     // lanes of a warp with an open gate: where the two ways cost the same
+constexpr float kOpenGate = -3.7f;
+
 template <bool kBf16, typename Pair>
-__device__ __forceinline__ void gated_pairs(uint32_t (&out)[8], Pair pair) {
+__device__ __forceinline__ void gated_pairs(uint32_t (&out)[8], Pair pair, bool& wide) {
   constexpr int kType = kBf16 ? HY3D_BF16 : HY3D_F16;
   uint32_t differ[8], any = 0;
 #pragma unroll
@@ -573,7 +584,9 @@ __device__ __forceinline__ void gated_pairs(uint32_t (&out)[8], Pair pair) {
     }
     if (kBf16) any = any | (differ[q] | differ[q + 1]) | (differ[q + 2] | differ[q + 3]);
   }
-  if (kBf16 && any) {
+  const uint32_t lanes = kBf16 ? __ballot_sync(0xffffffffu, any != 0) : 0;
+  if (lanes) {
+    wide = __popc(lanes) >= kWideEnter;
     uint32_t mask = 0;
 #pragma unroll
     for (int u = 0; u < 8; ++u) mask |= differ[u] ? 1u << u : 0u;
@@ -589,6 +602,19 @@ __device__ __forceinline__ void gated_pairs(uint32_t (&out)[8], Pair pair) {
       for (int u = 0; u < 8; ++u) out[u] = u == j ? w : out[u];
     }
   }
+}
+// The erf form for all of them (bf16); `wide` stays set while enough lanes have a gate the fast form leaves open.
+template <typename Pair>
+__device__ __forceinline__ void gated_pairs_wide(uint32_t (&out)[8], Pair pair, bool& wide) {
+  float least = 0.0f;
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    float2 v, g;
+    pair(u, v, g);
+    out[u] = pack2(v.x * gelu_erf(g.x), v.y * gelu_erf(g.y), HY3D_BF16);
+    least = fminf(least, fminf(g.x, g.y));
+  }
+  wide = __popc(__ballot_sync(0xffffffffu, least < kOpenGate)) >= kWideLeave;
 }
 template <bool kBf16>
 __device__ __forceinline__ float gated1(float v, float g) {

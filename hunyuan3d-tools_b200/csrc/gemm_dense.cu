@@ -134,7 +134,7 @@ __device__ __forceinline__ void slab_math(const uint32_t (&r)[32], float as, con
 template <bool kBf16>
 __device__ __forceinline__ void slab_math_geglu(const uint32_t (&rv)[16], const uint32_t (&rg)[16],
                                                 float as, const float* wsb, const float* bsb,
-                                                uint32_t (&packed8)[8]) {
+                                                uint32_t (&packed8)[8], bool& wide) {
   // `as * ws` and the fused multiply-add of two neighbouring columns, packed as in slab_math.
   const float2 as2 = make_float2(as, as);
   // (16-byte loads of the parameters: the two pairs that share one are unrolled next to each other)
@@ -149,7 +149,7 @@ __device__ __forceinline__ void slab_math_geglu(const uint32_t (&rv)[16], const 
     v = scaled2(rv + 2 * j, wsb + c, bsb + c, j & 1);
     g = scaled2(rg + 2 * j, wsb + 16 + c, bsb + 16 + c, j & 1);
   };
-  gated_pairs<kBf16>(packed8, pair);
+  if (kBf16 && wide) gated_pairs_wide(packed8, pair, wide); else gated_pairs<kBf16>(packed8, pair, wide);
 }
 
 // Writes one packed 32 x 32 slab row into the warp's staging buffer (64-byte swizzle: 16-byte
@@ -503,6 +503,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     // per-column scales / bias are refilled only when the tile column changes (with the grid
     // a multiple of the column count, a CTA keeps its column for the whole launch).
     float as_next = 0.0f;
+    bool wide_gates = false;
     // Tile coordinates advance by additions (tile += tile_step in the walk order), not by a
     // division per tile: (fast, slow) = (column, row unit) when N-fastest, else the reverse.
     const int fast_dim = p.n_fastest ? p.n_tiles : p.m_tiles;
@@ -617,8 +618,12 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         } else {
           for (int s = half; s < nslab; s += kWarpsPerQuarter) {
             const int c0 = s * acc_per_slab;
-            uint32_t packed[16];
-#pragma unroll
+            // Two groups of 16 outputs, by one copy of the gate's code: each goes to the staging buffer by itself
+            // (laid out as in slab_store).
+            const uint32_t buf_addr = stage_buf + sb * kSlabBytes;
+            const uint32_t row_addr = buf_addr + static_cast<uint32_t>(lane) * 64u;
+            const uint32_t sw = (static_cast<uint32_t>(lane) >> 1) & 3u;
+#pragma unroll 1
             for (int b = 0; b < 2; ++b) {
               uint32_t rv[16], rg[16], out[8];
               const int cb = c0 + 32 * b;
@@ -631,12 +636,20 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                 release_acc(smem_u32(&ctrl->tmem_empty[buf]));
                 arrived = true;
               }
-              slab_math_geglu<kBf16>(rv, rg, as, wsb + cb, bsb + cb, out);
-#pragma unroll
-              for (int j = 0; j < 8; ++j) packed[8 * b + j] = out[j];
+              slab_math_geglu<kBf16>(rv, rg, as, wsb + cb, bsb + cb, out, wide_gates);
+              if (b == 0) {
+                if (lane == 0) { if (pend) tma_store_wait_read<1>(); else tma_store_wait_read<0>(); }
+                __syncwarp();
+              }
+              st_shared_v4(row_addr + ((2 * b ^ sw) << 4), out[0], out[1], out[2], out[3]);
+              st_shared_v4(row_addr + (((2 * b + 1) ^ sw) << 4), out[4], out[5], out[6], out[7]);
             }
-            slab_store(packed, stage_buf + sb * kSlabBytes, lane, pend, &tm_o, ((n0 + c0) >> 1) * 2,
-                       out_row, rows_in && ((n0 + c0) >> 1) < ldo);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (rows_in && ((n0 + c0) >> 1) < ldo) tma_store_2d(&tm_o, buf_addr, ((n0 + c0) >> 1) * 2, out_row);
+              tma_store_commit();
+            }
             if (++sb == p.store_bufs) sb = 0;
           }
         }

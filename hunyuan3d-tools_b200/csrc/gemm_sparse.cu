@@ -265,7 +265,7 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     constexpr int kOutDtype = kBf16 ? HY3D_BF16 : HY3D_F16;
     const int64_t ldo = geglu ? (p.N >> 1) : p.N;
     const uint32_t stage_buf = staging_base + static_cast<uint32_t>(warp - 2) * kSlabBytes;
-    bool ok = true;
+    bool ok = true, wide_gates = false;
     int it = 0;
     for (int tile = first_tile; tile < total_tiles; tile += tile_step, ++it) {
       const int buf = it & 1;
@@ -357,7 +357,8 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
               v = scaled(ra[i], ra[i + 1], as2, h);
               g = scaled(rb[i], rb[i + 1], as2, 2 + h);
             };
-            gated_pairs<kBf16>(out, pair);
+            if (kBf16 && wide_gates) gated_pairs_wide(out, pair, wide_gates);
+            else gated_pairs<kBf16>(out, pair, wide_gates);
             __syncwarp();
             stmatrix_x4_trans(st_addr, out[0], out[1], out[2], out[3]);
             stmatrix_x4_trans(st_addr + 512u, out[4], out[5], out[6], out[7]);

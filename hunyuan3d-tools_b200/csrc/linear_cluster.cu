@@ -327,6 +327,7 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
   // the sparse GEMM: 64-byte rows with 64-byte swizzle, 32-byte rows with 32-byte swizzle after the gate.
   const uint32_t stage_buf = ring + static_cast<uint32_t>(warp) * kSlabBytes;
   float* asw = ctrl->slab_scale[warp];
+  bool wide_gates = false;                               // not asked for: a warp has a slab or two
   const int frag_tok = 2 * (lane & 3);
   const uint32_t st_row = static_cast<uint32_t>(lane) & 7u, st_mat = static_cast<uint32_t>(lane) >> 3;
   const uint32_t st_addr =
@@ -369,7 +370,7 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
         v = scaled(ra[i], ra[i + 1], as2, h);
         g = scaled(rb[i], rb[i + 1], as2, 2 + h);
       };
-      gated_pairs<kBf16>(out, pair);
+      gated_pairs<kBf16>(out, pair, wide_gates);
       __syncwarp();
       stmatrix_x4_trans(st_addr, out[0], out[1], out[2], out[3]);
       stmatrix_x4_trans(st_addr + 512u, out[4], out[5], out[6], out[7]);

@@ -430,7 +430,7 @@ linear_fused_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_const
     const int nmine = nslab > half ? (nslab - half + kEpiPerQuarter - 1) / kEpiPerQuarter : 0;
     const int ncols = nmine * kAps;                                  // <= 128
     const int pend = p.store_bufs - 1;
-    bool ok = true;
+    bool ok = true, wide_gates = false;
     int it = 0, blk = -1, prev_m = -1, sb = 0;
     float as = 0.0f;
     // Column scales and bias of every slab this warp will take from a tile: fetched one tile
@@ -532,7 +532,7 @@ linear_fused_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_const
               arrived = true;
             }
             uint32_t out[8];
-            dense::slab_math_geglu<kBf16>(rv, rg, as, wsb + j * kAps + 32 * b, bsb + j * kAps + 32 * b, out);
+            dense::slab_math_geglu<kBf16>(rv, rg, as, wsb + j * kAps + 32 * b, bsb + j * kAps + 32 * b, out, wide_gates);
             __syncwarp();
 #pragma unroll
             for (int u = 0; u < 8; ++u) packed[8 * b + u] = out[u];

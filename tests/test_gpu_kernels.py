@@ -669,3 +669,26 @@ def test_planned_split_takes_parameters_at_any_address(qu, tc, M, K, N):
         assert torch.equal(tc.int8_linear_tc(x, w, scale, bias), ref)
         assert torch.equal(tc.int8_gemm_tc(q, w, s, scale, bias, out_dtype=torch.bfloat16), ref)
         assert torch.equal(native.gemm_dense(q, s, w, scale, bias, 1, 0, (M, K)), ref)
+
+
+@pytest.mark.parametrize("sparse", [False, True])
+@pytest.mark.parametrize("M,K,N,block", [(3000, 64, 640, 97), (2500, 320, 2560, 400), (700, 1280, 96, 33)])
+def test_bf16_gate_keeps_its_bits_when_the_gates_width_changes(tc, sp, sparse, M, K, N, block):
+    """Warps that meet many strongly negative gates go over to the erf form and come back where the gates are narrow:
+    blocks of rows with gates of a standard deviation of 0.2, 2 and 12 in turn, the same bits throughout."""
+    g = torch.Generator(device=DEV).manual_seed(K + N)
+    q = torch.randint(-127, 128, (M, K), generator=g, device=DEV, dtype=torch.int8)
+    w = torch.randint(-127, 128, (N, K), generator=g, device=DEV, dtype=torch.int8)
+    comp, meta = sp.sparse_prune_and_pack(w) if sparse else (w, None)
+    s = torch.tensor([0.2, 2.0, 0.2, 12.0], device=DEV)[torch.arange(M, device=DEV) // block % 4]
+    ws = (torch.rand(N, generator=g, device=DEV) + 0.5) / (73.0 * 73.0 * K ** 0.5)
+    if sparse:
+        acc = sp.sparse_int8_gemm(q, None, comp, meta, None, None, out_dtype=torch.int32)
+        y = sp.sparse_int8_gemm(q, s, comp, meta, ws, None, out_dtype=torch.bfloat16, epilogue=2)
+    else:
+        acc = tc.int8_gemm_tc(q, w, None, None, None, out_dtype=torch.int32)
+        y = tc.int8_gemm_tc(q, w, s, ws, None, out_dtype=torch.bfloat16, epilogue=2)
+    v = (acc.double() * (s[:, None] * ws[None, :]).double()).float().view(M, N // 32, 2, 16)
+    value, gate = v[:, :, 0].reshape(M, -1), v[:, :, 1].reshape(M, -1)
+    ref = (value * (0.5 * gate * (1.0 + torch.erf(gate * 0.70710678118654752440)))).bfloat16()
+    assert torch.equal(y, ref)
