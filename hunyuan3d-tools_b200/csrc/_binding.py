@@ -28,6 +28,7 @@ _DTYPE_CODE = {torch.float16: F16, torch.bfloat16: BF16, torch.float32: F32, tor
 # check that the library exports exactly what the header declares.
 SIGNATURES = {
     "hy3d_quantize_rows": [c_void_p, c_int, c_int64, c_int64, c_int64, c_void_p, c_void_p, c_void_p],
+    "hy3d_gelu_enum_check": [ctypes.c_float, c_void_p, c_void_p, c_void_p],
     "hy3d_quantizer_enum_check": [c_int, c_void_p, c_void_p, c_void_p],
     "hy3d_layernorm_quantize": [c_void_p, c_int, c_int64, c_int64, c_int64, c_void_p, c_void_p, c_int,
                                 ctypes.c_float, c_void_p, c_void_p, c_void_p, c_void_p],
@@ -83,7 +84,7 @@ SIGNATURES = {
 }
 
 # The argument lists above belong to this ABI version of the library (hy3d_version()).
-ABI_VERSION = 203
+ABI_VERSION = 204
 
 
 def configure(lib: ctypes.CDLL) -> ctypes.CDLL:
@@ -245,6 +246,13 @@ class _Base:
             _DTYPE_CODE[dtype], ctypes.byref(pairs), ctypes.byref(bad),
             torch.cuda.current_stream().cuda_stream), "hy3d_quantizer_enum_check")
         return pairs.value, bad.value
+
+    def gelu_enum_check(self, bound):
+        """(values compared, values where the epilogues' GELU and the erf form differ by more than bound * |g|)."""
+        compared, outside = ctypes.c_ulonglong(0), ctypes.c_ulonglong(0)
+        self._check(self._lib.hy3d_gelu_enum_check(bound, ctypes.byref(compared), ctypes.byref(outside),
+                                                   torch.cuda.current_stream().cuda_stream), "hy3d_gelu_enum_check")
+        return compared.value, outside.value
 
     def _out_shape(self, M, N, epilogue):
         return (M, N // 2) if epilogue == EPI_GEGLU else (M, N)

@@ -149,6 +149,24 @@ __global__ void __launch_bounds__(512, 1) tmem_drain_kernel(int iters, uint32_t*
   }
 }
 
+// Enumeration behind the GEGLU gate's settled roundings: the fast form against the erf form over every fp32 g
+// of at least 2^-125 (below, where the products lose bits to underflow, the two differ by a denormal step).
+__device__ unsigned long long g_gelu_counts[2];   // [0] values compared, [1] further apart than bound * |g|
+
+__global__ void __launch_bounds__(256) gelu_enum_kernel(float bound) {
+  const uint32_t step = gridDim.x * blockDim.x;      // a power of two
+  const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned long long seen = 0, outside = 0;
+  for (uint32_t i = 0; i < (1u << 31) / step * 2; ++i) {
+    const float g = __uint_as_float(first + i * step);
+    if (!(fabsf(g) >= 2.350988701644575e-38f) || isinf(g)) continue;
+    ++seen;
+    if (!(fabsf(gelu_phi(g) - gelu_erf(g)) <= bound * fabsf(g))) ++outside;
+  }
+  atomicAdd(&g_gelu_counts[0], seen);
+  atomicAdd(&g_gelu_counts[1], outside);
+}
+
 }  // namespace
 }  // namespace probe
 }  // namespace hy3d
@@ -171,6 +189,23 @@ int hy3d_probe_mma_i8(int n, int groups, int sparse, int64_t* ops_out, void* str
   if (ops_out)
     *ops_out = static_cast<int64_t>(sms) * groups * 4 * 2 * 128 * n * (sparse ? 64 : 32);
   return cudaGetLastError() == cudaSuccess ? HY3D_OK : HY3D_ERR_CUDA;
+}
+
+int hy3d_gelu_enum_check(float bound, unsigned long long* compared_out, unsigned long long* outside_out, void* stream) {
+  using namespace hy3d;
+  if (!(bound >= 0.0f) || !compared_out || !outside_out) return HY3D_ERR_ARG;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  void* counts = nullptr;
+  unsigned long long h[2] = {0, 0};
+  if (cudaGetSymbolAddress(&counts, probe::g_gelu_counts) != cudaSuccess) return HY3D_ERR_CUDA;
+  if (cudaMemsetAsync(counts, 0, sizeof(h), s) != cudaSuccess) return HY3D_ERR_CUDA;
+  probe::gelu_enum_kernel<<<1024, 256, 0, s>>>(bound);
+  if (cudaGetLastError() != cudaSuccess) return HY3D_ERR_CUDA;
+  if (cudaMemcpyAsync(h, counts, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess) return HY3D_ERR_CUDA;
+  if (cudaStreamSynchronize(s) != cudaSuccess) return HY3D_ERR_CUDA;
+  *compared_out = h[0];
+  *outside_out = h[1];
+  return HY3D_OK;
 }
 
 int hy3d_probe_tmem_ld(int warps, int depth, int iters, int64_t* bytes_out, void* stream) {

@@ -149,6 +149,14 @@ int hy3d_add_layernorm_quantize(const void* x, const void* add, void* sum, int x
                                 void* stream);
 
 /*
+ * Self-check of the GELU that the GEMM epilogues evaluate (test hook, no reference counterpart): compares it on the
+ * device with 0.5 * g * (1 + erf(g / sqrt 2)) in fp32 for every fp32 g of magnitude 2^-125 and up, and counts the
+ * values where the two are further apart than bound * |g|.  The bf16 GEGLU epilogue rounds as that form does because
+ * none are at bound 2.1e-7.  Synchronises the stream (4.2e9 values, ~20 ms).
+ */
+int hy3d_gelu_enum_check(float bound, unsigned long long* compared_out, unsigned long long* outside_out, void* stream);
+
+/*
  * Self-check of the quantiser's rounding (test hook, no reference counterpart).  The kernel
  * above never divides; this call enumerates on the device every pair of 16-bit patterns
  * (amax, x) of x_dtype with |x| <= amax -- every input the quantiser can meet -- and counts the

@@ -692,3 +692,11 @@ def test_bf16_gate_keeps_its_bits_when_the_gates_width_changes(tc, sp, sparse, M
     value, gate = v[:, :, 0].reshape(M, -1), v[:, :, 1].reshape(M, -1)
     ref = (value * (0.5 * gate * (1.0 + torch.erf(gate * 0.70710678118654752440)))).bfloat16()
     assert torch.equal(y, ref)
+
+
+def test_gelu_and_erf_form_stay_within_the_gates_bound(ik):
+    """What the settled bf16 gate rests on, for every fp32 gate: 253 binades of two signs, none further from the erf
+    form than 2.1e-7 |g| -- and the count does notice a bound that does not hold."""
+    compared, outside = ik.gelu_enum_check(2.1e-7)
+    assert compared == 2 * 253 * 2 ** 23 and outside == 0
+    assert ik.gelu_enum_check(2.0e-7)[1] > 0
