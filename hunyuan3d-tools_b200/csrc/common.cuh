@@ -499,14 +499,25 @@ __device__ __forceinline__ float ex2_approx(float v) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
   return r;
 }
+// The smaller of two values, NaN if either is.
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 // kN pairs at once: every coefficient is set up once for all of them and their chains overlap.
-template <int kN>
+// kInf: +infinity gives +infinity, as with the erf form (whose -infinity is NaN, here too); |v| then stops at 64,
+// where 2^h has long been 0 -- infinity times that 0 would be NaN.  One more instruction a value, and these epilogues
+// are bound by issue: 49152 x 320 -> 1280 with GELU 52 -> 55 us.  Gates do without (49152 x 320 -> 2560 would go from
+// 83 to 86 us): a gate of +infinity gives NaN unless it is recomputed.
+template <int kN, bool kInf>
 __device__ __forceinline__ void gelu_phi2n(const float2 (&v)[kN], float2 (&out)[kN]) {
   float2 nt[kN], h[kN];              // nt = -|v|; the coefficients of odd powers carry the sign
 #pragma unroll
   for (int i = 0; i < kN; ++i) {
-    nt[i] = make_float2(__uint_as_float(__float_as_uint(v[i].x) | 0x80000000u),
-                        __uint_as_float(__float_as_uint(v[i].y) | 0x80000000u));
+    const float2 c = kInf ? make_float2(min_nan(v[i].x, 64.0f), min_nan(v[i].y, 64.0f)) : v[i];
+    nt[i] = make_float2(__uint_as_float(__float_as_uint(c.x) | 0x80000000u),
+                        __uint_as_float(__float_as_uint(c.y) | 0x80000000u));
     h[i] = make_float2(-8.168350404957891e-07f, -8.168350404957891e-07f);
   }
 #define HY3D_HORNER(c)  \
@@ -528,7 +539,7 @@ __device__ __forceinline__ void gelu_phi2n(const float2 (&v)[kN], float2 (&out)[
 __device__ __forceinline__ float2 gelu_phi2(float2 v) {
   const float2 in[1] = {v};
   float2 out[1];
-  gelu_phi2n<1>(in, out);
+  gelu_phi2n<1, true>(in, out);
   return out[0];
 }
 __device__ __forceinline__ float gelu_phi(float v) { return gelu_phi2(make_float2(v, v)).x; }
@@ -568,7 +579,7 @@ __device__ __forceinline__ void gated_pairs(uint32_t (&out)[8], Pair pair, bool&
     float2 v[4], g[4], y[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) pair(q + j, v[j], g[j]);
-    gelu_phi2n<4>(g, y);
+    gelu_phi2n<4, false>(g, y);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       y[j] = __fmul2_rn(v[j], y[j]);

@@ -700,3 +700,24 @@ def test_gelu_and_erf_form_stay_within_the_gates_bound(ik):
     compared, outside = ik.gelu_enum_check(2.1e-7)
     assert compared == 2 * 253 * 2 ** 23 and outside == 0
     assert ik.gelu_enum_check(2.0e-7)[1] > 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,N", [(5, 128, 144), (300, 128, 144), (1500, 64, 256), (257, 6144, 1536)])
+def test_gelu_of_infinite_pre_activations(qu, dtype, M, K, N):
+    """+infinity stays, -infinity and NaN give NaN, as in torch, and the columns beside them keep their bits: one launch,
+    two and three (split K), direct and bulk stores, dense and 2:4 sparse."""
+    torch.manual_seed(K)
+    lin = torch.nn.Linear(K, N).to(DEV).to(dtype)
+    x = torch.randn(M, K, device=DEV).to(dtype)
+    special = [float("inf"), float("-inf"), float("nan"), 3e4, -3e4]
+    for make in (qu.Int8Linear.from_linear, qu.Int8Linear.from_linear_sparse):
+        layer = make(lin)
+        layer.epilogue = "gelu"
+        ref = layer(x)
+        layer.bias = layer.bias.clone()
+        layer.bias[:5] = torch.tensor(special, device=DEV).to(dtype)
+        y = layer(x)
+        assert torch.equal(y[:, 5:], ref[:, 5:])
+        assert bool((y[:, 0] == float("inf")).all()) and bool(y[:, 1:3].isnan().all())
+        assert bool((y[:, 3] > 2.9e4).all()) and bool((y[:, 4] == 0).all())
