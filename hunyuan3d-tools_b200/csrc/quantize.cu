@@ -21,8 +21,11 @@
 #include "common.cuh"
 
 namespace hy3d {
+int device_sm_count();
 namespace quant {
 namespace {
+
+int sm_count() { return device_sm_count() > 0 ? device_sm_count() : 148; }
 
 constexpr int kQuantThreads = 256;
 struct True { static constexpr bool value = true; };
@@ -190,7 +193,7 @@ int launch_quantize(const void* x, const void* add, int64_t M, int64_t K, int64_
   // warp that holds a part of it -- unless the rows are too few to fill the chip that way.
   int lg = -1, maxv = 0;
   int64_t best = INT64_MAX;
-  const int64_t fill = static_cast<int64_t>(148) * 4 * kQuantThreads;
+  const int64_t fill = static_cast<int64_t>(sm_count()) * 4 * kQuantThreads;
   for (int l = 0; l <= 8; ++l) {
     const int64_t g = int64_t{1} << l;
     const int64_t v = (nvec + g - 1) / g;
@@ -405,7 +408,7 @@ int launch_layernorm_quantize(const void* x, const void* add, int64_t M, int64_t
   const int v = maxv <= 5 ? maxv : 8, out = add ? 2 : y_out ? 1 : 0;
   const KernelFn kernel = kernels[maxv <= 5 ? maxv - 1 : 5][(v << lg) == nvec ? 1 : 0][out];
   // One wave of resident blocks, evened out: every block walks the same number of row batches (or one less).
-  const int64_t wave = static_cast<int64_t>(148) * ln_blocks(v, out);
+  const int64_t wave = static_cast<int64_t>(sm_count()) * ln_blocks(v, out);
   const int64_t trips = (batches + wave - 1) / wave;
   const int64_t blocks = (batches + trips - 1) / trips;
   cudaLaunchConfig_t cfg = {};
@@ -552,7 +555,7 @@ int dequant_bias(const int32_t* acc, const float* act_scale, const void* w_scale
   if (M == 0) return HY3D_OK;
   const int64_t total = M * (N >> 3);
   int64_t blocks = (total + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
+  if (blocks > sm_count() * 16) blocks = sm_count() * 16;
   dequant_bias_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
       acc, act_scale, w_scale, ws_dtype, bias, bias_dtype, out, out_dtype, M, N);
   return cudaGetLastError() == cudaSuccess ? HY3D_OK : HY3D_ERR_CUDA;
