@@ -24,8 +24,8 @@ constexpr int kUnroll = 4;      // vectors a thread has in flight
 // one 32-bit division per thread and additions from there on.
 template <bool kBf16>
 __global__ void __launch_bounds__(kThreads)
-add_bias_kernel(const uint4* __restrict__ x, const uint4* __restrict__ bx, const uint4* __restrict__ h,
-                const uint4* __restrict__ bh, uint4* __restrict__ y, int64_t total, int vec_cols) {
+add_bias_kernel(const uint4* x, const uint4* __restrict__ bx, const uint4* h, const uint4* __restrict__ bh, uint4* y,
+                int64_t total, int vec_cols) {          // y may be x or h: a thread has read its vectors before it writes
   pdl_launch_dependents();
   const int64_t first = static_cast<int64_t>(blockIdx.x) * (kUnroll * kThreads);
   int col = static_cast<int>((first + threadIdx.x) % vec_cols);

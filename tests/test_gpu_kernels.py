@@ -721,3 +721,15 @@ def test_gelu_of_infinite_pre_activations(qu, dtype, M, K, N):
         assert torch.equal(y[:, 5:], ref[:, 5:])
         assert bool((y[:, 0] == float("inf")).all()) and bool(y[:, 1:3].isnan().all())
         assert bool((y[:, 3] > 2.9e4).all()) and bool((y[:, 4] == 0).all())
+
+
+@pytest.mark.parametrize("alias", ["x", "h"])
+def test_bias_pass_may_write_over_its_input(tc, alias):
+    torch.manual_seed(3)
+    x, h = (torch.randn(2, 40, 33, 17, device=DEV).bfloat16().contiguous(memory_format=torch.channels_last) for _ in range(2))
+    b = torch.randn(40, device=DEV).bfloat16()
+    ref = (x + b[:, None, None]) + (h + b[:, None, None])
+    y = x if alias == "x" else h
+    assert tc._lib.hy3d_add_bias_nhwc(x.data_ptr(), b.data_ptr(), h.data_ptr(), b.data_ptr(), 1, y.data_ptr(), 2 * 33 * 17, 40,
+                                      torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(y, ref)
