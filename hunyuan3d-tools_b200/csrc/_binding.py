@@ -211,8 +211,7 @@ class _Base:
 
     def groupnorm_nhwc(self, x, groups, gamma, beta, eps, silu=False, out=None, workspace=None, add=None):
         """GroupNorm (+ SiLU) of a channels_last (B, C, H, W) f16/bf16 tensor; the result has
-        the same shape and memory format.  ``workspace``: optional fp32 tensor of at least
-        ``groupnorm_workspace_floats(B, H*W, groups)`` elements (allocated when absent).
+        the same shape and memory format.  ``workspace`` is accepted and not used.
         ``add``: optional (B, C) tensor of x's dtype added per sample and channel first."""
         if x.dim() != 4 or x.dtype not in (torch.float16, torch.bfloat16) or not x.is_cuda:
             raise RuntimeError("groupnorm_nhwc: x must be a 4-D f16/bf16 CUDA tensor")
@@ -224,9 +223,6 @@ class _Base:
                 raise RuntimeError(f"groupnorm_nhwc: add must be a ({B}, {C}) CUDA tensor of {x.dtype}")
             add = add.contiguous()
         y = out if out is not None else torch.empty_like(x, memory_format=torch.channels_last)
-        need = self._lib.hy3d_groupnorm_workspace_floats(B, H * W, groups)
-        if workspace is None or workspace.numel() < need:
-            workspace = torch.empty(max(need, 1), dtype=torch.float32, device=x.device)
         if gamma is not None and beta is not None and gamma.dtype != beta.dtype:
             beta = beta.to(gamma.dtype)
         gb = gamma if gamma is not None else beta
@@ -236,7 +232,7 @@ class _Base:
                 x.data_ptr(), add.data_ptr() if add is not None else None, _DTYPE_CODE[x.dtype], B, H * W, C, groups,
                 gamma.data_ptr() if gamma is not None else None,
                 beta.data_ptr() if beta is not None else None, code, float(eps), 1 if silu else 0,
-                y.data_ptr(), workspace.data_ptr(), self._stream(x)), "hy3d_groupnorm_nhwc")
+                y.data_ptr(), None, self._stream(x)), "hy3d_groupnorm_nhwc")
         return y
 
     def quantizer_enum_check(self, dtype):

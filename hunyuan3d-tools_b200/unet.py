@@ -104,7 +104,6 @@ class GroupNormNHWC(nn.GroupNorm):
         self.silu = silu
         self.fused = False
         self._ik = None
-        self._ws = None
 
     def __call__(self, x, add=None):
         # The direct way to the kernel where no hook, subclass or tracer stands in it.
@@ -129,10 +128,8 @@ class GroupNormNHWC(nn.GroupNorm):
             if self._ik is None:
                 from .csrc.build import load_int8_kernels
                 self._ik = load_int8_kernels()
-            if self._ws is None or self._ws.device != x.device:
-                self._ws = torch.empty(1 << 16, dtype=torch.float32, device=x.device)
             return self._ik.groupnorm_nhwc(x, self.num_groups, self.weight, self.bias, self.eps,
-                                           silu=self.silu, workspace=self._ws, add=add)
+                                           silu=self.silu, add=add)
         if add is not None:
             x = x + add[:, :, None, None]
         y = super().forward(x)
