@@ -13,8 +13,9 @@
 //           of GroupNorm followed by SiLU as separate ops)
 // Results must not depend on how the work is spread: a statistic that moves in its last place changes some
 // rounding of the output, and behind an int8 quantiser a deep network turns that into 2 % of its result.  So
-// the order of every sum is a function of (B, HW, C, groups) alone -- row chunks, row lanes within a chunk,
-// channels within a group, chunk classes -- and slabs, ranks and sets only say who adds which part.
+// the order of every sum is a function of (B, HW, C, groups) and the device's SM count alone -- row chunks, row
+// lanes within a chunk, channels within a group, chunk classes -- and slabs, ranks and sets only say who adds
+// which part.
 // Bound by HBM at the large sizes (2 x 31.5 MB for 12 x 320 x 64 x 64: 9.7 us) beside two special-function
 // instructions per element of the SiLU (7 us), by latency at the small ones.  Two grid-wide launches with
 // partials in global memory took 27.1 us there and 11.5 us for 12 x 1280 x 8 x 8.

@@ -23,7 +23,8 @@
 // takes one contiguous range of it, so a block is quantised once per CTA that touches it.
 //
 // The arithmetic is that of quantize_rows_kernel and gemm_dense_kernel (same helper
-// functions), so the output is bit-identical to the two-launch path.
+// functions), so the output is bit-identical to the two-launch path.  It is slower than that on
+// every shape measured (see linear_path), so nothing takes it by itself: callers ask for it.
 #include "common.cuh"
 
 namespace hy3d {

@@ -5,9 +5,11 @@
 // layer below about 10 G multiply-adds.
 //
 // Every function answers Py_None, having done nothing, for arguments outside the plain case (another
-// dtype, a non-contiguous or CPU tensor, a tensor subclass, a size the kernels refuse); the caller then
-// takes the checked path of `_binding.py`, which either handles them or raises with its message.  Plain
-// CPython calling convention: no argument-conversion layer in between.
+// dtype, a non-contiguous or CPU tensor, a tensor subclass, a shape that does not fit); the caller then
+// takes the checked path of `_binding.py`, which either handles them or raises with its message.  What only
+// the library refuses (an address off a 16-byte boundary, K above a kernel's limit, GEGLU with N % 32 != 0)
+// raises here with the library's status, as it does there.  No gradient is recorded, whatever the grad mode.
+// Plain CPython calling convention: no argument-conversion layer in between.
 #include <Python.h>
 #include <dlfcn.h>
 

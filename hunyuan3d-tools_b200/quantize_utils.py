@@ -593,13 +593,14 @@ def _replace_linear_sparse(module, min_features, sparse_min_k, stats, choose=Non
 
 
 def sparse_pays(in_features: int, out_features: int) -> bool:
-    """Whether the 2:4-sparse kernel is the faster one for a layer of this size on B200.
-    Measured over the texture UNet's shapes: the sparse GEMM wins where the layer is bound by
-    the tensor pipe and shared-memory bandwidth (deep K and many weight rows -- 1280 -> 10240:
-    34.7 vs 39.1 us, 5120 -> 1280: 15.8 vs 18.7 us at 3072 tokens) and loses where the output
-    write or the per-tile fixed cost dominates (every K <= 640 layer, 1280 -> 320, 1280 -> 1280,
-    2560 -> 640).  The reference used one threshold on K (``sparse_min_k=640``, fitted on an
-    RTX 4090, quantize_utils.py:426)."""
+    """Whether ``quantize_model_mixed`` makes a layer of this size 2:4 sparse: deep K and many weight rows, where
+    the halved weight stream pays for the transposing epilogue.  At 3072 tokens, replayed from a graph, the GEMM takes
+    13.8 us sparse and 16.5 dense for 5120 -> 1280 (whole layer 22.6 / 24.6) and 32.5 / 33.2 for 1280 -> 10240
+    (37.3 / 36.7: even); elsewhere it loses (49152 x 320 -> 320 19.5 / 12.1, 49152 x 1280 -> 320 27.3 / 24.4,
+    12288 x 2560 -> 640 19.8 / 17.8, 12288 x 640 -> 5120 47.6 / 42.8) or ties (3072 x 1280 -> 1280 7.0 / 7.0).  A
+    whole UNet step takes the same time mixed and dense (22.2-22.3 ms); which layers are sparse is part of a model's
+    results, so the rule stays as it was when those layers won by 12 to 18 %.  The reference used one threshold
+    on K (``sparse_min_k=640``, fitted on an RTX 4090, quantize_utils.py:426)."""
     return in_features >= 1280 and in_features * out_features >= 5120 * 1280
 
 

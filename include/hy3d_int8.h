@@ -36,9 +36,11 @@ extern "C" {
 
 /* ---- GEMM epilogues ------------------------------------------------------------------ */
 #define HY3D_EPI_LINEAR  0  /* y = acc * (act_scale[m] * w_scale[n]) + bias[n]             */
-#define HY3D_EPI_GELU    1  /* y = gelu_erf(linear)                                        */
+#define HY3D_EPI_GELU    1  /* y = gelu(linear) = linear * Phi(linear), exact form         */
 #define HY3D_EPI_GEGLU   2  /* weights row-interleaved in blocks of 16 (value,gate):
-                               y[m, j] = value * gelu_erf(gate); output has N/2 columns   */
+                               y[m, j] = value * gelu(gate); output has N/2 columns.
+                               bf16 outputs round as 0.5 * g * (1 + erf(g / sqrt 2)) in
+                               fp32 does; fp16 ones and GELU may differ in the last place */
 
 /* ABI version (changes whenever an argument list or its meaning does), build architecture
  * ("sm_100a") and the digest of the sources the library was built from. */
@@ -196,7 +198,7 @@ int hy3d_gemm_w8a8_dense(const int8_t* A, const int8_t* B, const float* act_scal
  * formula and roundings, so the result equals hy3d_gemm_w8a8_dense bit for bit.
  * hy3d_dense_splitk_plan returns the number of ranges this library would use for a shape
  * (1 = do not split) and the workspace it needs.  out_dtype f16/bf16, epilogue linear or GELU,
- * N % 8 == 0; splits = 1 runs the plain kernel.
+ * N % 8 == 0; splits = 1 runs the plain kernel.  With splits > 1 w_scale and bias too must be 16-byte aligned.
  * Replaces: the split-K path and its reduce kernel of the reference's sparse GEMM
  * (csrc/int8_sparse_tc.cu:1730-1732 cost terms, split-K reduce) in the dense kernel's terms.
  */
@@ -233,8 +235,8 @@ int hy3d_linear_w8a8_dense(const void* x, int x_dtype, int64_t ldx,
  * pointers; anything else returns HY3D_ERR_SHAPE / HY3D_ERR_ARG and launches nothing.
  * scale_out: optional (M) f32 array that receives the per-token scales, or NULL.
  * block_n: 0 = choose, else the weight-tile width (multiple of 32, 64 for GEGLU, <= 256).
- * hy3d_linear_w8a8_dense takes this path by itself for the shapes where it is the faster one;
- * hy3d_linear_path(M, K, N, epilogue) tells which (1 = one launch, 0 = two launches).
+ * hy3d_linear_w8a8_dense would take this path by itself for shapes where it is the faster one, and
+ * hy3d_linear_path(M, K, N, epilogue) tells which (1 = one launch, 0 = two launches): today none, 0 for every shape.
  * Replaces: the fused quantise + GEMM path csrc/int8_sparse_tc.cu:657-734, 1934-2002
  * (sparse_gemm_fq_kernel, sp_use_fused, sparse_fq_launch) and the path query
  * csrc/int8_sparse_tc.cu:2065-2070 (sparse_int8_linear_path), for the dense layer.
