@@ -758,10 +758,9 @@ def unet_record(ctx: Ctx, args):
     mm = importlib.import_module(PKG + ".multimesh")
     out = {"config": "BASELINE configs[3]: SD2.1-architecture UNet, 2 (CFG) x 6 views x 64x64x4 latents, "
                      "multiview attention, random init", "unit": "ms/step", "steps": 20}
-    # "none": the stock PyTorch model (bf16 linears, torch GroupNorm); "none_nhwc_groupnorm": the
-    # same with this library's channels-last GroupNorm kernel, so that the INT8 linears' own
-    # contribution can be read off as (none_nhwc_groupnorm - dense); "mixed_torch_groupnorm":
-    # the INT8 model with torch's GroupNorm.
+    # "none": the stock PyTorch model (bf16 linears, torch GroupNorm); "none_nhwc_groupnorm": the same with this
+    # library's channels-last GroupNorm kernel and element-wise passes, so that the INT8 linears' own contribution
+    # can be read off as (none_nhwc_groupnorm - dense); "mixed_torch_groupnorm": the INT8 model with torch's.
     variants = (("dense", "dense", None), ("mixed", "mixed", None), ("none", "none", False),
                 ("none_nhwc_groupnorm", "none", True), ("mixed_torch_groupnorm", "mixed", False))
     for key, quant, fused_gn in variants:
