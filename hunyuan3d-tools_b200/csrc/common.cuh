@@ -682,4 +682,18 @@ inline cudaLaunchAttribute pdl_attribute() {
   return a;
 }
 
+// Host side: launch attribute that asks for no more shared memory per SM than `blocks` blocks of `bytes` each need
+// (the runtime keeps 1 KB of its own per block), so that the rest is L1.  Without it a kernel runs with whatever split
+// its predecessor left, if it fits: behind a GEMM that is 228 KB of shared memory and 28 KB of L1, too little for the
+// loads that a streaming kernel keeps in flight (quantiser of 49152 x 320 behind itself 7.6 us, with that split 12.1).
+// Whole layers from a graph, us: 49152 x 320 -> 320 22.0 -> 19.4, 12288 x 2560 -> 640 33.2 -> 29.7, 49152 x 1280 -> 320
+// 58.4 -> 50.7, LayerNorm + 12288 x 640 -> 1920 27.1 -> 24.7.
+inline cudaLaunchAttribute carveout_attribute(int64_t blocks, int64_t bytes) {
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  const int64_t percent = (blocks * (bytes + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024);
+  a.val.sharedMemCarveout = static_cast<unsigned>(percent > 100 ? 100 : percent);
+  return a;
+}
+
 }  // namespace hy3d

@@ -1171,10 +1171,9 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
     rcfg.gridDim = dim3(static_cast<unsigned>(blocks));
     rcfg.blockDim = dim3(256);
     rcfg.stream = stream;
-    cudaLaunchAttribute rattr[1];
-    rattr[0] = pdl_attribute();
+    cudaLaunchAttribute rattr[2] = {pdl_attribute(), carveout_attribute(8, 0)};
     rcfg.attrs = rattr;
-    rcfg.numAttrs = 1;
+    rcfg.numAttrs = 2;
     const int32_t* part = workspace;
     uint16_t* o16 = static_cast<uint16_t*>(final_out);
     const int Ni = static_cast<int>(N);

@@ -113,9 +113,9 @@ int launch(void (*kernel)(Params...), int64_t vectors, cudaStream_t stream, Args
   cfg.gridDim = dim3(static_cast<unsigned>(blocks));
   cfg.blockDim = dim3(kThreads);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1] = {pdl_attribute()};
+  cudaLaunchAttribute attr[2] = {pdl_attribute(), carveout_attribute(2048 / kThreads, 0)};
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   if (cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) != cudaSuccess) {
     cudaGetLastError();
     return HY3D_ERR_CUDA;

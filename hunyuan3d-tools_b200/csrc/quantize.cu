@@ -211,9 +211,9 @@ int launch_quantize(const void* x, const void* add, int64_t M, int64_t K, int64_
   cfg.gridDim = dim3(static_cast<unsigned>(blocks));
   cfg.blockDim = dim3(kQuantThreads);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1] = {pdl_attribute()};
+  cudaLaunchAttribute attr[2] = {pdl_attribute(), carveout_attribute(2048 / kQuantThreads, 32)};
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   using KernelFn = void (*)(const uint16_t*, const uint16_t*, int64_t, int8_t*, float*, int64_t, int, int);
 #define HY3D_Q(V)                                                                                      \
   {{quantize_rows_kernel<kBf16, V, false, false>, quantize_rows_kernel<kBf16, V, true, false>},        \
@@ -416,9 +416,9 @@ int launch_layernorm_quantize(const void* x, const void* add, int64_t M, int64_t
   cfg.blockDim = dim3(kQuantThreads);
   cfg.dynamicSmemBytes = static_cast<size_t>(2 * K) * sizeof(float);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1] = {pdl_attribute()};
+  cudaLaunchAttribute attr[2] = {pdl_attribute(), carveout_attribute(ln_blocks(v, out), 8 * K)};
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const uint16_t*>(x),
                                              reinterpret_cast<const uint16_t*>(add), ldx, gamma, beta, gb_dtype, eps, q, scale, reinterpret_cast<uint16_t*>(y_out), M, static_cast<int>(K), lg);
   if (err != cudaSuccess) {
