@@ -372,6 +372,32 @@ __device__ __forceinline__ void mma_sp_i8_2cta(uint32_t d_tmem, uint64_t desc_a,
       ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(e_tmem), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The sparse instructions with the descriptors as (low word, shared high word), like mma_i8_lohi.
+template <int kG>
+__device__ __forceinline__ void mma_sp_i8_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi,
+                                               uint32_t e_tmem, uint32_t idesc, uint32_t accumulate) {
+  if (kG == 1) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        ".reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "mov.b64 da, {%1, %3};\n\t"
+        "mov.b64 db, {%2, %3};\n\t"
+        "tcgen05.mma.sp.cta_group::1.kind::i8 [%0], da, db, [%4], %5, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(e_tmem), "r"(idesc), "r"(accumulate)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        ".reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "mov.b64 da, {%1, %3};\n\t"
+        "mov.b64 db, {%2, %3};\n\t"
+        "tcgen05.mma.sp.cta_group::2.kind::i8 [%0], da, db, [%4], %5, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(e_tmem), "r"(idesc), "r"(accumulate)
+        : "memory");
+  }
+}
 __device__ __forceinline__ void tmem_cp_128x128b_2cta(uint32_t dst_tmem, uint64_t src_desc) {
   asm volatile("tcgen05.cp.cta_group::2.128x128b [%0], %1;" ::"r"(dst_tmem), "l"(src_desc)
                : "memory");

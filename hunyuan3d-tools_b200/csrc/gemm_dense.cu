@@ -159,7 +159,7 @@ __device__ __forceinline__ void slab_math_geglu(const uint32_t (&rv)[16], const 
 __device__ __forceinline__ void slab_store(const uint32_t (&packed)[16], uint32_t buf_addr, int lane,
                                            int pending_ok, const CUtensorMap* tm_o, int x_bytes,
                                            int y_row, bool in_range) {
-  if (lane == 0) {
+  if (elect_one()) {
     if (pending_ok) tma_store_wait_read<1>(); else tma_store_wait_read<0>();
   }
   __syncwarp();
@@ -171,7 +171,7 @@ __device__ __forceinline__ void slab_store(const uint32_t (&packed)[16], uint32_
                  packed[4 * c + 3]);
   fence_proxy_async_smem();
   __syncwarp();
-  if (lane == 0) {
+  if (elect_one()) {
     if (in_range) tma_store_2d(tm_o, buf_addr, x_bytes, y_row);
     tma_store_commit();
   }
@@ -195,7 +195,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   // A stage holds kAtoms 128-byte-wide K blocks of each operand: [A0][A1..][B0][B1..].
   // Resident-B mode (one CTA per tile, one K block per stage): a stage holds A only, and the
   // CTA's B tile -- it keeps one tile column for the whole launch -- sits behind the ring.
-  const bool b_res = kG == 1 && kAtoms == 1 && p.b_resident;
+  const bool b_res = kAtoms == 1 && p.b_resident;
   const uint32_t stage_bytes = b_res ? a_bytes : static_cast<uint32_t>(kAtoms) * (a_bytes + b_bytes);
   const uint32_t b_res_base = smem_base + static_cast<uint32_t>(p.stages) * stage_bytes;
   const uint32_t b_res_bytes = b_res ? static_cast<uint32_t>(p.num_kb) * b_bytes : 0u;
@@ -263,16 +263,17 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   if (warp == 0) {
     // ---------------- TMA producer (all lanes walk the loop, lane 0 issues) ----------------
     {
-      const bool issuer = lane == 0;
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      if (b_res && first_tile < total_units && issuer) {
+      if (b_res && first_tile < total_units && elect_one()) {
         const uint32_t bf = smem_u32(&ctrl->b_full);
-        const int n0 = tile_n(first_tile) * p.block_n;
-        mbar_arrive_expect_tx(bf, b_res_bytes);
-        for (int kb = 0; kb < p.num_kb; ++kb)
-          tma_load_2d(b_res_base + kb * b_bytes, &tm_b, bf, kb * kBlockKBytes, n0);
+        const int n0 = tile_n(first_tile) * p.block_n + col_off;
+        if (leader) mbar_arrive_expect_tx(bf, static_cast<uint32_t>(kG) * b_res_bytes);
+        for (int kb = 0; kb < p.num_kb; ++kb) {
+          if (kG == 1) tma_load_2d(b_res_base + kb * b_bytes, &tm_b, bf, kb * kBlockKBytes, n0);
+          else tma_load_2d_pair(b_res_base + kb * b_bytes, &tm_b, map_to_cta(bf, 0), kb * kBlockKBytes, n0);
+        }
       }
       __syncwarp();
       for (int unit = first_tile; ok && unit < total_units; unit += tile_step) {
@@ -291,11 +292,16 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           if (b_res) {
             HY3D_TRACE_FINE(3, tr, 20, kb);
 #if defined(HY3D_TRACE) || defined(HY3D_KO)
-            if (p.debug & 1) { if (issuer) mbar_arrive(full); } else
+            if (p.debug & 1) { if (elect_one() && leader) mbar_arrive(full); } else
 #endif
-            if (issuer) {
-              mbar_arrive_expect_tx(full, a_bytes);
-              tma_load_2d(sa, &tm_a, full, kb * kBlockKBytes, m0);
+            if (elect_one()) {
+              if (kG == 1) {
+                mbar_arrive_expect_tx(full, a_bytes);
+                tma_load_2d(sa, &tm_a, full, kb * kBlockKBytes, m0);
+              } else {
+                if (leader) mbar_arrive_expect_tx(full, 2 * a_bytes);
+                tma_load_2d_pair(sa, &tm_a, map_to_cta(full, 0), kb * kBlockKBytes, m0);
+              }
             }
             HY3D_TRACE_FINE(3, tr, 21, kb);
             if (++stage == p.stages) { stage = 0; phase ^= 1; }
@@ -303,11 +309,11 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           }
 #if defined(HY3D_TRACE) || defined(HY3D_KO)
           if (p.debug & 1) {
-            if (leader && issuer) mbar_arrive(full);
+            if (leader && elect_one()) mbar_arrive(full);
           } else
 #endif
-          if (!issuer) {
-            // only lane 0 issues
+          if (!elect_one()) {
+            // only the elected lane issues
           } else if (kG == 1) {
             mbar_arrive_expect_tx(full, stage_bytes);
 #pragma unroll
@@ -338,7 +344,6 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     // spends between two issues is a cycle the pipe idles: the loop is kept to one barrier
     // probe, four issues and one commit per stage.
     if (leader) {
-      const bool issuer = lane == 0;
       const uint32_t idesc = make_idesc_i8(kTileM * kG, static_cast<uint32_t>(p.block_n), false);
       // Descriptor = (low word: address field + leading-dimension offset, high word: stride,
       // version, swizzle).  Only the 14-bit address field changes from stage to stage and from
@@ -395,42 +400,16 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after_sync();
-        if (issuer) HY3D_TRACE_EVENT(1, tr, 6, it);
+        if (elect_one()) HY3D_TRACE_EVENT(1, tr, 6, it);
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * p.acc_cols);
         uint32_t acc = 0;   // the first MMA of a tile overwrites the accumulator
-        if (b_res) {
-          // A from the ring, B from its resident block of the same K index.
-          uint32_t xb = b_res_lo0;
-          for (int kb = 0; kb < p.num_kb; ++kb) {
-            ok = wait_full();
-            if (!ok) break;
-            if (issuer) HY3D_TRACE_FINE(1, tr, 22, kb);
-            const int ksteps = kb + 1 < p.num_kb ? 4 : p.last_ksteps;
-            if (issuer) {
-              if (do_mma) {
-                for (int k = 0; k < ksteps; ++k)
-                  mma_i8_lohi<kG>(d_tmem, a_lo + 2 * k, xb + 2 * k, desc_hi, idesc, k ? 1u : acc);
-              }
-              commit_empty();
-              HY3D_TRACE_FINE(1, tr, 23, kb);
-            }
-            acc = 1u;
-            next_stage();
-            xb += b_atom;
-          }
-          if (ok && issuer) {
-            HY3D_TRACE_EVENT(1, tr, 3, it);
-            tc_commit_1cta(smem_u32(&ctrl->tmem_full[buf]));
-          }
-          __syncwarp();
-          continue;
-        }
+        uint32_t b_lo = b_res_lo0;   // resident mode: the K block of the same index
         for (int kb = 0; kb < full_kb; ++kb) {
           ok = wait_full();
           if (!ok) break;
-          if (issuer) {
+          if (elect_one()) {
             if (do_mma) {
-              uint32_t xa = a_lo, xb = a_lo + b_off;
+              uint32_t xa = a_lo, xb = b_res ? b_lo : a_lo + b_off;
 #pragma unroll
               for (int a = 0; a < kAtoms; ++a) {
                 mma_i8_lohi<kG>(d_tmem, xa, xb, desc_hi, idesc, a ? 1u : acc);
@@ -444,26 +423,29 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             commit_empty();
           }
           acc = 1u;
+          b_lo += b_atom;
           next_stage();
         }
         if (ok && full_kb < nkb) {   // ragged last stage: fewer K steps
           ok = wait_full();
           if (ok) {
-            if (issuer) {
+            if (elect_one()) {
               if (do_mma) {
-                for (int k = 0; k < p.last_ksteps; ++k) {
+                const uint32_t xb = b_res ? b_lo : a_lo + b_off;
+                mma_i8_lohi<kG>(d_tmem, a_lo, xb, desc_hi, idesc, acc);
+#pragma unroll
+                for (int k = 1; k < 4 * kAtoms - 1; ++k) {
                   const uint32_t at = static_cast<uint32_t>(k >> 2), kk = static_cast<uint32_t>(k & 3);
-                  mma_i8_lohi<kG>(d_tmem, a_lo + at * a_atom + 2 * kk,
-                                  a_lo + b_off + at * b_atom + 2 * kk, desc_hi, idesc, k ? 1u : acc);
+                  if (k < p.last_ksteps)
+                    mma_i8_lohi<kG>(d_tmem, a_lo + at * a_atom + 2 * kk, xb + at * b_atom + 2 * kk, desc_hi, idesc, 1u);
                 }
               }
               commit_empty();
             }
-            acc = 1u;
             next_stage();
           }
         }
-        if (ok && issuer) {
+        if (ok && elect_one()) {
           HY3D_TRACE_EVENT(1, tr, 3, it);
           if (kG == 1) tc_commit_1cta(smem_u32(&ctrl->tmem_full[buf]));
           else tc_commit_2cta(smem_u32(&ctrl->tmem_full[buf]), 3);
@@ -490,7 +472,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     auto release_acc = [&](uint32_t bar) {
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) {
+      if (elect_one()) {
         if (kG == 1 || leader) mbar_arrive(bar); else mbar_arrive_cluster(bar, 0);
       }
     };
@@ -597,10 +579,13 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         const bool rows_in = out_row < p.M;
         const int pend = p.store_bufs - 1;
         int sb = 0;
+        // Which slabs a warp takes moves on from tile to tile: with a number of slabs that four does not divide the
+        // same warps would always have one more.
+        const int first_slab = (half + it) & (kWarpsPerQuarter - 1);
         if (kEpi != HY3D_EPI_GEGLU) {
           // Each warp takes every kWarpsPerQuarter-th slab of its quarter; once its last
           // tcgen05.ld has landed the accumulator buffer is handed back to the MMA warp.
-          for (int s = half; s < nslab; s += kWarpsPerQuarter) {
+          for (int s = first_slab; s < nslab; s += kWarpsPerQuarter) {
             uint32_t r[32], packed[16];
             __syncwarp();
             tmem_ld_x32(t_row + s * kSlabCols, r);
@@ -616,7 +601,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             if (++sb == p.store_bufs) sb = 0;
           }
         } else {
-          for (int s = half; s < nslab; s += kWarpsPerQuarter) {
+          for (int s = first_slab; s < nslab; s += kWarpsPerQuarter) {
             const int c0 = s * acc_per_slab;
             // Two groups of 16 outputs, by one copy of the gate's code: each goes to the staging buffer by itself
             // (laid out as in slab_store).
@@ -638,7 +623,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
               }
               slab_math_geglu<kBf16>(rv, rg, as, wsb + cb, bsb + cb, out, wide_gates);
               if (b == 0) {
-                if (lane == 0) { if (pend) tma_store_wait_read<1>(); else tma_store_wait_read<0>(); }
+                if (elect_one()) { if (pend) tma_store_wait_read<1>(); else tma_store_wait_read<0>(); }
                 __syncwarp();
               }
               st_shared_v4(row_addr + ((2 * b ^ sw) << 4), out[0], out[1], out[2], out[3]);
@@ -646,7 +631,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             }
             fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0) {
+            if (elect_one()) {
               if (rows_in && ((n0 + c0) >> 1) < ldo) tma_store_2d(&tm_o, buf_addr, ((n0 + c0) >> 1) * 2, out_row);
               tma_store_commit();
             }
@@ -725,7 +710,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       HY3D_TRACE_RAW(4, acc_tile); HY3D_TRACE_RAW(5, acc_wait); HY3D_TRACE_RAW(6, it);
     }
     // Global writes of the bulk stores must be complete before the CTA retires.
-    if (p.tma_store && lane == 0) tma_store_wait_all<0>();
+    if (p.tma_store && elect_one()) tma_store_wait_all<0>();
   }
 
   // ---------------- teardown ----------------
@@ -1067,11 +1052,11 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
   // its tile column and the column's B tile fits beside at least four A stages, B is loaded
   // once and only A streams: 128 x K bytes per tile.
   const int a_stage = kTileM * kBlockKBytes;
-  const int b_tile_bytes = p.num_kb * block_n * kBlockKBytes;
+  const int b_tile_bytes = p.num_kb * (block_n / group) * kBlockKBytes;
   const int ctrl_bytes = static_cast<int>(sizeof(DenseCtrl));
   const int staging1 = kEpiWarps * kSlabBytes;
   int b_resident = 0, store_bufs = 2, stages = 0, stage_bytes = 0;
-  if (group == 1 && atoms == 1 && column_fixed && p.splits == 1 && total_tiles >= 2 * clusters) {
+  if (atoms == 1 && column_fixed && p.splits == 1 && total_tiles >= 2 * clusters) {
     // One staging buffer per epilogue warp: measured faster than two here (a warp that must
     // wait for its previous store to leave shared memory paces the store stream, and the
     // loads queue behind fewer stores).

@@ -147,7 +147,6 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   if (warp == 0) {
     // ---------------- TMA producer (all lanes walk the loop, lane 0 issues) ----------------
     {
-      const bool issuer = lane == 0;
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -161,8 +160,8 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
           const uint32_t full = smem_u32(&ctrl->full[stage]);
           const uint32_t sa = smem_base + stage * stage_bytes;
           const uint32_t sb = sa + kABytes + kEBytes;
-          if (!issuer) {
-            // only lane 0 issues
+          if (!elect_one()) {
+            // only the elected lane issues
           } else if (kG == 1) {
             mbar_arrive_expect_tx(full, stage_bytes);
             tma_load_2d(sa, &tm_w, full, kb * (kBlockK / 2), w0);
@@ -188,12 +187,18 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   } else if (warp == 1) {
     // ---------------- MMA issuer (one thread) ----------------
     if (leader) {
-      const bool issuer = lane == 0;
+      // One thread issues, named by elect.sync: the compiler then knows that there is one, and descriptors stay in
+      // uniform registers (behind `lane == 0` every issue converted them for whichever lanes were active).
+      // Descriptors advance as low words, see the dense kernel.
       const uint32_t idesc = make_idesc_i8(kTileW * kG, static_cast<uint32_t>(p.block_t), true);
-      const uint64_t desc128 = make_smem_desc(0, 1024, 128);
+      const uint64_t desc_const = make_smem_desc(0, 1024, 128);
+      const uint32_t desc_hi = static_cast<uint32_t>(desc_const >> 32);
       const uint64_t desc_e = make_smem_desc(0, 128, 0);
+      const uint32_t a_lo0 = static_cast<uint32_t>(desc_const) | ((smem_base & 0x3FFFFu) >> 4);
+      const uint32_t stage_step = stage_bytes >> 4, e_off = kABytes >> 4, b_off = (kABytes + kEBytes) >> 4, b_box = b_half >> 4;
+      const uint32_t e_tmem = tmem_base + e_col;
       int stage = 0;
-      uint32_t phase = 0;
+      uint32_t phase = 0, a_lo = a_lo0;
       bool ok = true;
       int it = 0;
       for (int tile = first_tile; ok && tile < total_tiles; tile += tile_step, ++it) {
@@ -205,48 +210,41 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * p.block_t);
+        uint32_t acc = 0;   // the first MMA of a tile overwrites the accumulator
         for (int kb = 0; kb < p.num_kb; ++kb) {
-          ok = mbar_wait<true>(smem_u32(&ctrl->full[stage]), phase, abort_flag, kDevTimeoutFull);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          const uint32_t sa = smem_base + stage * stage_bytes;
-          const uint32_t se = sa + kABytes;
-          const uint32_t sb = se + kEBytes;
-          const uint64_t da = desc128 | static_cast<uint64_t>((sa & 0x3FFFFu) >> 4);
-          const uint64_t db0 = desc128 | static_cast<uint64_t>((sb & 0x3FFFFu) >> 4);
-          const uint64_t db1 = desc128 | static_cast<uint64_t>(((sb + b_half) & 0x3FFFFu) >> 4);
-          // Metadata of the stage: two 128-lane x 128-bit copies = 8 columns = four K=64 steps.
-          const uint64_t de0 = desc_e | static_cast<uint64_t>((se & 0x3FFFFu) >> 4);
-          const uint64_t de1 = desc_e | static_cast<uint64_t>(((se + kEBytes / 2) & 0x3FFFFu) >> 4);
-          if (issuer) {
-          if (kG == 1) {
-            tmem_cp_128x128b_1cta(tmem_base + e_col, de0);
-            tmem_cp_128x128b_1cta(tmem_base + e_col + 4, de1);
-          } else {
-            tmem_cp_128x128b_2cta(tmem_base + e_col, de0);
-            tmem_cp_128x128b_2cta(tmem_base + e_col + 4, de1);
+          const uint32_t bar = smem_u32(&ctrl->full[stage]);
+          ok = mbar_test_wait(bar, phase);
+          if (!__all_sync(0xffffffffu, ok)) {
+            if (!ok) ok = mbar_wait<true>(bar, phase, abort_flag, kDevTimeoutFull);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
           }
-          const int nk = (kb == p.num_kb - 1) ? p.last_ksteps : 4;
-          // Per K=64 instruction: 32 compressed bytes of A (+2 address units), 64 bytes of B
-          // (+4; the second 128-byte box after two steps) and two metadata columns.
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if (k < nk) {
-              const uint64_t dbk = k < 2 ? db0 + 4 * k : db1 + 4 * (k - 2);
-              if (kG == 1)
-                mma_sp_i8_1cta(d_tmem, da + 2 * k, dbk, tmem_base + e_col + 2 * k, idesc,
-                               (kb | k) != 0 ? 1u : 0u);
-              else
-                mma_sp_i8_2cta(d_tmem, da + 2 * k, dbk, tmem_base + e_col + 2 * k, idesc,
-                               (kb | k) != 0 ? 1u : 0u);
+          const int nk = kb == p.num_kb - 1 ? p.last_ksteps : 4;
+          if (elect_one()) {
+            // Metadata of the stage: two 128-lane x 128-bit copies = 8 columns = four K=64 steps.
+            const uint64_t de0 = desc_e | ((a_lo + e_off) & 0x3FFFu), de1 = desc_e | ((a_lo + e_off + (kEBytes >> 5)) & 0x3FFFu);
+            if (kG == 1) {
+              tmem_cp_128x128b_1cta(e_tmem, de0);
+              tmem_cp_128x128b_1cta(e_tmem + 4, de1);
+            } else {
+              tmem_cp_128x128b_2cta(e_tmem, de0);
+              tmem_cp_128x128b_2cta(e_tmem + 4, de1);
             }
+            // Per K=64 instruction: 32 compressed bytes of A (+2 address units), 64 bytes of B
+            // (+4; the second 128-byte box after two steps) and two metadata columns.
+            const uint32_t b_lo = a_lo + b_off;
+            mma_sp_i8_lohi<kG>(d_tmem, a_lo, b_lo, desc_hi, e_tmem, idesc, acc);
+            if (nk > 1) mma_sp_i8_lohi<kG>(d_tmem, a_lo + 2, b_lo + 4, desc_hi, e_tmem + 2, idesc, 1u);
+            if (nk > 2) mma_sp_i8_lohi<kG>(d_tmem, a_lo + 4, b_lo + b_box, desc_hi, e_tmem + 4, idesc, 1u);
+            if (nk > 3) mma_sp_i8_lohi<kG>(d_tmem, a_lo + 6, b_lo + b_box + 4, desc_hi, e_tmem + 6, idesc, 1u);
+            if (kG == 1) tc_commit_1cta(smem_u32(&ctrl->empty[stage]));
+            else tc_commit_2cta(smem_u32(&ctrl->empty[stage]), 3);
           }
-          if (kG == 1) tc_commit_1cta(smem_u32(&ctrl->empty[stage]));
-          else tc_commit_2cta(smem_u32(&ctrl->empty[stage]), 3);
-          }   // issuer
-          if (++stage == p.stages) { stage = 0; phase ^= 1; }
+          acc = 1u;
+          a_lo += stage_step;
+          if (++stage == p.stages) { stage = 0; phase ^= 1; a_lo = a_lo0; }
         }
-        if (ok && issuer) {
+        if (ok && elect_one()) {
           if (kG == 1) tc_commit_1cta(smem_u32(&ctrl->tmem_full[buf]));
           else tc_commit_2cta(smem_u32(&ctrl->tmem_full[buf]), 3);
         }
@@ -341,7 +339,7 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
           tmem_ld_16x256b_x4(t_row + c0, ra);
           tmem_ld_16x256b_x4(t_row + (16u << 16) + c0, rb);
           tmem_ld_wait();
-          if (lane == 0) tma_store_wait_read<0>();
+          if (elect_one()) tma_store_wait_read<0>();
           __syncwarp();
           // `as * ws` and the fused multiply-add of two neighbouring tokens of one weight row
           auto scaled = [&](uint32_t a0, uint32_t a1, float2 as2, int i) {
@@ -375,7 +373,7 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
           }
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) {
+          if (elect_one()) {
             const int out_col = geglu ? ((w0 + quarter * 32) >> 1) : (w0 + quarter * 32);
             const int out_row = t0 + c0;
             if (out_col < ldo && out_row < p.M) tma_store_2d(&tm_o, stage_buf, out_col * 2, out_row);
@@ -421,13 +419,13 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       }
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) {
+      if (elect_one()) {
         // The accumulator buffer goes back to the leader's MMA warp (own CTA or the peer).
         if (kG == 1 || leader) mbar_arrive(smem_u32(&ctrl->tmem_empty[buf]));
         else mbar_arrive_cluster(smem_u32(&ctrl->tmem_empty[buf]), 0);
       }
     }
-    if (p.tma_store && lane == 0) tma_store_wait_all<0>();
+    if (p.tma_store && elect_one()) tma_store_wait_all<0>();
   }
 
   // ---------------- teardown ----------------

@@ -148,7 +148,7 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
       tma_load_2d(sa + kTileW * 144, &tm_e, full, (ku0 + u) * 32 + 16, w0);
     }
   };
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     for (int u = 0; u < nku && u < p.stages; ++u) load_stage(u);
   }
 
@@ -232,12 +232,11 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
       ok = mbar_wait(smem_u32(&ctrl->empty[u % p.stages]), static_cast<uint32_t>(u / p.stages - 1) & 1u, abort_flag,
                      kDevTimeoutEmpty);
       ok = __all_sync(0xffffffffu, ok);
-      if (ok && lane == 0) load_stage(u);
+      if (ok && elect_one()) load_stage(u);
     }
     __syncwarp();
   } else if (warp == 1) {
     tc_fence_after_sync();
-    const bool issuer = lane == 0;
     const uint32_t idesc = make_idesc_i8(kTileW, static_cast<uint32_t>(p.block_t), kSparse);
     const uint64_t desc_const = make_smem_desc(0, 1024, 128);
     const uint32_t desc_hi = static_cast<uint32_t>(desc_const >> 32), lo_const = static_cast<uint32_t>(desc_const);
@@ -256,7 +255,7 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
         if (!ok) ok = mbar_wait<true>(full, phase, abort_flag, kDevTimeoutFull);
         if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
       }
-      if (issuer) {
+      if (elect_one()) {
         if (kSparse) {
           const uint32_t se = (a_lo & 0x3FFFu) + kTileW * 128 / 16;
           tmem_cp_128x128b_1cta(e_col, desc_e | se);
@@ -280,7 +279,7 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
       a_lo += kStage >> 4;
       if (++s == p.stages) { s = 0; phase ^= 1; a_lo = a_first; }
     }
-    if (ok && issuer) tc_commit_1cta(smem_u32(&ctrl->tmem_full));
+    if (ok && elect_one()) tc_commit_1cta(smem_u32(&ctrl->tmem_full));
     __syncwarp();
   }
 
@@ -355,7 +354,7 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
         }
       }
     }
-    if (lane == 0) tma_store_wait_read<0>();
+    if (elect_one()) tma_store_wait_read<0>();
     __syncwarp();
     auto scaled = [&](uint32_t a0, uint32_t a1, float2 as2, int i) {
       return __ffma2_rn(make_float2(static_cast<float>(static_cast<int32_t>(a0)), static_cast<float>(static_cast<int32_t>(a1))),
@@ -387,14 +386,14 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     }
     fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0) {
+    if (elect_one()) {
       const int out_col = geglu ? ((w0 + quarter * 32) >> 1) : (w0 + quarter * 32);
       const int out_row = t0 + s * kSlab;
       if (out_col < ldo && out_row < p.M) tma_store_2d(&tm_o, stage_buf, out_col * 2, out_row);
       tma_store_commit();
     }
   }
-  if (lane == 0) tma_store_wait_all<0>();
+  if (elect_one()) tma_store_wait_all<0>();
 
   // ---------------- teardown ----------------
   tc_fence_before_sync();
