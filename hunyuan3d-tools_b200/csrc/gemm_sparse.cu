@@ -272,6 +272,20 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       const int t0 = (tile / p.w_tiles) * p.block_t;
       const int n = w0 + row_in_tile;
       const bool n_ok = n < p.N;
+      // Which slabs a warp takes moves on from tile to tile: with a number of slabs that four does not divide (seven
+      // of 224 tokens) the same warps would always have one more.
+      const int first_slab = (half + it) & (kWarpsPerQuarter - 1);
+      bool arrived = false;
+      // The accumulator buffer goes back to the leader's MMA warp (own CTA or the peer) once this warp's loads have landed.
+      auto release_acc = [&]() {
+        tc_fence_before_sync();
+        __syncwarp();
+        if (elect_one()) {
+          if (kG == 1 || leader) mbar_arrive(smem_u32(&ctrl->tmem_empty[buf]));
+          else mbar_arrive_cluster(smem_u32(&ctrl->tmem_empty[buf]), 0);
+        }
+        arrived = true;
+      };
       float ws = 0.0f, bs = 0.0f;                            // direct stores: weight row n
       float wsr[4] = {0.0f, 0.0f, 0.0f, 0.0f}, bsr[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // fragment rows
       float sc_next = 0.0f;
@@ -279,8 +293,8 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         if (p.tma_store) {
           // Each warp stages the 32 token scales of its own slab (fetched one slab ahead), so
           // the tile needs no CTA-wide barrier.
-          const int t = t0 + half * kSlabTokens + lane;
-          if (half * kSlabTokens < p.block_t && t < p.M) sc_next = p.act_scale[t];
+          const int t = t0 + first_slab * kSlabTokens + lane;
+          if (first_slab * kSlabTokens < p.block_t && t < p.M) sc_next = p.act_scale[t];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int nr = w0 + quarter * 32 + (lane >> 2) + 8 * i;
@@ -325,7 +339,7 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         const uint32_t st_addr =
             geglu ? stage_buf + (8u * (st_mat >> 1) + st_row) * 32u + (((st_mat & 1u) ^ ((st_row >> 2) & 1u)) << 4)
                   : stage_buf + st_row * 64u + ((st_mat ^ ((st_row >> 1) & 3u)) << 4);
-        for (int s = half; s < nslab; s += kWarpsPerQuarter) {
+        for (int s = first_slab; s < nslab; s += kWarpsPerQuarter) {
           const int c0 = s * kSlabTokens;
           uint32_t ra[16], rb[16];
           const float sc = sc_next;
@@ -339,6 +353,7 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
           tmem_ld_16x256b_x4(t_row + c0, ra);
           tmem_ld_16x256b_x4(t_row + (16u << 16) + c0, rb);
           tmem_ld_wait();
+          if (s + kWarpsPerQuarter >= nslab) release_acc();
           if (elect_one()) tma_store_wait_read<0>();
           __syncwarp();
           // `as * ws` and the fused multiply-add of two neighbouring tokens of one weight row
@@ -417,14 +432,9 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
           }
         }
       }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (elect_one()) {
-        // The accumulator buffer goes back to the leader's MMA warp (own CTA or the peer).
-        if (kG == 1 || leader) mbar_arrive(smem_u32(&ctrl->tmem_empty[buf]));
-        else mbar_arrive_cluster(smem_u32(&ctrl->tmem_empty[buf]), 0);
-      }
+      if (!arrived) release_acc();
     }
+    __syncwarp();
     if (p.tma_store && elect_one()) tma_store_wait_all<0>();
   }
 
