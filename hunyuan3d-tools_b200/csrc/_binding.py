@@ -36,6 +36,7 @@ SIGNATURES = {
                              c_void_p, c_int, c_int64, c_int64, c_int64, c_int, c_int, c_int,
                              c_void_p],
     "hy3d_dense_splitk_plan": [c_int64, c_int64, c_int64, c_int, c_void_p],
+    "hy3d_dense_layer_splitk_plan": [c_int64, c_int64, c_int64, c_int, c_void_p],
     "hy3d_gemm_w8a8_dense_splitk": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p,
                                     c_int, c_int64, c_int64, c_int64, c_int, c_int, c_void_p, c_int64, c_void_p],
     "hy3d_linear_w8a8_dense": [c_void_p, c_int, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -84,7 +85,7 @@ SIGNATURES = {
 }
 
 # The argument lists above belong to this ABI version of the library (hy3d_version()).
-ABI_VERSION = 204
+ABI_VERSION = 205
 
 
 def configure(lib: ctypes.CDLL) -> ctypes.CDLL:

@@ -288,12 +288,18 @@ int hy3d_gemm_w8a8_dense(const int8_t* A, const int8_t* B, const float* act_scal
                     N, K, epilogue, cta_group, block_n, static_cast<cudaStream_t>(stream));
 }
 
-int hy3d_dense_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, int64_t* workspace_bytes) {
+static int splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, bool layer, int64_t* workspace_bytes) {
   if (check_device() != HY3D_OK) return 1;
-  const int splits = dense_splitk_plan(M, N, K, epilogue);
+  const int splits = dense_splitk_plan(M, N, K, epilogue, layer);
   // every K range owns an M-padded (whole 128-row tiles) int32 matrix
   if (workspace_bytes) *workspace_bytes = splits > 1 ? static_cast<int64_t>(splits) * ((M + 127) / 128 * 128) * N * 4 : 0;
   return splits;
+}
+int hy3d_dense_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, int64_t* workspace_bytes) {
+  return splitk_plan(M, N, K, epilogue, false, workspace_bytes);
+}
+int hy3d_dense_layer_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, int64_t* workspace_bytes) {
+  return splitk_plan(M, N, K, epilogue, true, workspace_bytes);
 }
 
 int hy3d_gemm_w8a8_dense_splitk(const int8_t* A, const int8_t* B, const float* act_scale,

@@ -11,7 +11,7 @@
 
 #include "../../include/hy3d_int8.h"
 
-#define HY3D_ABI_VERSION 204
+#define HY3D_ABI_VERSION 205
 
 namespace hy3d {
 

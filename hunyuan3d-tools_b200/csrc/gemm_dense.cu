@@ -823,51 +823,70 @@ splitk_reduce_kernel(const int32_t* __restrict__ partial, int splits, int64_t sp
   }
 }
 
+// Stages of A that fit beside a resident B tile (one staging buffer per epilogue warp), and the fewest that pay.
+constexpr int kResidentStages = 4;
+constexpr int64_t kDeepK = 1024;         // pairs take two K blocks a stage from here on
+int64_t resident_stages(int64_t b_tile_bytes) {
+  return (kSmemLimit - static_cast<int64_t>(sizeof(DenseCtrl)) - kEpiWarps * kSlabBytes - b_tile_bytes) / (kTileM * kBlockKBytes);
+}
+
 struct TilePlan {
   int block_n = 0, group = 0;
   double us = 0.0;
 };
 
 // Tile width and CTA grouping for a launch of `splits` K ranges, with its expected device time.  Pairs halve the
-// B traffic into shared memory, which is what bounds the tensor pipe on deep K, and cost more per hand-off; wide
-// tiles re-read A less often, narrow ones spread few tiles over the chip.  All of it from one cost model, in
-// microseconds: rounds of the persistent grid x (K blocks x the slower of issue and operand fill + the tile's
-// epilogue) + operand traffic through L2 + a fixed part.  Fitted to 210 shapes x all tiles (6 % rms); the tile it
-// picks is 0.5 % from the best on average (4 % with the rule before it: tiles of 128 to 256 columns by rounds x
-// (width + 94), pairs by thresholds on K and the tile count): 7215 x 4800 -> 816 30.7 -> 25.5 us,
-// 902 x 2816 -> 4480 13.4 -> 11.4, 348 x 896 -> 912 5.2 -> 4.6.
-TilePlan search_tile(int64_t M, int64_t N, int64_t K, bool geglu, int cta_group, int block_n, int splits) {
+// B traffic into shared memory, which is what bounds the tensor pipe on deep K, and cost more per launch and per gate;
+// a resident B tile removes it; wide tiles re-read A less often, narrow ones spread few tiles over the chip.  All of
+// it from one cost model, in microseconds: rounds of the persistent grid x (K blocks x the slower of issue and operand
+// fill + the tile's epilogue) + operand traffic through L2 + the output + a fixed part.  Fitted to 170 shapes of random
+// size with each epilogue x all tiles (7 % rms near the best tile); the tile it picks is 1.2 % from the best on average.
+// (The model before, fitted when a pair's hand-over cost 2000 cycles and resident B was for single CTAs, is 3.7 % off
+// with today's kernel: 12288 x 640 -> 1920 18.8 -> 16.3 us, 1879 x 4800 -> 1024 14.7 -> 12.0, 40560 x 640 -> 176
+// 11.3 -> 9.8, 257 x 1536 -> 6144 7.5 -> 6.8.)
+TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group, int block_n, int splits) {
+  // K block: a + b x width / 100, at least c; one row per way the operands come
+  struct Block { double a, b, least; };
+  constexpr Block kStream = {0.0914, 0.0552, 0.1382}, kResident = {0.0554, 0.0, 0.1394};        // single CTAs
+  constexpr Block kPair = {0.0849, 0.0496, 0.005}, kPairResident = {0.0233, 0.007, 0.1102}, kPairDeep = {0.0332, 0.0743, 0.091};
   TilePlan best;
   best.us = 1e30;
+  const bool geglu = epilogue == HY3D_EPI_GEGLU;
   const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
   const int step = geglu ? 64 : 32;
   const int64_t nk = ((K + kBlockKBytes - 1) / kBlockKBytes + splits - 1) / splits;
   for (int g = 1; g <= 2; ++g) {
-    if (cta_group != 0 ? g != cta_group : (g == 2 && (K < 1024 || splits > 1))) continue;
+    if (cta_group != 0 ? g != cta_group : (g == 2 && (M <= kTileM || splits > 1))) continue;
     for (int bn = 64; bn <= 256; bn += step) {
       const int w = block_n != 0 ? block_n : N <= 128 ? static_cast<int>(N) : bn;
       if (w != bn && bn != 64) break;                    // a width that is given: once per group
       if (w == bn && bn >= N + 32 && bn > 64) break;
       if (g == 2 && (w & 31) && cta_group == 0) continue;
-      const int64_t nt = (N + w - 1) / w;
-      const int64_t tiles = ((M + kTileM * g - 1) / (kTileM * g)) * nt * splits;
-      int64_t slots = sms / g;
-      if (nt > 1 && nt <= slots / 4) slots -= slots % nt;     // every CTA keeps one tile column, see the launch
+      const int64_t nt = (N + w - 1) / w, mt = (M + kTileM * g - 1) / (kTileM * g);
+      const int64_t tiles = mt * nt * splits;
+      int64_t slots = sms / g < tiles ? sms / g : tiles;
+      bool column_fixed = nt == 1;
+      if (nt > 1 && nt <= slots / 4) { slots -= slots % nt; column_fixed = true; }     // see the launch
       const double rounds = static_cast<double>((tiles + slots - 1) / slots);
-      const bool resident = g == 1 && splits == 1 && nt <= sms / 4 && tiles >= 2 * slots &&
-                            nk * w * kBlockKBytes + 4 * kTileM * kBlockKBytes + 33000 <= kSmemLimit;
+      const bool deep = g == 2 && K >= kDeepK;
+      const bool resident = !deep && splits == 1 && column_fixed && tiles >= 2 * slots &&
+                            resident_stages(nk * (w / g) * kBlockKBytes) >= kResidentStages;
+      const Block& kb = g == 1 ? (resident ? kResident : kStream) : deep ? kPairDeep : resident ? kPairResident : kPair;
       const double c = w / 100.0;
-      double block = g == 2 ? 0.148 + 0.031 * c : resident ? 0.050 + 0.030 * c : 0.072 + 0.070 * c;
-      const double least = g == 2 ? 0.019 : resident ? 0.220 : 0.207;
-      if (block < least) block = least;
-      const double operand = tiles * g * static_cast<double>(nk) * kBlockKBytes * (kTileM + (resident ? 0.0 : static_cast<double>(w) / g)) / 1e7;
-      double us = 3.09 + rounds * (static_cast<double>(nk) * block + 0.124 + 0.423 * c) + 0.078 * operand + (g == 2 ? 1.19 : 0.0);
+      double block = kb.a + kb.b * c;
+      if (block < kb.least) block = kb.least;
+      if (M < kTileM) block += 0.0016 * (1.0 - static_cast<double>(M) / kTileM) * static_cast<double>(nt);   // many CTAs, few lines of A
+      const double gate = geglu ? (g == 2 ? 2.59 : 2.39) : epilogue == HY3D_EPI_GELU ? 2.65 : 1.0;
+      const double rows = static_cast<double>(M) / static_cast<double>(mt * g);
+      const double operand = static_cast<double>(tiles * g * nk) * kBlockKBytes *
+                             ((rows < kTileM ? rows : kTileM) + (resident ? 0.0 : static_cast<double>(w) / g)) / 1e7;
+      double us = 2.98 + (g == 1 ? 0.0 : deep ? 0.76 : resident ? 1.09 : 0.46) +
+                  rounds * (static_cast<double>(nk) * block + (g == 1 ? 0.282 : 0.292) * c * gate) + 0.136 * operand +
+                  (resident ? 0.092 * static_cast<double>(nk) * c / g : 0.0) +
+                  0.068 * static_cast<double>(M) * static_cast<double>(N) * (geglu ? 1.0 : 2.0) / 1e6;
       // A CTA does not fit beside a quantiser's, so a grid that wants nearly every SM starts late behind one: it
       // needs a few SMs to spare (257 x 1536 -> 4608, whole layer: 144 tiles 9.0 us, 108 tiles 8.1).
       if (splits == 1 && rounds == 1.0 && tiles * g * 5 > sms * 4) us += 0.7;
-      // Pairs lean less on L2, which the real operands' traffic shares: they win where the model sees them equal
-      // (49152 x 1280 -> 320 in the layer: 61.0 -> 58.6 us).
-      if (g == 2 && rounds >= 4.0) us *= 0.985;
       if (us < best.us) { best.us = us; best.block_n = w; best.group = g; }
     }
   }
@@ -888,42 +907,47 @@ struct Memo {
   }
 };
 
-TilePlan plan_tile(int64_t M, int64_t N, int64_t K, bool geglu, int cta_group, int block_n, int splits) {
+TilePlan plan_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group, int block_n, int splits) {
   static thread_local Memo<TilePlan> memo;
-  const int64_t rest = (geglu ? 1 : 0) | cta_group << 1 | block_n << 3 | static_cast<int64_t>(splits) << 12;
-  return memo.get(M, N, K, rest, [&] { return search_tile(M, N, K, geglu, cta_group, block_n, splits); });
+  const int64_t rest = epilogue | cta_group << 2 | block_n << 4 | static_cast<int64_t>(splits) << 13;
+  return memo.get(M, N, K, rest, [&] { return search_tile(M, N, K, epilogue, cta_group, block_n, splits); });
 }
 
 // What the calling thread spends on a layer of two launches (quantise, GEMM) and of three (and a reduction).
 constexpr double kTwoLaunchesUs = 7.5, kThreeLaunchesUs = 10.0;
 
 struct LayerPlan {
-  int splits = 1;
+  int splits = 1;        // K ranges of a layer
+  int gemm_splits = 1;   // what hy3d_dense_splitk_plan answers
   double us = 0.0;
 };
 
 // Split-K plan and expected time of a whole layer, quantisation included: the greater of the device's time and the
 // calling thread's.  A split pays one more launch, and every range writes and re-reads an M-padded int32 matrix
-// (~11 TB/s, it stays in L2).  Fitted to 130 layers of random size x all splits (0.6 us rms).
-//   257 x 6144 -> 1536 13.4 -> 11.0 us (GEMM), 132 x 4160 -> 1200 9.9 -> 8.2, 200 x 5952 -> 2992 13.4 -> 11.5
+// (~12 TB/s, it stays in L2).  Fitted to 90 layers of random size x all splits (0.8 us rms).  The single launch has
+// caught up since its MMAs are issued by an elected thread (257 x 6144 -> 1536, layer: 11.9 us against 12.0 in three
+// ranges; 13.8 and 13.7 before), so few layers split any more (512 x 8192 -> 1024 does).  A caller that asks for the
+// GEMM's plan is still told a split that is within 11 % of the single launch, as it was before.
 LayerPlan search_layer(int64_t M, int64_t N, int64_t K) {
   const int64_t num_kb = (K + kBlockKBytes - 1) / kBlockKBytes;
   const int64_t part_rows = (M + kTileM - 1) / kTileM * kTileM;
   const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
   const double act = static_cast<double>(M) * K / 1e6, weights = static_cast<double>(N) * K / 1e7;
   LayerPlan best;
-  best.us = 0.9 + search_tile(M, N, K, false, 0, 0, 1).us + 0.46 * act + 1.7 * weights;
-  if (best.us < kTwoLaunchesUs) best.us = kTwoLaunchesUs;
-  if (best.us <= kThreeLaunchesUs || num_kb < 16 || part_rows / kTileM * ((N + 255) / 256) * 2 > sms) return best;
-  const double part_us = 0.21 + 0.09 * static_cast<double>(part_rows) * N * 8.0 / 1e6;
-  const double single_us = best.us;
-  best.us *= 0.9;                                   // a split has to be worth its workspace
+  const double single_us = 0.39 + 1.18 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0, 0, 1).us + 0.36 * act + 0.07 * weights;
+  best.us = single_us > kTwoLaunchesUs ? single_us : kTwoLaunchesUs;
+  if (num_kb < 16 || part_rows / kTileM * ((N + 255) / 256) * 2 > sms) return best;
+  const double part_us = 0.21 + 0.078 * static_cast<double>(part_rows) * N * 8.0 / 1e6;
+  double gemm_us = 1.11 * single_us, layer_us = 0.97 * best.us;      // a split has to be worth its workspace
   for (int sp = 2; sp <= 16 && static_cast<int64_t>(sp) * 4 <= num_kb; ++sp) {
-    double us = 2.8 + search_tile(M, N, K, false, 1, 0, sp).us + sp * part_us + 0.42 * act + weights;
-    if (us < kThreeLaunchesUs) us = kThreeLaunchesUs + 0.01 * us;
-    if (us < best.us) { best.us = us; best.splits = sp; }
+    const double us = 3.48 + 0.98 * search_tile(M, N, K, HY3D_EPI_LINEAR, 1, 0, sp).us + sp * part_us + 0.35 * act + 0.45 * weights;
+    if (us < gemm_us) { gemm_us = us; best.gemm_splits = sp; }
+    if (us > kThreeLaunchesUs ? us < layer_us : kThreeLaunchesUs < layer_us) {
+      layer_us = us > kThreeLaunchesUs ? us : kThreeLaunchesUs;
+      best.splits = sp;
+    }
   }
-  if (best.splits == 1) best.us = single_us;
+  if (best.splits > 1) best.us = layer_us;
   return best;
 }
 
@@ -937,9 +961,10 @@ LayerPlan plan_layer(int64_t M, int64_t N, int64_t K) {
 // Split-K plan for a dense layer: how many K ranges pay (1 = none).  Splitting serves launches
 // whose tiles leave most SMs idle while each tile walks a long K alone (the M = 257 image-encoder
 // layers with K = 6144): the ranges run side by side and a second small kernel adds them up.
-int dense_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue) {
+int dense_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, bool layer) {
   if (epilogue == HY3D_EPI_GEGLU || (N & 7) || M <= 0 || N <= 0 || K <= 0) return 1;
-  return plan_layer(M, N, K).splits;
+  const LayerPlan p = plan_layer(M, N, K);
+  return layer ? p.splits : p.gemm_splits;
 }
 
 // Expected time of a layer that quantises and multiplies in separate launches, in microseconds.
@@ -975,7 +1000,7 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
 
   int group = cta_group;
   if (block_n == 0 || group == 0) {
-    const TilePlan t = plan_tile(M, N, K, geglu, cta_group, block_n, splits);
+    const TilePlan t = plan_tile(M, N, K, epilogue, cta_group, block_n, splits);
     block_n = t.block_n;
     group = t.group;
 #ifdef HY3D_TRACE
@@ -1003,7 +1028,7 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
   // Deep stages (two 128-byte K blocks, eight MMAs per barrier round trip) for CTA pairs on
   // deep K: a pair's per-stage hand-off crosses the cluster, and halving the number of
   // hand-offs is what lets pairs profit from their smaller shared-memory traffic.
-  const int atoms = (group == 2 && K >= 1024 && splits == 1) ? 2 : 1;
+  const int atoms = (group == 2 && K >= kDeepK && splits == 1) ? 2 : 1;
   p.atoms = atoms;
   const int stage_k = kBlockKBytes * atoms;
   p.num_kb = static_cast<int>((K + stage_k - 1) / stage_k);
@@ -1065,8 +1090,8 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
     // One staging buffer per epilogue warp: measured faster than two here (a warp that must
     // wait for its previous store to leave shared memory paces the store stream, and the
     // loads queue behind fewer stores).
-    const int st = (kSmemLimit - ctrl_bytes - staging1 - b_tile_bytes) / a_stage;
-    if (st >= 4) { b_resident = 1; store_bufs = 1; stages = st; stage_bytes = a_stage; }
+    const int st = static_cast<int>(resident_stages(b_tile_bytes));
+    if (st >= kResidentStages) { b_resident = 1; store_bufs = 1; stages = st; stage_bytes = a_stage; }
   }
 #if defined(HY3D_TRACE) || defined(HY3D_KO)
   if (const char* e = getenv("HY3D_B_RESIDENT")) { if (!atoi(e)) b_resident = 0; }

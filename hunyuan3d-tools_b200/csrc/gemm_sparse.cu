@@ -459,18 +459,18 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 // Tile shape.  CTA pairs (256 weight rows sharing one token tile) halve each CTA's activation traffic into
 // shared memory, which is what paces deep-K stages, and cost more per tile hand-off; a wide token tile
 // amortises the weights, a narrow one spreads few tokens over the chip.  Both come from one cost model, in
-// microseconds, fitted to 98 shapes x all tiles (7 % rms; the tile it picks is 1 % from the best on average,
-// where a fixed threshold for pairs and tiles of 128 tokens or more were 10 %):
-//   2335 x 4864 -> 688: 12.3 -> 10.6 us, 3451 x 3328 -> 640: 15.1 -> 8.7, 279 x 704 -> 1120: 4.8 -> 4.0
+// microseconds, fitted to 120 shapes of random size with each epilogue x all tiles (7 % rms); the tile it picks is
+// 0.6 % from the best on average (the model before, fitted when a pair's hand-over cost 2000 cycles: 1.3 %):
+//   2915 x 5120 -> 1296 with GELU: single CTAs of 128 tokens 21.1 us, pairs of 128 17.8
 struct SparseTile {
   int block_t = 0, group = 1;
   double us = 1e30;
 };
-SparseTile search_tile(int64_t M, int64_t N, int64_t K, int block_t) {
+SparseTile search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int block_t) {
   SparseTile best;
   const int64_t kblocks = (K + kBlockK - 1) / kBlockK;
   const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
-  for (int g = 1; g <= (K >= 1024 ? 2 : 1); ++g) {
+  for (int g = 1; g <= 2; ++g) {
     for (int bt = 32; bt <= 224; bt += 32) {
       if (block_t != 0 && bt != 32) break;             // the caller's width, one pass per group
       const int t = block_t != 0 ? block_t : bt;
@@ -480,11 +480,12 @@ SparseTile search_tile(int64_t M, int64_t N, int64_t K, int block_t) {
       const double tiles = static_cast<double>((N + kTileW * g - 1) / (kTileW * g)) * static_cast<double>((M + t - 1) / t);
       const double rounds = static_cast<double>((static_cast<int64_t>(tiles) + sms / g - 1) / (sms / g));
       const double w = t / 100.0;
-      double stage = g == 1 ? 0.196 + 0.130 * w : 0.327 + 0.036 * w;
-      const double floor_us = g == 1 ? 0.273 : 0.351;
-      if (stage < floor_us) stage = floor_us;
+      double stage = g == 1 ? 0.179 + 0.159 * w : 0.223 + 0.058 * w;
+      if (g == 1 && stage < 0.256) stage = 0.256;
+      const double gate = epilogue == HY3D_EPI_GEGLU ? 1.79 : epilogue == HY3D_EPI_GELU ? 2.23 : 1.0;
       const double operand_mb = tiles * g * static_cast<double>(kblocks) * (kABytes + kEBytes + 256.0 * t / g) / 1e7;
-      const double us = 3.0 + rounds * (static_cast<double>(kblocks) * stage + 0.08 + 0.55 * w) + 0.096 * operand_mb + (g == 2 ? 0.61 : 0.0);
+      const double us = 2.98 + rounds * (static_cast<double>(kblocks) * stage + (g == 1 ? 0.253 : 0.403) * w * gate) + 0.071 * operand_mb +
+                        (g == 2 ? 0.56 : 0.0) + 0.1 * static_cast<double>(M) * static_cast<double>(N) * (epilogue == HY3D_EPI_GEGLU ? 1.0 : 2.0) / 1e6;
       if (us < best.us) { best.us = us; best.block_t = t; best.group = g; }
     }
   }
@@ -496,7 +497,7 @@ SparseTile search_tile(int64_t M, int64_t N, int64_t K, int block_t) {
 // Expected time of a layer that quantises and multiplies in separate launches, in microseconds: the greater of
 // the device's and the calling thread's (7.5), fitted to 110 layers of random size (0.2 us rms).
 double sparse_layer_us(int64_t M, int64_t N, int64_t K) {
-  const double us = 1.271 * search_tile(M, N, K, 0).us + 0.424 * static_cast<double>(M) * K / 1e6 - 0.08;
+  const double us = 1.271 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0).us + 0.424 * static_cast<double>(M) * K / 1e6 - 0.08;
   return us > 7.5 ? us : 7.5;
 }
 
@@ -522,7 +523,7 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
        reinterpret_cast<uintptr_t>(w_meta) | reinterpret_cast<uintptr_t>(out)) & 15)
     return HY3D_ERR_SHAPE;
 
-  const SparseTile tile = search_tile(M, N, K, block_t);
+  const SparseTile tile = search_tile(M, N, K, epilogue, block_t);
   block_t = tile.block_t;
   int group = tile.group;
 #ifdef HY3D_TRACE

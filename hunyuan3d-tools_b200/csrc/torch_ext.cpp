@@ -34,7 +34,7 @@ namespace {
 struct Api {
   HY3D_FN(hy3d_linear_w8a8_dense);
   HY3D_FN(hy3d_gemm_w8a8_dense);
-  HY3D_FN(hy3d_dense_splitk_plan);
+  HY3D_FN(hy3d_dense_layer_splitk_plan);
   HY3D_FN(hy3d_gemm_w8a8_dense_splitk);
   HY3D_FN(hy3d_quantize_rows);
   HY3D_FN(hy3d_linear_cluster_plan);
@@ -149,7 +149,7 @@ bool one_launch(int64_t M, int64_t N, int64_t K, int sparse, int* block_t, int* 
 int dense_gemm(const int8_t* q, const float* s, const at::Tensor& w, const Params& p, void* out, int out_code,
                int64_t M, int64_t N, int64_t K, int epi, cudaStream_t st) {
   int64_t bytes = 0;
-  const int splits = p.may_split() ? api.hy3d_dense_splitk_plan(M, N, K, epi, &bytes) : 1;
+  const int splits = p.may_split() ? api.hy3d_dense_layer_splitk_plan(M, N, K, epi, &bytes) : 1;
   if (splits > 1) {
     Scratch part(static_cast<size_t>(bytes), st);
     return api.hy3d_gemm_w8a8_dense_splitk(q, w.const_data_ptr<int8_t>(), s, p.ws, p.ws_code, p.bias, p.bias_code,
@@ -185,7 +185,7 @@ PyObject* linear_dense_impl(PyObject* px, PyObject* pw, PyObject* pscale, PyObje
   const size_t codes = align256(static_cast<size_t>(M) * K);
   Scratch ws(codes + static_cast<size_t>(M) * 4, st);
   int64_t bytes = 0;
-  if (p.may_split() && api.hy3d_dense_splitk_plan(M, N, K, static_cast<int>(epi), &bytes) > 1) {
+  if (p.may_split() && api.hy3d_dense_layer_splitk_plan(M, N, K, static_cast<int>(epi), &bytes) > 1) {
     rc = api.hy3d_quantize_rows(x->const_data_ptr(), code, M, K, K, ws.at(0), reinterpret_cast<float*>(ws.at(codes)), st);
     if (rc == HY3D_OK)
       rc = dense_gemm(ws.at(0), reinterpret_cast<float*>(ws.at(codes)), *w, p, y.mutable_data_ptr(), code, M, N, K,
@@ -823,7 +823,7 @@ PyObject* open_library(PyObject*, PyObject* arg) {
   } while (0)
   HY3D_SYM(hy3d_linear_w8a8_dense);
   HY3D_SYM(hy3d_gemm_w8a8_dense);
-  HY3D_SYM(hy3d_dense_splitk_plan);
+  HY3D_SYM(hy3d_dense_layer_splitk_plan);
   HY3D_SYM(hy3d_gemm_w8a8_dense_splitk);
   HY3D_SYM(hy3d_quantize_rows);
   HY3D_SYM(hy3d_linear_cluster_plan);

@@ -203,6 +203,8 @@ int hy3d_gemm_w8a8_dense(const int8_t* A, const int8_t* B, const float* act_scal
  * (csrc/int8_sparse_tc.cu:1730-1732 cost terms, split-K reduce) in the dense kernel's terms.
  */
 int hy3d_dense_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, int64_t* workspace_bytes);
+/* The same for a whole layer, quantisation and the calling thread's launches counted: what the layers here take. */
+int hy3d_dense_layer_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, int64_t* workspace_bytes);
 int hy3d_gemm_w8a8_dense_splitk(const int8_t* A, const int8_t* B, const float* act_scale,
                                 const void* w_scale, int w_scale_dtype,
                                 const void* bias, int bias_dtype,

@@ -144,6 +144,26 @@ def test_dense_resident_b_tile_bit_exact(tc, M, K, N, bn):
 
 
 @pytest.mark.parametrize("M,K,N,bn", [
+    (40000, 320, 320, 160),   # two columns of pairs, K ends in half a block
+    (38001, 640, 1280, 256),  # five columns, five K blocks, six A stages; ragged last row tile
+    (39000, 976, 192, 192),   # one column, seven blocks and a K step: the fewest A stages beside them
+    (38100, 336, 176, 0),     # the library's own choice; last K block of one step, columns clipped
+])
+def test_dense_resident_b_tile_of_pairs_bit_exact(tc, M, K, N, bn):
+    """CTA pairs that keep their tile column hold half of the B tile each (K < 1024): integer sums of the oracle, and
+    the same bits as single CTAs that stream both operands."""
+    A, B = _rand_i8((M, K), M + K + 7), _rand_i8((N, K), N + K + 8)
+    acc = tc.int8_gemm_tc(A.to(DEV), B.to(DEV), None, None, None, out_dtype=torch.int32, cta_group=2, block_n=bn)
+    assert torch.equal(acc.cpu(), O.int32_matmul(A, B))
+    g = torch.Generator().manual_seed(M)
+    a_s, w_s = torch.rand(M, generator=g) * 0.05 + 1e-3, (torch.rand(N, generator=g) * 1e-3 + 1e-5).bfloat16()
+    y = [tc.int8_gemm_tc(A.to(DEV), B.to(DEV), a_s.to(DEV), w_s.to(DEV), None, out_dtype=torch.bfloat16, cta_group=c,
+                         block_n=b) for c, b in ((2, bn), (0, 0), (1, 256))]
+    assert torch.equal(y[0], y[1]) and torch.equal(y[0], y[2])
+    assert tc.device_status() == 0
+
+
+@pytest.mark.parametrize("M,K,N,bn", [
     (2600, 2064, 512, 0),     # K = 8 deep stages + a 16-element tail; ragged last row tile
     (300, 1024, 256, 256),    # exactly four deep stages, second CTA's rows half empty
     (1000, 1104, 320, 160),   # tail of 80: three K steps of the first block
