@@ -246,30 +246,38 @@ class Int8Linear(nn.Module):
     # -- construction ------------------------------------------------------------------
     @staticmethod
     def _assemble(linear, dt, codes, scale, comp=None, meta=None) -> "Int8Linear":
-        """A layer around finished buffers, without the placeholder tensors of ``__init__``."""
+        """A layer around finished buffers, without the placeholder tensors of ``__init__``.  The plain attributes go
+        straight into ``__dict__``: ``nn.Module.__setattr__`` looks through parameters, buffers and modules first, which
+        for six of them is a third of what a layer's conversion costs the calling thread."""
         layer = Int8Linear.__new__(Int8Linear)
-        layer._init_sizes(linear.in_features, linear.out_features)
-        b = layer._buffers
+        nn.Module.__init__(layer)
+        d = layer.__dict__
+        k, n = linear.in_features, linear.out_features
+        d["in_features"], d["out_features"] = k, n
+        d["_tc_ok"] = d["_sparse_ok"] = k % 64 == 0 and n % 16 == 0
+        b = d["_buffers"]
         b["weight_int8_nk"], b["weight_scale"] = codes, scale
         b["weight_sparse_comp"], b["weight_sparse_meta"] = comp, meta
-        if linear.bias is not None:
-            b["bias"] = linear.bias.data.to(dt)
+        bias = linear.bias
+        if bias is not None:
+            bias = bias.data
+            b["bias"] = bias if bias.dtype is dt else bias.to(dt)
         else:
-            layer.bias = None
+            d["bias"] = None
         if comp is not None:
-            layer.mode = "sparse"
+            d["mode"] = "sparse"
         return layer
 
     @staticmethod
     def from_linear(linear: nn.Linear) -> "Int8Linear":
         """Per-channel quantisation of an ``nn.Linear`` (reference: quantize_utils.py:203-223)."""
-        has_bias = linear.bias is not None
-        dt = _param_dtype(linear)
         weight = linear.weight
         if weight.is_cuda:
             got = (_NATIVE or _load_native()).quantize_weight(weight, False)
-            if got is not None:
-                return Int8Linear._assemble(linear, dt, got[0], got[1])
+            if got is not None:      # (codes, scales in the layer's type)
+                return Int8Linear._assemble(linear, got[1].dtype, got[0], got[1])
+        has_bias = linear.bias is not None
+        dt = _param_dtype(linear)
         layer = Int8Linear(linear.in_features, linear.out_features, bias=has_bias, dtype=dt)
         weight_f32 = weight.data.float()
         # Same expressions as the reference, evaluated on the weight's device.  (On CUDA torch
@@ -289,16 +297,17 @@ class Int8Linear(nn.Module):
         """2:4-sparse conversion (reference: quantize_utils.py:226-260): quantise with the
         scale of the UNPRUNED row, then prune on int8 magnitudes, compress and pack on the
         GPU."""
-        has_bias = linear.bias is not None
-        dt = _param_dtype(linear)
-        device = linear.weight.device
-        if device.type != "cuda":
+        weight = linear.weight
+        if not weight.is_cuda:
             raise RuntimeError("from_linear_sparse needs the layer on a CUDA device "
                                "(pruning and packing run on the GPU)")
-        got = (_NATIVE or _load_native()).quantize_weight(linear.weight, True)
-        if got is not None:
-            return Int8Linear._assemble(linear, dt, torch.empty(0, dtype=torch.int8, device=device), got[2],
-                                        got[0], got[1])
+        got = (_NATIVE or _load_native()).quantize_weight(weight, True)
+        if got is not None:          # its scales have the layer's type; no dense codes
+            comp, meta, scale = got
+            return Int8Linear._assemble(linear, scale.dtype, comp.new_empty(0), scale, comp, meta)
+        has_bias = linear.bias is not None
+        dt = _param_dtype(linear)
+        device = weight.device
         sp_mod = _load_sp()
         layer = Int8Linear(linear.in_features, linear.out_features, bias=has_bias, dtype=dt)
         weight_f32 = linear.weight.data.float()
