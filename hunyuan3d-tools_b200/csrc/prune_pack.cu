@@ -114,6 +114,13 @@ __device__ __forceinline__ float max_nan(float a, float b) {
   return r;
 }
 
+// The same for two 16-bit values at once, into a running pair of maxima whose signs mean nothing.
+template <int kType>
+__device__ __forceinline__ void absmax_nan2(uint32_t w, uint32_t& acc) {
+  if (kType == HY3D_BF16) asm("max.NaN.xorsign.abs.bf16x2 %0, %0, %1;" : "+r"(acc) : "r"(w));
+  else asm("max.NaN.xorsign.abs.f16x2 %0, %0, %1;" : "+r"(acc) : "r"(w));
+}
+
 // Sixteen bytes of weights as floats: 8 values of a 16-bit type, 4 of fp32.
 template <int kType>
 __device__ __forceinline__ void widen16(const uint4& v, float (&f)[kType == HY3D_F32 ? 4 : 8]) {
@@ -146,9 +153,11 @@ __device__ __forceinline__ void quotient2(float2 w, float scale, float inv, uint
 }
 
 // Per-output-channel quantisation of a weight matrix, optionally 2:4 pruned and packed, in one pass
-// over HBM.  G threads share a row: 16-byte loads for the row's absmax, then every thread quantises
-// 32 adjacent K elements at a time from L1 / L2 and writes 32 codes, or 16 survivors and one metadata
-// word.  The arithmetic is torch's, operation by operation, so the buffers equal those of the torch
+// over HBM.  G threads share a row: 16-byte loads for the row's absmax (two 16-bit values an instruction), then every
+// thread quantises eight adjacent K elements at a time and writes 8 codes, or 4 survivors and the byte of
+// metadata that four lanes put together to a word.  Neighbouring lanes take neighbouring elements: loads and
+// stores are contiguous, and a row of 1280 fills a warp five times (in pieces of 32 elements a thread it was two
+// rounds, the second a quarter full).  The arithmetic is torch's, operation by operation, so the buffers equal those of the torch
 // expressions: |w| max; dense: max(amax * (1/127), 1e-8), sparse: max(amax, 1e-8) * (1/127) (torch on
 // CUDA multiplies by the reciprocal of a Python divisor); rint of the IEEE quotient w / scale.
 // The quotient comes from the correctly rounded reciprocal and two residual corrections, two values per
@@ -156,10 +165,13 @@ __device__ __forceinline__ void quotient2(float2 w, float scale, float inv, uint
 // functions on the IBM RISC System/6000 processor", 1990) the second then gives the correctly rounded
 // one.  |w| <= amax keeps the code within +-127.  Rows whose scale is not finite (a NaN or an infinity
 // among the weights) divide one by one; a NaN quotient becomes 0 as in torch's cast.
-// Bound by instruction issue (29 slots a weight with pruning, the ALU pipe two thirds busy).  10240 x 1280 bf16 with pruning: the
-// torch form, 11 launches over fp32 temporaries, took 160 us, this kernel with __fdiv_rn 26.8 us.
-template <int kType, bool kSparse>
-__global__ void __launch_bounds__(256)
+// Bound by instruction issue, most of it the pruning network on the half-rate ALU pipe.  10240 x 1280 bf16 with pruning:
+// the torch form, 11 launches over fp32 temporaries, took 160 us, pieces of 32 elements a thread 17.2 us (12.5
+// without pruning), this kernel 13.9 (9.1), of which 6 are HBM time; fp32 26.6 -> 19.5 (27.2 -> 17.0).
+// kKeep > 0 (16-bit types): a thread has at most that many vectors of its row and keeps them in registers between the
+// two passes; otherwise (fp32, rows of more than 16384) the second pass reads them again.
+template <int kType, bool kSparse, int kKeep>
+__global__ void __launch_bounds__(256, kKeep > 5 ? 4 : 5)
 quantize_weight_kernel(const void* __restrict__ w, int64_t N, int K, int8_t* __restrict__ codes,
                        uint32_t* __restrict__ meta, int meta_ld, void* __restrict__ scale_out, int scale_dtype, int G) {
   constexpr int kPer = kType == HY3D_F32 ? 4 : 8;       // elements of a 16-byte vector
@@ -169,13 +181,41 @@ quantize_weight_kernel(const void* __restrict__ w, int64_t N, int K, int8_t* __r
   const bool ok = row < N;
   const uint4* src = reinterpret_cast<const uint4*>(w) + (ok ? row : 0) * (K / kPer);
   float amax = 0.0f;
+  uint4 kept[kKeep > 0 ? kKeep : 1];
   if (ok) {
+    if constexpr (kType == HY3D_F32) {
 #pragma unroll 4
-    for (int c = sub; c < K / kPer; c += G) {
-      float f[kPer];
-      widen16<kType>(__ldg(src + c), f);
+      for (int c = sub; c < K / kPer; c += G) {
+        float f[kPer];
+        widen16<kType>(__ldg(src + c), f);
 #pragma unroll
-      for (int j = 0; j < kPer; ++j) amax = max_nan(amax, fabsf(f[j]));
+        for (int j = 0; j < kPer; ++j) amax = max_nan(amax, fabsf(f[j]));
+      }
+    } else {
+      uint32_t acc = 0;
+      auto fold = [&](const uint4& v) {
+        absmax_nan2<kType>(v.x, acc);
+        absmax_nan2<kType>(v.y, acc);
+        absmax_nan2<kType>(v.z, acc);
+        absmax_nan2<kType>(v.w, acc);
+      };
+      if constexpr (kKeep > 0) {
+#pragma unroll
+        for (int i = 0; i < kKeep; ++i)
+          kept[i] = sub + i * G < K / kPer ? __ldcs(src + sub + i * G) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int i = 0; i < kKeep; ++i) fold(kept[i]);
+      } else {
+#pragma unroll 4
+        for (int c = sub; c < K / kPer; c += G) fold(__ldg(src + c));
+      }
+      acc &= 0x7FFF7FFFu;
+      if constexpr (kType == HY3D_BF16) {
+        amax = max_nan(__uint_as_float(acc << 16), __uint_as_float(acc & 0xFFFF0000u));
+      } else {
+        const float2 t = __half22float2(*reinterpret_cast<const __half2*>(&acc));
+        amax = max_nan(t.x, t.y);
+      }
     }
   }
   for (int off = 16; off > 0; off >>= 1) amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, off));
@@ -196,47 +236,55 @@ quantize_weight_kernel(const void* __restrict__ w, int64_t N, int K, int8_t* __r
   }
   const bool finite = scale < __int_as_float(0x7F800000);   // false for NaN too
   const float inv = __frcp_rn(scale);
-  const int chunks = K >> 5;
-  for (int chunk = sub; chunk < (kSparse ? meta_ld : chunks); chunk += G) {
-    if (kSparse && chunk >= chunks) {       // padding word: any valid 2:4 pattern (indices 0,1)
-      meta[row * meta_ld + chunk] = 0x44444444u;
-      continue;
-    }
-    uint32_t words[8];
+  // K / 8 is a multiple of four, so the four lanes of a metadata word are in range together; every lane of a warp
+  // walks the same rounds.
+  const int units = K >> 3;
+  auto work = [&](int u, auto vector) {
+    const bool in = u < units;
+    uint32_t words[2] = {0, 0};
+    if (in) {
 #pragma unroll
-    for (int v = 0; v < 32 / kPer; ++v) {
-      float f[kPer];
-      widen16<kType>(__ldg(src + chunk * (32 / kPer) + v), f);
+      for (int v = 0; v < 8 / kPer; ++v) {
+        float f[kPer];
+        widen16<kType>(vector(v), f);
 #pragma unroll
-      for (int j = 0; j < kPer; j += 4) {
-        uint32_t b[4];
-        if (finite) {
-          quotient2(make_float2(f[j], f[j + 1]), scale, inv, b[0], b[1]);
-          quotient2(make_float2(f[j + 2], f[j + 3]), scale, inv, b[2], b[3]);
-        } else {
+        for (int j = 0; j < kPer; j += 4) {
+          uint32_t b[4];
+          if (finite) {
+            quotient2(make_float2(f[j], f[j + 1]), scale, inv, b[0], b[1]);
+            quotient2(make_float2(f[j + 2], f[j + 3]), scale, inv, b[2], b[3]);
+          } else {
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            b[u] = static_cast<uint32_t>(max(-128, min(127, __float2int_rn(__fdiv_rn(f[j + u], scale)))));
+            for (int t = 0; t < 4; ++t)
+              b[t] = static_cast<uint32_t>(max(-128, min(127, __float2int_rn(__fdiv_rn(f[j + t], scale)))));
+          }
+          words[(v * kPer + j) >> 2] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
         }
-        words[(v * kPer + j) >> 2] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
       }
     }
     if constexpr (kSparse) {
-      uint32_t packed = 0, out[4] = {0, 0, 0, 0};
-#pragma unroll
-      for (int g = 0; g < 8; ++g) {
-        uint32_t two;
-        packed |= prune_word(words[g], two) << (4 * g);
-        out[g >> 1] |= two << (16 * (g & 1));
-      }
-      *reinterpret_cast<uint4*>(codes + row * (K >> 1) + (chunk << 4)) = make_uint4(out[0], out[1], out[2], out[3]);
-      meta[row * meta_ld + chunk] = packed;
-    } else {
-      uint4* dst = reinterpret_cast<uint4*>(codes + row * static_cast<int64_t>(K) + (chunk << 5));
-      dst[0] = make_uint4(words[0], words[1], words[2], words[3]);
-      dst[1] = make_uint4(words[4], words[5], words[6], words[7]);
+      uint32_t two0, two1;
+      const uint32_t n0 = prune_word(words[0], two0), n1 = prune_word(words[1], two1);
+      if (in) *reinterpret_cast<uint32_t*>(codes + row * (K >> 1) + 4 * u) = two0 | two1 << 16;
+      uint32_t packed = (n0 | n1 << 4) << (8 * (sub & 3));
+      packed |= __shfl_xor_sync(0xffffffffu, packed, 1);
+      packed |= __shfl_xor_sync(0xffffffffu, packed, 2);
+      if (in && (sub & 3) == 0) meta[row * meta_ld + (u >> 2)] = packed;
+    } else if (in) {
+      *reinterpret_cast<uint2*>(codes + row * static_cast<int64_t>(K) + 8 * u) = make_uint2(words[0], words[1]);
     }
+  };
+  if constexpr (kKeep > 0) {
+#pragma unroll
+    for (int i = 0; i < kKeep; ++i)
+      if (i * G < units) work(sub + i * G, [&](int) { return kept[i]; });
+  } else {
+#pragma unroll 2
+    for (int first = 0; first < units; first += G)
+      work(first + sub, [&](int v) { return __ldg(src + (first + sub) * (8 / kPer) + v); });
   }
+  if constexpr (kSparse)                    // padding words: any valid 2:4 pattern (indices 0,1)
+    for (int c = (K >> 5) + sub; c < meta_ld; c += G) meta[row * meta_ld + c] = 0x44444444u;
 }
 
 // Any K % 4 == 0: one thread per group, byte accesses (small / odd matrices only).
@@ -291,19 +339,26 @@ int quantize_weight(const void* w, int w_dtype, int64_t N, int64_t K, int8_t* co
   if (N == 0) return HY3D_OK;
   if (!w || !codes || !scale) return HY3D_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(codes)) & 15) return HY3D_ERR_SHAPE;
-  // Threads per row: a warp while a row is at most 64 chunks of 32 elements, then up to the block, so
+  // Threads per row: a warp while that is at most eight rounds of eight elements a thread, then up to the block, so
   // that long rows of few channels still spread over the chip.
   int G = 32;
-  while (G < 256 && (K >> 5) > 2 * G) G <<= 1;
+  while (G < 256 && (K >> 3) > 8 * G) G <<= 1;
   const int64_t blocks = (N + 256 / G - 1) / (256 / G);
   if (blocks > 0x7FFFFFFF) return HY3D_ERR_SHAPE;
   using KernelFn = void (*)(const void*, int64_t, int, int8_t*, uint32_t*, int, void*, int, int);
-  static const KernelFn kernels[3][2] = {
-      {quantize_weight_kernel<HY3D_F16, false>, quantize_weight_kernel<HY3D_F16, true>},
-      {quantize_weight_kernel<HY3D_BF16, false>, quantize_weight_kernel<HY3D_BF16, true>},
-      {quantize_weight_kernel<HY3D_F32, false>, quantize_weight_kernel<HY3D_F32, true>}};
-  kernels[w_dtype][meta ? 1 : 0]<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
-      w, N, static_cast<int>(K), codes, meta, static_cast<int>(meta_ld), scale, scale_dtype, G);
+#define HY3D_QW(T) {{quantize_weight_kernel<T, false, 2>, quantize_weight_kernel<T, true, 2>},  \
+                    {quantize_weight_kernel<T, false, 5>, quantize_weight_kernel<T, true, 5>},  \
+                    {quantize_weight_kernel<T, false, 8>, quantize_weight_kernel<T, true, 8>},  \
+                    {quantize_weight_kernel<T, false, 0>, quantize_weight_kernel<T, true, 0>}}
+  static const KernelFn kernels[2][4][2] = {HY3D_QW(HY3D_F16), HY3D_QW(HY3D_BF16)};
+#undef HY3D_QW
+  static const KernelFn wide[2] = {quantize_weight_kernel<HY3D_F32, false, 0>, quantize_weight_kernel<HY3D_F32, true, 0>};
+  const int64_t rounds = ((K >> 3) + G - 1) / G;
+  const int sp = meta ? 1 : 0;
+  const KernelFn kernel = w_dtype == HY3D_F32 ? wide[sp]
+                                              : kernels[w_dtype == HY3D_BF16][rounds <= 2 ? 0 : rounds <= 5 ? 1 : rounds <= 8 ? 2 : 3][sp];
+  kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(w, N, static_cast<int>(K), codes, meta,
+                                                            static_cast<int>(meta_ld), scale, scale_dtype, G);
   return cudaGetLastError() == cudaSuccess ? HY3D_OK : HY3D_ERR_CUDA;
 }
 
