@@ -490,7 +490,7 @@ linear_fused_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_const
           tmem_ld_wait();
           tmem_ld_x16(t_row + chunk_col(c + 1), rb);
           const uint32_t sbuf = stage_buf + sb * kSlabBytes;
-          if (lane == 0) { if (pend) tma_store_wait_read<1>(); else tma_store_wait_read<0>(); }
+          if (elect_one()) { if (pend) tma_store_wait_read<1>(); else tma_store_wait_read<0>(); }
           __syncwarp();
           chunk_math_store<kBf16, kEpi>(ra, as, wsb + (c << 4), bsb + (c << 4), sbuf, lane, 0);
           // ---- second half (registers rb) ----
@@ -507,7 +507,7 @@ linear_fused_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_const
           chunk_math_store<kBf16, kEpi>(rb, as, wsb + (c << 4) + 16, bsb + (c << 4) + 16, sbuf, lane, 1);
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) {
+          if (elect_one()) {
             const int out_col = n0 + chunk_col(c);
             if (rows_in && out_col < p.N) tma_store_2d(&tm_o, sbuf, out_col * 2, out_row);
             tma_store_commit();
@@ -552,7 +552,8 @@ linear_fused_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_const
       if (threadIdx.x == 64) HY3D_TRACE_EVENT(2, tr, 4, u - unit_lo);
     }
     // Global writes of the bulk stores must be complete before the CTA retires.
-    if (lane == 0) tma_store_wait_all<0>();
+    __syncwarp();
+    if (elect_one()) tma_store_wait_all<0>();      // the lane that issued the stores, as in slab_store
   } else {
     // ---------------- quantiser ----------------
     const int qw = warp - 2 - kEpiWarps;
