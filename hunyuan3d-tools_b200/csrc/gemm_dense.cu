@@ -483,6 +483,9 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     };
     bool ok = true;
     int it = 0;
+    // The staging buffer to write next goes on through the tiles: with two of them a warp waits for all its stores but
+    // the latest, which reads the other buffer only as long as they alternate (a warp may have an odd number of slabs).
+    int sb = 0;
     int cur_n0 = -1;
     long long acc_tile = 0, acc_wait = 0;   // per-role cycle totals of a -DHY3D_TRACE build
     const bool scaled = p.out_dtype != HY3D_S32;
@@ -563,7 +566,6 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         const int nslab16 = p.block_n >> 4;
         const int out_row = split * p.m_rows_pad + m0 + quarter * 32;
         const int pend = p.store_bufs - 1;
-        int sb = 0;
         for (int s = half; s < nslab16; s += kWarpsPerQuarter) {
           uint32_t r16[16];
           __syncwarp();
@@ -583,7 +585,6 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         const int out_row = m0 + quarter * 32;
         const bool rows_in = out_row < p.M;
         const int pend = p.store_bufs - 1;
-        int sb = 0;
         // Which slabs a warp takes moves on from tile to tile: with a number of slabs that four does not divide the
         // same warps would always have one more.
         const int first_slab = (half + it) & (kWarpsPerQuarter - 1);

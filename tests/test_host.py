@@ -291,3 +291,28 @@ def test_checkpoint_of_separate_projections_loads_into_the_stacked_model(qu, pkg
         delattr(stock, attr)
     with torch.no_grad():
         assert stock(torch.randn(1, 4, 8, 8), torch.tensor([3]), torch.randn(1, 3, 16)).shape == (1, 4, 8, 8)
+
+
+def test_dense_staging_buffers_alternate_across_tiles():
+    """A dense epilogue warp with two staging buffers waits for all its stores but the latest, so no slab may go to the
+    buffer of the one before it.  Walks the slabs that the kernel gives a warp, tile after tile; which buffer comes next
+    is read from the kernel's text, since a store that is overwritten early need not show in any result."""
+    text = open(os.path.join(ROOT, "hunyuan3d-tools_b200", "csrc", "gemm_dense.cu")).read()
+    epilogue = text[text.index("// ---------------- epilogue ----------------"):text.index("// ---------------- teardown ----------------")]
+    tiles = epilogue[epilogue.index("for (int tile = first_tile;"):]
+    assert len(re.findall(r"if \(\+\+sb == p\.store_bufs\) sb = 0;", tiles)) == 3      # bulk, GEGLU and split-K stores
+
+    def overwritten(per_tile):
+        for slabs in range(1, 17):
+            for half in range(4):
+                for rotate in (0, 1):
+                    sb, latest = 0, None
+                    for it in range(12):
+                        sb = 0 if per_tile else sb
+                        for _ in range((half + rotate * it) % 4, slabs, 4):
+                            if sb == latest:
+                                return True
+                            latest, sb = sb, (sb + 1) % 2
+        return False
+    assert overwritten(per_tile=True)
+    assert not overwritten(per_tile=bool(re.search(r"\bint sb\b", tiles)))
