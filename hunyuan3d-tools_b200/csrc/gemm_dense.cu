@@ -993,6 +993,7 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
     if (!workspace || out_dtype == HY3D_S32 || epilogue == HY3D_EPI_GEGLU || (N & 7)) return HY3D_ERR_ARG;
     if ((reinterpret_cast<uintptr_t>(workspace) & 15) || !act_scale || !w_scale) return HY3D_ERR_ARG;
     if ((reinterpret_cast<uintptr_t>(w_scale) | reinterpret_cast<uintptr_t>(bias)) & 15) return HY3D_ERR_SHAPE;
+    if (K <= kBlockKBytes) splits = 1;     // one K block is one range: no partials, the launch writes the output itself
   }
   if (out_dtype != HY3D_S32 && (!act_scale || !w_scale)) return HY3D_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) |

@@ -509,6 +509,8 @@ def test_groupnorm_nhwc_argument_checks(ik):
     (100, 3152, 272, 3, 0),         # ragged last K block in the last range, ragged columns
     (924, 1024, 320, 4, 0),         # two stages per range
     (130, 4096, 64, 16, 0),         # one narrow tile column, sixteen ranges
+    (200, 128, 256, 4, 0),          # one K block cannot be split: the single launch
+    (65, 48, 96, 2, 1),
 ])
 def test_dense_splitk_equals_single_launch(tc, dtype, M, K, N, splits, epi):
     """Split-K (int32 partials per K range + reduce/epilogue kernel) gives the bits of the
