@@ -291,17 +291,18 @@ class Int8KernelsModule(_Base):
 class TcGemmModule(_Base):
     """Counterpart of the reference's ``int8_gemm_tc`` extension (csrc/int8_gemm_tc.cu)."""
 
-    def dense_splitk_plan(self, M, N, K, epilogue=EPI_LINEAR):
-        """(K ranges this library would use for the shape -- 1 = no split --, workspace bytes)."""
+    def dense_splitk_plan(self, M, N, K, epilogue=EPI_LINEAR, layer=False):
+        """(K ranges this library would use for the shape -- 1 = no split --, workspace bytes): for the GEMM by
+        itself, or with ``layer`` for a layer that quantises its input first."""
         nbytes = ctypes.c_int64(0)
-        splits = self._lib.hy3d_dense_splitk_plan(M, N, K, epilogue, ctypes.byref(nbytes))
-        return int(splits), int(nbytes.value)
+        plan = self._lib.hy3d_dense_layer_splitk_plan if layer else self._lib.hy3d_dense_splitk_plan
+        return int(plan(M, N, K, epilogue, ctypes.byref(nbytes))), int(nbytes.value)
 
-    def _planned_splits(self, M, N, K, epilogue, w_scale, bias):
+    def _planned_splits(self, M, N, K, epilogue, w_scale, bias, layer=False):
         """The plan's K ranges, or 1 where the reduction behind them could not read the parameters: it takes
         scales and bias by 16-byte vectors, the single launch at any address."""
         addresses = (w_scale.data_ptr() if w_scale is not None else 0) | (self._opt_bias(bias)[0] or 0)
-        return self.dense_splitk_plan(M, N, K, epilogue)[0] if addresses % 16 == 0 else 1
+        return self.dense_splitk_plan(M, N, K, epilogue, layer)[0] if addresses % 16 == 0 else 1
 
     def int8_gemm_tc(self, A, B, act_scale, w_scale, bias, out_dtype=None, epilogue=EPI_LINEAR,
                      cta_group=0, block_n=0, splits=None):
@@ -382,9 +383,10 @@ class TcGemmModule(_Base):
         N = w_int8.shape[0]
         if w_int8.shape[1] != K:
             raise RuntimeError(f"K mismatch: x has {K}, w_int8 has {w_int8.shape[1]}")
-        if cta_group == 0 and block_n == 0 and self._planned_splits(M, N, K, epilogue, w_scale, bias) > 1:
+        splits = self._planned_splits(M, N, K, epilogue, w_scale, bias, True) if cta_group == 0 and block_n == 0 else 1
+        if splits > 1:
             q, s = self._quantize(x)                     # few rows, deep K: split-K GEMM
-            return self.int8_gemm_tc(q, w_int8, s, w_scale, bias, out_dtype=x.dtype, epilogue=epilogue)
+            return self.int8_gemm_tc(q, w_int8, s, w_scale, bias, out_dtype=x.dtype, epilogue=epilogue, splits=splits)
         q = torch.empty((M, K), dtype=torch.int8, device=x.device)
         s = torch.empty((M,), dtype=torch.float32, device=x.device)
         out = torch.empty(self._out_shape(M, N, epilogue), dtype=x.dtype, device=x.device)

@@ -918,35 +918,53 @@ TilePlan plan_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group,
 constexpr double kTwoLaunchesUs = 7.5, kThreeLaunchesUs = 10.0;
 
 struct LayerPlan {
-  int splits = 1;        // K ranges of a layer
-  int gemm_splits = 1;   // what hy3d_dense_splitk_plan answers
+  int splits = 1;
   double us = 0.0;
 };
+
+// Splitting serves a K of 16 blocks or more under tiles for at most half the SMs; every range keeps four blocks.
+bool can_split(int64_t M, int64_t N, int64_t K) {
+  const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
+  return K > 15 * kBlockKBytes && (M + kTileM - 1) / kTileM * ((N + 255) / 256) * 2 <= sms;
+}
+bool has_range(int splits, int64_t K) { return splits <= 16 && static_cast<int64_t>(splits) * 4 <= (K + kBlockKBytes - 1) / kBlockKBytes; }
+// The int32 matrix of one range, written and read again, in MB (M padded to whole tiles).
+double partial_mb(int64_t M, int64_t N) { return static_cast<double>((M + kTileM - 1) / kTileM * kTileM) * static_cast<double>(N) * 8.0 / 1e6; }
+
+// Split-K plan of the GEMM by itself, for callers that have the codes: device time of the launch and its reduction
+// against the single launch.  Fitted to 110 shapes (2048 <= K, M <= 1300) x all splits, 0.7 us rms either way; asks for a
+// twentieth, since a split also takes a workspace and a launch.  The split that it picks is 1.4 % from the best on
+// average, never splitting 13 %: 64 x 8192 -> 512 12.7 us, in 7 ranges 7.6; 1117 x 7616 -> 224 11.5, in 4 ranges 9.6;
+// not so 257 x 6144 -> 1536 (9.0 against 9.6 in 3) and 358 x 5760 -> 4480 (11.7 against 15.0 in 2).
+int search_gemm_splits(int64_t M, int64_t N, int64_t K) {
+  if (!can_split(M, N, K)) return 1;
+  double best_us = 0.95 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0, 0, 1).us;
+  int best = 1;
+  for (int sp = 2; has_range(sp, K); ++sp) {
+    const double us = 2.16 + 0.963 * search_tile(M, N, K, HY3D_EPI_LINEAR, 1, 0, sp).us + sp * (0.12 + 0.0795 * partial_mb(M, N)) +
+                      0.31 * static_cast<double>(N) * K / 1e7;
+    if (us < best_us) { best_us = us; best = sp; }
+  }
+  return best;
+}
 
 // Split-K plan and expected time of a whole layer, quantisation included: the greater of the device's time and the
 // calling thread's.  A split pays one more launch, and every range writes and re-reads an M-padded int32 matrix
 // (~12 TB/s, it stays in L2).  Fitted to 90 layers of random size x all splits (0.8 us rms).  The single launch has
 // caught up since its MMAs are issued by an elected thread (257 x 6144 -> 1536, layer: 11.9 us against 12.0 in three
-// ranges; 13.8 and 13.7 before), so few layers split any more (512 x 8192 -> 1024 does).  A caller that asks for the
-// GEMM's plan is still told a split that is within 11 % of the single launch, as it was before.
+// ranges; 13.8 and 13.7 before), so few layers split any more (512 x 8192 -> 1024 does).
 LayerPlan search_layer(int64_t M, int64_t N, int64_t K) {
-  const int64_t num_kb = (K + kBlockKBytes - 1) / kBlockKBytes;
-  const int64_t part_rows = (M + kTileM - 1) / kTileM * kTileM;
-  const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
   const double act = static_cast<double>(M) * K / 1e6, weights = static_cast<double>(N) * K / 1e7;
   LayerPlan best;
   const double single_us = 0.39 + 1.18 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0, 0, 1).us + 0.36 * act + 0.07 * weights;
   best.us = single_us > kTwoLaunchesUs ? single_us : kTwoLaunchesUs;
-  if (num_kb < 16 || part_rows / kTileM * ((N + 255) / 256) * 2 > sms) return best;
-  const double part_us = 0.21 + 0.078 * static_cast<double>(part_rows) * N * 8.0 / 1e6;
-  double gemm_us = 1.11 * single_us, layer_us = 0.97 * best.us;      // a split has to be worth its workspace
-  for (int sp = 2; sp <= 16 && static_cast<int64_t>(sp) * 4 <= num_kb; ++sp) {
-    const double us = 3.48 + 0.98 * search_tile(M, N, K, HY3D_EPI_LINEAR, 1, 0, sp).us + sp * part_us + 0.35 * act + 0.45 * weights;
-    if (us < gemm_us) { gemm_us = us; best.gemm_splits = sp; }
-    if (us > kThreeLaunchesUs ? us < layer_us : kThreeLaunchesUs < layer_us) {
-      layer_us = us > kThreeLaunchesUs ? us : kThreeLaunchesUs;
-      best.splits = sp;
-    }
+  if (!can_split(M, N, K)) return best;
+  double layer_us = 0.97 * best.us;      // a split has to be worth its workspace
+  for (int sp = 2; has_range(sp, K); ++sp) {
+    double us = 3.48 + 0.98 * search_tile(M, N, K, HY3D_EPI_LINEAR, 1, 0, sp).us + sp * (0.21 + 0.078 * partial_mb(M, N)) +
+                0.35 * act + 0.45 * weights;
+    if (us < kThreeLaunchesUs) us = kThreeLaunchesUs;
+    if (us < layer_us) { layer_us = us; best.splits = sp; }
   }
   if (best.splits > 1) best.us = layer_us;
   return best;
@@ -959,13 +977,15 @@ LayerPlan plan_layer(int64_t M, int64_t N, int64_t K) {
 
 }  // namespace
 
-// Split-K plan for a dense layer: how many K ranges pay (1 = none).  Splitting serves launches
-// whose tiles leave most SMs idle while each tile walks a long K alone (the M = 257 image-encoder
-// layers with K = 6144): the ranges run side by side and a second small kernel adds them up.
+// Split-K plan: how many K ranges pay (1 = none) for the GEMM by itself or for a layer that quantises first.
+// Splitting serves launches whose tiles leave most SMs idle while each tile walks a long K alone (64 x 8192 -> 512):
+// the ranges run side by side and a second small kernel adds them up.  A layer gains less: its calling thread then has
+// a third launch to make (59 x 4096 -> 64 as a GEMM 7.7 -> 6.6 us, as a layer 10.8 and 10.3).
 int dense_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, bool layer) {
   if (epilogue == HY3D_EPI_GEGLU || (N & 7) || M <= 0 || N <= 0 || K <= 0) return 1;
-  const LayerPlan p = plan_layer(M, N, K);
-  return layer ? p.splits : p.gemm_splits;
+  if (layer) return plan_layer(M, N, K).splits;
+  static thread_local Memo<int> memo;
+  return memo.get(M, N, K, 0, [&] { return search_gemm_splits(M, N, K); });
 }
 
 // Expected time of a layer that quantises and multiplies in separate launches, in microseconds.

@@ -191,19 +191,20 @@ int hy3d_gemm_w8a8_dense(const int8_t* A, const int8_t* B, const float* act_scal
 
 /*
  * Split-K form of the GEMM above for launches whose tiles leave most SMs idle while each walks
- * a long K alone (few rows, deep K: the image encoder's M = 257, K = 6144 layer): the K blocks
+ * a long K alone (few rows, few columns, deep K: 64 x 8192 -> 512): the K blocks
  * are cut into `splits` ranges that run side by side as int32 partials in `workspace`
  * (splits x ceil(M/128)*128 x N x 4 bytes, 16-byte aligned, no initialisation needed), and a second kernel
  * adds the partials -- exactly, in int32 -- and applies the epilogue with the GEMM kernel's own
  * formula and roundings, so the result equals hy3d_gemm_w8a8_dense bit for bit.
- * hy3d_dense_splitk_plan returns the number of ranges this library would use for a shape
+ * hy3d_dense_splitk_plan returns the number of ranges that is expected to be the fastest for this GEMM by itself
  * (1 = do not split) and the workspace it needs.  out_dtype f16/bf16, epilogue linear or GELU,
  * N % 8 == 0; splits = 1 runs the plain kernel.  With splits > 1 w_scale and bias too must be 16-byte aligned.
  * Replaces: the split-K path and its reduce kernel of the reference's sparse GEMM
  * (csrc/int8_sparse_tc.cu:1730-1732 cost terms, split-K reduce) in the dense kernel's terms.
  */
 int hy3d_dense_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, int64_t* workspace_bytes);
-/* The same for a whole layer, quantisation and the calling thread's launches counted: what the layers here take. */
+/* The same for a whole layer: quantisation and the calling thread's launches count too, so fewer shapes split.  What
+ * the layers here take. */
 int hy3d_dense_layer_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, int64_t* workspace_bytes);
 int hy3d_gemm_w8a8_dense_splitk(const int8_t* A, const int8_t* B, const float* act_scale,
                                 const void* w_scale, int w_scale_dtype,

@@ -1,6 +1,8 @@
 """GPU parity tests of the CUDA kernels, called through the C ABI (ctypes binding), against
 the CPU oracle.  Integer results must be bit-exact; floating-point outputs are compared with
 the tolerance written in each test."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -10,6 +12,12 @@ from conftest import as_half
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
+
+
+def _runs_as_one_launch(tc, M, N, K, sparse=0):
+    """Whether a layer of this size takes the one-launch kernel (outside a graph capture)."""
+    block_t, ks = ctypes.c_int(0), ctypes.c_int(0)
+    return tc._lib.hy3d_linear_cluster_plan(M, N, K, sparse, ctypes.byref(block_t), ctypes.byref(ks)) == 1
 
 
 # ------------------------------------------------------------------ activation quantiser
@@ -504,7 +512,7 @@ def test_groupnorm_nhwc_argument_checks(ik):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,K,N,splits,epi", [
-    (257, 6144, 1536, None, 0),     # the image encoder's deep-K layer: the library's own plan
+    (109, 8064, 752, None, 0),      # the library's own plan
     (257, 6144, 1536, 5, 1),        # GELU, five ranges (48 K blocks: 10 + 10 + 10 + 10 + 8)
     (100, 3152, 272, 3, 0),         # ragged last K block in the last range, ragged columns
     (924, 1024, 320, 4, 0),         # two stages per range
@@ -553,7 +561,19 @@ def test_staging_buffers_over_many_tiles_of_odd_slab_counts(tc, M, K, N, epi, sp
 def test_dense_splitk_plan_leaves_the_unet_shapes_alone(tc):
     for M, K, N in [(49152, 320, 320), (12288, 640, 5120), (3072, 5120, 1280), (924, 1024, 1280)]:
         assert tc.dense_splitk_plan(M, N, K)[0] == 1
-    assert tc.dense_splitk_plan(257, 1536, 6144)[0] > 1
+
+
+@pytest.mark.parametrize("M,K,N,gemm,layer", [
+    (257, 6144, 1536, False, False), (358, 5760, 4480, False, False), (123, 3520, 3392, False, False),
+    (59, 4096, 64, True, False), (109, 8064, 752, True, True), (298, 7936, 384, True, True),
+])
+def test_dense_splitk_plans_split_where_it_is_faster(tc, M, K, N, gemm, layer):
+    """Shapes of which the split form was measured more than 5 % slower or faster than the single launch, as a GEMM and
+    as a layer: us of the GEMM 9.0 and 9.6 split, 11.7 and 15.0, 7.5 and 8.5; 7.7 and 6.6 (layer 10.8 and 10.3),
+    12.7 and 7.8, 9.3 and 8.1."""
+    for of_layer, want in ((False, gemm), (True, layer)):
+        splits, nbytes = tc.dense_splitk_plan(M, N, K, layer=of_layer)
+        assert (splits > 1) == want and nbytes == (splits * ((M + 127) // 128 * 128) * N * 4 if want else 0)
 
 
 @pytest.mark.parametrize("sparse", [False, True])
@@ -693,19 +713,21 @@ def test_residual_quantisers_equal_adding_first(qu, ik, dtype, M, K):
         assert torch.equal(total, x + h) and torch.equal(z.q, ref.q) and torch.equal(z.scale, ref.scale)
 
 
-@pytest.mark.parametrize("M,K,N", [(132, 4160, 1200), (257, 6144, 1536)])
+@pytest.mark.parametrize("M,K,N", [(298, 7936, 384), (173, 8448, 640)])
 def test_planned_split_takes_parameters_at_any_address(qu, tc, M, K, N):
     """Scales and bias that do not start on 16 bytes: the reduction behind a split K refuses them, so a shape the
-    plan would split runs as one launch, with the same bits."""
-    assert tc.dense_splitk_plan(M, N, K)[0] > 1
+    plan would split runs as one launch, with the same bits.  With parameters that do it runs split, here and in the
+    native path."""
+    assert tc.dense_splitk_plan(M, N, K)[0] > 1 and tc.dense_splitk_plan(M, N, K, layer=True)[0] > 1
+    assert not _runs_as_one_launch(tc, M, N, K)
     g = torch.Generator(device=DEV).manual_seed(K)
     x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
     w = torch.randint(-127, 128, (N, K), generator=g, device=DEV, dtype=torch.int8)
     ws, b = (torch.rand(N + 1, generator=g, device=DEV).bfloat16() for _ in range(2))
-    ref = tc.int8_linear_tc(x, w, ws[1:].clone(), b[1:].clone())
     q, s = tc._quantize(x)
+    ref = tc.int8_gemm_tc(q, w, s, ws[1:].clone(), b[1:].clone(), out_dtype=torch.bfloat16, splits=1)
     native = qu._load_native()
-    for scale, bias in ((ws[1:], b[1:]), (ws[1:].clone(), b[1:]), (ws[1:], b[1:].clone())):
+    for scale, bias in ((ws[1:].clone(), b[1:].clone()), (ws[1:], b[1:]), (ws[1:].clone(), b[1:]), (ws[1:], b[1:].clone())):
         assert torch.equal(tc.int8_linear_tc(x, w, scale, bias), ref)
         assert torch.equal(tc.int8_gemm_tc(q, w, s, scale, bias, out_dtype=torch.bfloat16), ref)
         assert torch.equal(native.gemm_dense(q, s, w, scale, bias, 1, 0, (M, K)), ref)
@@ -743,10 +765,12 @@ def test_gelu_and_erf_form_stay_within_the_gates_bound(ik):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("M,K,N", [(5, 128, 144), (300, 128, 144), (1500, 64, 256), (257, 6144, 1536)])
-def test_gelu_of_infinite_pre_activations(qu, dtype, M, K, N):
+@pytest.mark.parametrize("M,K,N", [(5, 128, 144), (300, 128, 144), (1500, 64, 256), (298, 7936, 384)])
+def test_gelu_of_infinite_pre_activations(qu, tc, dtype, M, K, N):
     """+infinity stays, -infinity and NaN give NaN, as in torch, and the columns beside them keep their bits: one launch,
     two and three (split K), direct and bulk stores, dense and 2:4 sparse."""
+    if K == 7936:
+        assert tc.dense_splitk_plan(M, N, K, 1, layer=True)[0] > 1 and not _runs_as_one_launch(tc, M, N, K)
     torch.manual_seed(K)
     lin = torch.nn.Linear(K, N).to(DEV).to(dtype)
     x = torch.randn(M, K, device=DEV).to(dtype)
