@@ -953,16 +953,20 @@ int search_gemm_splits(int64_t M, int64_t N, int64_t K) {
 // (~12 TB/s, it stays in L2).  Fitted to 90 layers of random size x all splits (0.8 us rms).  The single launch has
 // caught up since its MMAs are issued by an elected thread (257 x 6144 -> 1536, layer: 11.9 us against 12.0 in three
 // ranges; 13.8 and 13.7 before), so few layers split any more (512 x 8192 -> 1024 does).
+// Few tokens on many weights take longer than the tile's model says (every CTA reads the same few lines of A), up to 8 us
+// at 60 MB; without `few` such layers were left to two launches where one is shorter (7 x 3200 -> 9632 15.9 us against
+// 10.7).  With it no layer of 930 got slower by more than 4 %, 18 got faster.
 LayerPlan search_layer(int64_t M, int64_t N, int64_t K) {
   const double act = static_cast<double>(M) * K / 1e6, weights = static_cast<double>(N) * K / 1e7;
+  const double few = M < kTileM ? weights * (1.0 - static_cast<double>(M) / kTileM) : 0.0;
   LayerPlan best;
-  const double single_us = 0.39 + 1.18 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0, 0, 1).us + 0.36 * act + 0.07 * weights;
+  const double single_us = 0.39 + 1.18 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0, 0, 1).us + 0.36 * act + 0.07 * weights + few;
   best.us = single_us > kTwoLaunchesUs ? single_us : kTwoLaunchesUs;
   if (!can_split(M, N, K)) return best;
   double layer_us = 0.97 * best.us;      // a split has to be worth its workspace
   for (int sp = 2; has_range(sp, K); ++sp) {
     double us = 3.48 + 0.98 * search_tile(M, N, K, HY3D_EPI_LINEAR, 1, 0, sp).us + sp * (0.21 + 0.078 * partial_mb(M, N)) +
-                0.35 * act + 0.45 * weights;
+                0.35 * act + 0.45 * weights + few;
     if (us < kThreeLaunchesUs) us = kThreeLaunchesUs;
     if (us < layer_us) { layer_us = us; best.splits = sp; }
   }

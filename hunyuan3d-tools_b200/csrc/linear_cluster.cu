@@ -496,7 +496,7 @@ bool linear_cluster_plan(int64_t M, int64_t N, int64_t K, bool sparse, int* bloc
     const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
     // A layer takes the one launch where it is expected to be the shorter one: below the host's time for two
     // launches, and for few tokens and many dense weights, which the cluster's K split streams over the whole
-    // chip (5 x 2816 -> 7872 14.5 -> 10.5 us, 13 x 4736 -> 5440 14.7 -> 11.4).
+    // chip (7 x 3200 -> 9632 15.9 -> 10.7 us, 2 x 7680 -> 7520 19.6 -> 15.0, 7 x 1216 -> 9760 10.6 -> 7.1).
     double best = sparse ? sparse_layer_us(M, N, K) : dense_layer_us(M, N, K);
     // more than 148 blocks of 160 tokens and one weight tile: never one wave
     for (int bt = M <= 16 ? 16 : 32; M > 0 && M <= 148 * 160 && K <= 16384 && bt <= 160; bt = bt == 16 ? 32 : bt + 32) {

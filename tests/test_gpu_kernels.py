@@ -615,6 +615,16 @@ def test_one_launch_layer_equals_two_launches(tc, sp, sparse, M, K, N, block_t, 
             assert rc == 0 and torch.equal(out, ref)
 
 
+@pytest.mark.parametrize("M,K,N,one", [
+    (7, 3200, 9632, True), (4, 2368, 6160, True), (10, 2048, 9456, True), (2, 7680, 7520, True), (7, 1216, 9760, True),
+    (12, 1280, 640, True), (924, 1024, 2560, False), (257, 6144, 1536, False), (53, 4544, 3728, False),
+])
+def test_dense_layers_take_the_shorter_form(tc, M, K, N, one):
+    """One launch or two by what was measured, us: 10.7 and 15.9, 9.0 and 12.5, 8.5 and 11.4, 15.0 and 19.6, 7.1 and 10.6;
+    7.1 and 7.6; two where one takes 14.7 against 12.1, or has no plan."""
+    assert _runs_as_one_launch(tc, M, N, K) == one
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_gelu_epilogue_over_its_whole_range(tc, dtype):
     """Pre-activations from -14 to 14 in steps of 1/512 (accumulator k, scale 1/512): v * Phi(v) in double
