@@ -8,6 +8,8 @@
 // and optionally 8 raw nibble bytes.  Traffic: N*K read, N*K/2 + N*K/8 written.
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace hy3d {
 namespace prune {
 namespace {
@@ -155,7 +157,7 @@ __device__ __forceinline__ void quotient2(float2 w, float scale, float inv, uint
 // Per-output-channel quantisation of a weight matrix, optionally 2:4 pruned and packed, in one pass
 // over HBM.  G threads share a row: 16-byte loads for the row's absmax (two 16-bit values an instruction), then every
 // thread quantises eight adjacent K elements at a time and writes 8 codes, or 4 survivors and the byte of
-// metadata that four lanes put together to a word.  Neighbouring lanes take neighbouring elements: loads and
+// metadata that belongs to them.  Neighbouring lanes take neighbouring elements: loads and
 // stores are contiguous, and a row of 1280 fills a warp five times (in pieces of 32 elements a thread it was two
 // rounds, the second a quarter full).  The arithmetic is torch's, operation by operation, so the buffers equal those of the torch
 // expressions: |w| max; dense: max(amax * (1/127), 1e-8), sparse: max(amax, 1e-8) * (1/127) (torch on
@@ -164,12 +166,15 @@ __device__ __forceinline__ void quotient2(float2 w, float scale, float inv, uint
 // instruction: the first makes it faithful, and by Markstein's theorem ("Computation of elementary
 // functions on the IBM RISC System/6000 processor", 1990) the second then gives the correctly rounded
 // one.  |w| <= amax keeps the code within +-127.  Rows whose scale is not finite (a NaN or an infinity
-// among the weights) divide one by one; a NaN quotient becomes 0 as in torch's cast.
+// among the weights) divide one by one in a loop of their own; a NaN quotient becomes 0 as in torch's cast.
 // Bound by instruction issue, most of it the pruning network on the half-rate ALU pipe.  10240 x 1280 bf16 with pruning:
-// the torch form, 11 launches over fp32 temporaries, took 160 us, pieces of 32 elements a thread 17.2 us (12.5
-// without pruning), this kernel 13.9 (9.1), of which 6 are HBM time; fp32 26.6 -> 19.5 (27.2 -> 17.0).
+// the torch form, 11 launches over fp32 temporaries, took 160 us, this kernel 11.4 (without pruning 8.2), of which 6 are
+// HBM time.  Pieces of 32 elements a thread took 16.1; four lanes that shuffle a metadata word together, and the
+// question whether the row is finite at every four elements, 13.2, and were slower than those pieces where a row fills
+// them (10240 x 2048 17.0, 19.4 and 16.7 now; 1536 x 8192 12.5, 14.1 and 12.1).
 // kKeep > 0 (16-bit types): a thread has at most that many vectors of its row and keeps them in registers between the
-// two passes; otherwise (fp32, rows of more than 16384) the second pass reads them again.
+// two passes (five fill five blocks an SM, eight leave four); otherwise (fp32, rows of more than 16384) the second pass
+// reads them again, which costs more than the fifth block brings (10240 x 4096 46.5 us against 35.5).
 template <int kType, bool kSparse, int kKeep>
 __global__ void __launch_bounds__(256, kKeep > 5 ? 4 : 5)
 quantize_weight_kernel(const void* __restrict__ w, int64_t N, int K, int8_t* __restrict__ codes,
@@ -236,10 +241,8 @@ quantize_weight_kernel(const void* __restrict__ w, int64_t N, int K, int8_t* __r
   }
   const bool finite = scale < __int_as_float(0x7F800000);   // false for NaN too
   const float inv = __frcp_rn(scale);
-  // K / 8 is a multiple of four, so the four lanes of a metadata word are in range together; every lane of a warp
-  // walks the same rounds.
   const int units = K >> 3;
-  auto work = [&](int u, auto vector) {
+  auto work = [&](int u, auto is_finite, auto vector) {
     const bool in = u < units;
     uint32_t words[2] = {0, 0};
     if (in) {
@@ -250,7 +253,7 @@ quantize_weight_kernel(const void* __restrict__ w, int64_t N, int K, int8_t* __r
 #pragma unroll
         for (int j = 0; j < kPer; j += 4) {
           uint32_t b[4];
-          if (finite) {
+          if constexpr (is_finite.value) {
             quotient2(make_float2(f[j], f[j + 1]), scale, inv, b[0], b[1]);
             quotient2(make_float2(f[j + 2], f[j + 3]), scale, inv, b[2], b[3]);
           } else {
@@ -265,23 +268,26 @@ quantize_weight_kernel(const void* __restrict__ w, int64_t N, int K, int8_t* __r
     if constexpr (kSparse) {
       uint32_t two0, two1;
       const uint32_t n0 = prune_word(words[0], two0), n1 = prune_word(words[1], two1);
-      if (in) *reinterpret_cast<uint32_t*>(codes + row * (K >> 1) + 4 * u) = two0 | two1 << 16;
-      uint32_t packed = (n0 | n1 << 4) << (8 * (sub & 3));
-      packed |= __shfl_xor_sync(0xffffffffu, packed, 1);
-      packed |= __shfl_xor_sync(0xffffffffu, packed, 2);
-      if (in && (sub & 3) == 0) meta[row * meta_ld + (u >> 2)] = packed;
+      if (in) {
+        *reinterpret_cast<uint32_t*>(codes + row * (K >> 1) + 4 * u) = two0 | two1 << 16;
+        reinterpret_cast<uint8_t*>(meta + row * meta_ld)[u] = static_cast<uint8_t>(n0 | n1 << 4);
+      }
     } else if (in) {
       *reinterpret_cast<uint2*>(codes + row * static_cast<int64_t>(K) + 8 * u) = make_uint2(words[0], words[1]);
     }
   };
-  if constexpr (kKeep > 0) {
+  if (!finite) {
+#pragma unroll 1
+    for (int first = 0; first < units; first += G)
+      work(first + sub, std::false_type{}, [&](int v) { return __ldg(src + (first + sub) * (8 / kPer) + v); });
+  } else if constexpr (kKeep > 0) {
 #pragma unroll
     for (int i = 0; i < kKeep; ++i)
-      if (i * G < units) work(sub + i * G, [&](int) { return kept[i]; });
+      if (i * G < units) work(sub + i * G, std::true_type{}, [&](int) { return kept[i]; });
   } else {
 #pragma unroll 2
     for (int first = 0; first < units; first += G)
-      work(first + sub, [&](int v) { return __ldg(src + (first + sub) * (8 / kPer) + v); });
+      work(first + sub, std::true_type{}, [&](int v) { return __ldg(src + (first + sub) * (8 / kPer) + v); });
   }
   if constexpr (kSparse)                    // padding words: any valid 2:4 pattern (indices 0,1)
     for (int c = (K >> 5) + sub; c < meta_ld; c += G) meta[row * meta_ld + c] = 0x44444444u;
@@ -346,6 +352,7 @@ int quantize_weight(const void* w, int w_dtype, int64_t N, int64_t K, int8_t* co
   const int64_t blocks = (N + 256 / G - 1) / (256 / G);
   if (blocks > 0x7FFFFFFF) return HY3D_ERR_SHAPE;
   using KernelFn = void (*)(const void*, int64_t, int, int8_t*, uint32_t*, int, void*, int, int);
+  // Vectors a thread keeps, by the rounds that a row takes: two (rows up to 512), five (1280 and its doublings), eight.
 #define HY3D_QW(T) {{quantize_weight_kernel<T, false, 2>, quantize_weight_kernel<T, true, 2>},  \
                     {quantize_weight_kernel<T, false, 5>, quantize_weight_kernel<T, true, 5>},  \
                     {quantize_weight_kernel<T, false, 8>, quantize_weight_kernel<T, true, 8>},  \

@@ -143,7 +143,7 @@ def test_weight_conversion_equals_the_torch_expressions(qu, sp, dtype, N, K):
             assert torch.equal(layer.weight_int8_nk, codes)
 
 
-@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("N,K", [(9, 32), (40, 544), (24, 1312), (17, 2560), (3, 16416)])
 def test_weight_conversion_in_registers_and_with_values_that_are_not_finite(qu, sp, dtype, N, K):
     """Rows of one round, of three and six of the five and eight that a thread keeps, of more threads than a warp, and
@@ -159,7 +159,7 @@ def test_weight_conversion_in_registers_and_with_values_that_are_not_finite(qu, 
     for sparse, scale in ((False, (amax / 127.0).clamp(min=1e-8)), (True, amax.clamp(min=1e-8) / 127.0)):
         got = native.quantize_weight(w, sparse)
         codes = torch.nan_to_num((f / scale[:, None]).round()).clamp(-128, 127).to(torch.int8)
-        assert torch.equal(torch.nan_to_num(got[-1]), torch.nan_to_num(scale.to(dtype)))
+        assert torch.equal(torch.nan_to_num(got[-1]), torch.nan_to_num(scale.to(torch.float16 if dtype == torch.float32 else dtype)))
         assert torch.equal(torch.isnan(got[-1]), torch.isnan(scale))
         if sparse:
             comp, meta = sp.sparse_prune_and_pack(codes)
