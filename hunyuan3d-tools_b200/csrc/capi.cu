@@ -405,7 +405,7 @@ int hy3d_linear_w8a8_sparse24(const void* x, int x_dtype, int64_t ldx, int8_t* q
   int rc = check_device();
   if (rc != HY3D_OK) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  rc = quantize_rows(x, nullptr, x_dtype, M, K, ldx, q_ws, scale_ws, s);
+  rc = quantize_rows(x, nullptr, x_dtype, M, K, ldx, q_ws, scale_ws, s, sparse_l1_elements(M, N, K, epilogue, block_m));
   if (rc != HY3D_OK) return rc;
   return gemm_sparse24(q_ws, scale_ws, w_comp, w_meta, meta_ld, w_scale, w_scale_dtype, bias,
                        bias_dtype, out, out_dtype, M, N, K, epilogue, block_m, s);

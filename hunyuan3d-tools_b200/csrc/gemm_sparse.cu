@@ -494,6 +494,18 @@ SparseTile search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int block_
 
 }  // namespace
 
+// Where the GEMM of a layer is a single round of the grid, its quantiser asks for L1 from here on only: the round waits
+// for the last SM's change of split (584 x 2752 -> 2064 11.0 us, 12.0 with L1; 2863 x 2240 -> 192 10.7 and 11.5; from eight
+// million elements on 0.96 of the time without).
+double sparse_l1_elements(int64_t M, int64_t N, int64_t K, int epilogue, int block_t) {
+  constexpr double kSingleRound = 8e6;
+  const double elements = static_cast<double>(M) * static_cast<double>(K);
+  if (M <= 0 || N <= 0 || K <= 0 || elements < kL1Elements || elements >= kSingleRound) return kL1Elements;
+  const SparseTile t = search_tile(M, N, K, epilogue, block_t);
+  const int64_t tiles = t.block_t > 0 ? (N + kTileW * t.group - 1) / (kTileW * t.group) * ((M + t.block_t - 1) / t.block_t) : 0;
+  return tiles * t.group <= device_sm_count() ? kSingleRound : kL1Elements;
+}
+
 // Expected time of a layer that quantises and multiplies in separate launches, in microseconds: the greater of
 // the device's and the calling thread's (7.5), fitted to 184 layers of random size that wait for the device (7 % rms).
 // With the coefficients of an earlier tile model the wrong one of one launch and two was taken more often: 51 of 549
@@ -619,6 +631,7 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
 }  // namespace sparse
 
 using sparse::gemm_sparse24;
+using sparse::sparse_l1_elements;
 using sparse::sparse_layer_us;
 
 }  // namespace hy3d
