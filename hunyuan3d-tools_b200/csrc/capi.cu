@@ -3,6 +3,7 @@
 #include "common.cuh"
 
 #include <cudaTypedefs.h>
+#include <atomic>
 #include <mutex>
 
 namespace hy3d {
@@ -95,6 +96,38 @@ int ensure_max_smem(const void* kernel, int bytes) {
     ++n_seen;
   }
   return HY3D_OK;
+}
+
+// Stands in for any kernel in the question below; never launched.
+__global__ void occupancy_probe_kernel() {}
+
+// Clusters of `ranks` CTAs that run at the same time with room for `per_sm` CTAs on an SM: the GPCs have 16 to 20 SMs, and
+// what is left over in each stays idle (148 SMs: 15 clusters of eight, 45 of three; with two CTAs an SM 33 and 93).
+int resident_clusters(int ranks, int per_sm) {
+  constexpr int kMost = 8;
+  static std::atomic<int> known[kMost + 1][kMost + 1];
+  if (ranks < 1 || ranks > kMost || per_sm < 1 || per_sm > kMost) return 0;
+  int n = known[per_sm][ranks].load(std::memory_order_relaxed);
+  if (n == 0) {
+    const void* kernel = reinterpret_cast<const void*>(occupancy_probe_kernel);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(ranks) * 64);
+    cfg.blockDim = dim3(32);
+    cfg.dynamicSmemBytes = static_cast<size_t>(228 / per_sm - 1) * 1024;     // 1 KB of each CTA's share is the runtime's
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(ranks);
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (ensure_max_smem(kernel, 227 * 1024) != HY3D_OK || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = device_sm_count() * per_sm * 3 / 4 / ranks;
+    }
+    known[per_sm][ranks].store(n, std::memory_order_relaxed);
+  }
+  return n;
 }
 
 // 2-D byte tensor: `rows` rows of `inner_bytes` bytes, `pitch_bytes` apart; the box is

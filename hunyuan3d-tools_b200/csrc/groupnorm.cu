@@ -24,6 +24,7 @@
 
 namespace hy3d {
 int device_sm_count();
+int resident_clusters(int ranks, int per_sm);
 int ensure_max_smem(const void* kernel, int bytes);
 namespace gnorm {
 namespace {
@@ -31,6 +32,15 @@ namespace {
 // Three CTAs per SM: 56 registers a thread, 64 with terms to add, which would spill otherwise.
 __host__ __device__ constexpr int narrow_threads(bool add) { return add ? 320 : 384; }
 constexpr int kWideThreads = 1024;
+// Registers that the launch bounds leave a thread: 56, 64 with terms to add, 64 in a wide CTA.  The compiler cannot use
+// more, so at least this many CTAs of `warps` warps are resident on an SM (64 K registers, 64 warps, 32 CTAs).
+constexpr int bounded_registers(bool wide, bool add) { return 65536 / (wide ? kWideThreads : 3 * narrow_threads(add)) / 8 * 8; }
+static_assert(bounded_registers(false, false) == 56 && bounded_registers(true, false) == 64, "");
+int64_t resident_ctas(bool wide, bool add, int64_t warps) {
+  int64_t n = 65536 / (bounded_registers(wide, add) * 32 * warps);
+  if (n > 64 / warps) n = 64 / warps;
+  return n < 32 ? n : 32;
+}
 constexpr int kOrderThreads = 320;    // lanes of a chunk: what 320 threads over whole rows make
 constexpr int kMaxRanks = 8;          // portable cluster size
 
@@ -303,9 +313,7 @@ int groupnorm_nhwc(const void* x, const void* pre, const void* add, int64_t add_
         const int64_t threads = static_cast<int64_t>(per_rank) * order.lanes * vec;
         if (threads > (w ? kWideThreads : narrow_threads(add != nullptr))) continue;
         const int64_t warps = (threads + 31) / 32;
-        int64_t resident = 65536 / ((w || add ? 64 : 56) * 32 * warps);        // by registers
-        if (resident > 64 / warps) resident = 64 / warps;
-        if (resident > 32) resident = 32;
+        const int64_t resident = resident_ctas(w != 0, add != nullptr, warps);
         const int64_t ctas = static_cast<int64_t>(r) * (groups / g) * B;
         if (ctas * 20 > sms * resident * 19) continue;                  // clusters leave a few slots empty
         slab_groups = g; ranks = r; sets = per_rank; wide = w != 0;
@@ -362,14 +370,21 @@ int groupnorm_nhwc(const void* x, const void* pre, const void* add, int64_t add_
   cfg.blockDim = dim3(static_cast<unsigned>(vec_cols * k));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  // Shared memory for the CTAs that an SM gets, L1 with what is left: 12 x 320 x 64 x 64 with room for one CTA fewer
-  // 35.6 us, with all of it shared 30.6, as here 25.1.
-  const int64_t ctas = static_cast<int64_t>(ranks) * (groups / slab_groups) * B;
-  const int64_t per_sm = (ctas + sms - 1) / sms;
-  const int64_t most = wide ? 1 : 65536 / ((add ? 64 : 56) * 32 * ((vec_cols * k + 31) / 32));
+  // Shared memory for as few CTAs an SM as run all clusters at the same time, L1 with what is left: 12 x 320 x 64 x 64 with
+  // room for one CTA fewer 35.6 us, with all of it shared 30.6, as here 25.1.  Clusters leave SMs of a GPC empty, so an
+  // even share of the CTAs is not always enough: 6 x 960 x 64 x 64 (48 clusters of six) 42.4 us with room for two CTAs, 30.5
+  // for three, 2 x 320 x 32 x 32 (16 of eight) 10.8 for one, 6.8 for two.  From two CTAs on the scheduler leaves a few more.
+  const int64_t clusters = static_cast<int64_t>(groups / slab_groups) * B;
+  const int64_t most = resident_ctas(wide, add != nullptr, (vec_cols * k + 31) / 32);
+  int64_t room = (clusters * ranks + sms - 1) / sms;
+  auto holds = [&](int64_t per_sm) {
+    const int64_t n = resident_clusters(ranks, static_cast<int>(per_sm));
+    return n == 0 || (per_sm == 1 ? clusters <= n : clusters * 20 <= n * 19);
+  };
+  while (room < most && !holds(room)) ++room;
   cudaLaunchAttribute attr[3];
   attr[0] = pdl_attribute();
-  attr[2] = carveout_attribute(per_sm < most ? per_sm : most, static_cast<int64_t>(smem));
+  attr[2] = carveout_attribute(room < most ? room : most, static_cast<int64_t>(smem));
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = static_cast<unsigned>(ranks);
   attr[1].val.clusterDim.y = 1;

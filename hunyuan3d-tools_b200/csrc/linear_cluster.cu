@@ -19,10 +19,10 @@
 // The CTAs of a cluster wait for one another only at hardware cluster barriers; every mbarrier wait is
 // bounded as in the other kernels.
 #include "common.cuh"
-#include <atomic>
 #include <cstdlib>
 
 namespace hy3d {
+int resident_clusters(int ranks, int per_sm);   // in capi.cu
 namespace lincl {
 namespace {
 
@@ -460,34 +460,6 @@ double plan_layer_us(const Plan& p, int64_t M, int64_t N, int64_t K, bool sparse
                 : 1.156 * plan_us(p, M, false) - 0.4 + 0.25 * weights + (p.ks > 1 ? 0.2 : 0.0);
 }
 
-// Clusters of `ks` CTAs that run at the same time, one CTA an SM: the GPCs have 16 to 20 SMs, and what is left
-// over in each stays idle.  A second wave doubles the time (253 x 1792 -> 224 in 16 clusters of 7: 14.3 us, two
-// launches 7.8).
-int resident_clusters(int ks, int sms) {
-  static std::atomic<int> known[kMaxRanks + 1];
-  int n = known[ks].load(std::memory_order_relaxed);
-  if (n == 0) {
-    const void* kernel = reinterpret_cast<const void*>(linear_cluster_kernel<false, false, HY3D_EPI_LINEAR>);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(ks) * 64);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmemLimit;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = static_cast<unsigned>(ks);
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    if (ensure_max_smem(kernel, kSmemLimit) != HY3D_OK || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
-      cudaGetLastError();
-      n = sms * 3 / 4 / ks;
-    }
-    known[ks].store(n, std::memory_order_relaxed);
-  }
-  return n;
-}
-
 }  // namespace
 
 // Whether a layer of this size should run as one launch, and with which plan.  Sizes recur in every step of
@@ -511,7 +483,8 @@ bool linear_cluster_plan(int64_t M, int64_t N, int64_t K, bool sparse, int* bloc
         p.block_t = bt; p.ks = k;
         if (!complete(&p, M, N, K, sparse)) continue;
         const int64_t clusters = static_cast<int64_t>(p.t_tiles) * p.w_tiles;
-        if (clusters * k > (k > 1 ? sms * 7 / 8 : sms) || (k > 1 && clusters > resident_clusters(k, sms))) continue;
+        // a second wave doubles the time (253 x 1792 -> 224 in 16 clusters of 7: 14.3 us, two launches 7.8)
+        if (clusters * k > (k > 1 ? sms * 7 / 8 : sms) || (k > 1 && clusters > resident_clusters(k, 1))) continue;
         const double t = plan_order_us(p, M, sparse);
         if (!best.block_t || t < best_us) { best_us = t; best = p; }
       }
