@@ -844,7 +844,9 @@ struct TilePlan {
 // size with each epilogue x all tiles (7 % rms near the best tile); the tile it picks is 1.2 % from the best on average.
 // (The model before, fitted when a pair's hand-over cost 2000 cycles and resident B was for single CTAs, is 3.7 % off
 // with today's kernel: 12288 x 640 -> 1920 18.8 -> 16.3 us, 1879 x 4800 -> 1024 14.7 -> 12.0, 40560 x 640 -> 176
-// 11.3 -> 9.8, 257 x 1536 -> 6144 7.5 -> 6.8.)
+// 11.3 -> 9.8, 257 x 1536 -> 6144 7.5 -> 6.8.)  Gates and a short K were rare in that fit; over 490 shapes, most with
+// K <= 1152, x all tiles: `tile_us`, dearer GELU in pairs and no pairs for GEGLU below deep K (1463 x 64 -> 3840 with GEGLU
+// 12.7 -> 7.7 us, 1300 x 128 -> 5024 7.1 -> 5.6, 6873 x 896 -> 5952 with GELU 42.5 -> 38.1, with GEGLU 48.5 -> 41.5).
 TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group, int block_n, int splits) {
   // K block: a + b x width / 100, at least c; one row per way the operands come
   struct Block { double a, b, least; };
@@ -857,7 +859,7 @@ TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_grou
   const int step = geglu ? 64 : 32;
   const int64_t nk = ((K + kBlockKBytes - 1) / kBlockKBytes + splits - 1) / splits;
   for (int g = 1; g <= 2; ++g) {
-    if (cta_group != 0 ? g != cta_group : (g == 2 && (M <= kTileM || splits > 1))) continue;
+    if (cta_group != 0 ? g != cta_group : (g == 2 && (M <= kTileM || splits > 1 || (geglu && K < kDeepK)))) continue;
     for (int bn = 64; bn <= 256; bn += step) {
       const int w = block_n != 0 ? block_n : N <= 128 ? static_cast<int>(N) : bn;
       if (w != bn && bn != 64) break;                    // a width that is given: once per group
@@ -877,12 +879,15 @@ TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_grou
       double block = kb.a + kb.b * c;
       if (block < kb.least) block = kb.least;
       if (M < kTileM) block += 0.0016 * (1.0 - static_cast<double>(M) / kTileM) * static_cast<double>(nt);   // many CTAs, few lines of A
-      const double gate = geglu ? (g == 2 ? 2.59 : 2.39) : epilogue == HY3D_EPI_GELU ? 2.65 : 1.0;
+      const double gate = geglu ? (g == 2 ? 2.59 : 2.39) : epilogue == HY3D_EPI_GELU ? (g == 2 && !deep ? 3.1 : 2.65) : 1.0;
+      // A tile too narrow to give all sixteen warps a slab takes longer than its share; one of a single K block does not
+      // hide the column parameters that it waits for.
+      const double tile_us = (gate > 1.0 ? 0.15 : 0.0) + (column_fixed || nk > 1 ? 0.0 : 0.1);
       const double rows = static_cast<double>(M) / static_cast<double>(mt * g);
       const double operand = static_cast<double>(tiles * g * nk) * kBlockKBytes *
                              ((rows < kTileM ? rows : kTileM) + (resident ? 0.0 : static_cast<double>(w) / g)) / 1e7;
       double us = 2.98 + (g == 1 ? 0.0 : deep ? 0.76 : resident ? 1.09 : 0.46) +
-                  rounds * (static_cast<double>(nk) * block + (g == 1 ? 0.282 : 0.292) * c * gate) + 0.136 * operand +
+                  rounds * (static_cast<double>(nk) * block + (g == 1 ? 0.282 : 0.292) * c * gate + tile_us) + 0.136 * operand +
                   (resident ? 0.092 * static_cast<double>(nk) * c / g : 0.0) +
                   0.068 * static_cast<double>(M) * static_cast<double>(N) * (geglu ? 1.0 : 2.0) / 1e6;
       // A CTA does not fit beside a quantiser's, so a grid that wants nearly every SM starts late behind one: it

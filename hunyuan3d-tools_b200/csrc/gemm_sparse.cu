@@ -484,7 +484,7 @@ SparseTile search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int block_
       if (g == 1 && stage < 0.256) stage = 0.256;
       const double gate = epilogue == HY3D_EPI_GEGLU ? 1.79 : epilogue == HY3D_EPI_GELU ? 2.23 : 1.0;
       const double operand_mb = tiles * g * static_cast<double>(kblocks) * (kABytes + kEBytes + 256.0 * t / g) / 1e7;
-      const double us = 2.98 + rounds * (static_cast<double>(kblocks) * stage + (g == 1 ? 0.253 : 0.403) * w * gate) + 0.071 * operand_mb +
+      const double us = 2.98 + rounds * (static_cast<double>(kblocks) * stage + (g == 1 ? 0.253 : 0.403) * w * gate + (gate > 1.0 ? 0.1 : 0.0)) + 0.071 * operand_mb +
                         (g == 2 ? 0.56 : 0.0) + 0.1 * static_cast<double>(M) * static_cast<double>(N) * (epilogue == HY3D_EPI_GEGLU ? 1.0 : 2.0) / 1e6;
       if (us < best.us) { best.us = us; best.block_t = t; best.group = g; }
     }
