@@ -237,24 +237,20 @@ class Int8Linear(nn.Module):
 
     def _init_sizes(self, in_features: int, out_features: int):
         super().__init__()
-        self.in_features = in_features
-        self.out_features = out_features
+        # Plain attributes go straight into ``__dict__``: ``nn.Module.__setattr__`` looks through parameters, buffers and
+        # modules first, which for six of them is a third of what a layer's conversion costs the calling thread.
+        d = self.__dict__
+        d["in_features"], d["out_features"] = in_features, out_features
         # The reference's eligibility rule (quantize_utils.py:175-178).
-        self._tc_ok = (in_features % 64 == 0) and (out_features % 16 == 0)
-        self._sparse_ok = (in_features % 64 == 0) and (out_features % 16 == 0)
+        d["_tc_ok"] = d["_sparse_ok"] = in_features % 64 == 0 and out_features % 16 == 0
 
     # -- construction ------------------------------------------------------------------
     @staticmethod
     def _assemble(linear, dt, codes, scale, comp=None, meta=None) -> "Int8Linear":
-        """A layer around finished buffers, without the placeholder tensors of ``__init__``.  The plain attributes go
-        straight into ``__dict__``: ``nn.Module.__setattr__`` looks through parameters, buffers and modules first, which
-        for six of them is a third of what a layer's conversion costs the calling thread."""
+        """A layer around finished buffers, without the placeholder tensors of ``__init__``."""
         layer = Int8Linear.__new__(Int8Linear)
-        nn.Module.__init__(layer)
+        layer._init_sizes(linear.in_features, linear.out_features)
         d = layer.__dict__
-        k, n = linear.in_features, linear.out_features
-        d["in_features"], d["out_features"] = k, n
-        d["_tc_ok"] = d["_sparse_ok"] = k % 64 == 0 and n % 16 == 0
         b = d["_buffers"]
         b["weight_int8_nk"], b["weight_scale"] = codes, scale
         b["weight_sparse_comp"], b["weight_sparse_meta"] = comp, meta

@@ -316,3 +316,15 @@ def test_dense_staging_buffers_alternate_across_tiles():
         return False
     assert overwritten(per_tile=True)
     assert not overwritten(per_tile=bool(re.search(r"\bint sb\b", tiles)))
+
+
+def test_assembled_layers_have_the_attributes_of_constructed_ones(qu):
+    """A layer that a GPU conversion puts together around finished buffers, against one from the constructor."""
+    lin = nn.Linear(128, 48).half()
+    made = qu.Int8Linear(128, 48)
+    for comp in (None, torch.zeros(48, 64, dtype=torch.int8)):
+        layer = qu.Int8Linear._assemble(lin, torch.float16, made.weight_int8_nk, made.weight_scale, comp, comp)
+        assert set(layer.__dict__) == set(made.__dict__) | ({"mode"} if comp is not None else set())
+        assert set(layer._buffers) == set(made._buffers)
+        assert all(layer.__dict__[k] == made.__dict__[k] for k in ("in_features", "out_features", "_tc_ok", "_sparse_ok", "training"))
+    assert qu.Int8Linear._assemble(nn.Linear(128, 48, bias=False), torch.float16, None, None).bias is None
