@@ -360,19 +360,9 @@ __device__ __forceinline__ void mma_sp_i8_1cta(uint32_t d_tmem, uint64_t desc_a,
       ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(e_tmem), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// CTA-pair forms: A is 256 rows (128 per CTA), B is split by columns between the CTAs, each
-// CTA's metadata sits in its own tensor memory.
-__device__ __forceinline__ void mma_sp_i8_2cta(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b,
-                                               uint32_t e_tmem, uint32_t idesc,
-                                               uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "tcgen05.mma.sp.cta_group::2.kind::i8 [%0], %1, %2, [%3], %4, p;\n\t}"
-      ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(e_tmem), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The sparse instructions with the descriptors as (low word, shared high word), like mma_i8_lohi.
+// The sparse instruction with the descriptors as (low word, shared high word), like mma_i8_lohi.  In the CTA-pair form
+// A is 256 rows (128 per CTA), B is split by columns between the CTAs, and each CTA's metadata sits in its own tensor
+// memory.
 template <int kG>
 __device__ __forceinline__ void mma_sp_i8_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi,
                                                uint32_t e_tmem, uint32_t idesc, uint32_t accumulate) {

@@ -153,7 +153,7 @@ __device__ __forceinline__ void slab_math_geglu(const uint32_t (&rv)[16], const 
 }
 
 // Writes one packed 32 x 32 slab row into the warp's staging buffer (64-byte swizzle: 16-byte
-// chunk c of row r sits at c ^ ((r >> 1) & 3)) and lets lane 0 issue the TMA store.
+// chunk c of row r sits at c ^ ((r >> 1) & 3)) and lets one lane issue the TMA store.
 // `pending_ok` = number of earlier bulk groups of this warp that may still be reading
 // shared memory (1 with two staging buffers, 0 with one).
 __device__ __forceinline__ void slab_store(const uint32_t (&packed)[16], uint32_t buf_addr, int lane,
@@ -261,7 +261,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   pdl_wait();
 
   if (warp == 0) {
-    // ---------------- TMA producer (all lanes walk the loop, lane 0 issues) ----------------
+    // ---------------- TMA producer (all lanes walk the loop, the elected one issues) ----------------
     {
       int stage = 0;
       uint32_t phase = 0;
@@ -347,7 +347,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     // one, where behind `lane == 0` every issue first gathered its operands for whichever lanes were
     // active.  MMAs alone (no loads, no epilogue), 12288 x 640 -> 1920: resident B, 192 columns
     // 14.9 -> 11.5 us, pairs of 256 15.2 -> 11.8; 49152 x 320 -> 2560 29.7 -> 25.6 (24.0 is the pipe's own time
-    // and the launch).  The same at the TMA sites of all roles.
+    // and the launch).  The same at the TMA sites of this kernel's roles.
     if (leader) {
       const uint32_t idesc = make_idesc_i8(kTileM * kG, static_cast<uint32_t>(p.block_n), false);
       // Descriptor = (low word: address field + leading-dimension offset, high word: stride,
@@ -405,7 +405,9 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after_sync();
+#ifdef HY3D_TRACE
         if (elect_one()) HY3D_TRACE_EVENT(1, tr, 6, it);
+#endif
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * p.acc_cols);
         uint32_t acc = 0;   // the first MMA of a tile overwrites the accumulator
         uint32_t b_lo = b_res_lo0;   // resident mode: the K block of the same index
@@ -472,7 +474,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     const int acc_per_slab = geglu ? 2 * kSlabCols : kSlabCols;
     // The accumulator buffer is handed back to the leader's MMA warp (its own CTA or the peer).
     // One arrival per warp: every lane's tcgen05.ld has completed (its own wait::ld), the
-    // warp converges, then lane 0 signals.  (An arrival per thread would put 512 serialised
+    // warp converges, then the elected lane signals.  (An arrival per thread would put 512 serialised
     // updates of one shared-memory word on the epilogue's critical path.)
     auto release_acc = [&](uint32_t bar) {
       tc_fence_before_sync();

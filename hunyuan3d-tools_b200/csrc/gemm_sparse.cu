@@ -97,7 +97,7 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   volatile int* abort_flag = &ctrl->abort_flag;
 
   // Warp index through a shuffle: known warp-uniform to the compiler, so the producer and MMA
-  // roles run as warp-uniform loops (all lanes wait, lane 0 issues) with their descriptors and
+  // roles run as warp-uniform loops (all lanes wait, the elected one issues) with their descriptors and
   // coordinates in uniform registers.
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
@@ -145,7 +145,7 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   pdl_wait();
 
   if (warp == 0) {
-    // ---------------- TMA producer (all lanes walk the loop, lane 0 issues) ----------------
+    // ---------------- TMA producer (all lanes walk the loop, the elected one issues) ----------------
     {
       int stage = 0;
       uint32_t phase = 0;
