@@ -121,15 +121,23 @@ def test_dense_accumulators_bit_exact(tc, M, K, N, bn):
     assert torch.equal(acc.cpu(), O.int32_matmul(A, B))
 
 
+def _dense_by_slices(tc, A, B, a_s, w_s, bias):
+    """The layer's output from single-CTA launches of 2048 rows: fewer than two tiles per CTA, so both operands stream."""
+    return torch.cat([tc.int8_gemm_tc(A[i:i + 2048], B, a_s[i:i + 2048], w_s, bias, out_dtype=torch.bfloat16, cta_group=1)
+                      for i in range(0, A.shape[0], 2048)])
+
+
 @pytest.mark.parametrize("M,K,N,bn", [
     (40000, 192, 256, 0),     # one tile column, 313 row tiles (last one ragged), two K blocks
     (38000, 320, 640, 0),     # three columns of 224; ragged last K block
     (37900, 640, 160, 160),   # five K blocks resident
     (40000, 320, 2560, 256),  # ten columns
+    (39000, 1024, 128, 128),  # eight K blocks: the fewest A stages (four) fit beside them
+    (39000, 1040, 128, 128),  # nine do not leave four: both operands stream
 ])
 def test_dense_resident_b_tile_bit_exact(tc, M, K, N, bn):
     """Launches that keep one tile column per CTA with at least two tiles each load their B tile
-    once and stream only A (single-CTA tiles; K = 192 / 320 / 640 with two, three and five K
+    once and stream only A (single-CTA tiles; two to eight K
     blocks, ragged last row tile, ragged last K block, one and several tile columns)."""
     A, B = _rand_i8((M, K), M + K + 5), _rand_i8((N, K), N + K + 6)
     acc = tc.int8_gemm_tc(A.to(DEV), B.to(DEV), None, None, None, out_dtype=torch.int32,
@@ -143,31 +151,31 @@ def test_dense_resident_b_tile_bit_exact(tc, M, K, N, bn):
                         out_dtype=torch.bfloat16, cta_group=1, block_n=bn)
     ref = O.epilogue(O.int32_matmul(A, B), a_s, w_s, bias, torch.bfloat16, "linear")
     assert O.rel_l2(y, ref) < 2e-3          # same accumulators and formula; fma contraction only
-    # and the resident-B launch equals the streaming one bit for bit (pairs stream both operands)
-    if K >= 64 and N % 32 == 0:
-        y2 = tc.int8_gemm_tc(A.to(DEV), B.to(DEV), a_s.to(DEV), w_s.to(DEV), bias.to(DEV),
-                             out_dtype=torch.bfloat16, cta_group=2, block_n=bn)
-        assert torch.equal(y, y2)
+    # and the resident-B launch equals streaming ones, and pairs, bit for bit
+    operands = (A.to(DEV), B.to(DEV), a_s.to(DEV), w_s.to(DEV), bias.to(DEV))
+    assert torch.equal(y, _dense_by_slices(tc, *operands))
+    assert torch.equal(y, tc.int8_gemm_tc(*operands, out_dtype=torch.bfloat16, cta_group=2, block_n=bn))
     assert tc.device_status() == 0
 
 
 @pytest.mark.parametrize("M,K,N,bn", [
     (40000, 320, 320, 160),   # two columns of pairs, K ends in half a block
-    (38001, 640, 1280, 256),  # five columns, five K blocks, six A stages; ragged last row tile
-    (39000, 976, 192, 192),   # one column, seven blocks and a K step: the fewest A stages beside them
-    (38100, 336, 176, 0),     # the library's own choice; last K block of one step, columns clipped
+    (38001, 640, 1280, 256),  # five columns, five K blocks, seven A stages; ragged last row tile
+    (39000, 976, 192, 192),   # one column, eight K blocks of which the last has three steps, six A stages
+    (39000, 1008, 256, 256),  # the most that pairs with one block a stage keep: four A stages beside eight blocks
+    (38100, 336, 176, 0),     # the library's own width; last K block of three steps, columns clipped
 ])
 def test_dense_resident_b_tile_of_pairs_bit_exact(tc, M, K, N, bn):
     """CTA pairs that keep their tile column hold half of the B tile each (K < 1024): integer sums of the oracle, and
-    the same bits as single CTAs that stream both operands."""
+    the same bits as single CTAs that stream both operands and as the library's own choice."""
     A, B = _rand_i8((M, K), M + K + 7), _rand_i8((N, K), N + K + 8)
     acc = tc.int8_gemm_tc(A.to(DEV), B.to(DEV), None, None, None, out_dtype=torch.int32, cta_group=2, block_n=bn)
     assert torch.equal(acc.cpu(), O.int32_matmul(A, B))
     g = torch.Generator().manual_seed(M)
     a_s, w_s = torch.rand(M, generator=g) * 0.05 + 1e-3, (torch.rand(N, generator=g) * 1e-3 + 1e-5).bfloat16()
-    y = [tc.int8_gemm_tc(A.to(DEV), B.to(DEV), a_s.to(DEV), w_s.to(DEV), None, out_dtype=torch.bfloat16, cta_group=c,
-                         block_n=b) for c, b in ((2, bn), (0, 0), (1, 256))]
-    assert torch.equal(y[0], y[1]) and torch.equal(y[0], y[2])
+    operands = (A.to(DEV), B.to(DEV), a_s.to(DEV), w_s.to(DEV), None)
+    y = tc.int8_gemm_tc(*operands, out_dtype=torch.bfloat16, cta_group=2, block_n=bn)
+    assert torch.equal(y, _dense_by_slices(tc, *operands)) and torch.equal(y, tc.int8_gemm_tc(*operands, out_dtype=torch.bfloat16))
     assert tc.device_status() == 0
 
 
@@ -310,8 +318,9 @@ def test_sparse_tile_known_answer_from_reference_tests(sp, golden):
     (4096, 320, 320, 0), (12288, 2560, 640, 240), (3, 1280, 1280, 0), (64, 640, 5120, 0),
     (257, 1536, 4608, 0), (500, 64, 16, 0), (2772, 1024, 320, 128), (1, 64, 16, 0),
     (700, 5120, 1280, 224),
-    # deep K, M >= 2048: the CTA-pair variant (256 weight rows per tile), full and ragged tiles
-    (2304, 1024, 512, 0), (2100, 2560, 640, 0), (3000, 1280, 1296, 192), (2048, 5120, 1280, 64),
+    (2304, 1024, 512, 0), (2100, 2560, 640, 0),
+    # CTA pairs (256 weight rows per tile), full and ragged tiles, deep K and short
+    (2500, 2560, 1312, 0), (3000, 1280, 1296, 192), (2048, 5120, 1280, 64), (8119, 576, 1696, 0), (13021, 896, 672, 0),
 ])
 def test_sparse_accumulators_bit_exact(sp, M, K, N, bt):
     X, W = _rand_i8((M, K), M + K), _rand_i8((N, K), N + K + 5)
@@ -324,8 +333,8 @@ def test_sparse_accumulators_bit_exact(sp, M, K, N, bt):
 
 @pytest.mark.parametrize("mode,code", [("linear", 0), ("gelu", 1), ("geglu", 2)])
 def test_sparse_pair_variant_epilogues(sp, mode, code):
-    """Scaled outputs of the CTA-pair variant (chosen for K >= 1024, M >= 2048)."""
-    M, K, N = 2500, 1280, 768
+    """Scaled outputs of the CTA-pair variant: the cost model has pairs of 224 tokens 6 to 12 % ahead of single CTAs here."""
+    M, K, N = 2500, 2560, 1312
     A, B = _rand_i8((M, K), 31), _rand_i8((N, K), 32)
     g = torch.Generator().manual_seed(33)
     a_s = torch.rand(M, generator=g) * 0.05 + 1e-3
