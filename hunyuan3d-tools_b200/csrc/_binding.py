@@ -524,8 +524,8 @@ class SparseTcModule(_Base):
 
     def sparse_int8_linear_path(self, M, K, N):
         """csrc/int8_sparse_tc.cu:2065-2070 reported which of two code paths a shape takes
-        (1 = quantiser fused into the GEMM).  The sparse layer here always runs its
-        quantiser and its GEMM as two launches."""
+        (1 = quantiser fused into the GEMM).  The sparse layer here runs its quantiser and its
+        GEMM as two launches, small layers as one outside a stream capture."""
         return 0
 
     def test_mma_sp(self, a_comp, b, meta):

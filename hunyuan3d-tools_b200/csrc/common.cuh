@@ -707,7 +707,8 @@ inline cudaLaunchAttribute pdl_attribute() {
 // its predecessor left, if it fits: behind a GEMM that is 228 KB of shared memory and 28 KB of L1, too little for the
 // loads that a streaming kernel keeps in flight (quantiser of 49152 x 320 behind itself 7.6 us, with that split 12.1).
 // Whole layers from a graph, us: 49152 x 320 -> 320 22.0 -> 19.4, 12288 x 2560 -> 640 33.2 -> 29.7, 49152 x 1280 -> 320
-// 58.4 -> 50.7, LayerNorm + 12288 x 640 -> 1920 27.1 -> 24.7.
+// 58.4 -> 50.7, LayerNorm + 12288 x 640 -> 1920 27.1 -> 24.7.  The kernel behind starts later, since the SMs change their
+// split in between: the quantiser of a small layer leaves the attribute out.
 inline cudaLaunchAttribute carveout_attribute(int64_t blocks, int64_t bytes) {
   cudaLaunchAttribute a = {};
   a.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
