@@ -507,11 +507,9 @@ double sparse_l1_elements(int64_t M, int64_t N, int64_t K, int epilogue, int blo
 }
 
 // Expected time of a layer that quantises and multiplies in separate launches, in microseconds: the greater of
-// the device's and the calling thread's (7.5), fitted to 184 layers of random size that wait for the device (7 % rms).
-// With the coefficients of an earlier tile model the wrong one of one launch and two was taken more often: 51 of 549
-// layers by more than 5 %, 18 now (78 x 2048 -> 272 8.6 us in one, 7.2 in two).
+// the device's and the calling thread's (7.5), fitted to 110 layers of random size (0.2 us rms).
 double sparse_layer_us(int64_t M, int64_t N, int64_t K) {
-  const double us = 2.44 + 0.98 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0).us + 0.37 * static_cast<double>(M) * K / 1e6;
+  const double us = 1.271 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0).us + 0.424 * static_cast<double>(M) * K / 1e6 - 0.08;
   return us > 7.5 ? us : 7.5;
 }
 

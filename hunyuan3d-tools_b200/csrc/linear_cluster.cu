@@ -447,16 +447,11 @@ double plan_us(const Plan& p, int64_t M, bool sparse) {
          (p.ks > 1 ? 1.5 + 0.41 * slabs : 0.0) + 0.23 * slabs;
 }
 
-// What the plans of one layer are compared by: a K split costs a caller a little more than the device time says, sparse
-// ones less (2 x 1856 -> 128 in eight ranges 7.5 us, in one 8.7).
-double plan_order_us(const Plan& p, int64_t M, bool sparse) { return plan_us(p, M, sparse) + (p.ks > 1 ? (sparse ? -0.36 : 0.17) : 0.0); }
-
-// What a caller sees of the best of them beside dense_layer_us / sparse_layer_us: fitted to 117 dense and 258 sparse
-// layers of random size (sparse 7 % rms).  The sparse MMA's metadata chain makes one CTA's K units dearer where there
-// are many weights.
+// What a caller sees of a plan beside dense_layer_us / sparse_layer_us: fitted to 117 dense and 110 sparse layers
+// of random size.  The sparse MMA's metadata chain makes one CTA's K units dearer where there are many weights.
 double plan_layer_us(const Plan& p, int64_t M, int64_t N, int64_t K, bool sparse) {
   const double weights = static_cast<double>(N) * K / 1e7;
-  return sparse ? 1.165 * plan_us(p, M, true) - 0.39 + 0.2 * weights + (p.ks > 1 ? 0.52 : 0.0)
+  return sparse ? 1.289 * plan_us(p, M, true) - 0.96 + 0.38 * weights - (p.ks > 1 ? 0.46 : 0.0)
                 : 1.156 * plan_us(p, M, false) - 0.4 + 0.25 * weights + (p.ks > 1 ? 0.2 : 0.0);
 }
 
@@ -474,8 +469,7 @@ bool linear_cluster_plan(int64_t M, int64_t N, int64_t K, bool sparse, int* bloc
     // A layer takes the one launch where it is expected to be the shorter one: below the host's time for two
     // launches, and for few tokens and many dense weights, which the cluster's K split streams over the whole
     // chip (7 x 3200 -> 9632 15.9 -> 10.7 us, 2 x 7680 -> 7520 19.6 -> 15.0, 7 x 1216 -> 9760 10.6 -> 7.1).
-    Plan best;
-    double best_us = 0.0;
+    double best = sparse ? sparse_layer_us(M, N, K) : dense_layer_us(M, N, K);
     // more than 148 blocks of 160 tokens and one weight tile: never one wave
     for (int bt = M <= 16 ? 16 : 32; M > 0 && M <= 148 * 160 && K <= 16384 && bt <= 160; bt = bt == 16 ? 32 : bt + 32) {
       for (int k = 1; k <= kMaxRanks; ++k) {
@@ -485,14 +479,10 @@ bool linear_cluster_plan(int64_t M, int64_t N, int64_t K, bool sparse, int* bloc
         const int64_t clusters = static_cast<int64_t>(p.t_tiles) * p.w_tiles;
         // a second wave doubles the time (253 x 1792 -> 224 in 16 clusters of 7: 14.3 us, two launches 7.8)
         if (clusters * k > (k > 1 ? sms * 7 / 8 : sms) || (k > 1 && clusters > resident_clusters(k, 1))) continue;
-        const double t = plan_order_us(p, M, sparse);
-        if (!best.block_t || t < best_us) { best_us = t; best = p; }
+        const double t = plan_layer_us(p, M, N, K, sparse);
+        if (t < best) { best = t; e.block_t = bt; e.ks = k; }
       }
       if (bt >= M) break;
-    }
-    if (best.block_t && plan_layer_us(best, M, N, K, sparse) < (sparse ? sparse_layer_us(M, N, K) : dense_layer_us(M, N, K))) {
-      e.block_t = best.block_t;
-      e.ks = best.ks;
     }
   }
   *block_t = e.block_t;

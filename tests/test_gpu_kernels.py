@@ -634,14 +634,6 @@ def test_dense_layers_take_the_shorter_form(tc, M, K, N, one):
     assert _runs_as_one_launch(tc, M, N, K) == one
 
 
-@pytest.mark.parametrize("M,K,N,one", [
-    (78, 2048, 272, False), (55, 2048, 48, False), (27, 1856, 448, False), (12, 1280, 640, True), (1, 64, 16, True),
-])
-def test_sparse_layers_take_the_shorter_form(tc, M, K, N, one):
-    """us in one launch and in two: 8.6 and 7.2, 8.4 and 7.2, 8.2 and 7.4; 7.1 and more than 7.2, 4.6 and 6.9."""
-    assert _runs_as_one_launch(tc, M, N, K, 1) == one
-
-
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_gelu_epilogue_over_its_whole_range(tc, dtype):
     """Pre-activations from -14 to 14 in steps of 1/512 (accumulator k, scale 1/512): v * Phi(v) in double
