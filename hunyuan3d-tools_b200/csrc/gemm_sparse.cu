@@ -494,20 +494,21 @@ SparseTile search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int block_
 
 }  // namespace
 
-// Where the GEMM of a layer is a single round of the grid, its quantiser asks for L1 from here on only: the round waits
-// for the last SM's change of split (584 x 2752 -> 2064 11.0 us, 12.0 with L1; 2863 x 2240 -> 192 10.7 and 11.5; from eight
-// million elements on 0.96 of the time without).
+// The same for a sparse layer, whose GEMM waits more for the change of split, most of all where it is a single round of
+// the grid: 1138 x 640 -> 3600 8.3 us, 9.3 with L1; 584 x 2752 -> 2064 10.2 and 11.2 (inputs in L2), 4375 x 1088 -> 528 12.2
+// and 10.7 (from HBM).  More rounds gain from a million elements on (2 to 4 million 0.97 of the time), one from three.
 double sparse_l1_elements(int64_t M, int64_t N, int64_t K, int epilogue, int block_t) {
-  constexpr double kSingleRound = 8e6;
+  constexpr double kRounds = 1e6, kSingleRound = 3e6;
   const double elements = static_cast<double>(M) * static_cast<double>(K);
-  if (M <= 0 || N <= 0 || K <= 0 || elements < kL1Elements || elements >= kSingleRound) return kL1Elements;
+  if (M <= 0 || N <= 0 || K <= 0 || elements < kRounds || elements >= kSingleRound) return kRounds;
   const SparseTile t = search_tile(M, N, K, epilogue, block_t);
   const int64_t tiles = t.block_t > 0 ? (N + kTileW * t.group - 1) / (kTileW * t.group) * ((M + t.block_t - 1) / t.block_t) : 0;
-  return tiles * t.group <= device_sm_count() ? kSingleRound : kL1Elements;
+  return tiles * t.group <= device_sm_count() ? kSingleRound : kRounds;
 }
 
 // Expected time of a layer that quantises and multiplies in separate launches, in microseconds: the greater of
-// the device's and the calling thread's (7.5), fitted to 110 layers of random size (0.2 us rms).
+// the device's and the calling thread's (7.5).  The coefficients were fitted over an earlier tile model; against calls of
+// today's library they are 10 % rms off where a layer waits for the device.
 double sparse_layer_us(int64_t M, int64_t N, int64_t K) {
   const double us = 1.271 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0).us + 0.424 * static_cast<double>(M) * K / 1e6 - 0.08;
   return us > 7.5 ? us : 7.5;

@@ -497,9 +497,10 @@ dequant_bias_kernel(const int32_t* __restrict__ acc, const float* __restrict__ a
 }  // namespace
 
 // Elements from which the quantiser asks for L1.  It gains by it where the loads in flight bound it, and the GEMM behind
-// it starts later, since the SMs change their split in between: layers of 1 to 2 million elements take 0.995 of the time
-// without (16 to 32 million 0.90), smaller ones the same or, 2:4-sparse, up to 1.13 (1138 x 640 -> 3600 8.5 -> 9.6 us).
-constexpr double kL1Elements = 1e6;
+// it may start later, since the SMs change their split in between.  Dense layers, time with it over time without, inputs
+// from HBM / from L2: 0.6 to 1 million elements 0.99 / 1.00, 2 to 4 million 0.97 / 0.99, from 8 million on 0.94 / 0.95;
+// fewer 1.00, up to 1.05.  (2:4-sparse layers: sparse_l1_elements.)
+constexpr double kL1Elements = 6e5;
 
 int quantize_rows(const void* x, const void* add, int x_dtype, int64_t M, int64_t K, int64_t ldx, int8_t* q,
                   float* scale, cudaStream_t stream, double l1_elements = kL1Elements) {
