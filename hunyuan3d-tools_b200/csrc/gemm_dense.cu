@@ -487,6 +487,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     int it = 0;
     // The staging buffer to write next goes on through the tiles: with two of them a warp waits for all its stores but
     // the latest, which reads the other buffer only as long as they alternate (a warp may have an odd number of slabs).
+    // Starting at buffer 0 in every tile gave 27648 x 128 -> 128 (one slab a warp) a few wrong slabs in some launches.
     int sb = 0;
     int cur_n0 = -1;
     long long acc_tile = 0, acc_wait = 0;   // per-role cycle totals of a -DHY3D_TRACE build

@@ -296,7 +296,7 @@ def test_checkpoint_of_separate_projections_loads_into_the_stacked_model(qu, pkg
 def test_dense_staging_buffers_alternate_across_tiles():
     """A dense epilogue warp with two staging buffers waits for all its stores but the latest, so no slab may go to the
     buffer of the one before it.  Walks the slabs that the kernel gives a warp, tile after tile; which buffer comes next
-    is read from the kernel's text, since a store that is overwritten early need not show in any result."""
+    is read from the kernel's text, since a store that is overwritten early shows in some launches only."""
     text = open(os.path.join(ROOT, "hunyuan3d-tools_b200", "csrc", "gemm_dense.cu")).read()
     epilogue = text[text.index("// ---------------- epilogue ----------------"):text.index("// ---------------- teardown ----------------")]
     tiles = epilogue[epilogue.index("for (int tile = first_tile;"):]
