@@ -39,6 +39,11 @@ constexpr int kSlabTokens = 32;                       // tokens per TMA store
 constexpr int kSlabBytes = kSlabTokens * 64;          // 32 tokens x 32 columns x 2 B
 constexpr int kSmemLimit = 227 * 1024;
 constexpr int kMaxBlockT = 240;      // 2 * 240 accumulator columns + 8 metadata columns <= 512
+// With one accumulator buffer, for launches in which no CTA has a second tile.  A stage of a pair then brings 52 KB for 512
+// cycles of MMA instead of 36 KB for 256 at 128 tokens, and the fill of shared memory is what paces deep stages:
+// 2915 x 5120 -> 1296 in one round of 72 tiles 14.4 us, in two rounds of 128 tokens 17.1 (with GELU 15.7 and 17.8);
+// 256 x 1280 -> 18944 8.4 -> 7.6.
+constexpr int kWideBlockT = 256;
 
 struct SparseArgs {
   const float* act_scale;
@@ -109,7 +114,7 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   const int row_off = static_cast<int>(cta_rank) * kTileW;                 // this CTA's weight rows
   const int tok_off = static_cast<int>(cta_rank) * (p.block_t / kG);       // this CTA's share of B
   const uint32_t tmem_cols = 512;
-  const uint32_t e_col = static_cast<uint32_t>(2 * p.block_t);
+  const uint32_t e_col = static_cast<uint32_t>((p.block_t > kMaxBlockT ? 1 : 2) * p.block_t);     // behind the accumulators
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
@@ -461,7 +466,8 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 // amortises the weights, a narrow one spreads few tokens over the chip.  Both come from one cost model, in
 // microseconds, fitted to 120 shapes of random size with each epilogue x all tiles (7 % rms); the tile it picks is
 // 0.6 % from the best on average (the model before, fitted when a pair's hand-over cost 2000 cycles: 1.3 %):
-//   2915 x 5120 -> 1296 with GELU: single CTAs of 128 tokens 21.1 us, pairs of 128 17.8
+//   2915 x 5120 -> 1296 with GELU: single CTAs of 128 tokens 21.1 us, pairs of 128 17.8, one round of 256 15.7
+// (the same constants hold for those: over 54 shapes that could take them none got slower by more than 2 %).
 struct SparseTile {
   int block_t = 0, group = 1;
   double us = 1e30;
@@ -471,14 +477,15 @@ SparseTile search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int block_
   const int64_t kblocks = (K + kBlockK - 1) / kBlockK;
   const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
   for (int g = 1; g <= 2; ++g) {
-    for (int bt = 32; bt <= 224; bt += 32) {
+    for (int bt = 32; bt <= kWideBlockT; bt += 32) {
       if (block_t != 0 && bt != 32) break;             // the caller's width, one pass per group
       const int t = block_t != 0 ? block_t : bt;
-      if (t < 16 || t > kMaxBlockT || (t & 15) || (g == 2 && (t & 31))) continue;
+      if (t < 16 || t > kWideBlockT || (t & 15) || (g == 2 && (t & 31))) continue;
       if (block_t == 0 && bt > 32 && bt >= M + 32) break;
       if (block_t == 0 && bt == 32 && M > 1024) continue;      // one store per 32 tokens and 32 columns
       const double tiles = static_cast<double>((N + kTileW * g - 1) / (kTileW * g)) * static_cast<double>((M + t - 1) / t);
       const double rounds = static_cast<double>((static_cast<int64_t>(tiles) + sms / g - 1) / (sms / g));
+      if (t > kMaxBlockT && (rounds > 1.0 || block_t != 0)) continue;
       const double w = t / 100.0;
       double stage = g == 1 ? 0.179 + 0.159 * w : 0.223 + 0.058 * w;
       if (g == 1 && stage < 0.256) stage = 0.256;
@@ -542,7 +549,7 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
 #ifdef HY3D_TRACE
   if (const char* e = getenv("HY3D_SPARSE_CTA_GROUP")) group = atoi(e) == 2 ? 2 : 1;
 #endif
-  if (block_t < 16 || block_t > kMaxBlockT || (block_t & 15)) return HY3D_ERR_SHAPE;
+  if (block_t < 16 || block_t > kWideBlockT || (block_t & 15)) return HY3D_ERR_SHAPE;
   if (group == 2 && (block_t & 31)) group = 1;
 
   SparseArgs p;

@@ -331,6 +331,26 @@ def test_sparse_accumulators_bit_exact(sp, M, K, N, bt):
     assert torch.equal(acc.cpu(), O.int32_matmul(X, O.expand_24(co, no)))
 
 
+# 256-token tiles with one accumulator buffer: launches of one round, pairs (2817 tokens and more) and single CTAs, whole and
+# ragged tiles, deep K and K of a block and less.
+@pytest.mark.parametrize("M,K,N", [(2817, 2560, 1312), (3072, 640, 1536), (2915, 5120, 1296), (250, 576, 18944), (497, 704, 9216), (256, 64, 18944)])
+def test_sparse_one_round_of_wide_tiles(sp, M, K, N):
+    X, W = _rand_i8((M, K), M + K).to(DEV), _rand_i8((N, K), N + K + 5).to(DEV)
+    comp, meta = sp.sparse_prune_and_pack(W)
+    wp = O.expand_24(*O.prune_compress(W.cpu()))
+    acc = sp.sparse_int8_gemm(X, None, comp, meta, None, None, out_dtype=torch.int32)
+    rows = torch.cat([torch.arange(3), torch.arange(M - 40, M), torch.randperm(M, generator=torch.Generator().manual_seed(M))[:60]])
+    assert torch.equal(acc[rows.to(DEV)].cpu(), O.int32_matmul(X[rows.to(DEV)].cpu(), wp))
+    g = torch.Generator().manual_seed(33)
+    a_s, w_s = (torch.rand(M, generator=g) * 0.05 + 1e-3).to(DEV), (torch.rand(N, generator=g) * 1e-3 + 1e-5).bfloat16().to(DEV)
+    bias = (torch.randn(N, generator=g) * 0.1).bfloat16().to(DEV)
+    for epi in (0, 1, 2) if N % 32 == 0 else (0, 1):      # the epilogue is the narrow tiles': the same bits
+        y = sp.sparse_int8_gemm(X, a_s, comp, meta, w_s, bias, out_dtype=torch.bfloat16, epilogue=epi)
+        assert torch.equal(y, sp.sparse_int8_gemm(X, a_s, comp, meta, w_s, bias, out_dtype=torch.bfloat16, epilogue=epi, force_tile=128))
+    with pytest.raises(RuntimeError):      # 256 is the rule's to choose
+        sp.sparse_int8_gemm(X, None, comp, meta, None, None, out_dtype=torch.int32, force_tile=256)
+
+
 @pytest.mark.parametrize("mode,code", [("linear", 0), ("gelu", 1), ("geglu", 2)])
 def test_sparse_pair_variant_epilogues(sp, mode, code):
     """Scaled outputs of the CTA-pair variant: the cost model has pairs of 224 tokens 6 to 12 % ahead of single CTAs here."""
