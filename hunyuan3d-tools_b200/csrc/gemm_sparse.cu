@@ -53,7 +53,9 @@ struct SparseArgs {
   int ws_dtype, bias_dtype, out_dtype, epilogue;
   int M, N, K;
   int block_t, stages, tma_store;
-  int w_tiles, t_tiles, num_kb, last_ksteps;
+  int num_kb, last_ksteps;
+  int fast_tiles, total_tiles, w_fastest;     // tile order: weight or token tiles run fastest (see tokens_fastest)
+  int share, rest;        // tokens fastest: tiles of a CTA's (pair's) contiguous range; the first `rest` have one more
 };
 
 struct __align__(16) SparseCtrl {
@@ -106,11 +108,12 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   // coordinates in uniform registers.
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
-  const int total_tiles = p.w_tiles * p.t_tiles;       // w_tiles counts 128*kG-row units
   const uint32_t cta_rank = kG == 2 ? cluster_cta_rank() : 0u;
   const bool leader = cta_rank == 0;
-  const int first_tile = static_cast<int>(blockIdx.x) / kG;
-  const int tile_step = static_cast<int>(gridDim.x) / kG;
+  const int walker = static_cast<int>(blockIdx.x) / kG;
+  const int first_tile = p.w_fastest ? walker : walker * p.share + min(walker, p.rest);
+  const int end_tile = p.w_fastest ? p.total_tiles : first_tile + p.share + (walker < p.rest ? 1 : 0);
+  const int tile_step = p.w_fastest ? static_cast<int>(gridDim.x) / kG : 1;
   const int row_off = static_cast<int>(cta_rank) * kTileW;                 // this CTA's weight rows
   const int tok_off = static_cast<int>(cta_rank) * (p.block_t / kG);       // this CTA's share of B
   const uint32_t tmem_cols = 512;
@@ -155,9 +158,10 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = first_tile; ok && tile < total_tiles; tile += tile_step) {
-        const int w0 = (tile % p.w_tiles) * (kTileW * kG) + row_off;
-        const int t0 = (tile / p.w_tiles) * p.block_t + tok_off;
+      for (int tile = first_tile; ok && tile < end_tile; tile += tile_step) {
+        const int slow = tile / p.fast_tiles, fast = tile - slow * p.fast_tiles;
+        const int w0 = (p.w_fastest ? fast : slow) * (kTileW * kG) + row_off;
+        const int t0 = (p.w_fastest ? slow : fast) * p.block_t + tok_off;
         for (int kb = 0; kb < p.num_kb; ++kb) {
           ok = mbar_wait(smem_u32(&ctrl->empty[stage]), phase ^ 1, abort_flag, kDevTimeoutEmpty);
           ok = __all_sync(0xffffffffu, ok);
@@ -206,7 +210,7 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       uint32_t phase = 0, a_lo = a_lo0;
       bool ok = true;
       int it = 0;
-      for (int tile = first_tile; ok && tile < total_tiles; tile += tile_step, ++it) {
+      for (int tile = first_tile; ok && tile < end_tile; tile += tile_step, ++it) {
         const int buf = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
         ok = mbar_wait(smem_u32(&ctrl->tmem_empty[buf]), acc_phase ^ 1, abort_flag,
@@ -270,11 +274,14 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     const uint32_t stage_buf = staging_base + static_cast<uint32_t>(warp - 2) * kSlabBytes;
     bool ok = true, wide_gates = false;
     int it = 0;
-    for (int tile = first_tile; tile < total_tiles; tile += tile_step, ++it) {
+    float wsr[4] = {0.0f, 0.0f, 0.0f, 0.0f}, bsr[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // of the fragment rows of w0
+    int cur_w0 = -1;
+    for (int tile = first_tile; tile < end_tile; tile += tile_step, ++it) {
       const int buf = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
-      const int w0 = (tile % p.w_tiles) * (kTileW * kG) + row_off;
-      const int t0 = (tile / p.w_tiles) * p.block_t;
+      const int slow = tile / p.fast_tiles, fast = tile - slow * p.fast_tiles;
+      const int w0 = (p.w_fastest ? fast : slow) * (kTileW * kG) + row_off;
+      const int t0 = (p.w_fastest ? slow : fast) * p.block_t;
       const int n = w0 + row_in_tile;
       const bool n_ok = n < p.N;
       // Which slabs a warp takes moves on from tile to tile: with a number of slabs that four does not divide (seven
@@ -292,7 +299,6 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         arrived = true;
       };
       float ws = 0.0f, bs = 0.0f;                            // direct stores: weight row n
-      float wsr[4] = {0.0f, 0.0f, 0.0f, 0.0f}, bsr[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // fragment rows
       float sc_next = 0.0f;
       if (p.out_dtype != HY3D_S32) {
         if (p.tma_store) {
@@ -300,12 +306,13 @@ gemm_sparse_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
           // the tile needs no CTA-wide barrier.
           const int t = t0 + first_slab * kSlabTokens + lane;
           if (first_slab * kSlabTokens < p.block_t && t < p.M) sc_next = p.act_scale[t];
+          if (w0 != cur_w0) {
+            cur_w0 = w0;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int nr = w0 + quarter * 32 + (lane >> 2) + 8 * i;
-            if (nr < p.N) {
-              wsr[i] = load_scalar(p.w_scale, p.ws_dtype, nr);
-              bsr[i] = p.bias ? load_scalar(p.bias, p.bias_dtype, nr) : 0.0f;
+            for (int i = 0; i < 4; ++i) {
+              const int nr = w0 + quarter * 32 + (lane >> 2) + 8 * i;
+              wsr[i] = nr < p.N ? load_scalar(p.w_scale, p.ws_dtype, nr) : 0.0f;
+              bsr[i] = nr < p.N && p.bias ? load_scalar(p.bias, p.bias_dtype, nr) : 0.0f;
             }
           }
         } else {
@@ -499,6 +506,24 @@ SparseTile search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int block_
   return best;
 }
 
+// Tile order of launches of several rounds.  Weights fastest: the CTAs share a token block, which comes from HBM once, but
+// each of them goes to other weight rows with every tile, loads their scales and bias anew, and neighbours write their
+// pieces of the output's rows side by side.  Tokens fastest, a contiguous range for each CTA: the weight rows change once or
+// twice a launch, and the tokens are read once per column of weight tiles, from L2 as long as they stay there.  Over 75
+// shapes of several rounds, time with weights fastest over time with tokens fastest:
+//   GEGLU, codes below 10 MB 0.99 to 1.19, 1.074 on average (3072 x 1280 -> 10240 37.0 -> 34.3 us, 12288 x 640 -> 5120 62.7 -> 56.2);
+//     10 to 25 MB 0.97 to 1.12, below 1 where N is under 1024
+//   GELU, codes below 10 MB 0.99 to 1.15, 1.045 on average; more 0.87 to 1.07
+//   plain, codes below 10 MB, M below 10,000 and K below 1600 0.975 to 1.12, 1.049 on average; the others 0.82 to 1.10, since
+//     the output's stream displaces the tokens (49152 x 640 -> 640 27.6 us and 31.9)
+bool tokens_fastest(int64_t M, int64_t N, int64_t K, int epilogue, bool rounds) {
+  const int64_t codes = M * K;
+  if (!rounds) return false;
+  if (epilogue == HY3D_EPI_GEGLU && N >= 1024) return codes < 25000000;
+  if (epilogue != HY3D_EPI_LINEAR) return codes < 10000000;
+  return codes < 10000000 && M < 10000 && K < 1600;
+}
+
 }  // namespace
 
 // The same for a sparse layer, whose GEMM waits more for the change of split, most of all where it is a single round of
@@ -557,8 +582,9 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
   p.ws_dtype = ws_dtype; p.bias_dtype = bias_dtype; p.out_dtype = out_dtype; p.epilogue = epilogue;
   p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.K = static_cast<int>(K);
   p.block_t = block_t;
-  p.w_tiles = static_cast<int>((N + kTileW * group - 1) / (kTileW * group));
-  p.t_tiles = static_cast<int>((M + block_t - 1) / block_t);
+  const int w_tiles = static_cast<int>((N + kTileW * group - 1) / (kTileW * group));
+  const int t_tiles = static_cast<int>((M + block_t - 1) / block_t);
+  p.total_tiles = w_tiles * t_tiles;
   p.num_kb = static_cast<int>(kblocks);
   const int k_last = static_cast<int>(K - (kblocks - 1) * kBlockK);
   p.last_ksteps = (k_last + 63) / 64;
@@ -611,9 +637,12 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
   if (rc != HY3D_OK) return rc;
   const int sms = device_sm_count();
   if (sms <= 0) return HY3D_ERR_CUDA;
-  const int total_tiles = p.w_tiles * p.t_tiles;
   const int max_clusters = sms / group;
-  const int clusters = total_tiles < max_clusters ? total_tiles : max_clusters;
+  const int clusters = p.total_tiles < max_clusters ? p.total_tiles : max_clusters;
+  p.w_fastest = tokens_fastest(M, N, K, epilogue, p.total_tiles > clusters) ? 0 : 1;
+  p.fast_tiles = p.w_fastest ? w_tiles : t_tiles;
+  p.share = p.total_tiles / clusters;
+  p.rest = p.total_tiles - p.share * clusters;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(group * clusters));
   cfg.blockDim = dim3(kThreads);

@@ -331,6 +331,32 @@ def test_sparse_accumulators_bit_exact(sp, M, K, N, bt):
     assert torch.equal(acc.cpu(), O.int32_matmul(X, O.expand_24(co, no)))
 
 
+# Tokens fastest in contiguous ranges: a range that ends inside a column of weight tiles, at its end and beyond it, ragged last
+# tiles both ways, more columns than CTAs, pairs and single CTAs; widths that the cost model does not choose.
+@pytest.mark.parametrize("M,K,N,bt", [(3072, 1280, 10240, 0), (1500, 640, 10240, 0), (4444, 640, 3040, 0), (2000, 1024, 4096, 160),
+                                      (333, 320, 20000, 0), (9000, 384, 1056, 64), (1100, 128, 9600, 32)])
+def test_sparse_token_ranges(sp, M, K, N, bt):
+    X, W = _rand_i8((M, K), M + K).to(DEV), _rand_i8((N, K), N + K + 5).to(DEV)
+    comp, meta = sp.sparse_prune_and_pack(W)
+    acc = sp.sparse_int8_gemm(X, None, comp, meta, None, None, out_dtype=torch.int32, force_tile=bt)
+    rows = torch.cat([torch.arange(2), torch.arange(M - 20, M), torch.randperm(M, generator=torch.Generator().manual_seed(M))[:40]])
+    assert torch.equal(acc[rows.to(DEV)].cpu(), O.int32_matmul(X[rows.to(DEV)].cpu(), O.expand_24(*O.prune_compress(W.cpu()))))
+    g = torch.Generator().manual_seed(33)
+    a_s, w_s = (torch.rand(M, generator=g) * 0.05 + 1e-3).to(DEV), (torch.rand(N, generator=g) * 1e-4 + 1e-5).bfloat16().to(DEV)
+    bias = (torch.randn(N, generator=g) * 0.1).bfloat16().to(DEV)
+    base = torch.addcmul(bias.double(), acc.double(), (a_s[:, None] * w_s.float()[None]).double()).float()   # one rounding, as fma
+    for epi in (0, 1, 2):
+        y = sp.sparse_int8_gemm(X, a_s, comp, meta, w_s, bias, out_dtype=torch.bfloat16, epilogue=epi, force_tile=bt)
+        if epi == 0:
+            ref = base
+        elif epi == 1:
+            ref = torch.nn.functional.gelu(base)
+        else:
+            v, gate = base.view(M, N // 32, 2, 16).unbind(2)
+            ref = (v * torch.nn.functional.gelu(gate)).reshape(M, N // 2)
+        assert O.rel_l2(y, ref) < 2.5e-3      # one rounding to bf16: 2^-9 / sqrt(3) on average, 1.2e-3
+
+
 # 256-token tiles with one accumulator buffer: launches of one round, pairs (2817 tokens and more) and single CTAs, whole and
 # ragged tiles, deep K and K of a block and less.
 @pytest.mark.parametrize("M,K,N", [(2817, 2560, 1312), (3072, 640, 1536), (2915, 5120, 1296), (250, 576, 18944), (497, 704, 9216), (256, 64, 18944)])
