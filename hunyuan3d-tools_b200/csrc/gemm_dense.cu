@@ -70,6 +70,7 @@ struct __align__(16) DenseCtrl {
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint64_t b_full;      // resident-B mode: the whole B tile has landed
+  uint64_t b_empty;     // ... and the MMAs of its tile column are done with it (ranges only)
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -177,7 +178,7 @@ __device__ __forceinline__ void slab_store(const uint32_t (&packed)[16], uint32_
   }
 }
 
-template <bool kBf16, int kEpi, int kG, int kAtoms>
+template <bool kBf16, int kEpi, int kG, int kAtoms, bool kRanges>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                   const __grid_constant__ CUtensorMap tm_o, const DenseArgs p) {
@@ -219,8 +220,14 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   // tile, so a large A is fetched from HBM once); see the host-side choice.
   auto tile_m = [&](int t) { return p.n_fastest ? t / p.n_tiles : t % p.m_tiles; };
   auto tile_n = [&](int t) { return p.n_fastest ? t % p.n_tiles : t / p.m_tiles; };
-  const int first_tile = static_cast<int>(blockIdx.x) / kG;
-  const int tile_step = static_cast<int>(gridDim.x) / kG;
+  // Unit walk of this CTA (pair): first_tile, first_tile + tile_step, ... below end_unit.  With kRanges it is a contiguous
+  // range of tiles, numbered down the columns.  (A kernel of its own: anything in the MMA loop that is not the same for the
+  // whole launch costs the others 2 to 10 %.)
+  const int walkers = static_cast<int>(gridDim.x) / kG, walker = static_cast<int>(blockIdx.x) / kG;
+  const int range_len = total_units / walkers, range_rest = total_units - range_len * walkers;
+  const int first_tile = kRanges ? walker * range_len + min(walker, range_rest) : walker;
+  const int end_unit = kRanges ? first_tile + range_len + (walker < range_rest ? 1 : 0) : total_units;
+  const int tile_step = kRanges ? 1 : walkers;
   const int row_off = static_cast<int>(cta_rank) * kTileM;
   const int col_off = static_cast<int>(cta_rank) * (p.block_n / kG);
 
@@ -234,6 +241,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       mbar_init(smem_u32(&ctrl->tmem_empty[b]), kG * kEpiWarps);   // one arrival per epilogue warp
     }
     mbar_init(smem_u32(&ctrl->b_full), 1);
+    mbar_init(smem_u32(&ctrl->b_empty), 1);
     ctrl->abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tm_a);
@@ -266,23 +274,34 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      if (b_res && first_tile < total_units && elect_one()) {
+      auto load_b = [&](int n0) {
         const uint32_t bf = smem_u32(&ctrl->b_full);
-        const int n0 = tile_n(first_tile) * p.block_n + col_off;
         if (leader) mbar_arrive_expect_tx(bf, static_cast<uint32_t>(kG) * b_res_bytes);
         for (int kb = 0; kb < p.num_kb; ++kb) {
           if (kG == 1) tma_load_2d(b_res_base + kb * b_bytes, &tm_b, bf, kb * kBlockKBytes, n0);
           else tma_load_2d_pair(b_res_base + kb * b_bytes, &tm_b, map_to_cta(bf, 0), kb * kBlockKBytes, n0);
         }
-      }
+      };
+      if (b_res && first_tile < end_unit && elect_one()) load_b(tile_n(first_tile) * p.block_n + col_off);
       __syncwarp();
-      for (int unit = first_tile; ok && unit < total_units; unit += tile_step) {
+      int col_left = kRanges ? p.m_tiles - first_tile % p.m_tiles : 0;     // tiles up to the next column
+      uint32_t b_phase = 0;
+      for (int unit = first_tile; ok && unit < end_unit; unit += tile_step) {
         const int split = p.splits > 1 ? unit / total_tiles : 0;
         const int tile = unit - split * total_tiles;
         const int kb0 = split * p.kb_per_split;
         const int nkb = p.splits > 1 ? min(p.kb_per_split, p.num_kb - kb0) : p.num_kb;
         const int m0 = tile_m(tile) * (kTileM * kG) + row_off;
         const int n0 = tile_n(tile) * p.block_n + col_off;
+        if (kRanges && col_left-- == 0) {        // another column: its B tile, once the MMAs are done with the last one
+          ok = mbar_wait(smem_u32(&ctrl->b_empty), b_phase, abort_flag, kDevTimeoutEmpty);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          b_phase ^= 1;
+          col_left = p.m_tiles - 1;
+          if (elect_one()) load_b(n0);
+          __syncwarp();
+        }
         for (int kb = 0; kb < nkb; ++kb) {
           ok = mbar_wait(smem_u32(&ctrl->empty[stage]), phase ^ 1, abort_flag, kDevTimeoutEmpty);
           ok = __all_sync(0xffffffffu, ok);
@@ -388,12 +407,14 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         else tc_commit_2cta(smem_u32(&ctrl->empty[stage]), 3);
       };
       const uint32_t b_res_lo0 = lo_const | ((b_res_base & 0x3FFFFu) >> 4);
-      if (b_res && first_tile < total_units) {
+      if (b_res && first_tile < end_unit) {
         ok = mbar_wait(smem_u32(&ctrl->b_full), 0, abort_flag, kDevTimeoutFull);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after_sync();
       }
-      for (int unit = first_tile; ok && unit < total_units; unit += tile_step, ++it) {
+      int col_left = kRanges ? p.m_tiles - first_tile % p.m_tiles : 0;
+      uint32_t b_phase = 1;
+      for (int unit = first_tile; ok && unit < end_unit; unit += tile_step, ++it) {
         const int buf = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
         // K range of this unit; only the last range of a matrix can end in a ragged stage
@@ -457,6 +478,19 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           if (kG == 1) tc_commit_1cta(smem_u32(&ctrl->tmem_full[buf]));
           else tc_commit_2cta(smem_u32(&ctrl->tmem_full[buf]), 3);
         }
+        if (kRanges && --col_left == 0 && unit + 1 < end_unit) {
+          // The next tile starts another column: B goes back to the producers and comes anew.
+          col_left = p.m_tiles;
+          if (ok && elect_one()) {
+            if (kG == 1) tc_commit_1cta(smem_u32(&ctrl->b_empty));
+            else tc_commit_2cta(smem_u32(&ctrl->b_empty), 3);
+          }
+          __syncwarp();
+          if (ok) ok = mbar_wait(smem_u32(&ctrl->b_full), b_phase, abort_flag, kDevTimeoutFull);
+          ok = __all_sync(0xffffffffu, ok);
+          tc_fence_after_sync();
+          b_phase ^= 1;
+        }
         __syncwarp();
       }
     }
@@ -502,13 +536,13 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     const int fast_dim = p.n_fastest ? p.n_tiles : p.m_tiles;
     const int step_slow = tile_step / fast_dim, step_fast = tile_step - step_slow * fast_dim;
     int t_fast = 0, t_slow = 0;
-    if (first_tile < total_tiles && p.splits == 1) {
+    if (first_tile < end_unit && p.splits == 1) {
       t_slow = first_tile / fast_dim;
       t_fast = first_tile - t_slow * fast_dim;
       const int m_first = (p.n_fastest ? t_slow : t_fast) * (kTileM * kG) + row_off + row_in_tile;
       if (scaled && m_first < p.M) as_next = p.act_scale[m_first];
     }
-    for (int tile = first_tile; tile < total_units; tile += tile_step, ++it) {
+    for (int tile = first_tile; tile < end_unit; tile += tile_step, ++it) {
       const int buf = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
       int split = 0;
@@ -526,7 +560,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         t_slow += step_slow;
         if (t_fast >= fast_dim) { t_fast -= fast_dim; ++t_slow; }
         as_next = 0.0f;
-        if (scaled && tile + tile_step < total_tiles) {
+        if (scaled && tile + tile_step < end_unit) {
           const int mn = (p.n_fastest ? t_slow : t_fast) * (kTileM * kG) + row_off + row_in_tile;
           if (mn < p.M) as_next = p.act_scale[mn];
         }
@@ -834,6 +868,45 @@ int64_t resident_stages(int64_t b_tile_bytes) {
   return (kSmemLimit - static_cast<int64_t>(sizeof(DenseCtrl)) - kEpiWarps * kSlabBytes - b_tile_bytes) / (kTileM * kBlockKBytes);
 }
 
+// How a launch walks its tiles of `w` columns: strided over the grid, N-fastest, with the grid rounded down to a multiple of
+// the tile columns where that keeps every CTA in one of them, or in contiguous ranges down the columns.  Ranges use every SM
+// and keep B resident whatever the number of columns, but for a reload where a range goes on into the next column.  CTAs
+// that run together then write pieces of other rows: behind GEGLU, which is bound by the gate's instructions, that does not
+// show, plain layers lose by it (49152 x 320 -> 2560 54.3 us, 56.6 in ranges; 49152 x 320 -> 960 22.7 and 24.5).
+// With GEGLU, us strided / in ranges: 49152 x 320 -> 2560 95.9 / 90.1 (140 SMs, 28 rounds; 148 and 26), 24576 x 320 -> 2560
+// 50.5 / 47.8, 12288 x 640 -> 5120 57.2 / 50.8 (in pairs), 5000 x 512 -> 4096 21.5 / 20.8.  A must stay in L2, since every
+// column reads it again at its own time.
+struct Walk {
+  int clusters = 0;
+  bool column_fixed = false, resident = false, ranges = false;
+  double rounds = 0.0;       // tiles that the busiest CTA works through
+};
+constexpr int64_t kRangesMaxA = 64000000;
+Walk plan_walk(int64_t M, int64_t N, int64_t K, int g, int w, int splits, int epilogue) {
+  const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
+  const int64_t nk = (K + kBlockKBytes - 1) / kBlockKBytes;
+  const int64_t nt = (N + w - 1) / w, mt = (M + kTileM * g - 1) / (kTileM * g);
+  const int64_t units = mt * nt * splits, most = sms / g < units ? sms / g : units;
+  Walk walk;
+  int64_t slots = most;
+  walk.column_fixed = nt == 1;
+  if (nt > 1 && nt <= slots / 4) { slots -= slots % nt; walk.column_fixed = true; }
+  walk.rounds = static_cast<double>((units + slots - 1) / slots);
+  const bool shallow = !(g == 2 && K >= kDeepK) && splits == 1;       // one K block a stage
+  const bool fits = shallow && resident_stages(nk * (w / g) * kBlockKBytes) >= kResidentStages;
+  walk.resident = fits && walk.column_fixed && units >= 2 * slots;
+  if (epilogue == HY3D_EPI_GEGLU && fits && nt > 1 && w % (2 * kSlabCols) == 0 && units >= 2 * most && M * K <= kRangesMaxA) {
+    const double rounds = static_cast<double>((units + most - 1) / most);
+    if (rounds <= static_cast<double>(mt) && (!walk.resident || rounds < walk.rounds)) {     // two columns a CTA at most
+      walk.ranges = walk.resident = true;
+      walk.rounds = rounds;
+      slots = most;
+    }
+  }
+  walk.clusters = static_cast<int>(slots);
+  return walk;
+}
+
 struct TilePlan {
   int block_n = 0, group = 0;
   double us = 0.0;
@@ -862,7 +935,7 @@ TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_grou
   const int step = geglu ? 64 : 32;
   const int64_t nk = ((K + kBlockKBytes - 1) / kBlockKBytes + splits - 1) / splits;
   for (int g = 1; g <= 2; ++g) {
-    if (cta_group != 0 ? g != cta_group : (g == 2 && (M <= kTileM || splits > 1 || (geglu && K < kDeepK)))) continue;
+    if (cta_group != 0 ? g != cta_group : (g == 2 && (M <= kTileM || splits > 1))) continue;
     for (int bn = 64; bn <= 256; bn += step) {
       const int w = block_n != 0 ? block_n : N <= 128 ? static_cast<int>(N) : bn;
       if (w != bn && bn != 64) break;                    // a width that is given: once per group
@@ -870,13 +943,14 @@ TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_grou
       if (g == 2 && (w & 31) && cta_group == 0) continue;
       const int64_t nt = (N + w - 1) / w, mt = (M + kTileM * g - 1) / (kTileM * g);
       const int64_t tiles = mt * nt * splits;
-      int64_t slots = sms / g < tiles ? sms / g : tiles;
-      bool column_fixed = nt == 1;
-      if (nt > 1 && nt <= slots / 4) { slots -= slots % nt; column_fixed = true; }     // see the launch
-      const double rounds = static_cast<double>((tiles + slots - 1) / slots);
+      const Walk walk = plan_walk(M, N, K, g, w, splits, epilogue);
+      const bool column_fixed = walk.column_fixed || walk.ranges, resident = walk.resident;
+      const double rounds = walk.rounds;
       const bool deep = g == 2 && K >= kDeepK;
-      const bool resident = !deep && splits == 1 && column_fixed && tiles >= 2 * slots &&
-                            resident_stages(nk * (w / g) * kBlockKBytes) >= kResidentStages;
+      // GEGLU in pairs below deep K only in ranges of some length, where a single CTA's B tile does not fit: 12288 x 640 ->
+      // 5120 53.0 us in single CTAs, 50.8 in pairs; 24576 x 320 -> 2560 48.0 and 49.3, 8000 x 768 -> 3200 26.4 and 27.5.
+      if (g == 2 && cta_group == 0 && geglu && !deep &&
+          !(walk.ranges && rounds >= 8.0 && resident_stages(nk * 256 * kBlockKBytes) < kResidentStages)) continue;
       const Block& kb = g == 1 ? (resident ? kResident : kStream) : deep ? kPairDeep : resident ? kPairResident : kPair;
       const double c = w / 100.0;
       double block = kb.a + kb.b * c;
@@ -1083,7 +1157,7 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
   p.tma_store = (out_dtype != HY3D_S32 && block_n % (geglu ? 2 * kSlabCols : kSlabCols) == 0) ? 1 : 0;
   if (p.splits > 1) p.tma_store = 1;   // 64-byte slabs of int32 partials (block_n is a multiple of 16)
 
-  // Grid and tile order.  Tiles are walked N-fastest: CTAs running together share an A tile (a
+  // Grid and tile order (plan_walk).  Strided, tiles are walked N-fastest: CTAs running together share an A tile (a
   // large activation matrix is then fetched from HBM once, while the small B stays
   // L2-resident), and with the grid rounded down to a multiple of the column count every CTA
   // keeps ONE tile column for the whole launch, so its per-column scales and bias are staged
@@ -1091,24 +1165,9 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
   // equal on every sweep shape).
   const int sms = device_sm_count();
   if (sms <= 0) return HY3D_ERR_CUDA;
-  const int total_tiles = p.m_tiles * p.n_tiles;
-  const int total_units = total_tiles * p.splits;
-  const int max_clusters = sms / group;
-  int clusters = total_units < max_clusters ? total_units : max_clusters;
-  bool column_fixed = p.n_tiles == 1;
-  p.n_fastest = 0;
-  if (p.n_tiles > 1) {
-    p.n_fastest = 1;
-    if (p.n_tiles <= clusters / 4) { clusters -= clusters % p.n_tiles; column_fixed = true; }
-  }
-#ifdef HY3D_TRACE
-  if (const char* e = getenv("HY3D_ORDER")) {
-    p.n_fastest = atoi(e) ? 1 : 0;
-    clusters = total_tiles < max_clusters ? total_tiles : max_clusters;
-    column_fixed = p.n_tiles == 1;
-    if (p.n_fastest && p.n_tiles <= clusters / 4) { clusters -= clusters % p.n_tiles; column_fixed = true; }
-  }
-#endif
+  const Walk walk = plan_walk(M, N, K, group, block_n, p.splits, epilogue);
+  const int clusters = walk.clusters;
+  p.n_fastest = p.n_tiles > 1 && !walk.ranges ? 1 : 0;
 
   // Shared memory: [pipeline stages][resident B tile][store staging][control block].
   // A single CTA's load rate from L2 (about 64 bytes per clock) is what paces short-K tiles:
@@ -1120,16 +1179,15 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
   const int ctrl_bytes = static_cast<int>(sizeof(DenseCtrl));
   const int staging1 = kEpiWarps * kSlabBytes;
   int b_resident = 0, store_bufs = 2, stages = 0, stage_bytes = 0;
-  if (atoms == 1 && column_fixed && p.splits == 1 && total_tiles >= 2 * clusters) {
+  if (walk.resident) {
     // One staging buffer per epilogue warp: measured faster than two here (a warp that must
     // wait for its previous store to leave shared memory paces the store stream, and the
     // loads queue behind fewer stores).
-    const int st = static_cast<int>(resident_stages(b_tile_bytes));
-    if (st >= kResidentStages) { b_resident = 1; store_bufs = 1; stages = st; stage_bytes = a_stage; }
+    b_resident = 1;
+    store_bufs = 1;
+    stages = static_cast<int>(resident_stages(b_tile_bytes));
+    stage_bytes = a_stage;
   }
-#if defined(HY3D_TRACE) || defined(HY3D_KO)
-  if (const char* e = getenv("HY3D_B_RESIDENT")) { if (!atoi(e)) b_resident = 0; }
-#endif
   if (!b_resident) {
     stage_bytes = atoms * (a_stage + (block_n / group) * kBlockKBytes);
     // Two staging buffers per epilogue warp unless that costs one of fewer than four pipeline stages.
@@ -1181,17 +1239,20 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
 
   using KernelFn = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const DenseArgs);
   // [0]: one CTA per tile, [1]: CTA pairs, [2]: CTA pairs with deep (two-block) stages.
-#define HY3D_DENSE_ROW(G, A)                                                              \
-  {{gemm_dense_kernel<false, HY3D_EPI_LINEAR, G, A>, gemm_dense_kernel<false, HY3D_EPI_GELU, G, A>, \
-    gemm_dense_kernel<false, HY3D_EPI_GEGLU, G, A>},                                        \
-   {gemm_dense_kernel<true, HY3D_EPI_LINEAR, G, A>, gemm_dense_kernel<true, HY3D_EPI_GELU, G, A>,   \
-    gemm_dense_kernel<true, HY3D_EPI_GEGLU, G, A>}}
+#define HY3D_DENSE_ROW(G, A)                                                                        \
+  {{gemm_dense_kernel<false, HY3D_EPI_LINEAR, G, A, false>, gemm_dense_kernel<false, HY3D_EPI_GELU, G, A, false>, \
+    gemm_dense_kernel<false, HY3D_EPI_GEGLU, G, A, false>},                                          \
+   {gemm_dense_kernel<true, HY3D_EPI_LINEAR, G, A, false>, gemm_dense_kernel<true, HY3D_EPI_GELU, G, A, false>,   \
+    gemm_dense_kernel<true, HY3D_EPI_GEGLU, G, A, false>}}
   static const KernelFn kernels[3][2][3] = {HY3D_DENSE_ROW(1, 1), HY3D_DENSE_ROW(2, 1), HY3D_DENSE_ROW(2, 2)};
 #undef HY3D_DENSE_ROW
+  static const KernelFn in_ranges[2][2] = {
+      {gemm_dense_kernel<false, HY3D_EPI_GEGLU, 1, 1, true>, gemm_dense_kernel<true, HY3D_EPI_GEGLU, 1, 1, true>},
+      {gemm_dense_kernel<false, HY3D_EPI_GEGLU, 2, 1, true>, gemm_dense_kernel<true, HY3D_EPI_GEGLU, 2, 1, true>}};
   // Raw int32 output runs the direct-store path of the <false, LINEAR> instance.
   const int ki = out_dtype == HY3D_BF16 ? 1 : 0;
   const int variant = (group == 2 && atoms == 2) ? 2 : group - 1;
-  const KernelFn kernel = kernels[variant][ki][epilogue];
+  const KernelFn kernel = walk.ranges ? in_ranges[group - 1][ki] : kernels[variant][ki][epilogue];
   rc = ensure_max_smem(reinterpret_cast<const void*>(kernel), kSmemLimit);
   if (rc != HY3D_OK) return rc;
   const int grid = group * clusters;

@@ -331,6 +331,21 @@ def test_sparse_accumulators_bit_exact(sp, M, K, N, bt):
     assert torch.equal(acc.cpu(), O.int32_matmul(X, O.expand_24(co, no)))
 
 
+# GEGLU in contiguous ranges down the tile columns: B loaded again inside a range, ragged rows and columns, single CTAs and
+# pairs, both types, against the direct-store form (32-column tiles walk strided); the last walks strided.
+@pytest.mark.parametrize("M,K,N,group,bn", [(5000, 512, 4096, 0, 0), (24576, 320, 2560, 0, 0), (12288, 640, 5120, 0, 0), (5003, 272, 1888, 1, 128),
+                                            (9001, 400, 1312, 2, 64), (3000, 128, 5120, 1, 64), (2600, 640, 3968, 2, 256), (49152, 64, 192, 1, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_dense_geglu_ranges(tc, M, K, N, group, bn, dtype):
+    A, B = _rand_i8((M, K), M + K).to(DEV), _rand_i8((N, K), N + K + 5).to(DEV)
+    g = torch.Generator().manual_seed(33)
+    a_s, w_s = (torch.rand(M, generator=g) * 0.05 + 1e-3).to(DEV), (torch.rand(N, generator=g) * 1e-4 + 1e-5).to(dtype).to(DEV)
+    bias = (torch.randn(N, generator=g) * 0.1).to(dtype).to(DEV)
+    for _ in range(3):
+        y = tc.int8_gemm_tc(A, B, a_s, w_s, bias, out_dtype=dtype, epilogue=2, cta_group=group, block_n=bn)
+        assert torch.equal(y, tc.int8_gemm_tc(A, B, a_s, w_s, bias, out_dtype=dtype, epilogue=2, cta_group=1, block_n=32))
+
+
 # Tokens fastest in contiguous ranges: a range that ends inside a column of weight tiles, at its end and beyond it, ragged last
 # tiles both ways, more columns than CTAs, pairs and single CTAs; widths that the cost model does not choose.
 @pytest.mark.parametrize("M,K,N,bt", [(3072, 1280, 10240, 0), (1500, 640, 10240, 0), (4444, 640, 3040, 0), (2000, 1024, 4096, 160),
