@@ -162,19 +162,25 @@ __device__ __forceinline__ void quotient2(float2 w, float scale, float inv, uint
 // rounds, the second a quarter full).  The arithmetic is torch's, operation by operation, so the buffers equal those of the torch
 // expressions: |w| max; dense: max(amax * (1/127), 1e-8), sparse: max(amax, 1e-8) * (1/127) (torch on
 // CUDA multiplies by the reciprocal of a Python divisor); rint of the IEEE quotient w / scale.
-// The quotient comes from the correctly rounded reciprocal and two residual corrections, two values per
+// 16-bit weights take one fused multiply-add, w * mul + 1.5 * 2^23, with the nudged reciprocal of the activation
+// quantiser: the argument in quantize.cu's header holds for this scale too, which is within 1.3e-7 of amax / 127 (w / amax
+// times 127 is at least 1.9e-6 of itself away from a half-integer, 11 significant bits each, unless it is one; scale,
+// reciprocal and nudge move it by 4.2e-7).  Half-integers at w = amax / 2 are told by the nudge; there are others where 127
+// divides the significand of amax, and anywhere where the scale is the floor of 1e-8: such rows, and fp32 weights, divide.
+// Their quotient comes from the correctly rounded reciprocal and two residual corrections, two values per
 // instruction: the first makes it faithful, and by Markstein's theorem ("Computation of elementary
 // functions on the IBM RISC System/6000 processor", 1990) the second then gives the correctly rounded
 // one.  |w| <= amax keeps the code within +-127.  Rows whose scale is not finite (a NaN or an infinity
 // among the weights) divide one by one in a loop of their own; a NaN quotient becomes 0 as in torch's cast.
 // Bound by instruction issue, most of it the pruning network on the half-rate ALU pipe.  10240 x 1280 bf16 with pruning:
-// the torch form, 11 launches over fp32 temporaries, took 160 us, this kernel 11.4 (without pruning 8.2), of which 6 are
-// HBM time.  Pieces of 32 elements a thread took 16.1; four lanes that shuffle a metadata word together, and the
-// question whether the row is finite at every four elements, 13.2, and were slower than those pieces where a row fills
-// them (10240 x 2048 17.0, 19.4 and 16.7 now; 1536 x 8192 12.5, 14.1 and 12.1).
+// the torch form, 11 launches over fp32 temporaries, took 160 us, this kernel 10.7 (without pruning 7.3), of which 6 are
+// HBM time; with the corrected quotient for every weight, six packed instructions a pair instead of one, 11.6 and 8.9
+// (8192 x 2048 14.3 and 10.2, now 12.7 and 8.4).  Pieces of 32 elements a thread took 16.1; four lanes that shuffle a metadata
+// word together, and the question whether the row is finite at every four elements, 13.2 (both with that quotient).
 // kKeep > 0 (16-bit types): a thread has at most that many vectors of its row and keeps them in registers between the
 // two passes (five fill five blocks an SM, eight leave four); otherwise (fp32, rows of more than 16384) the second pass
 // reads them again, which costs more than the fifth block brings (10240 x 4096 46.5 us against 35.5).
+enum { kNudged, kDivided, kNotFinite };      // how a row's codes are found
 template <int kType, bool kSparse, int kKeep>
 __global__ void __launch_bounds__(256, kKeep > 5 ? 4 : 5)
 quantize_weight_kernel(const void* __restrict__ w, int64_t N, int K, int8_t* __restrict__ codes,
@@ -241,8 +247,16 @@ quantize_weight_kernel(const void* __restrict__ w, int64_t N, int K, int8_t* __r
   }
   const bool finite = scale < __int_as_float(0x7F800000);   // false for NaN too
   const float inv = __frcp_rn(scale);
+  float mul = inv;
+  bool divide = kType == HY3D_F32;
+  if constexpr (kType != HY3D_F32) {
+    const float a = kSparse ? fmaxf(amax, 1e-8f) : amax;
+    const float rest = fmaf(scale, -127.0f, a);         // exact: a few units in the scale's last place, times 127
+    mul = __int_as_float(__float_as_int(inv) + (fmaf(scale, 3.814697265625e-6f, rest) >= 0.0f ? 2 : -2));
+    divide = fmaf(__fdiv_rn(a, 127.0f), -127.0f, a) == 0.0f || (!kSparse && __fmul_rn(amax, inv127) < 1e-8f);
+  }
   const int units = K >> 3;
-  auto work = [&](int u, auto is_finite, auto vector) {
+  auto work = [&](int u, auto how, auto vector) {
     const bool in = u < units;
     uint32_t words[2] = {0, 0};
     if (in) {
@@ -253,7 +267,10 @@ quantize_weight_kernel(const void* __restrict__ w, int64_t N, int K, int8_t* __r
 #pragma unroll
         for (int j = 0; j < kPer; j += 4) {
           uint32_t b[4];
-          if constexpr (is_finite.value) {
+          if constexpr (how.value == kNudged) {
+            const float2 t0 = quant::fast_code2(make_float2(f[j], f[j + 1]), mul), t1 = quant::fast_code2(make_float2(f[j + 2], f[j + 3]), mul);
+            b[0] = __float_as_uint(t0.x); b[1] = __float_as_uint(t0.y); b[2] = __float_as_uint(t1.x); b[3] = __float_as_uint(t1.y);
+          } else if constexpr (how.value == kDivided) {
             quotient2(make_float2(f[j], f[j + 1]), scale, inv, b[0], b[1]);
             quotient2(make_float2(f[j + 2], f[j + 3]), scale, inv, b[2], b[3]);
           } else {
@@ -276,18 +293,22 @@ quantize_weight_kernel(const void* __restrict__ w, int64_t N, int K, int8_t* __r
       *reinterpret_cast<uint2*>(codes + row * static_cast<int64_t>(K) + 8 * u) = make_uint2(words[0], words[1]);
     }
   };
+  using Nudged = std::integral_constant<int, kNudged>;
+  using Divided = std::integral_constant<int, kDivided>;
+  auto again = [&](int first) { return [=](int v) { return __ldg(src + (first + sub) * (8 / kPer) + v); }; };
   if (!finite) {
 #pragma unroll 1
-    for (int first = 0; first < units; first += G)
-      work(first + sub, std::false_type{}, [&](int v) { return __ldg(src + (first + sub) * (8 / kPer) + v); });
+    for (int first = 0; first < units; first += G) work(first + sub, std::integral_constant<int, kNotFinite>{}, again(first));
+  } else if (divide) {
+#pragma unroll 2
+    for (int first = 0; first < units; first += G) work(first + sub, Divided{}, again(first));
   } else if constexpr (kKeep > 0) {
 #pragma unroll
     for (int i = 0; i < kKeep; ++i)
-      if (i * G < units) work(sub + i * G, std::true_type{}, [&](int) { return kept[i]; });
-  } else {
+      if (i * G < units) work(sub + i * G, Nudged{}, [&](int) { return kept[i]; });
+  } else if constexpr (kType != HY3D_F32) {
 #pragma unroll 2
-    for (int first = 0; first < units; first += G)
-      work(first + sub, std::true_type{}, [&](int v) { return __ldg(src + (first + sub) * (8 / kPer) + v); });
+    for (int first = 0; first < units; first += G) work(first + sub, Nudged{}, again(first));
   }
   if constexpr (kSparse)                    // padding words: any valid 2:4 pattern (indices 0,1)
     for (int c = (K >> 5) + sub; c < meta_ld; c += G) meta[row * meta_ld + c] = 0x44444444u;

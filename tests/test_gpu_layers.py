@@ -143,6 +143,29 @@ def test_weight_conversion_equals_the_torch_expressions(qu, sp, dtype, N, K):
             assert torch.equal(layer.weight_int8_nk, codes)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("K", [768, 16384 + 512])      # kept in registers, read again
+def test_weight_conversion_at_the_ties(qu, dtype, K):
+    """Codes of weights around every half-integer multiple of the scale: rows of every significand of the largest weight (127
+    divides some), of a scale at its floor and below the type's normal range; the neighbours on both sides of each tie."""
+    bits = 7 if dtype == torch.bfloat16 else 10
+    amax = torch.cat([1 + torch.arange(2 ** bits) / 2 ** bits, torch.tensor([1.27e-6, 1.2e-6, 3e-7, 6e-8, 1e-3, 254 / 4096])]).to(dtype)
+    k = torch.arange(127)
+    tie = (amax.double()[:, None] * (2 * k + 1) / 254).to(dtype)
+    near = torch.cat([tie, torch.nextafter(tie, torch.zeros_like(tie)), torch.nextafter(tie, amax[:, None].expand_as(tie))], 1)
+    near = torch.cat([near, -near, amax[:, None], -amax[:, None]], 1)
+    w = torch.zeros(amax.numel(), K, dtype=dtype)
+    w[:, :near.shape[1]] = torch.minimum(near.abs(), amax[:, None]).copysign(near)
+    lin = torch.nn.Linear(K, w.shape[0], bias=False, dtype=dtype, device=DEV)
+    lin.weight.data.copy_(w)
+    wf, am = w.to(DEV).float(), w.to(DEV).float().abs().amax(1, keepdim=True)
+    dense = qu.Int8Linear.from_linear(lin)
+    assert torch.equal(dense.weight_int8_nk, torch.round(wf / (am / 127.0).clamp(min=1e-8)).clamp(-128, 127).to(torch.int8))
+    codes = torch.round(wf / (am.clamp(min=1e-8) / 127.0)).clamp(-128, 127).to(torch.int8)
+    comp, _ = O.prune_compress(codes.cpu())
+    assert torch.equal(qu.Int8Linear.from_linear_sparse(lin).weight_sparse_comp.cpu(), comp)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("N,K", [(9, 32), (40, 544), (24, 1312), (17, 2560), (3, 16416)])
 def test_weight_conversion_in_registers_and_with_values_that_are_not_finite(qu, sp, dtype, N, K):
