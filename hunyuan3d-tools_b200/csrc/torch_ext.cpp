@@ -437,7 +437,7 @@ PyObject* groupnorm_nhwc(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return groupnorm_impl(a[0], groups, a[2], a[3], PyFloat_AS_DOUBLE(a[4]), a[5] == Py_True, a[6], Py_None);
 }
 
-// quantize_weight(w (N,K), sparse) -> (codes, scale) or (compressed codes, metadata, scale) | None
+// quantize_weight(w (N,K), sparse) -> (codes, scale) or (compressed codes, metadata, the layer's empty dense codes, scale) | None
 PyObject* quantize_weight(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 2) return none();
@@ -451,10 +451,13 @@ PyObject* quantize_weight(PyObject*, PyObject* const* a, Py_ssize_t n) {
   cudaStream_t st = c10::cuda::getCurrentCUDAStream(w->device().index()).stream();
   const auto dev = w->device();
   const int64_t ld = 4 * ((K + 127) / 128);
-  at::Tensor out[3];
+  at::Tensor out[4];
   int count = 0;
   out[count++] = at::Tensor(at::detail::empty_cuda({N, sparse ? K / 2 : K}, at::kChar, dev, std::nullopt));
-  if (sparse) out[count++] = at::Tensor(at::detail::empty_cuda({N, ld}, at::kInt, dev, std::nullopt));
+  if (sparse) {
+    out[count++] = at::Tensor(at::detail::empty_cuda({N, ld}, at::kInt, dev, std::nullopt));
+    out[count++] = at::Tensor(at::detail::empty_cuda({0}, at::kChar, dev, std::nullopt));
+  }
   const at::ScalarType st_type = w->scalar_type() == at::kBFloat16 ? at::kBFloat16 : at::kHalf;
   out[count++] = at::Tensor(at::detail::empty_cuda({N}, st_type, dev, std::nullopt));
   const int rc = api.hy3d_quantize_weight(

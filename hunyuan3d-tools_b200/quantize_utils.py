@@ -299,8 +299,8 @@ class Int8Linear(nn.Module):
                                "(pruning and packing run on the GPU)")
         got = (_NATIVE or _load_native()).quantize_weight(weight, True)
         if got is not None:          # its scales have the layer's type; no dense codes
-            comp, meta, scale = got
-            return Int8Linear._assemble(linear, scale.dtype, comp.new_empty(0), scale, comp, meta)
+            comp, meta, codes, scale = got
+            return Int8Linear._assemble(linear, scale.dtype, codes, scale, comp, meta)
         has_bias = linear.bias is not None
         dt = _param_dtype(linear)
         device = weight.device
