@@ -70,7 +70,7 @@ __device__ __forceinline__ void cluster_sync_release() {
 
 // Floats of a chunk's per-channel sums in shared memory.  Padded, so that chunks start in different banks: the threads that
 // add a group's channels take one chunk each, and with slices of 160 floats sixteen of them met in one bank (12 x 1280 x 16 x 16
-// 12.3 -> 10.5 us, 12 x 2560 x 16 x 16 17.0 -> 13.5, 12 x 1280 x 8 x 8 7.3 -> 6.4, 12 x 640 x 32 x 32 17.6 -> 17.0).
+// 12.3 -> 11.2 us, 12 x 2560 x 16 x 16 17.0 -> 13.6, 12 x 1280 x 8 x 8 7.3 -> 6.7, 12 x 640 x 32 x 32 17.7 -> 17.4).
 __host__ __device__ constexpr int slice_floats(int lanes, int slab) { return (lanes * 2 * slab + 31) / 32 * 32 + 2; }
 
 // How a sample's sums are ordered: `chunks` ranges of `rows` rows; `lanes` row lanes walk a chunk with a
@@ -78,6 +78,24 @@ __host__ __device__ constexpr int slice_floats(int lanes, int slab) { return (la
 // `classes` running sums (chunk modulo classes), added in order last.
 struct Order {
   int chunks, rows, lanes, classes;
+};
+
+// i / by for 0 <= i and i * by < 2^31: a multiplication by ceil(2^31 / by), which is above 2^31 / by by less than one, so
+// that the product errs by less than i / 2^31 < 1 / by.  The indices divided here are below 2^15 and `by` is at most 5120.
+// Integer division takes some twenty instructions in a row, and every phase of the kernel began with one or two: with
+// these and loops that count rows, 12 x 320 x 64 x 64 25.3 -> 24.3 us, 12 x 1280 x 16 x 16 11.2 -> 9.8, 4 x 128 x 11 x 12
+// 4.6 -> 4.2.
+struct Divisor {
+  uint32_t magic;
+  explicit Divisor(int by) : magic(static_cast<uint32_t>(((1ll << 31) + by - 1) / by)) {}
+  __device__ int operator()(int i) const { return static_cast<int>(__umulhi(2u * static_cast<uint32_t>(i), magic)); }
+};
+
+// What the cut into slabs, ranks and sets gives every thread to know.
+struct Cut {
+  int sets;                 // chunks that a CTA works on at a time
+  float inv_n;              // 1 / elements of a group
+  Divisor vec_cols, lanes, width, pairs, cpg;       // vectors of a slab's row, order.lanes, 2 * slab, 2 * slab_groups
 };
 
 // Threads are laid out as (row lane ty, vector column tx): tx = tid % (slab / 8) owns 8 adjacent channels.
@@ -91,7 +109,7 @@ template <bool kBf16, int kAdd, bool kSilu, bool kWide>
 __global__ void __launch_bounds__(kWide ? kWideThreads : narrow_threads(kAdd > 0), kWide ? 1 : 3)
 groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ pre, const uint16_t* __restrict__ add,
                  int64_t add_ld, int64_t HW, int C, int cpg,
-                 int slab_groups, int rows_per_cta, int chunks_per_rank, int reps, Order order,
+                 int slab_groups, int rows_per_cta, int chunks_per_rank, int reps, Order order, Cut cut,
                  const void* __restrict__ gamma, const void* __restrict__ beta, int gb_dtype, float eps,
                  uint16_t* __restrict__ y) {
   // [chunks][2 * slab_groups] group partials, [classes][2 * slab_groups] their class sums, then the fold's
@@ -99,9 +117,9 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ pr
   extern __shared__ float smem[];
   const int slab = slab_groups * cpg;
   const int vec_cols = slab >> 3, row_vecs = C >> 3;
-  const int k = blockDim.x / vec_cols, sets = k / order.lanes;
-  const int tx = threadIdx.x % vec_cols, ty = threadIdx.x / vec_cols;
-  const int set = ty / order.lanes, lane = ty - set * order.lanes;
+  const int sets = cut.sets, k = sets * order.lanes;
+  const int ty = cut.vec_cols(threadIdx.x), tx = threadIdx.x - ty * vec_cols;
+  const int set = cut.lanes(ty), lane = ty - set * order.lanes;
   const int S = gridDim.x, rank = blockIdx.x, b = blockIdx.z;
   const int c0 = static_cast<int>(blockIdx.y) * slab + 8 * tx;      // this thread's first channel
   float* s_part = smem;
@@ -138,16 +156,16 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ pr
       const int64_t r0 = static_cast<int64_t>(first + slot) * order.rows;
       const int rows = static_cast<int>(r0 + order.rows < HW ? order.rows : HW - r0);
       const int step = order.lanes * row_vecs;                        // at most 320 vectors and a row
-      int left = (rows - lane + order.lanes - 1) / order.lanes;       // rows of this lane (may be < 1)
+      int left = rows - lane;                                         // rows from this lane's on (may be < 1)
       const uint4* in = src + (r0 + lane) * row_vecs;
-      for (; left > 0; left -= 4, in += 4 * step) {                   // four rows in flight per thread, to the last
+      for (; left > 0; left -= 4 * order.lanes, in += 4 * step) {    // four rows in flight per thread, to the last
         uint4 v[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-          if (u < left) v[u] = in[u * step];
+          if (u * order.lanes < left) v[u] = in[u * step];
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-          if (u < left) accumulate(v[u]);
+          if (u * order.lanes < left) accumulate(v[u]);
       }
       // every row lane parks its sums in its own slice
       float* mine = s_acc + slot * set_floats + lane * 2 * slab + 8 * tx;
@@ -161,16 +179,13 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ pr
     // Channel c adds the lanes of its chunk in order, group g its channels in order; the group sums of the
     // chunk go to every rank of the cluster.
     if (order.lanes > 1) {
-      const int width = 2 * slab, cols = min(width, static_cast<int>(blockDim.x)), side = blockDim.x / cols;   // whole slots side by side
-      const int row = threadIdx.x / cols;
-      for (int slot = row < side ? row : here; slot < here; slot += side) {
-        for (int i = threadIdx.x - row * cols; i < width; i += cols) {
-          float* p = s_acc + slot * set_floats + i;
-          float a = *p;
+      for (int i = threadIdx.x; i < here * 2 * slab; i += blockDim.x) {
+        const int slot = cut.width(i);
+        float* p = s_acc + slot * set_floats + i - slot * 2 * slab;
+        float a = *p;
 #pragma unroll 4
-          for (int l = 1; l < order.lanes; ++l) a += p[l * width];
-          *p = a;
-        }
+        for (int l = 1; l < order.lanes; ++l) a += p[l * 2 * slab];
+        *p = a;
       }
     }
     __syncwarp();          // the fold's trip counts differ by thread; the barrier is for converged warps
@@ -178,10 +193,10 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ pr
     peers_run = true;
     __syncthreads();
     for (int i = threadIdx.x; i < here * 2 * slab_groups; i += blockDim.x) {    // sums, then sums of squares
-      const int slot = i / (2 * slab_groups), g = i - slot * 2 * slab_groups;
+      const int slot = cut.pairs(i), g = i - slot * 2 * slab_groups;
       const float* p = s_acc + slot * set_floats + g * cpg;
       float a = 0.0f;
-#pragma unroll 8
+#pragma unroll 4
       for (int c = 0; c < cpg; ++c) a += p[c];
       const uint32_t at = smem_u32(s_part + (first + slot) * 2 * slab_groups + g);
       for (int peer = 0; peer < S; ++peer)
@@ -192,7 +207,7 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ pr
   if (!peers_run) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // a rank without chunks
   if (S > 1) cluster_sync_release(); else __syncthreads();
   for (int i = threadIdx.x; i < order.classes * 2 * slab_groups; i += blockDim.x) {
-    const int cls = i / (2 * slab_groups), g = i - cls * 2 * slab_groups;
+    const int cls = cut.pairs(i), g = i - cls * 2 * slab_groups;
     float a = 0.0f;
 #pragma unroll 4
     for (int ch = cls; ch < order.chunks; ch += order.classes) a += s_part[ch * 2 * slab_groups + g];
@@ -200,16 +215,15 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ pr
   }
   __syncthreads();
   // One thread per channel of the slab turns the class sums into scale and shift.
-  const float inv_n = 1.0f / (static_cast<float>(HW) * static_cast<float>(cpg));
   for (int c = threadIdx.x; c < slab; c += blockDim.x) {
-    const int g = c / cpg;
+    const int g = cut.cpg(c);
     float a = 0.0f, q = 0.0f;
     for (int cls = 0; cls < order.classes; ++cls) {
       a += s_class[cls * 2 * slab_groups + g];
       q += s_class[cls * 2 * slab_groups + slab_groups + g];
     }
-    const float mean = a * inv_n;
-    const float rstd = rsqrtf(fmaxf(fmaf(-mean, mean, q * inv_n), 0.0f) + eps);
+    const float mean = a * cut.inv_n;
+    const float rstd = rsqrtf(fmaxf(fmaf(-mean, mean, q * cut.inv_n), 0.0f) + eps);
     const int ch = static_cast<int>(blockIdx.y) * slab + c;
     const float ga = gamma ? load_scalar(gamma, gb_dtype, ch) : 1.0f;
     const float be = beta ? load_scalar(beta, gb_dtype, ch) : 0.0f;
@@ -248,17 +262,17 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ pr
   const int rows = static_cast<int>(r0 + rows_per_cta < HW ? rows_per_cta : HW - r0);
   const int64_t at0 = (r0 + ty) * row_vecs;
   const int step = k * row_vecs;
-  int left = (rows - ty + k - 1) / k;                                 // may be < 1
+  int left = rows - ty;                                               // may be < 1
   const uint4* in = src + at0;
   uint4* out = dst + at0;
-  for (; left > 0; left -= 4, in += 4 * step, out += 4 * step) {
+  for (; left > 0; left -= 4 * k, in += 4 * step, out += 4 * step) {
     uint4 v[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (u < left) v[u] = __ldcs(in + u * step);
+      if (u * k < left) v[u] = __ldcs(in + u * step);
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (u < left) out[u * step] = transform(v[u]);
+      if (u * k < left) out[u * step] = transform(v[u]);
   }
 }
 
@@ -359,7 +373,7 @@ int groupnorm_nhwc(const void* x, const void* pre, const void* add, int64_t add_
                        static_cast<size_t>(reps) * sets * slice_floats(order.lanes, slab)) * sizeof(float);
   if (rows_per_cta > 0x7FFFFFFF || B > 65535 || groups / slab_groups > 65535) return HY3D_ERR_SHAPE;
 
-  using KernelFn = void (*)(const uint16_t*, const uint16_t*, const uint16_t*, int64_t, int64_t, int, int, int, int, int, int, Order, const void*,
+  using KernelFn = void (*)(const uint16_t*, const uint16_t*, const uint16_t*, int64_t, int64_t, int, int, int, int, int, int, Order, Cut, const void*,
                             const void*, int, float, uint16_t*);
 #define HY3D_GN_ADD(BF, A, W) {groupnorm_kernel<BF, A, false, W>, groupnorm_kernel<BF, A, true, W>}
 #define HY3D_GN_ROW(W)                                                                    \
@@ -391,6 +405,8 @@ int groupnorm_nhwc(const void* x, const void* pre, const void* add, int64_t add_
     return n == 0 || (per_sm == 1 ? clusters <= n : clusters * 20 <= n * 19);
   };
   while (room < most && !holds(room)) ++room;
+  const Cut cut{sets, 1.0f / (static_cast<float>(HW) * static_cast<float>(cpg)), Divisor(vec_cols), Divisor(order.lanes),
+                Divisor(2 * slab), Divisor(2 * slab_groups), Divisor(cpg)};
   cudaLaunchAttribute attr[3];
   attr[0] = pdl_attribute();
   attr[2] = carveout_attribute(room < most ? room : most, static_cast<int64_t>(smem));
@@ -402,7 +418,7 @@ int groupnorm_nhwc(const void* x, const void* pre, const void* add, int64_t add_
   cfg.numAttrs = 3;
   const cudaError_t err = cudaLaunchKernelEx(
       &cfg, kernel, static_cast<const uint16_t*>(x), static_cast<const uint16_t*>(pre), static_cast<const uint16_t*>(add), add_ld, HW, static_cast<int>(C), cpg,
-      slab_groups, static_cast<int>(rows_per_cta), chunks_per_rank, reps, order, gamma, beta, gb_dtype, eps, static_cast<uint16_t*>(y));
+      slab_groups, static_cast<int>(rows_per_cta), chunks_per_rank, reps, order, cut, gamma, beta, gb_dtype, eps, static_cast<uint16_t*>(y));
   if (err != cudaSuccess) {
     cudaGetLastError();
     return HY3D_ERR_CUDA;
