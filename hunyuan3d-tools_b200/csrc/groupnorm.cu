@@ -80,6 +80,12 @@ struct Order {
   int chunks, rows, lanes, classes;
 };
 
+// Sets that work side by side when `most` could: evened out over the rounds that a rank's chunks take.
+int even_sets(int chunks, int ranks, int most) {
+  const int per_rank = (chunks + ranks - 1) / ranks, rounds = (per_rank + most - 1) / most;
+  return (per_rank + rounds - 1) / rounds;
+}
+
 // i / by for 0 <= i and i * by < 2^31: a multiplication by ceil(2^31 / by), which is above 2^31 / by by less than one, so
 // that the product errs by less than i / 2^31 < 1 / by.  The indices divided here are below 2^15 and `by` is at most 5120.
 // Integer division takes some twenty instructions in a row, and every phase of the kernel began with one or two: with
@@ -359,12 +365,23 @@ int groupnorm_nhwc(const void* x, const void* pre, const void* add, int64_t add_
     wide = static_cast<int64_t>(ranks) * (groups / slab_groups) * B <= sms;
     sets = (wide ? kWideThreads : narrow_threads(add != nullptr)) / ((slab_groups * cpg >> 3) * order.lanes);
     if (sets < 1) return HY3D_ERR_SHAPE;
+    // Clusters that do not all run at the same time make a second wave: as many ranks as prevent it, if any number does.
+    // 8 x 96 x 89 x 86 (16 wide clusters of eight, 15 run) 24.6 us, with six ranks 16.4; 8 x 640 x 40 x 40 20.3 and 17.0
+    // (seven), 9 x 832 x 53 x 42 29.2 and 25.7; of 140 drawn shapes it changes seven, all of them faster, 1.14x to 1.50x.
+    auto one_wave = [&](int r) {
+      const int64_t warps = (((slab_groups * cpg >> 3) * order.lanes * even_sets(order.chunks, r, sets)) + 31) / 32;
+      const int64_t most = resident_ctas(wide, add != nullptr, warps);
+      const int n = resident_clusters(r, static_cast<int>(most < 8 ? most : 8));
+      return n == 0 || B * (groups / slab_groups) <= n;
+    };
+    for (int r = ranks; r >= 1; --r)
+      if (one_wave(r)) { ranks = r; break; }
   }
   const int slab = slab_groups * cpg, vec_cols = slab >> 3;
   // As many rounds as 42 KB of slices hold between two folds (two of 12 x 320 x 64 x 64; a fold less is worth 1 us there).
   const int chunks_per_rank = (order.chunks + ranks - 1) / ranks;
   const int rounds = (chunks_per_rank + sets - 1) / sets;
-  sets = (chunks_per_rank + rounds - 1) / rounds;
+  sets = even_sets(order.chunks, ranks, sets);
   const int k = sets * order.lanes;
   int reps = 42 * 1024 / (sets * slice_floats(order.lanes, slab) * 4);
   reps = reps < 1 ? 1 : reps > rounds ? rounds : reps;

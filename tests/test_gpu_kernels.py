@@ -567,6 +567,20 @@ def test_groupnorm_nhwc_matches_torch_fp32(ik, dtype, silu, shape):
     assert float((ya.float() - refa.float()).abs().max()) <= 2 * ulpa
 
 
+@pytest.mark.parametrize("shape", [(8, 96, 89, 86), (8, 640, 40, 40), (9, 832, 21, 42)])     # fewer ranks, so that one wave does
+def test_groupnorm_nhwc_fewer_ranks(ik, shape):
+    B, C, H, W = shape
+    g = torch.Generator(device=DEV).manual_seed(C)
+    x = (torch.randn(B, C, H, W, generator=g, device=DEV) * 2 + 0.7).bfloat16().contiguous(memory_format=torch.channels_last)
+    gamma, beta = 1 + 0.2 * torch.randn(C, generator=g, device=DEV), 0.2 * torch.randn(C, generator=g, device=DEV)
+    add = (torch.randn(B, C, generator=g, device=DEV) * 0.5).bfloat16()
+    for term in (None, add):
+        xs = x if term is None else x + term[:, :, None, None]
+        ref = torch.nn.functional.group_norm(xs.float(), 32, gamma, beta, 1e-5).bfloat16()
+        y = ik.groupnorm_nhwc(x, 32, gamma, beta, 1e-5, silu=True, add=term)
+        assert O.rel_l2(y, torch.nn.functional.silu(ref.float()).bfloat16()) < 3e-3
+
+
 def test_groupnorm_nhwc_argument_checks(ik):
     x = torch.randn(2, 64, 4, 4, device=DEV).bfloat16()
     with pytest.raises(RuntimeError):
