@@ -516,6 +516,19 @@ def test_layernorm_quantize_equals_quantising_its_own_output(ik, dtype, M, K):
     assert torch.equal(q3, q) and torch.equal(s3, s)
 
 
+@pytest.mark.parametrize("batches,rows", [(1, 1), (1, 0), (2, 0), (2, 7)])     # row batches of every block, and rows beyond them
+def test_layernorm_quantize_uneven_trips(ik, batches, rows):
+    K = 1280                                                                  # eight rows a batch, three blocks an SM
+    M = 3 * torch.cuda.get_device_properties(0).multi_processor_count * 8 * batches + rows
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x = (torch.randn(M, K, generator=g, device=DEV) * 3 + 0.5).bfloat16()
+    gamma, beta = 1 + 0.1 * torch.randn(K, generator=g, device=DEV), 0.1 * torch.randn(K, generator=g, device=DEV)
+    q, s = ik.layernorm_quantize(x, gamma, beta, 1e-5)
+    for lo in range(0, M, 1000):                                              # a block of these makes one trip
+        qo, so = ik.layernorm_quantize(x[lo:lo + 1000], gamma, beta, 1e-5)
+        assert torch.equal(q[lo:lo + 1000], qo) and torch.equal(s.reshape(-1)[lo:lo + 1000], so.reshape(-1))
+
+
 def test_layernorm_quantize_without_affine_and_argument_checks(ik):
     x = torch.randn(64, 256).bfloat16().to(DEV)
     q, s, y = ik.layernorm_quantize(x, None, None, 1e-6, return_normalised=True)
