@@ -910,6 +910,7 @@ Walk plan_walk(int64_t M, int64_t N, int64_t K, int g, int w, int splits, int ep
 struct TilePlan {
   int block_n = 0, group = 0;
   double us = 0.0;
+  Walk walk;
 };
 
 // Tile width and CTA grouping for a launch of `splits` K ranges, with its expected device time.  Pairs halve the
@@ -970,7 +971,7 @@ TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_grou
       // A CTA does not fit beside a quantiser's, so a grid that wants nearly every SM starts late behind one: it
       // needs a few SMs to spare (257 x 1536 -> 4608, whole layer: 144 tiles 9.0 us, 108 tiles 8.1).
       if (splits == 1 && rounds == 1.0 && tiles * g * 5 > sms * 4) us += 0.7;
-      if (us < best.us) { best.us = us; best.block_n = w; best.group = g; }
+      if (us < best.us) { best.us = us; best.block_n = w; best.group = g; best.walk = walk; }
     }
   }
   return best;
@@ -1107,12 +1108,16 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
     return HY3D_ERR_SHAPE;
 
   int group = cta_group;
+  Walk walk;
+  bool walk_known = false;
   if (block_n == 0 || group == 0) {
     const TilePlan t = plan_tile(M, N, K, epilogue, cta_group, block_n, splits);
     block_n = t.block_n;
     group = t.group;
+    walk = t.walk;
+    walk_known = splits == 1;
 #ifdef HY3D_TRACE
-    if (const char* e = getenv("HY3D_CTA_GROUP")) group = atoi(e) == 2 ? 2 : 1;
+    if (const char* e = getenv("HY3D_CTA_GROUP")) { group = atoi(e) == 2 ? 2 : 1; walk_known = false; }
 #endif
   }
   if (block_n < 16 || block_n > 256 || (block_n & 15) || (geglu && (block_n & 31)))
@@ -1121,6 +1126,7 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
   if (group == 2 && (block_n & 31)) {
     if (cta_group == 2) return HY3D_ERR_SHAPE;
     group = 1;
+    walk_known = false;
   }
 
   DenseArgs p;
@@ -1165,7 +1171,7 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
   // equal on every sweep shape).
   const int sms = device_sm_count();
   if (sms <= 0) return HY3D_ERR_CUDA;
-  const Walk walk = plan_walk(M, N, K, group, block_n, p.splits, epilogue);
+  if (!walk_known) walk = plan_walk(M, N, K, group, block_n, p.splits, epilogue);
   const int clusters = walk.clusters;
   p.n_fastest = p.n_tiles > 1 && !walk.ranges ? 1 : 0;
 
