@@ -411,7 +411,7 @@ int groupnorm_nhwc(const void* x, const void* pre, const void* add, int64_t add_
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   // Shared memory for as few CTAs an SM as run all clusters at the same time, L1 with what is left: 12 x 320 x 64 x 64 with
-  // room for one CTA fewer 35.6 us, with all of it shared 30.6, as here 25.1.  Clusters leave SMs of a GPC empty, so an
+  // room for one CTA fewer 35.6 us, with all of it shared 30.6, as here 25.1 (24.3 since).  Clusters leave SMs of a GPC empty, so an
   // even share of the CTAs is not always enough: 6 x 960 x 64 x 64 (48 clusters of six) 42.4 us with room for two CTAs, 30.5
   // for three, 2 x 320 x 32 x 32 (16 of eight) 10.8 for one, 6.8 for two.  From two CTAs on the scheduler leaves a few more.
   const int64_t clusters = static_cast<int64_t>(groups / slab_groups) * B;
