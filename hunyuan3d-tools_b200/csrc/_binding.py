@@ -35,6 +35,7 @@ SIGNATURES = {
     "hy3d_gemm_w8a8_dense": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int,
                              c_void_p, c_int, c_int64, c_int64, c_int64, c_int, c_int, c_int,
                              c_void_p],
+    "hy3d_gemm_plan": [c_int64, c_int64, c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "hy3d_dense_splitk_plan": [c_int64, c_int64, c_int64, c_int, c_void_p],
     "hy3d_dense_layer_splitk_plan": [c_int64, c_int64, c_int64, c_int, c_void_p],
     "hy3d_gemm_w8a8_dense_splitk": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p,

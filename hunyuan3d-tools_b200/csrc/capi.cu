@@ -68,6 +68,12 @@ int device_sm_count() {
   return query_device(&sms, &major) == HY3D_OK ? sms : -1;
 }
 
+// What a plan reckons with: the device's SMs, without a device a whole B200's.
+int planned_sms() {
+  const int sms = device_sm_count();
+  return sms > 0 ? sms : 148;
+}
+
 int current_device() {
   int dev = 0;
   return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
@@ -102,12 +108,14 @@ int ensure_max_smem(const void* kernel, int bytes) {
 __global__ void occupancy_probe_kernel() {}
 
 // Clusters of `ranks` CTAs that run at the same time with room for `per_sm` CTAs on an SM: the GPCs have 16 to 20 SMs, and
-// what is left over in each stays idle (148 SMs: 15 clusters of eight, 45 of three; with two CTAs an SM 33 and 93).
+// what is left over in each stays idle (148 SMs: 15 clusters of eight, 45 of three; with two CTAs an SM 33 and 93).  Asked
+// once per device.
 int resident_clusters(int ranks, int per_sm) {
   constexpr int kMost = 8;
-  static std::atomic<int> known[kMost + 1][kMost + 1];
-  if (ranks < 1 || ranks > kMost || per_sm < 1 || per_sm > kMost) return 0;
-  int n = known[per_sm][ranks].load(std::memory_order_relaxed);
+  static std::atomic<int> known[kMaxDevices][kMost + 1][kMost + 1];
+  const int dev = current_device();
+  if (dev < 0 || dev >= kMaxDevices || ranks < 1 || ranks > kMost || per_sm < 1 || per_sm > kMost) return 0;
+  int n = known[dev][per_sm][ranks].load(std::memory_order_relaxed);
   if (n == 0) {
     const void* kernel = reinterpret_cast<const void*>(occupancy_probe_kernel);
     cudaLaunchConfig_t cfg = {};
@@ -125,7 +133,7 @@ int resident_clusters(int ranks, int per_sm) {
       cudaGetLastError();
       n = device_sm_count() * per_sm * 3 / 4 / ranks;
     }
-    known[per_sm][ranks].store(n, std::memory_order_relaxed);
+    known[dev][per_sm][ranks].store(n, std::memory_order_relaxed);
   }
   return n;
 }
@@ -333,6 +341,14 @@ int hy3d_dense_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, int64_
 }
 int hy3d_dense_layer_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, int64_t* workspace_bytes) {
   return splitk_plan(M, N, K, epilogue, true, workspace_bytes);
+}
+
+int hy3d_gemm_plan(int64_t M, int64_t N, int64_t K, int epilogue, int sparse, int cta_group, int block, int sms, int* plan) {
+  if (!plan || epilogue < HY3D_EPI_LINEAR || epilogue > HY3D_EPI_GEGLU || cta_group < 0 || cta_group > 2 || sms < 0) return HY3D_ERR_ARG;
+  if (M <= 0 || N <= 0 || K <= 0) return HY3D_ERR_SHAPE;
+  if (sms == 0) sms = planned_sms();
+  return sparse ? sparse_gemm_plan(M, N, K, epilogue, block, sms, plan)
+                : dense_gemm_plan(M, N, K, epilogue, cta_group, block, sms, plan);
 }
 
 int hy3d_gemm_w8a8_dense_splitk(const int8_t* A, const int8_t* B, const float* act_scale,

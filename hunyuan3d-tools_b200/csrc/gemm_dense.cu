@@ -26,6 +26,7 @@ namespace hy3d {
 int encode_tmap_2d_u8(CUtensorMap* map, const void* base, uint64_t inner_bytes, uint64_t rows,
                       uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_rows, int swizzle_bytes);
 int device_sm_count();
+int planned_sms();
 int current_device();
 // Raises a kernel's dynamic shared-memory limit once per (device, kernel); thread-safe.
 int ensure_max_smem(const void* kernel, int bytes);
@@ -882,8 +883,7 @@ struct Walk {
   double rounds = 0.0;       // tiles that the busiest CTA works through
 };
 constexpr int64_t kRangesMaxA = 64000000;
-Walk plan_walk(int64_t M, int64_t N, int64_t K, int g, int w, int splits, int epilogue) {
-  const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
+Walk plan_walk(int64_t M, int64_t N, int64_t K, int g, int w, int splits, int epilogue, int sms) {
   const int64_t nk = (K + kBlockKBytes - 1) / kBlockKBytes;
   const int64_t nt = (N + w - 1) / w, mt = (M + kTileM * g - 1) / (kTileM * g);
   const int64_t units = mt * nt * splits, most = sms / g < units ? sms / g : units;
@@ -924,7 +924,7 @@ struct TilePlan {
 // 11.3 -> 9.8, 257 x 1536 -> 6144 7.5 -> 6.8.)  Gates and a short K were rare in that fit; over 490 shapes, most with
 // K <= 1152, x all tiles: `tile_us`, dearer GELU in pairs and no pairs for GEGLU below deep K (1463 x 64 -> 3840 with GEGLU
 // 12.7 -> 7.7 us, 1300 x 128 -> 5024 7.1 -> 5.6, 6873 x 896 -> 5952 with GELU 42.5 -> 38.1, with GEGLU 48.5 -> 41.5).
-TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group, int block_n, int splits) {
+TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group, int block_n, int splits, int sms) {
   // K block: a + b x width / 100, at least c; one row per way the operands come
   struct Block { double a, b, least; };
   constexpr Block kStream = {0.0914, 0.0552, 0.1382}, kResident = {0.0554, 0.0, 0.1394};        // single CTAs
@@ -932,7 +932,6 @@ TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_grou
   TilePlan best;
   best.us = 1e30;
   const bool geglu = epilogue == HY3D_EPI_GEGLU;
-  const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
   const int step = geglu ? 64 : 32;
   const int64_t nk = ((K + kBlockKBytes - 1) / kBlockKBytes + splits - 1) / splits;
   for (int g = 1; g <= 2; ++g) {
@@ -944,7 +943,7 @@ TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_grou
       if (g == 2 && (w & 31) && cta_group == 0) continue;
       const int64_t nt = (N + w - 1) / w, mt = (M + kTileM * g - 1) / (kTileM * g);
       const int64_t tiles = mt * nt * splits;
-      const Walk walk = plan_walk(M, N, K, g, w, splits, epilogue);
+      const Walk walk = plan_walk(M, N, K, g, w, splits, epilogue, sms);
       const bool column_fixed = walk.column_fixed || walk.ranges, resident = walk.resident;
       const double rounds = walk.rounds;
       const bool deep = g == 2 && K >= kDeepK;
@@ -978,23 +977,23 @@ TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_grou
 }
 
 // Sizes recur in every step of a model, so each thread keeps its last few answers (a search takes ~0.3 us, a
-// split-K plan fifteen of them).
+// split-K plan fifteen of them).  They hold for devices of as many SMs as the search was made for.
 template <typename Value>
 struct Memo {
-  struct Entry { int64_t M, N, K, rest; Value value; } entries[64] = {};
+  struct Entry { int64_t M, N, K, rest; int sms; Value value; } entries[64] = {};
   template <typename Search>
-  Value get(int64_t M, int64_t N, int64_t K, int64_t rest, Search search) {
+  Value get(int64_t M, int64_t N, int64_t K, int64_t rest, int sms, Search search) {
     Entry& e = entries[(static_cast<uint64_t>(M) * 31 + static_cast<uint64_t>(N) * 7 + static_cast<uint64_t>(K >> 4) * 3 +
                         static_cast<uint64_t>(rest) * 5) & 63];
-    if (e.M != M || e.N != N || e.K != K || e.rest != rest) e = {M, N, K, rest, search()};
+    if (e.M != M || e.N != N || e.K != K || e.rest != rest || e.sms != sms) e = {M, N, K, rest, sms, search()};
     return e.value;
   }
 };
 
-TilePlan plan_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group, int block_n, int splits) {
+TilePlan plan_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group, int block_n, int splits, int sms) {
   static thread_local Memo<TilePlan> memo;
   const int64_t rest = epilogue | cta_group << 2 | block_n << 4 | static_cast<int64_t>(splits) << 13;
-  return memo.get(M, N, K, rest, [&] { return search_tile(M, N, K, epilogue, cta_group, block_n, splits); });
+  return memo.get(M, N, K, rest, sms, [&] { return search_tile(M, N, K, epilogue, cta_group, block_n, splits, sms); });
 }
 
 // What the calling thread spends on a layer of two launches (quantise, GEMM) and of three (and a reduction).
@@ -1006,8 +1005,7 @@ struct LayerPlan {
 };
 
 // Splitting serves a K of 16 blocks or more under tiles for at most half the SMs; every range keeps four blocks.
-bool can_split(int64_t M, int64_t N, int64_t K) {
-  const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
+bool can_split(int64_t M, int64_t N, int64_t K, int sms) {
   return K > 15 * kBlockKBytes && (M + kTileM - 1) / kTileM * ((N + 255) / 256) * 2 <= sms;
 }
 bool has_range(int splits, int64_t K) { return splits <= 16 && static_cast<int64_t>(splits) * 4 <= (K + kBlockKBytes - 1) / kBlockKBytes; }
@@ -1019,12 +1017,12 @@ double partial_mb(int64_t M, int64_t N) { return static_cast<double>((M + kTileM
 // twentieth, since a split also takes a workspace and a launch.  The split that it picks is 1.4 % from the best on
 // average, never splitting 13 %: 64 x 8192 -> 512 12.7 us, in 7 ranges 7.6; 1117 x 7616 -> 224 11.5, in 4 ranges 9.6;
 // not so 257 x 6144 -> 1536 (9.0 against 9.6 in 3) and 358 x 5760 -> 4480 (11.7 against 15.0 in 2).
-int search_gemm_splits(int64_t M, int64_t N, int64_t K) {
-  if (!can_split(M, N, K)) return 1;
-  double best_us = 0.95 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0, 0, 1).us;
+int search_gemm_splits(int64_t M, int64_t N, int64_t K, int sms) {
+  if (!can_split(M, N, K, sms)) return 1;
+  double best_us = 0.95 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0, 0, 1, sms).us;
   int best = 1;
   for (int sp = 2; has_range(sp, K); ++sp) {
-    const double us = 2.16 + 0.963 * search_tile(M, N, K, HY3D_EPI_LINEAR, 1, 0, sp).us + sp * (0.12 + 0.0795 * partial_mb(M, N)) +
+    const double us = 2.16 + 0.963 * search_tile(M, N, K, HY3D_EPI_LINEAR, 1, 0, sp, sms).us + sp * (0.12 + 0.0795 * partial_mb(M, N)) +
                       0.31 * static_cast<double>(N) * K / 1e7;
     if (us < best_us) { best_us = us; best = sp; }
   }
@@ -1039,16 +1037,16 @@ int search_gemm_splits(int64_t M, int64_t N, int64_t K) {
 // Few tokens on many weights take longer than the tile's model says (every CTA reads the same few lines of A), up to 8 us
 // at 60 MB; without `few` such layers were left to two launches where one is shorter (7 x 3200 -> 9632 15.9 us against
 // 10.7).  With it no layer of 930 got slower by more than 4 %, 18 got faster.
-LayerPlan search_layer(int64_t M, int64_t N, int64_t K) {
+LayerPlan search_layer(int64_t M, int64_t N, int64_t K, int sms) {
   const double act = static_cast<double>(M) * K / 1e6, weights = static_cast<double>(N) * K / 1e7;
   const double few = M < kTileM ? weights * (1.0 - static_cast<double>(M) / kTileM) : 0.0;
   LayerPlan best;
-  const double single_us = 0.39 + 1.18 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0, 0, 1).us + 0.36 * act + 0.07 * weights + few;
+  const double single_us = 0.39 + 1.18 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0, 0, 1, sms).us + 0.36 * act + 0.07 * weights + few;
   best.us = single_us > kTwoLaunchesUs ? single_us : kTwoLaunchesUs;
-  if (!can_split(M, N, K)) return best;
+  if (!can_split(M, N, K, sms)) return best;
   double layer_us = 0.97 * best.us;      // a split has to be worth its workspace
   for (int sp = 2; has_range(sp, K); ++sp) {
-    double us = 3.48 + 0.98 * search_tile(M, N, K, HY3D_EPI_LINEAR, 1, 0, sp).us + sp * (0.21 + 0.078 * partial_mb(M, N)) +
+    double us = 3.48 + 0.98 * search_tile(M, N, K, HY3D_EPI_LINEAR, 1, 0, sp, sms).us + sp * (0.21 + 0.078 * partial_mb(M, N)) +
                 0.35 * act + 0.45 * weights + few;
     if (us < kThreeLaunchesUs) us = kThreeLaunchesUs;
     if (us < layer_us) { layer_us = us; best.splits = sp; }
@@ -1059,7 +1057,8 @@ LayerPlan search_layer(int64_t M, int64_t N, int64_t K) {
 
 LayerPlan plan_layer(int64_t M, int64_t N, int64_t K) {
   static thread_local Memo<LayerPlan> memo;
-  return memo.get(M, N, K, 0, [&] { return search_layer(M, N, K); });
+  const int sms = planned_sms();
+  return memo.get(M, N, K, 0, sms, [&] { return search_layer(M, N, K, sms); });
 }
 
 }  // namespace
@@ -1072,11 +1071,50 @@ int dense_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, bool layer)
   if (epilogue == HY3D_EPI_GEGLU || (N & 7) || M <= 0 || N <= 0 || K <= 0) return 1;
   if (layer) return plan_layer(M, N, K).splits;
   static thread_local Memo<int> memo;
-  return memo.get(M, N, K, 0, [&] { return search_gemm_splits(M, N, K); });
+  const int sms = planned_sms();
+  return memo.get(M, N, K, 0, sms, [&] { return search_gemm_splits(M, N, K, sms); });
 }
 
 // Expected time of a layer that quantises and multiplies in separate launches, in microseconds.
 double dense_layer_us(int64_t M, int64_t N, int64_t K) { return plan_layer(M, N, K).us; }
+
+// Tile, grouping and walk of a launch, what the caller gave (block_n, cta_group; 0 = choose) kept.
+int plan_launch(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group, int block_n, int splits, int sms, TilePlan* plan) {
+  plan->block_n = block_n;
+  plan->group = cta_group;
+  bool walk_known = false;
+  if (block_n == 0 || cta_group == 0) {
+    *plan = plan_tile(M, N, K, epilogue, cta_group, block_n, splits, sms);
+    walk_known = true;
+#ifdef HY3D_TRACE
+    if (const char* e = getenv("HY3D_CTA_GROUP")) { plan->group = atoi(e) == 2 ? 2 : 1; walk_known = false; }
+#endif
+  }
+  const int w = plan->block_n;
+  if (w < 16 || w > 256 || (w & 15) || (epilogue == HY3D_EPI_GEGLU && (w & 31))) return HY3D_ERR_SHAPE;
+  // CTA pairs need an even split of the B tile into two multiples of 16 rows.
+  if (plan->group == 2 && (w & 31)) {
+    if (cta_group == 2) return HY3D_ERR_SHAPE;
+    plan->group = 1;
+    walk_known = false;
+  }
+  if (!walk_known) plan->walk = plan_walk(M, N, K, plan->group, w, splits, epilogue, sms);
+  return HY3D_OK;
+}
+
+// The plan of a launch in whole numbers (hy3d_gemm_plan).
+int dense_gemm_plan(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group, int block_n, int sms, int* out) {
+  if (N <= 0 || (N & 15) || K <= 0 || (K & 15)) return HY3D_ERR_SHAPE;
+  TilePlan plan;
+  const int rc = plan_launch(M, N, K, epilogue, cta_group, block_n, 1, sms, &plan);
+  if (rc != HY3D_OK) return rc;
+  out[0] = plan.block_n;
+  out[1] = plan.group;
+  out[2] = plan.walk.clusters;
+  out[3] = static_cast<int>(plan.walk.rounds);
+  out[4] = plan.walk.ranges ? 1 : 0;
+  return HY3D_OK;
+}
 
 int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const void* w_scale,
                int ws_dtype, const void* bias, int bias_dtype, void* out, int out_dtype, int64_t M,
@@ -1107,27 +1145,13 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
        reinterpret_cast<uintptr_t>(out)) & 15)
     return HY3D_ERR_SHAPE;
 
-  int group = cta_group;
-  Walk walk;
-  bool walk_known = false;
-  if (block_n == 0 || group == 0) {
-    const TilePlan t = plan_tile(M, N, K, epilogue, cta_group, block_n, splits);
-    block_n = t.block_n;
-    group = t.group;
-    walk = t.walk;
-    walk_known = splits == 1;
-#ifdef HY3D_TRACE
-    if (const char* e = getenv("HY3D_CTA_GROUP")) { group = atoi(e) == 2 ? 2 : 1; walk_known = false; }
-#endif
-  }
-  if (block_n < 16 || block_n > 256 || (block_n & 15) || (geglu && (block_n & 31)))
-    return HY3D_ERR_SHAPE;
-  // CTA pairs need an even split of the B tile into two multiples of 16 rows.
-  if (group == 2 && (block_n & 31)) {
-    if (cta_group == 2) return HY3D_ERR_SHAPE;
-    group = 1;
-    walk_known = false;
-  }
+  const int sms = device_sm_count();
+  if (sms <= 0) return HY3D_ERR_CUDA;
+  TilePlan plan;
+  int rc = plan_launch(M, N, K, epilogue, cta_group, block_n, splits, sms, &plan);
+  if (rc != HY3D_OK) return rc;
+  block_n = plan.block_n;
+  const int group = plan.group;
 
   DenseArgs p;
   p.act_scale = act_scale; p.w_scale = w_scale; p.bias = bias; p.out = out;
@@ -1169,9 +1193,7 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
   // keeps ONE tile column for the whole launch, so its per-column scales and bias are staged
   // once and the epilogue warps never meet at a CTA-wide barrier again (measured faster or
   // equal on every sweep shape).
-  const int sms = device_sm_count();
-  if (sms <= 0) return HY3D_ERR_CUDA;
-  if (!walk_known) walk = plan_walk(M, N, K, group, block_n, p.splits, epilogue);
+  const Walk walk = p.splits > 1 ? plan_walk(M, N, K, group, block_n, p.splits, epilogue, sms) : plan.walk;
   const int clusters = walk.clusters;
   p.n_fastest = p.n_tiles > 1 && !walk.ranges ? 1 : 0;
 
@@ -1222,7 +1244,7 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
   const int smem_bytes = stages * stage_bytes + fixed;
 
   CUtensorMap tm_a, tm_b, tm_o;
-  int rc = encode_tmap_2d_u8(&tm_a, A, static_cast<uint64_t>(K), static_cast<uint64_t>(M),
+  rc = encode_tmap_2d_u8(&tm_a, A, static_cast<uint64_t>(K), static_cast<uint64_t>(M),
                              static_cast<uint64_t>(K), kBlockKBytes, kTileM, 128);
   if (rc != HY3D_OK) return rc;
   rc = encode_tmap_2d_u8(&tm_b, B, static_cast<uint64_t>(K), static_cast<uint64_t>(N),
@@ -1313,6 +1335,7 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
 }  // namespace dense
 
 using dense::gemm_dense;
+using dense::dense_gemm_plan;
 using dense::dense_layer_us;
 using dense::dense_splitk_plan;
 

@@ -487,10 +487,9 @@ struct SparseTile {
   int block_t = 0, group = 1;
   double us = 1e30;
 };
-SparseTile search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int block_t) {
+SparseTile search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int block_t, int sms) {
   SparseTile best;
   const int64_t kblocks = (K + kBlockK - 1) / kBlockK;
-  const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
   for (int g = 1; g <= 2; ++g) {
     for (int bt = 32; bt <= kWideBlockT; bt += 32) {
       if (block_t != 0 && bt != 32) break;             // the caller's width, one pass per group
@@ -541,19 +540,62 @@ double sparse_l1_elements(int64_t M, int64_t N, int64_t K, int epilogue, int blo
   constexpr double kRounds = 1e6, kSingleRound = 3e6;
   const double elements = static_cast<double>(M) * static_cast<double>(K);
   if (M <= 0 || N <= 0 || K <= 0 || elements < kRounds || elements >= kSingleRound) return kRounds;
-  const SparseTile t = search_tile(M, N, K, epilogue, block_t);
+  const int sms = planned_sms();
+  const SparseTile t = search_tile(M, N, K, epilogue, block_t, sms);
   const int64_t tiles = t.block_t > 0 ? (N + kTileW * t.group - 1) / (kTileW * t.group) * ((M + t.block_t - 1) / t.block_t) : 0;
-  return tiles * t.group <= device_sm_count() ? kSingleRound : kRounds;
+  return tiles * t.group <= sms ? kSingleRound : kRounds;
 }
 
 // Expected time of a layer that quantises and multiplies in separate launches, in microseconds: the greater of
 // the device's and the calling thread's (7.5).  The coefficients were fitted over an earlier tile model; against calls of
 // today's library they are 10 % rms off where a layer waits for the device.
 double sparse_layer_us(int64_t M, int64_t N, int64_t K) {
-  const double us = 1.271 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0).us + 0.424 * static_cast<double>(M) * K / 1e6 - 0.08;
+  const double us = 1.271 * search_tile(M, N, K, HY3D_EPI_LINEAR, 0, planned_sms()).us + 0.424 * static_cast<double>(M) * K / 1e6 - 0.08;
   return us > 7.5 ? us : 7.5;
 }
 
+namespace {
+
+// A launch's tiles and walk.
+struct SparsePlan {
+  int block_t = 0, group = 1;
+  int w_tiles = 0, t_tiles = 0, total_tiles = 0;
+  int clusters = 0;           // CTAs, or pairs
+  bool in_ranges = false;     // tokens fastest
+};
+int plan_launch(int64_t M, int64_t N, int64_t K, int epilogue, int block_t, int sms, SparsePlan* p) {
+  const SparseTile tile = search_tile(M, N, K, epilogue, block_t, sms);
+  p->block_t = tile.block_t;
+  p->group = tile.group;
+#ifdef HY3D_TRACE
+  if (const char* e = getenv("HY3D_SPARSE_CTA_GROUP")) p->group = atoi(e) == 2 ? 2 : 1;
+#endif
+  if (p->block_t < 16 || p->block_t > kWideBlockT || (p->block_t & 15)) return HY3D_ERR_SHAPE;
+  if (p->group == 2 && (p->block_t & 31)) p->group = 1;
+  p->w_tiles = static_cast<int>((N + kTileW * p->group - 1) / (kTileW * p->group));
+  p->t_tiles = static_cast<int>((M + p->block_t - 1) / p->block_t);
+  p->total_tiles = p->w_tiles * p->t_tiles;
+  const int most = sms / p->group;
+  p->clusters = p->total_tiles < most ? p->total_tiles : most;
+  p->in_ranges = tokens_fastest(M, N, K, epilogue, p->total_tiles > p->clusters);
+  return HY3D_OK;
+}
+
+}  // namespace
+
+// The plan of a launch in whole numbers (hy3d_gemm_plan).
+int sparse_gemm_plan(int64_t M, int64_t N, int64_t K, int epilogue, int block_t, int sms, int* out) {
+  if (N <= 0 || (N & 15) || K <= 0 || (K & 63)) return HY3D_ERR_SHAPE;
+  SparsePlan plan;
+  const int rc = plan_launch(M, N, K, epilogue, block_t, sms, &plan);
+  if (rc != HY3D_OK) return rc;
+  out[0] = plan.block_t;
+  out[1] = plan.group;
+  out[2] = plan.clusters;
+  out[3] = (plan.total_tiles + plan.clusters - 1) / plan.clusters;
+  out[4] = plan.in_ranges ? 1 : 0;
+  return HY3D_OK;
+}
 
 int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
                   const uint32_t* w_meta, int64_t meta_ld, const void* w_scale, int ws_dtype,
@@ -576,23 +618,20 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
        reinterpret_cast<uintptr_t>(w_meta) | reinterpret_cast<uintptr_t>(out)) & 15)
     return HY3D_ERR_SHAPE;
 
-  const SparseTile tile = search_tile(M, N, K, epilogue, block_t);
-  block_t = tile.block_t;
-  int group = tile.group;
-#ifdef HY3D_TRACE
-  if (const char* e = getenv("HY3D_SPARSE_CTA_GROUP")) group = atoi(e) == 2 ? 2 : 1;
-#endif
-  if (block_t < 16 || block_t > kWideBlockT || (block_t & 15)) return HY3D_ERR_SHAPE;
-  if (group == 2 && (block_t & 31)) group = 1;
+  const int sms = device_sm_count();
+  if (sms <= 0) return HY3D_ERR_CUDA;
+  SparsePlan plan;
+  int rc = plan_launch(M, N, K, epilogue, block_t, sms, &plan);
+  if (rc != HY3D_OK) return rc;
+  block_t = plan.block_t;
+  const int group = plan.group, clusters = plan.clusters;
 
   SparseArgs p;
   p.act_scale = act_scale; p.w_scale = w_scale; p.bias = bias; p.out = out;
   p.ws_dtype = ws_dtype; p.bias_dtype = bias_dtype; p.out_dtype = out_dtype; p.epilogue = epilogue;
   p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.K = static_cast<int>(K);
   p.block_t = block_t;
-  const int w_tiles = static_cast<int>((N + kTileW * group - 1) / (kTileW * group));
-  const int t_tiles = static_cast<int>((M + block_t - 1) / block_t);
-  p.total_tiles = w_tiles * t_tiles;
+  p.total_tiles = plan.total_tiles;
   p.num_kb = static_cast<int>(kblocks);
   const int k_last = static_cast<int>(K - (kblocks - 1) * kBlockK);
   p.last_ksteps = (k_last + 63) / 64;
@@ -609,7 +648,7 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
   if (smem_bytes < 120 * 1024) smem_bytes = 120 * 1024;
 
   CUtensorMap tm_w, tm_e, tm_x, tm_o;
-  int rc = encode_tmap_2d_u8(&tm_w, w_comp, static_cast<uint64_t>(K / 2), static_cast<uint64_t>(N),
+  rc = encode_tmap_2d_u8(&tm_w, w_comp, static_cast<uint64_t>(K / 2), static_cast<uint64_t>(N),
                              static_cast<uint64_t>(K / 2), 128, kTileW, 128);
   if (rc != HY3D_OK) return rc;
   rc = encode_tmap_2d_u8(&tm_e, w_meta, static_cast<uint64_t>(meta_ld * 4), static_cast<uint64_t>(N),
@@ -643,14 +682,9 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
   const KernelFn kernel = kernels[group - 1][out_dtype == HY3D_BF16 ? 1 : 0][epilogue];
   rc = ensure_max_smem(reinterpret_cast<const void*>(kernel), kSmemLimit);
   if (rc != HY3D_OK) return rc;
-  const int sms = device_sm_count();
-  if (sms <= 0) return HY3D_ERR_CUDA;
-  const int max_clusters = sms / group;
-  const int clusters = p.total_tiles < max_clusters ? p.total_tiles : max_clusters;
-  const bool in_ranges = tokens_fastest(M, N, K, epilogue, p.total_tiles > clusters);
-  p.fast_tiles = in_ranges ? t_tiles : w_tiles;
-  p.share = in_ranges ? p.total_tiles / clusters : 0;
-  p.rest = in_ranges ? p.total_tiles - p.share * clusters : 0;
+  p.fast_tiles = plan.in_ranges ? plan.t_tiles : plan.w_tiles;
+  p.share = plan.in_ranges ? p.total_tiles / clusters : 0;
+  p.rest = plan.in_ranges ? p.total_tiles - p.share * clusters : 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(group * clusters));
   cfg.blockDim = dim3(kThreads);
@@ -674,6 +708,7 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
 }  // namespace sparse
 
 using sparse::gemm_sparse24;
+using sparse::sparse_gemm_plan;
 using sparse::sparse_l1_elements;
 using sparse::sparse_layer_us;
 

@@ -460,12 +460,12 @@ double plan_layer_us(const Plan& p, int64_t M, int64_t N, int64_t K, bool sparse
 // Whether a layer of this size should run as one launch, and with which plan.  Sizes recur in every step of
 // a model, so each thread keeps the answers for the last few.
 bool linear_cluster_plan(int64_t M, int64_t N, int64_t K, bool sparse, int* block_t, int* ks) {
-  struct Entry { int64_t M, N, K; int sparse, block_t, ks; };
+  struct Entry { int64_t M, N, K; int sparse, sms, block_t, ks; };
   static thread_local Entry memo[64] = {};
   Entry& e = memo[(static_cast<uint64_t>(M) * 31 + static_cast<uint64_t>(N) * 7 + static_cast<uint64_t>(K >> 4) * 3 + sparse) & 63];
-  if (e.M != M || e.N != N || e.K != K || e.sparse != (sparse ? 1 : 0)) {
-    e = {M, N, K, sparse ? 1 : 0, 0, 0};
-    const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
+  const int sms = planned_sms();
+  if (e.M != M || e.N != N || e.K != K || e.sparse != (sparse ? 1 : 0) || e.sms != sms) {
+    e = {M, N, K, sparse ? 1 : 0, sms, 0, 0};
     // A layer takes the one launch where it is expected to be the shorter one: below the host's time for two
     // launches, and for few tokens and many dense weights, which the cluster's K split streams over the whole
     // chip (7 x 3200 -> 9632 15.9 -> 10.7 us, 2 x 7680 -> 7520 19.6 -> 15.0, 7 x 1216 -> 9760 10.6 -> 7.1).

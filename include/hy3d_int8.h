@@ -189,6 +189,12 @@ int hy3d_gemm_w8a8_dense(const int8_t* A, const int8_t* B, const float* act_scal
                          int64_t M, int64_t N, int64_t K,
                          int epilogue, int cta_group, int block_n, void* stream);
 
+/* Test hook (no reference counterpart): what a GEMM of this size launches.  plan[0] tile width (dense: output columns, sparse:
+ * tokens), [1] CTAs that share a tile, [2] CTAs or pairs of the grid, [3] tiles of the busiest of them, [4] 1 where each
+ * walks a contiguous range of tiles.  cta_group (dense only) and block as for the GEMM, 0 = choose.  sms: SMs to plan for,
+ * 0 = this device's.  Needs no GPU.  Returns HY3D_OK, or the status with which the launch refuses the tile. */
+int hy3d_gemm_plan(int64_t M, int64_t N, int64_t K, int epilogue, int sparse, int cta_group, int block, int sms, int* plan);
+
 /*
  * Split-K form of the GEMM above for launches whose tiles leave most SMs idle while each walks
  * a long K alone (few rows, few columns, deep K: 64 x 8192 -> 512): the K blocks
@@ -206,6 +212,7 @@ int hy3d_dense_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, int64_
 /* The same for a whole layer: quantisation and the calling thread's launches count too, so fewer shapes split.  What
  * the layers here take. */
 int hy3d_dense_layer_splitk_plan(int64_t M, int64_t N, int64_t K, int epilogue, int64_t* workspace_bytes);
+
 int hy3d_gemm_w8a8_dense_splitk(const int8_t* A, const int8_t* B, const float* act_scale,
                                 const void* w_scale, int w_scale_dtype,
                                 const void* bias, int bias_dtype,

@@ -44,6 +44,24 @@ def test_library_identity(build_mod):
     assert b"alignment" in lib.hy3d_status_string(2)
 
 
+def _gemm_plan(build_mod, M, K, N, epilogue=0, sparse=0, group=0, block=0, sms=148):
+    """(tile width, CTAs a tile, CTAs or pairs, tiles of the busiest, contiguous ranges) of a launch."""
+    binding = importlib.import_module("hunyuan3d-tools_b200.csrc._binding")
+    plan = (ctypes.c_int * 5)()
+    rc = binding.configure(build_mod.load_library()).hy3d_gemm_plan(M, N, K, epilogue, sparse, group, block, sms, plan)
+    assert rc == 0, rc
+    return tuple(plan)
+
+
+@pytest.mark.parametrize("M,K,N,epilogue,sparse", [(49152, 320, 320, 0, 0), (24576, 320, 2560, 2, 0), (3000, 512, 2048, 1, 0), (3072, 1280, 10240, 2, 1)])
+def test_plans_are_kept_per_sm_count(build_mod, M, K, N, epilogue, sparse):
+    """A thread that goes from one device to another of fewer SMs gets a grid for that one."""
+    whole = _gemm_plan(build_mod, M, K, N, epilogue, sparse, sms=148)
+    part = _gemm_plan(build_mod, M, K, N, epilogue, sparse, sms=74)
+    assert part[1] * part[2] <= 74 < whole[1] * whole[2]
+    assert _gemm_plan(build_mod, M, K, N, epilogue, sparse, sms=148) == whole
+
+
 def test_build_flags_are_sm100a_only(build_mod):
     flags = " ".join(build_mod.cuda_flags())
     assert "arch=compute_100a,code=sm_100a" in flags
