@@ -347,7 +347,7 @@ int hy3d_gemm_plan(int64_t M, int64_t N, int64_t K, int epilogue, int sparse, in
   if (!plan || epilogue < HY3D_EPI_LINEAR || epilogue > HY3D_EPI_GEGLU || cta_group < 0 || cta_group > 2 || sms < 0) return HY3D_ERR_ARG;
   if (M <= 0 || N <= 0 || K <= 0) return HY3D_ERR_SHAPE;
   if (sms == 0) sms = planned_sms();
-  return sparse ? sparse_gemm_plan(M, N, K, epilogue, block, sms, plan)
+  return sparse ? sparse_gemm_plan(M, N, K, epilogue, cta_group, block, sms, plan)
                 : dense_gemm_plan(M, N, K, epilogue, cta_group, block, sms, plan);
 }
 

@@ -487,10 +487,11 @@ struct SparseTile {
   int block_t = 0, group = 1;
   double us = 1e30;
 };
-SparseTile search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int block_t, int sms) {
+SparseTile search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int block_t, int sms, int cta_group = 0) {
   SparseTile best;
   const int64_t kblocks = (K + kBlockK - 1) / kBlockK;
   for (int g = 1; g <= 2; ++g) {
+    if (cta_group != 0 && g != cta_group) continue;
     for (int bt = 32; bt <= kWideBlockT; bt += 32) {
       if (block_t != 0 && bt != 32) break;             // the caller's width, one pass per group
       const int t = block_t != 0 ? block_t : bt;
@@ -563,20 +564,21 @@ struct SparsePlan {
   int clusters = 0;           // CTAs, or pairs
   bool in_ranges = false;     // tokens fastest
 };
-int plan_launch(int64_t M, int64_t N, int64_t K, int epilogue, int block_t, int sms, SparsePlan* p) {
-  const SparseTile tile = search_tile(M, N, K, epilogue, block_t, sms);
+int plan_launch(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group, int block_t, int sms, SparsePlan* p) {
+#ifdef HY3D_TRACE
+  if (const char* e = getenv("HY3D_SPARSE_CTA_GROUP")) cta_group = atoi(e) == 2 ? 2 : 1;
+#endif
+  const SparseTile tile = search_tile(M, N, K, epilogue, block_t, sms, cta_group);
   p->block_t = tile.block_t;
   p->group = tile.group;
-#ifdef HY3D_TRACE
-  if (const char* e = getenv("HY3D_SPARSE_CTA_GROUP")) p->group = atoi(e) == 2 ? 2 : 1;
-#endif
   if (p->block_t < 16 || p->block_t > kWideBlockT || (p->block_t & 15)) return HY3D_ERR_SHAPE;
-  if (p->group == 2 && (p->block_t & 31)) p->group = 1;
   p->w_tiles = static_cast<int>((N + kTileW * p->group - 1) / (kTileW * p->group));
   p->t_tiles = static_cast<int>((M + p->block_t - 1) / p->block_t);
   p->total_tiles = p->w_tiles * p->t_tiles;
   const int most = sms / p->group;
   p->clusters = p->total_tiles < most ? p->total_tiles : most;
+  // The second accumulator buffer of so wide a tile would lie on the metadata columns and beyond the allocation.
+  if (p->block_t > kMaxBlockT && p->total_tiles > p->clusters) return HY3D_ERR_SHAPE;
   p->in_ranges = tokens_fastest(M, N, K, epilogue, p->total_tiles > p->clusters);
   return HY3D_OK;
 }
@@ -584,10 +586,10 @@ int plan_launch(int64_t M, int64_t N, int64_t K, int epilogue, int block_t, int 
 }  // namespace
 
 // The plan of a launch in whole numbers (hy3d_gemm_plan).
-int sparse_gemm_plan(int64_t M, int64_t N, int64_t K, int epilogue, int block_t, int sms, int* out) {
+int sparse_gemm_plan(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group, int block_t, int sms, int* out) {
   if (N <= 0 || (N & 15) || K <= 0 || (K & 63)) return HY3D_ERR_SHAPE;
   SparsePlan plan;
-  const int rc = plan_launch(M, N, K, epilogue, block_t, sms, &plan);
+  const int rc = plan_launch(M, N, K, epilogue, cta_group, block_t, sms, &plan);
   if (rc != HY3D_OK) return rc;
   out[0] = plan.block_t;
   out[1] = plan.group;
@@ -621,7 +623,7 @@ int gemm_sparse24(const int8_t* X, const float* act_scale, const int8_t* w_comp,
   const int sms = device_sm_count();
   if (sms <= 0) return HY3D_ERR_CUDA;
   SparsePlan plan;
-  int rc = plan_launch(M, N, K, epilogue, block_t, sms, &plan);
+  int rc = plan_launch(M, N, K, epilogue, 0, block_t, sms, &plan);
   if (rc != HY3D_OK) return rc;
   block_t = plan.block_t;
   const int group = plan.group, clusters = plan.clusters;

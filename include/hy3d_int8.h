@@ -191,7 +191,8 @@ int hy3d_gemm_w8a8_dense(const int8_t* A, const int8_t* B, const float* act_scal
 
 /* Test hook (no reference counterpart): what a GEMM of this size launches.  plan[0] tile width (dense: output columns, sparse:
  * tokens), [1] CTAs that share a tile, [2] CTAs or pairs of the grid, [3] tiles of the busiest of them, [4] 1 where each
- * walks a contiguous range of tiles.  cta_group (dense only) and block as for the GEMM, 0 = choose.  sms: SMs to plan for,
+ * walks a contiguous range of tiles.  cta_group (1 or 2; the sparse GEMM itself always chooses) and block as for
+ * the GEMM, 0 = choose.  sms: SMs to plan for,
  * 0 = this device's.  Needs no GPU.  Returns HY3D_OK, or the status with which the launch refuses the tile. */
 int hy3d_gemm_plan(int64_t M, int64_t N, int64_t K, int epilogue, int sparse, int cta_group, int block, int sms, int* plan);
 

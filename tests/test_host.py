@@ -62,6 +62,26 @@ def test_plans_are_kept_per_sm_count(build_mod, M, K, N, epilogue, sparse):
     assert _gemm_plan(build_mod, M, K, N, epilogue, sparse, sms=148) == whole
 
 
+@pytest.mark.parametrize("sms", [148, 74])
+@pytest.mark.parametrize("group", [0, 1, 2])
+def test_sparse_tiles_of_256_tokens_have_a_cta_to_themselves(build_mod, sms, group):
+    """They have one accumulator buffer: a second tile of the same CTA would write over the metadata.  The last size is one
+    round of such tiles in single CTAs, two in pairs; a caller's own 256 is refused."""
+    seen = 0
+    for M, K, N in [(2915, 5120, 1296), (256, 1280, 18944), (250, 576, 18944), (3072, 640, 1536), (1450, 5120, 1296), (128, 1280, 18944),
+                    (250, 576, 9472), (148 * 256, 2048, 128)]:
+        for epilogue in (0, 1, 2):
+            if epilogue == 2 and N % 32:
+                continue
+            width, g, _, tiles, _ = _gemm_plan(build_mod, M, K, N, epilogue, 1, group=group, sms=sms)
+            assert group in (0, g) and (width <= 240 or tiles == 1)
+            seen += width == 256
+    assert seen
+    binding = importlib.import_module("hunyuan3d-tools_b200.csrc._binding")
+    lib = binding.configure(build_mod.load_library())
+    assert lib.hy3d_gemm_plan(256, 1280, 18944, 0, 1, group, 256, sms, (ctypes.c_int * 5)()) == 2      # shape
+
+
 def test_build_flags_are_sm100a_only(build_mod):
     flags = " ".join(build_mod.cuda_flags())
     assert "arch=compute_100a,code=sm_100a" in flags
