@@ -875,15 +875,13 @@ int64_t resident_stages(int64_t b_tile_bytes) {
 // that run together then write pieces of other rows: behind GEGLU, which is bound by the gate's instructions, that does not
 // show, plain layers lose by it (49152 x 320 -> 2560 54.3 us, 56.6 in ranges; 49152 x 320 -> 960 22.7 and 24.5).
 // With GEGLU, us strided / in ranges: 49152 x 320 -> 2560 95.9 / 90.1 (140 SMs, 28 rounds; 148 and 26), 24576 x 320 -> 2560
-// 50.5 / 47.8, 12288 x 640 -> 5120 57.2 / 50.8 (in pairs), 5000 x 512 -> 4096 21.5 / 20.8.  A must stay in L2, since every
-// column reads it again at its own time.
+// 50.5 / 47.8, 12288 x 640 -> 5120 57.2 / 50.8 (in pairs).
 struct Walk {
   int clusters = 0;
   bool column_fixed = false, resident = false, ranges = false;
   double rounds = 0.0;       // tiles that the busiest CTA works through
 };
-constexpr int64_t kRangesMaxA = 64000000;
-Walk plan_walk(int64_t M, int64_t N, int64_t K, int g, int w, int splits, int epilogue, int sms) {
+Walk plan_walk(int64_t M, int64_t N, int64_t K, int g, int w, int splits, int sms) {
   const int64_t nk = (K + kBlockKBytes - 1) / kBlockKBytes;
   const int64_t nt = (N + w - 1) / w, mt = (M + kTileM * g - 1) / (kTileM * g);
   const int64_t units = mt * nt * splits, most = sms / g < units ? sms / g : units;
@@ -895,16 +893,26 @@ Walk plan_walk(int64_t M, int64_t N, int64_t K, int g, int w, int splits, int ep
   const bool shallow = !(g == 2 && K >= kDeepK) && splits == 1;       // one K block a stage
   const bool fits = shallow && resident_stages(nk * (w / g) * kBlockKBytes) >= kResidentStages;
   walk.resident = fits && walk.column_fixed && units >= 2 * slots;
-  if (epilogue == HY3D_EPI_GEGLU && fits && nt > 1 && w % (2 * kSlabCols) == 0 && units >= 2 * most && M * K <= kRangesMaxA) {
-    const double rounds = static_cast<double>((units + most - 1) / most);
-    if (rounds <= static_cast<double>(mt) && (!walk.resident || rounds < walk.rounds)) {     // two columns a CTA at most
-      walk.ranges = walk.resident = true;
-      walk.rounds = rounds;
-      slots = most;
-    }
-  }
   walk.clusters = static_cast<int>(slots);
   return walk;
+}
+
+// The walk in ranges behind GEGLU, if it can be had and takes fewer rounds than a strided walk that keeps B resident.
+// Every column reads A again at its own time, from L2 as long as A stays there.  Time of a layer strided over its time in
+// ranges, average over 20 to 90 sizes each: single CTAs, A below 6 MB 1.07, to 16 MB 1.04, to 32 MB 1.01, beyond 0.995 (three of
+// 19 lose 4 to 7 %: 82323 x 576 -> 2080 131 and 139 us); pairs 1.18, 1.19, 1.17 and to 64 MB 1.12.  From K = 1024 on wide
+// tiles with a streamed B, or pairs with deep stages, are faster than the narrow ones that fit beside the stages: 41 of 50
+// sizes lose, up to 30 % (57035 x 1024 -> 3104 179 us, in ranges 239).
+constexpr int64_t kRangesMaxA = 32000000, kPairRangesMaxA = 64000000;
+bool plan_ranges(int64_t M, int64_t N, int64_t K, int g, int w, int epilogue, int sms, const Walk& strided, Walk* walk) {
+  const int64_t nt = (N + w - 1) / w, mt = (M + kTileM * g - 1) / (kTileM * g), units = mt * nt, most = sms / g;
+  if (epilogue != HY3D_EPI_GEGLU || nt < 2 || w % (2 * kSlabCols) || units < 2 * most || M * K > (g == 1 ? kRangesMaxA : kPairRangesMaxA) || K >= kDeepK ||
+      resident_stages((K + kBlockKBytes - 1) / kBlockKBytes * (w / g) * kBlockKBytes) < kResidentStages)
+    return false;
+  walk->clusters = static_cast<int>(most);
+  walk->rounds = static_cast<double>((units + most - 1) / most);
+  walk->column_fixed = walk->resident = walk->ranges = true;
+  return walk->rounds <= static_cast<double>(mt) && (!strided.resident || walk->rounds < strided.rounds);     // two columns a CTA at most
 }
 
 struct TilePlan {
@@ -922,15 +930,15 @@ struct TilePlan {
 // (The model before, fitted when a pair's hand-over cost 2000 cycles and resident B was for single CTAs, is 3.7 % off
 // with today's kernel: 12288 x 640 -> 1920 18.8 -> 16.3 us, 1879 x 4800 -> 1024 14.7 -> 12.0, 40560 x 640 -> 176
 // 11.3 -> 9.8, 257 x 1536 -> 6144 7.5 -> 6.8.)  Gates and a short K were rare in that fit; over 490 shapes, most with
-// K <= 1152, x all tiles: `tile_us`, dearer GELU in pairs and no pairs for GEGLU below deep K (1463 x 64 -> 3840 with GEGLU
+// K <= 1152, x all tiles: `tile_us`, dearer GELU in pairs and no strided pairs for GEGLU below deep K (1463 x 64 -> 3840 with GEGLU
 // 12.7 -> 7.7 us, 1300 x 128 -> 5024 7.1 -> 5.6, 6873 x 896 -> 5952 with GELU 42.5 -> 38.1, with GEGLU 48.5 -> 41.5).
 TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group, int block_n, int splits, int sms) {
   // K block: a + b x width / 100, at least c; one row per way the operands come
   struct Block { double a, b, least; };
   constexpr Block kStream = {0.0914, 0.0552, 0.1382}, kResident = {0.0554, 0.0, 0.1394};        // single CTAs
   constexpr Block kPair = {0.0849, 0.0496, 0.005}, kPairResident = {0.0233, 0.007, 0.1102}, kPairDeep = {0.0332, 0.0743, 0.091};
-  TilePlan best;
-  best.us = 1e30;
+  TilePlan best, ranged;       // strided, and in ranges
+  best.us = ranged.us = 1e30;
   const bool geglu = epilogue == HY3D_EPI_GEGLU;
   const int step = geglu ? 64 : 32;
   const int64_t nk = ((K + kBlockKBytes - 1) / kBlockKBytes + splits - 1) / splits;
@@ -943,37 +951,58 @@ TilePlan search_tile(int64_t M, int64_t N, int64_t K, int epilogue, int cta_grou
       if (g == 2 && (w & 31) && cta_group == 0) continue;
       const int64_t nt = (N + w - 1) / w, mt = (M + kTileM * g - 1) / (kTileM * g);
       const int64_t tiles = mt * nt * splits;
-      const Walk walk = plan_walk(M, N, K, g, w, splits, epilogue, sms);
-      const bool column_fixed = walk.column_fixed || walk.ranges, resident = walk.resident;
-      const double rounds = walk.rounds;
       const bool deep = g == 2 && K >= kDeepK;
-      // GEGLU in pairs below deep K only in ranges of some length, where a single CTA's B tile does not fit: 12288 x 640 ->
-      // 5120 53.0 us in single CTAs, 50.8 in pairs; 24576 x 320 -> 2560 48.0 and 49.3, 8000 x 768 -> 3200 26.4 and 27.5.
-      if (g == 2 && cta_group == 0 && geglu && !deep &&
-          !(walk.ranges && rounds >= 8.0 && resident_stages(nk * 256 * kBlockKBytes) < kResidentStages)) continue;
-      const Block& kb = g == 1 ? (resident ? kResident : kStream) : deep ? kPairDeep : resident ? kPairResident : kPair;
       const double c = w / 100.0;
-      double block = kb.a + kb.b * c;
-      if (block < kb.least) block = kb.least;
-      if (M < kTileM) block += 0.0016 * (1.0 - static_cast<double>(M) / kTileM) * static_cast<double>(nt);   // many CTAs, few lines of A
-      const double gate = geglu ? (g == 2 ? 2.59 : 2.39) : epilogue == HY3D_EPI_GELU ? (g == 2 && !deep ? 3.1 : 2.65) : 1.0;
-      // A tile too narrow to give all sixteen warps a slab takes longer than its share; one of a single K block does not
-      // hide the column parameters that it waits for.
-      const double tile_us = (gate > 1.0 ? 0.15 : 0.0) + (column_fixed || nk > 1 ? 0.0 : 0.1);
-      const double rows = static_cast<double>(M) / static_cast<double>(mt * g);
-      const double operand = static_cast<double>(tiles * g * nk) * kBlockKBytes *
-                             ((rows < kTileM ? rows : kTileM) + (resident ? 0.0 : static_cast<double>(w) / g)) / 1e7;
-      double us = 2.98 + (g == 1 ? 0.0 : deep ? 0.76 : resident ? 1.09 : 0.46) +
-                  rounds * (static_cast<double>(nk) * block + (g == 1 ? 0.282 : 0.292) * c * gate + tile_us) + 0.136 * operand +
-                  (resident ? 0.092 * static_cast<double>(nk) * c / g : 0.0) +
-                  0.068 * static_cast<double>(M) * static_cast<double>(N) * (geglu ? 1.0 : 2.0) / 1e6;
-      // A CTA does not fit beside a quantiser's, so a grid that wants nearly every SM starts late behind one: it
-      // needs a few SMs to spare (257 x 1536 -> 4608, whole layer: 144 tiles 9.0 us, 108 tiles 8.1).
-      if (splits == 1 && rounds == 1.0 && tiles * g * 5 > sms * 4) us += 0.7;
-      if (us < best.us) { best.us = us; best.block_n = w; best.group = g; best.walk = walk; }
+      auto consider = [&](const Walk& walk, TilePlan* plan) {
+        const bool column_fixed = walk.column_fixed, resident = walk.resident;
+        const double rounds = walk.rounds;
+        const Block& kb = g == 1 ? (resident ? kResident : kStream) : deep ? kPairDeep : resident ? kPairResident : kPair;
+        double block = kb.a + kb.b * c;
+        if (block < kb.least) block = kb.least;
+        if (M < kTileM) block += 0.0016 * (1.0 - static_cast<double>(M) / kTileM) * static_cast<double>(nt);   // many CTAs, few lines of A
+        const double gate = geglu ? (g == 2 ? 2.59 : 2.39) : epilogue == HY3D_EPI_GELU ? (g == 2 && !deep ? 3.1 : 2.65) : 1.0;
+        // A tile too narrow to give all sixteen warps a slab takes longer than its share; one of a single K block does not
+        // hide the column parameters that it waits for.
+        const double tile_us = (gate > 1.0 ? 0.15 : 0.0) + (column_fixed || nk > 1 ? 0.0 : 0.1);
+        const double rows = static_cast<double>(M) / static_cast<double>(mt * g);
+        const double operand = static_cast<double>(tiles * g * nk) * kBlockKBytes *
+                               ((rows < kTileM ? rows : kTileM) + (resident ? 0.0 : static_cast<double>(w) / g)) / 1e7;
+        double us = 2.98 + (g == 1 ? 0.0 : deep ? 0.76 : resident ? 1.09 : 0.46) +
+                    rounds * (static_cast<double>(nk) * block + (g == 1 ? 0.282 : 0.292) * c * gate + tile_us) + 0.136 * operand +
+                    (resident ? 0.092 * static_cast<double>(nk) * c / g : 0.0) +
+                    0.068 * static_cast<double>(M) * static_cast<double>(N) * (geglu ? 1.0 : 2.0) / 1e6;
+        // A CTA does not fit beside a quantiser's, so a grid that wants nearly every SM starts late behind one: it
+        // needs a few SMs to spare (257 x 1536 -> 4608, whole layer: 144 tiles 9.0 us, 108 tiles 8.1).
+        if (splits == 1 && rounds == 1.0 && tiles * g * 5 > sms * 4) us += 0.7;
+        if (us < plan->us) *plan = {w, g, us, walk};
+      };
+      const Walk strided = plan_walk(M, N, K, g, w, splits, sms);
+      const bool gated_pair = g == 2 && cta_group == 0 && geglu && !deep;
+      if (!gated_pair) consider(strided, &best);
+      // GEGLU in pairs below deep K only in ranges of some length, where a single CTA's B tile does not fit: 12288 x 640 ->
+      // 5120 53.0 us in single CTAs, 50.8 in pairs; 24576 x 320 -> 2560 48.0 and 49.3.  How wide they must be depends on what
+      // a streamed B costs the single CTAs.  Its rows of 128 bytes lie in two lines each where K is no multiple of 128, and in
+      // five sectors for four where it is none of 32.  Strided over ranges, on average: K % 128 == 0 128 wide 0.88, 192 0.98, 256
+      // 1.07; K % 32 == 0 128 wide 0.98, 192 1.09, 256 1.15; other K 1.2, 1.33 and 1.47.
+      Walk walk;
+      if (splits > 1 || !plan_ranges(M, N, K, g, w, epilogue, sms, strided, &walk)) continue;
+      if (gated_pair && (walk.rounds < 8.0 || w < (K % 128 == 0 ? 256 : K % 32 == 0 ? 192 : 128) ||
+                         resident_stages(nk * 256 * kBlockKBytes) >= kResidentStages)) continue;
+      consider(walk, &ranged);
     }
   }
-  return best;
+  // Ranges with the strided walk's own tile are taken as the model says, and so are those that take the place of a streamed B
+  // whose rows are not whole sectors (K % 32): it comes at half the rate that the model has for it.  Another tile has to
+  // promise 2 % in pairs and in ten rounds or more of wide tiles, 10 % in fewer, and narrow tiles are not worth a change: the
+  // model is not that exact.  Over 650 sizes that could take ranges (1 to 64 MB of A, K 64 to 1072) the layer's time with
+  // strided walks over its time: 0.92 to 1.65, 1.085 on average, six below 0.985; the model alone, pairs of any width and
+  // any K, 0.73 to 1.64, 1.073, 95 below (61684 x 1024 -> 2144 136 us strided, 195 as the model has it; 10105 x 896 -> 3456
+  // 33.2 and 38.9).
+  const bool same = ranged.block_n == best.block_n && ranged.group == best.group;
+  const bool slow_stream = K % 32 != 0 && !best.walk.resident;
+  const bool sure = ranged.group == 2 || (ranged.block_n >= 192 && ranged.walk.rounds >= 10.0);
+  const double margin = same || slow_stream ? 1.0 : sure ? 1.02 : ranged.block_n >= 192 ? 1.1 : 1e30;
+  return margin * ranged.us < best.us ? ranged : best;
 }
 
 // Sizes recur in every step of a model, so each thread keeps its last few answers (a search takes ~0.3 us, a
@@ -1098,7 +1127,10 @@ int plan_launch(int64_t M, int64_t N, int64_t K, int epilogue, int cta_group, in
     plan->group = 1;
     walk_known = false;
   }
-  if (!walk_known) plan->walk = plan_walk(M, N, K, plan->group, w, splits, epilogue, sms);
+  if (!walk_known) {
+    const Walk strided = plan_walk(M, N, K, plan->group, w, splits, sms);
+    if (splits > 1 || !plan_ranges(M, N, K, plan->group, w, epilogue, sms, strided, &plan->walk)) plan->walk = strided;
+  }
   return HY3D_OK;
 }
 
@@ -1193,7 +1225,7 @@ int gemm_dense(const int8_t* A, const int8_t* B, const float* act_scale, const v
   // keeps ONE tile column for the whole launch, so its per-column scales and bias are staged
   // once and the epilogue warps never meet at a CTA-wide barrier again (measured faster or
   // equal on every sweep shape).
-  const Walk walk = p.splits > 1 ? plan_walk(M, N, K, group, block_n, p.splits, epilogue, sms) : plan.walk;
+  const Walk walk = p.splits > 1 ? plan_walk(M, N, K, group, block_n, p.splits, sms) : plan.walk;
   const int clusters = walk.clusters;
   p.n_fastest = p.n_tiles > 1 && !walk.ranges ? 1 : 0;
 

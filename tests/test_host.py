@@ -82,6 +82,28 @@ def test_sparse_tiles_of_256_tokens_have_a_cta_to_themselves(build_mod, sms, gro
     assert lib.hy3d_gemm_plan(256, 1280, 18944, 0, 1, group, 256, sms, (ctypes.c_int * 5)()) == 2      # shape
 
 
+def test_geglu_walks_in_ranges_only_where_that_is_faster(build_mod):
+    """Sizes of both sides of the rules behind the ranges (tile columns, CTAs a tile, ranges)."""
+    def plan(M, K, N):
+        p = _gemm_plan(build_mod, M, K, N, 2)
+        return p[0], p[1], p[4]
+    # measured faster in ranges: the strided walk's own tile, wide pairs, a B whose rows are not whole sectors
+    assert plan(49152, 320, 2560) == (256, 1, 1) and plan(24576, 320, 2560) == (256, 1, 1)
+    assert plan(12288, 640, 5120) == (256, 2, 1) and plan(11843, 592, 4832) == (256, 2, 1)
+    assert plan(53314, 912, 768)[2] == 1 and plan(4219, 1008, 5664)[2] == 1
+    # K of 1024 and more
+    for M, N in [(55985, 2176), (61684, 2144), (57035, 3104), (9662, 4480), (1810, 6144)]:
+        assert plan(M, 1024, N)[2] == 0
+    # narrow pairs with a K of whole lines and of whole sectors
+    for M, K, N in [(10105, 896, 3456), (7932, 896, 2656), (5218, 896, 4384), (40169, 768, 992), (10255, 768, 2752), (26741, 704, 1856)]:
+        width, group, ranges = plan(M, K, N)
+        assert not ranges or (group == 2 and width >= (256 if K % 128 == 0 else 192))
+    # another, narrower tile for next to nothing; a large A under single CTAs
+    for M, K, N in [(8127, 832, 2016), (5163, 240, 2112), (82218, 336, 1120), (10341, 896, 2304), (64243, 528, 2016)]:
+        assert plan(M, K, N)[2] == 0
+    assert plan(82323, 576, 2080)[1:] != (1, 1)
+
+
 def test_build_flags_are_sm100a_only(build_mod):
     flags = " ".join(build_mod.cuda_flags())
     assert "arch=compute_100a,code=sm_100a" in flags
