@@ -331,12 +331,18 @@ def test_sparse_accumulators_bit_exact(sp, M, K, N, bt):
     assert torch.equal(acc.cpu(), O.int32_matmul(X, O.expand_24(co, no)))
 
 
-# GEGLU in contiguous ranges down the tile columns: B loaded again inside a range, ragged rows and columns, single CTAs and
-# pairs, both types, against the direct-store form (32-column tiles walk strided); the last walks strided.
-@pytest.mark.parametrize("M,K,N,group,bn", [(5000, 512, 4096, 0, 0), (24576, 320, 2560, 0, 0), (12288, 640, 5120, 0, 0), (5003, 272, 1888, 1, 128),
-                                            (9001, 400, 1312, 2, 64), (3000, 128, 5120, 1, 64), (2600, 640, 3968, 2, 256), (49152, 64, 192, 1, 64)])
+# GEGLU in contiguous ranges down the tile columns: B loaded again inside a range, ragged rows, columns and last K stages,
+# single CTAs and pairs, the library's own tile and given ones, both types, against the direct-store form (32-column tiles
+# walk strided).  The plan tells that these sizes do walk in ranges on 148 SMs; the last two walk strided.
+@pytest.mark.parametrize("M,K,N,group,bn,ranges", [
+    (24576, 320, 2560, 0, 0, 1), (12288, 640, 5120, 0, 0, 1), (4219, 1008, 5664, 0, 0, 1), (5000, 512, 4096, 1, 192, 1), (4750, 272, 1888, 1, 128, 1),
+    (5003, 272, 1888, 1, 64, 1), (3000, 128, 5120, 1, 64, 1), (9001, 400, 1312, 2, 64, 1), (3073, 640, 3968, 2, 256, 1), (3073, 624, 3968, 2, 256, 1),
+    (5003, 272, 1888, 1, 128, 0), (49152, 64, 192, 1, 64, 0)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-def test_dense_geglu_ranges(tc, M, K, N, group, bn, dtype):
+def test_dense_geglu_ranges(tc, M, K, N, group, bn, ranges, dtype):
+    sms, plan = torch.cuda.get_device_properties(0).multi_processor_count, (ctypes.c_int * 5)()
+    assert tc._lib.hy3d_gemm_plan(M, N, K, 2, 0, group, bn, 0, plan) == 0
+    assert plan[4] == ranges or sms != 148
     A, B = _rand_i8((M, K), M + K).to(DEV), _rand_i8((N, K), N + K + 5).to(DEV)
     g = torch.Generator().manual_seed(33)
     a_s, w_s = (torch.rand(M, generator=g) * 0.05 + 1e-3).to(DEV), (torch.rand(N, generator=g) * 1e-4 + 1e-5).to(dtype).to(DEV)
