@@ -72,6 +72,7 @@ SIGNATURES = {
     "hy3d_probe_mma_i8": [c_int, c_int, c_int, c_void_p, c_void_p],
     "hy3d_probe_hbm": [c_int, c_void_p, c_void_p, c_int64, c_void_p],
     "hy3d_probe_tmem_ld": [c_int, c_int, c_int, c_void_p, c_void_p],
+    "hy3d_groupnorm_ranks": [c_int64, c_int64, c_int64, c_int, c_int],
     "hy3d_groupnorm_nhwc": [c_void_p, c_void_p, c_int, c_int64, c_int64, c_int64, c_int, c_void_p, c_void_p,
                             c_int, ctypes.c_float, c_int, c_void_p, c_void_p, c_void_p],
     "hy3d_groupnorm_nhwc_terms": [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int64, c_int64, c_int64, c_int, c_void_p,

@@ -233,6 +233,10 @@ int hy3d_groupnorm_nhwc_terms(const void* x, const void* bias, const void* add, 
                                static_cast<cudaStream_t>(stream));
 }
 
+int hy3d_groupnorm_ranks(int64_t B, int64_t HW, int64_t C, int groups, int add) {
+  return gnorm::ranks_of(B, HW, C, groups, add != 0);
+}
+
 int hy3d_add_bias_nhwc(const void* x, const void* bias_x, const void* h, const void* bias_h, int dtype, void* y,
                        int64_t rows, int64_t C, void* stream) {
   const int rc = check_device();

@@ -23,7 +23,7 @@
 #include "common.cuh"
 
 namespace hy3d {
-int device_sm_count();
+int planned_sms();
 int resident_clusters(int ranks, int per_sm);
 int ensure_max_smem(const void* kernel, int bytes);
 namespace gnorm {
@@ -282,31 +282,17 @@ groupnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ pr
   }
 }
 
-}  // namespace
-
-// Nothing needs global scratch any more; callers of the C ABI still pass a workspace of this size.
-int64_t workspace_floats(int64_t B, int64_t HW, int groups) {
-  (void)HW;
-  return B * groups * 2;
-}
-
-int groupnorm_nhwc(const void* x, const void* pre, const void* add, int64_t add_ld, int x_dtype, int64_t B, int64_t HW,
-                   int64_t C, int groups, const void* gamma, const void* beta, int gb_dtype, float eps, int silu,
-                   void* y, cudaStream_t stream) {
-  if (x_dtype != HY3D_F16 && x_dtype != HY3D_BF16) return HY3D_ERR_ARG;
-  if ((gamma || beta) && (gb_dtype < HY3D_F16 || gb_dtype > HY3D_F32)) return HY3D_ERR_ARG;
-  if (B < 0 || HW <= 0 || C <= 0 || groups <= 0 || (C & 7) || C % groups) return HY3D_ERR_SHAPE;
-  if (C > 2560 || B > 65535 || HW > (1ll << 31)) return HY3D_ERR_SHAPE;
-  if (B == 0) return HY3D_OK;
-  if (!x || !y || (pre && !add)) return HY3D_ERR_ARG;
-  if (add && (add_ld < C || (add_ld & 7))) return HY3D_ERR_SHAPE;
-  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(add) | reinterpret_cast<uintptr_t>(pre)) & 15)
-    return HY3D_ERR_SHAPE;
+// How a call is spread over the device: slabs of whole groups, ranks of a cluster, chunks that a CTA could work on at a time.
+struct Spread {
+  Order order;
+  int slab_groups = 0, ranks = 0, sets = 0;
+  bool wide = false;
+};
+bool spread_call(int64_t B, int64_t HW, int64_t C, int groups, bool add, int sms, Spread* spread) {
   const int cpg = static_cast<int>(C / groups);
   // The order of the sums (see Order), fixed by the shape: chunks so that 320-thread blocks of whole rows
   // would fill four per SM, at least eight rows each.
-  const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
-  Order order;
+  Order& order = spread->order;
   {
     int64_t want = static_cast<int64_t>(sms) * 4 / B;
     want = want < 1 ? 1 : want > 64 ? 64 : want;
@@ -340,9 +326,9 @@ int groupnorm_nhwc(const void* x, const void* pre, const void* add, int64_t add_
         const int per_rank = (order.chunks + r - 1) / r;
         if (r > 1 && (r - 1) * per_rank >= order.chunks) continue;      // a rank without chunks
         const int64_t threads = static_cast<int64_t>(per_rank) * order.lanes * vec;
-        if (threads > (w ? kWideThreads : narrow_threads(add != nullptr))) continue;
+        if (threads > (w ? kWideThreads : narrow_threads(add))) continue;
         const int64_t warps = (threads + 31) / 32;
-        const int64_t resident = resident_ctas(w != 0, add != nullptr, warps);
+        const int64_t resident = resident_ctas(w != 0, add, warps);
         const int64_t ctas = static_cast<int64_t>(r) * (groups / g) * B;
         if (ctas * 20 > sms * resident * 19) continue;                  // clusters leave a few slots empty
         slab_groups = g; ranks = r; sets = per_rank; wide = w != 0;
@@ -363,20 +349,66 @@ int groupnorm_nhwc(const void* x, const void* pre, const void* add, int64_t add_
     ranks = kMaxRanks;
     while (ranks > 1 && (order.chunks < ranks || HW < static_cast<int64_t>(16) * ranks)) ranks >>= 1;
     wide = static_cast<int64_t>(ranks) * (groups / slab_groups) * B <= sms;
-    sets = (wide ? kWideThreads : narrow_threads(add != nullptr)) / ((slab_groups * cpg >> 3) * order.lanes);
-    if (sets < 1) return HY3D_ERR_SHAPE;
+    sets = (wide ? kWideThreads : narrow_threads(add)) / ((slab_groups * cpg >> 3) * order.lanes);
+    if (sets < 1) return false;
     // Clusters that do not all run at the same time make a second wave: as many ranks as prevent it, if any number does.
     // 8 x 96 x 89 x 86 (16 wide clusters of eight, 15 run) 24.6 us, with six ranks 16.4; 8 x 640 x 40 x 40 20.3 and 17.0
-    // (seven), 9 x 832 x 53 x 42 29.2 and 25.7; of 140 drawn shapes it changes seven, all of them faster, 1.14x to 1.50x.
-    auto one_wave = [&](int r) {
+    // (seven).  Narrow CTAs with much to read hide the second wave and lose by the lanes that fewer ranks leave, the more so
+    // the fewer clusters are left for it: 9 x 1920 x 65 x 34 (72 clusters, 71 run) 57.3 us, with six ranks 71.3.  260 sizes
+    // that it concerns, time with a second wave over time without: wide 1.54 on average, 1.46 at least; narrow below 16 million
+    // elements 1.26, 0.99 at least (below 8 million where at most a twentieth of the clusters is left over); the other narrow
+    // ones 1.00, 41 of 94 below 0.985 and down to 0.80.
+    const int64_t clusters = B * (groups / slab_groups), elements = B * HW * C;
+    auto running = [&](int r) {
       const int64_t warps = (((slab_groups * cpg >> 3) * order.lanes * even_sets(order.chunks, r, sets)) + 31) / 32;
-      const int64_t most = resident_ctas(wide, add != nullptr, warps);
+      const int64_t most = resident_ctas(wide, add, warps);
       const int n = resident_clusters(r, static_cast<int>(most < 8 ? most : 8));
-      return n == 0 || B * (groups / slab_groups) <= n;
+      return n == 0 ? clusters : static_cast<int64_t>(n);
     };
-    for (int r = ranks; r >= 1; --r)
-      if (one_wave(r)) { ranks = r; break; }
+    const int64_t first_wave = running(ranks);
+    if (wide || elements < (clusters * 20 <= first_wave * 21 ? 8000000 : 16000000))
+      for (int r = ranks; r >= 1; --r)
+        if (clusters <= running(r)) { ranks = r; break; }
   }
+  spread->slab_groups = slab_groups; spread->ranks = ranks; spread->sets = sets; spread->wide = wide;
+  return true;
+}
+
+}  // namespace
+
+// Nothing needs global scratch any more; callers of the C ABI still pass a workspace of this size.
+int64_t workspace_floats(int64_t B, int64_t HW, int groups) {
+  (void)HW;
+  return B * groups * 2;
+}
+
+// Ranks of the clusters of a call (hy3d_groupnorm_ranks), 0 where it is refused.
+int ranks_of(int64_t B, int64_t HW, int64_t C, int groups, bool add) {
+  if (B <= 0 || HW <= 0 || C <= 0 || groups <= 0 || (C & 7) || C % groups || C > 2560 || B > 65535 || HW > (1ll << 31)) return 0;
+  Spread spread;
+  return spread_call(B, HW, C, groups, add, planned_sms(), &spread) ? spread.ranks : 0;
+}
+
+int groupnorm_nhwc(const void* x, const void* pre, const void* add, int64_t add_ld, int x_dtype, int64_t B, int64_t HW,
+                   int64_t C, int groups, const void* gamma, const void* beta, int gb_dtype, float eps, int silu,
+                   void* y, cudaStream_t stream) {
+  if (x_dtype != HY3D_F16 && x_dtype != HY3D_BF16) return HY3D_ERR_ARG;
+  if ((gamma || beta) && (gb_dtype < HY3D_F16 || gb_dtype > HY3D_F32)) return HY3D_ERR_ARG;
+  if (B < 0 || HW <= 0 || C <= 0 || groups <= 0 || (C & 7) || C % groups) return HY3D_ERR_SHAPE;
+  if (C > 2560 || B > 65535 || HW > (1ll << 31)) return HY3D_ERR_SHAPE;
+  if (B == 0) return HY3D_OK;
+  if (!x || !y || (pre && !add)) return HY3D_ERR_ARG;
+  if (add && (add_ld < C || (add_ld & 7))) return HY3D_ERR_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(add) | reinterpret_cast<uintptr_t>(pre)) & 15)
+    return HY3D_ERR_SHAPE;
+  const int cpg = static_cast<int>(C / groups);
+  const int sms = planned_sms();
+  Spread spread;
+  if (!spread_call(B, HW, C, groups, add != nullptr, sms, &spread)) return HY3D_ERR_SHAPE;
+  const Order& order = spread.order;
+  const int slab_groups = spread.slab_groups, ranks = spread.ranks;
+  int sets = spread.sets;
+  const bool wide = spread.wide;
   const int slab = slab_groups * cpg, vec_cols = slab >> 3;
   // As many rounds as 42 KB of slices hold between two folds (two of 12 x 320 x 64 x 64; a fold less is worth 1 us there).
   const int chunks_per_rank = (order.chunks + ranks - 1) / ranks;

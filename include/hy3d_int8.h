@@ -117,6 +117,8 @@ int hy3d_groupnorm_nhwc(const void* x, const void* add, int x_dtype, int64_t B, 
                         int groups, const void* gamma, const void* beta, int gb_dtype, float eps,
                         int silu, void* y, float* workspace, void* stream);
 int64_t hy3d_groupnorm_workspace_floats(int64_t B, int64_t HW, int groups);
+/* Test hook (no reference counterpart): CTAs of a cluster, which share a sample's slab of groups; 0 for sizes that are refused. */
+int hy3d_groupnorm_ranks(int64_t B, int64_t HW, int64_t C, int groups, int add);
 
 /*
  * The same with another optional term: `bias` (C), of x_dtype, is added to every pixel before `add`, rounded as

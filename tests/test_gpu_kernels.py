@@ -600,6 +600,24 @@ def test_groupnorm_nhwc_fewer_ranks(ik, shape):
         assert O.rel_l2(y, torch.nn.functional.silu(ref.float()).bfloat16()) < 3e-3
 
 
+@pytest.mark.parametrize("shape,add,fewer", [((8, 96, 89, 86), 0, 1), ((8, 640, 40, 40), 0, 1), ((8, 320, 86, 10), 1, 1),       # wide; narrow and small
+                                             ((9, 1920, 65, 34), 1, 0), ((9, 960, 44, 81), 1, 0), ((7, 1280, 56, 86), 1, 0),   # narrow and large
+                                             ((9, 1920, 40, 17), 1, 0)])                                                        # a twentieth left over
+def test_groupnorm_nhwc_second_wave(ik, shape, add, fewer):
+    """Fewer ranks keep clusters from a second wave, except where narrow CTAs have enough to read to hide it."""
+    B, C, H, W = shape
+    ranks = ik._lib.hy3d_groupnorm_ranks(B, H * W, C, 32, add)
+    assert 0 < ranks < 8 if fewer else ranks == 8
+    g = torch.Generator(device=DEV).manual_seed(C)
+    x = (torch.randn(B, C, H, W, generator=g, device=DEV) * 2 + 0.7).bfloat16().contiguous(memory_format=torch.channels_last)
+    gamma, beta = 1 + 0.2 * torch.randn(C, generator=g, device=DEV), 0.2 * torch.randn(C, generator=g, device=DEV)
+    term = (torch.randn(B, C, generator=g, device=DEV) * 0.5).bfloat16() if add else None
+    xs = x + term[:, :, None, None] if add else x
+    ref = torch.nn.functional.group_norm(xs.float(), 32, gamma, beta, 1e-5).bfloat16()
+    y = ik.groupnorm_nhwc(x, 32, gamma, beta, 1e-5, silu=True, add=term)
+    assert O.rel_l2(y, torch.nn.functional.silu(ref.float()).bfloat16()) < 3e-3
+
+
 def test_groupnorm_nhwc_argument_checks(ik):
     x = torch.randn(2, 64, 4, 4, device=DEV).bfloat16()
     with pytest.raises(RuntimeError):
