@@ -166,7 +166,8 @@ __device__ __forceinline__ void quotient2(float2 w, float scale, float inv, uint
 // quantiser: the argument in quantize.cu's header holds for this scale too, which is within 1.3e-7 of amax / 127 (w / amax
 // times 127 is at least 1.9e-6 of itself away from a half-integer, 11 significant bits each, unless it is one; scale,
 // reciprocal and nudge move it by 4.2e-7).  Half-integers at w = amax / 2 are told by the nudge; there are others where 127
-// divides the significand of amax, and anywhere where the scale is the floor of 1e-8: such rows, and fp32 weights, divide.
+// divides the significand of amax, and where the scale comes from the floor of 1e-8 nothing says how near a quotient lies to
+// one: such rows, and fp32 weights, divide.
 // Their quotient comes from the correctly rounded reciprocal and two residual corrections, two values per
 // instruction: the first makes it faithful, and by Markstein's theorem ("Computation of elementary
 // functions on the IBM RISC System/6000 processor", 1990) the second then gives the correctly rounded
@@ -250,10 +251,10 @@ quantize_weight_kernel(const void* __restrict__ w, int64_t N, int K, int8_t* __r
   float mul = inv;
   bool divide = kType == HY3D_F32;
   if constexpr (kType != HY3D_F32) {
-    const float a = kSparse ? fmaxf(amax, 1e-8f) : amax;
-    const float rest = fmaf(scale, -127.0f, a);         // exact: a few units in the scale's last place, times 127
+    const float rest = fmaf(scale, -127.0f, amax);      // exact: a few units in the scale's last place, times 127
     mul = __int_as_float(__float_as_int(inv) + (fmaf(scale, 3.814697265625e-6f, rest) >= 0.0f ? 2 : -2));
-    divide = fmaf(__fdiv_rn(a, 127.0f), -127.0f, a) == 0.0f || (!kSparse && __fmul_rn(amax, inv127) < 1e-8f);
+    const bool floored = kSparse ? amax < 1e-8f : __fmul_rn(amax, inv127) < 1e-8f;
+    divide = floored || fmaf(__fdiv_rn(amax, 127.0f), -127.0f, amax) == 0.0f;
   }
   const int units = K >> 3;
   auto work = [&](int u, auto how, auto vector) {

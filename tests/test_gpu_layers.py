@@ -147,11 +147,15 @@ def test_weight_conversion_equals_the_torch_expressions(qu, sp, dtype, N, K):
 @pytest.mark.parametrize("K", [768, 16384 + 512])      # kept in registers, read again
 def test_weight_conversion_at_the_ties(qu, dtype, K):
     """Codes of weights around every half-integer multiple of the scale: rows of every significand of the largest weight (127
-    divides some), of a scale at its floor and below the type's normal range; the neighbours on both sides of each tie."""
+    divides some), of a scale at its floor in either form and below the type's normal range; the neighbours on both sides of
+    each tie."""
     bits = 7 if dtype == torch.bfloat16 else 10
-    amax = torch.cat([1 + torch.arange(2 ** bits) / 2 ** bits, torch.tensor([1.27e-6, 1.2e-6, 3e-7, 6e-8, 1e-3, 254 / 4096])]).to(dtype)
+    plain = torch.cat([1 + torch.arange(2 ** bits) / 2 ** bits, torch.tensor([1.27e-6, 1.2e-6, 3e-7, 6e-8, 1e-3, 254 / 4096])]).to(dtype)
+    dense_floor, sparse_floor = torch.tensor([1.2e-6, 3e-7, 6e-8, 1e-8]).to(dtype), torch.tensor([9.9e-9, 9e-9, 1e-9, 5e-11]).to(dtype)
+    amax = torch.cat([plain, dense_floor, sparse_floor])      # the last four are zero in fp16
+    unit = torch.cat([plain.double() / 127, torch.full((4,), 1e-8, dtype=torch.double), torch.full((4,), 1e-8 / 127, dtype=torch.double)])
     k = torch.arange(127)
-    tie = (amax.double()[:, None] * (2 * k + 1) / 254).to(dtype)
+    tie = (unit[:, None] * (2 * k + 1) / 2).to(dtype)
     near = torch.cat([tie, torch.nextafter(tie, torch.zeros_like(tie)), torch.nextafter(tie, amax[:, None].expand_as(tie))], 1)
     near = torch.cat([near, -near, amax[:, None], -amax[:, None]], 1)
     w = torch.zeros(amax.numel(), K, dtype=dtype)
