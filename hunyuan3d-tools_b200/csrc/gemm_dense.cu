@@ -3,8 +3,9 @@
 // One persistent CTA per SM walks 128 x block_n output tiles.  Roles by warp:
 //   warp 0      TMA producer: A (128 x 128 B) and B (block_n x 128 B) boxes, 128-byte swizzle,
 //               into a ring of shared-memory stages, signalled through "full" mbarriers.  Where
-//               the CTA keeps one tile column and its B tile fits, B is loaded once and stays
-//               resident; only A streams.
+//               the CTA keeps one tile column, or walks down the columns in a contiguous range,
+//               and its B tile fits, B stays resident and only A streams (loaded once, or once
+//               per column that the range touches).
 //   warp 1      owns tensor memory; issues tcgen05.mma kind::i8 (128 x block_n x 32 per
 //               instruction, int32 accumulators in tensor memory) and commits each stage back
 //               to its "empty" mbarrier.
@@ -57,7 +58,7 @@ struct DenseArgs {
   int kb_per_split;  // ... of this many pipeline stages each, writing raw int32 partials ...
   int64_t split_stride;   // ... `split_stride` elements apart behind `out`
   int m_rows_pad;         // rows of one partial matrix (M rounded up to whole tiles)
-  int b_resident;  // the CTA's B tile (all K blocks) is loaded once and stays in shared memory
+  int b_resident;  // the B tile of the CTA's column (all K blocks) stays in shared memory
   int m_tiles, n_tiles, num_kb, last_ksteps, n_fastest;
   int atoms;   // 128-byte K blocks per pipeline stage (1 or 2)
   int debug;   // knock-out switches of -DHY3D_TRACE / -DHY3D_KO diagnostic builds (always 0 in the shipped library)
@@ -196,7 +197,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   const uint32_t b_bytes = static_cast<uint32_t>(p.block_n / kG) * kBlockKBytes;
   // A stage holds kAtoms 128-byte-wide K blocks of each operand: [A0][A1..][B0][B1..].
   // Resident-B mode (one K block per stage): a stage holds A only, and the
-  // CTA's B tile -- it keeps one tile column for the whole launch -- sits behind the ring.
+  // B tile of the CTA's column -- the same for the whole launch, except in ranges -- sits behind the ring.
   const bool b_res = kAtoms == 1 && p.b_resident;
   const uint32_t stage_bytes = b_res ? a_bytes : static_cast<uint32_t>(kAtoms) * (a_bytes + b_bytes);
   const uint32_t b_res_base = smem_base + static_cast<uint32_t>(p.stages) * stage_bytes;

@@ -86,7 +86,8 @@ int even_sets(int chunks, int ranks, int most) {
   return (per_rank + rounds - 1) / rounds;
 }
 
-// i / by for 0 <= i and i * by < 2^31: a multiplication by ceil(2^31 / by), which is above 2^31 / by by less than one, so
+// i / by for 0 <= i and i * by < 2^31 (after Granlund and Montgomery, "Division by invariant integers using multiplication",
+// 1994): a multiplication by ceil(2^31 / by), which is above 2^31 / by by less than one, so
 // that the product errs by less than i / 2^31 < 1 / by.  The indices divided here are below 2^15 and `by` is at most 5120.
 // Integer division takes some twenty instructions in a row, and every phase of the kernel began with one or two: with
 // these and loops that count rows, 12 x 320 x 64 x 64 25.3 -> 24.3 us, 12 x 1280 x 16 x 16 11.2 -> 9.8, 4 x 128 x 11 x 12
@@ -410,7 +411,9 @@ int groupnorm_nhwc(const void* x, const void* pre, const void* add, int64_t add_
   int sets = spread.sets;
   const bool wide = spread.wide;
   const int slab = slab_groups * cpg, vec_cols = slab >> 3;
-  // As many rounds as 42 KB of slices hold between two folds (two of 12 x 320 x 64 x 64; a fold less is worth 1 us there).
+  // As many rounds as 42 KB of slices hold between two folds.  Over 150 sizes, with and without a term, 40 KB, which the
+  // padding just fills with one round less at times, take 0.7 % longer on average and up to 9 % (10 x 256 x 13 x 55 8.9 -> 9.7
+  // us), 36 KB 1.1 % and up to 19 %; 46 KB are no faster.
   const int chunks_per_rank = (order.chunks + ranks - 1) / ranks;
   const int rounds = (chunks_per_rank + sets - 1) / sets;
   sets = even_sets(order.chunks, ranks, sets);
